@@ -20,20 +20,21 @@ extern "C" {
  * paths and its per-ISA kernels inside xnor_nn_init_convolution (src/implementation.cpp:16-24,
  * src/bcast_convolution.cpp:92-117); this is the same decision for the GPU. `auto` honours the
  * environment variable XNOR_NN_B200_KERNEL (popc | tcgen05_i8 | tcgen05_i8_rows) and otherwise
- * picks by shape. Both tcgen05 kernels read the same packed operands (+-1 bytes), so chained
- * layers and single executors work with either.
+ * picks by shape. Both tcgen05 kernels read the same packed operands (+-1 as 4-bit floats, two to
+ * a byte), so chained layers and single executors work with either; the names date from an 8-bit
+ * operand layout and stand for the same kernels.
  * (The value 1 is not used: the mma.sync b1 path it once named was measured slower than the
  * integer pipe and never built; a request for an unknown value is treated as `auto`.) */
 typedef enum {
     xnor_nn_b200_kernel_auto = -1,
     xnor_nn_b200_kernel_popc = 0,            /* LOP3+POPC integer pipe; every shape and format */
-    xnor_nn_b200_kernel_tcgen05_i8 = 2,      /* tcgen05.mma kind::i8, tiles of 128 frame
+    xnor_nn_b200_kernel_tcgen05_i8 = 2,      /* tcgen05.mma kind::mxf4, tiles of 128 frame
                                                 positions x up to 256 filters; unit stride,
                                                 padding smaller than the filter. Shapes it cannot
                                                 serve go to the rows kernel, then to popc. */
-    xnor_nn_b200_kernel_tcgen05_i8_rows = 3  /* tcgen05.mma kind::i8, tiles of 128 filters x
-                                                whole output rows of one image; unit stride,
-                                                rows of at most 256 pixels, any padding */
+    xnor_nn_b200_kernel_tcgen05_i8_rows = 3  /* tcgen05.mma kind::mxf4, tiles of 128 filters
+                                                x whole output rows of one image; unit stride,
+                                                rows of at most 240 pixels, any padding */
 } xnor_nn_b200_kernel_t;
 
 /* xnor_nn_init_convolution (src/common_convolution.cpp:9-63) with the kernel family stated.

@@ -1,7 +1,7 @@
 // Activation-side kernels: sign packing with the fused mean-|x| map, and the K box filter.
 //
 // All three are bound by HBM bandwidth: the fp32 source (4 B per element) is read exactly once
-// and 1/32 (bits) or 1/4 (int8) of that is written. One thread owns one pixel and walks its
+// and 1/32 (bits) or 1/8 (4-bit values) of that is written. One thread owns one pixel and walks its
 // channels in ascending order, so the mean-|x| sum is accumulated in the very order upstream
 // uses (src/bcast_calculate_k.cpp:55-65) and rounds identically; with an NCHW source the 32
 // lanes of a warp read 32 neighbouring pixels of one channel plane, a full 128-byte line.
@@ -21,7 +21,7 @@ __device__ __forceinline__ float ld_stream(const float *p) {
 }
 
 
-enum OutKind { kBitsDense = 0, kBytesFramed = 2 };
+enum OutKind { kBitsDense = 0, kNibblesFramed = 2 };
 
 struct BinArgs {
     const float *src;
@@ -33,7 +33,7 @@ struct BinArgs {
     long c_stride;    // elements between channels of one pixel
     long px_stride;   // elements between pixels of one image
     float inv_ic;
-    int words;        // 32-bit words per packed row (icw, or icp/4 for bytes)
+    int words;        // 32-bit words per packed row (icw, or icp/4 for nibbles)
     int wp, hp, lead, ih;
 };
 
@@ -70,15 +70,10 @@ __global__ void __launch_bounds__(128) binarize_kernel(const BinArgs g) {
             for (int i = 0; i < 32; i++) acc = __fadd_rn(acc, __fmul_rn(fabsf(v[i]), g.inv_ic));
         }
         if (WITH_PACK) {
-            if (KIND == kBytesFramed) {
+            if (KIND == kNibblesFramed) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    uint32_t w = 0;
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        w |= (sign_clear(v[4 * j + i]) ? 0x01u : 0xFFu) << (8 * i);
-                    row[c / 4 + j] = w;
-                }
+                for (int j = 0; j < 4; j++)
+                    row[c / 8 + j] = sign_nibbles(reinterpret_cast<const uint32_t *>(v) + 8 * j);
             } else {
                 uint32_t w = 0;
 #pragma unroll
@@ -89,74 +84,57 @@ __global__ void __launch_bounds__(128) binarize_kernel(const BinArgs g) {
     }
     if (c < g.ic) {  // channel tail: absent channels pack as zero
         uint32_t wbits = 0;
-        uint32_t wbytes[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint32_t wnib[4] = {0, 0, 0, 0};
         for (int i = 0; i < 32; i++) {
             unsigned bit = 0;
             if (c + i < g.ic) {
                 const float x = __ldg(p + (long)(c + i) * g.c_stride);
                 if (WITH_A) acc = __fadd_rn(acc, __fmul_rn(fabsf(x), g.inv_ic));
                 bit = sign_clear(x);
-                wbytes[i / 4] |= (bit ? 0x01u : 0xFFu) << (8 * (i % 4));
+                wnib[i / 8] |= (bit ? 0x2u : 0xAu) << (4 * (i % 8));
             }
             wbits = (wbits << 1) | bit;
         }
         if (WITH_PACK) {
-            if (KIND == kBytesFramed) {
+            if (KIND == kNibblesFramed) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) row[c / 4 + j] = wbytes[j];
+                for (int j = 0; j < 4; j++) row[c / 8 + j] = wnib[j];
             } else {
                 row[c / 32] = wbits;
             }
         }
-        c += 32;
-    }
-    if (WITH_PACK && KIND == kBytesFramed) {
-        // chunk padding beyond the last 32-channel group stays zero
-        for (int j = c / 4; j < g.words; j++) row[j] = 0u;
     }
     if (WITH_A) g.a[px] = acc;
 }
 
-// ---- NCHW source, +-1 bytes on the frame: the layout the tensor-core convolution reads -------
+// ---- +-1 nibbles on the frame: the layout the tensor-core convolution reads -------------------
 //
-// A block of four warps owns 32 neighbouring pixels and walks the channels in chunks of 128.
-// All warps load (lane = pixel, warp w the w-th quarter of the chunk's channels, so a load
-// instruction reads one 128-byte line of a channel plane; 32 independent loads per thread, issued
-// one chunk ahead so that they are in flight while the previous chunk is consumed). |x|/IC goes
-// to a float tile and the sign byte to a byte tile in shared memory, both pixel-major. Warp 0 then
-// adds the float tile up channel by channel, one lane per pixel, which keeps upstream's summation
-// order, while the other warps copy the byte tile out, 8 bytes per lane, a pixel's 128-byte line
-// per half warp. Five blocks are resident per SM (nine of the 96-channel kind): the shared-memory
+// A block of four warps owns 32 neighbouring pixels and walks the channels in chunks of TCC. All
+// warps load, one chunk ahead, so that a chunk's loads are in flight while the previous one is
+// consumed. |x|/IC goes to a float tile and the sign nibbles to a second tile in shared memory,
+// both pixel-major. Warp 0 then adds the float tile up channel by channel, one lane per pixel,
+// which keeps upstream's summation order, while the other warps copy the nibbles out, 8 bytes per
+// lane. Five blocks are resident per SM (nine of the 96-channel kind): the shared-memory
 // carve-out is sized for that, see launch_bin().
 //
-// The kernel is as much bound by instruction issue as by memory (a profile of the first version
-// on the 96-channel AlexNet layer: 29 instructions issued per global load, the schedulers busy
-// in 69 % of the active cycles, DRAM at 31 %). Hence: the sign bytes of four floats come from
-// three byte permutes and one logic operation; both tiles are written and read with 8- and
-// 16-byte shared-memory accesses, their rows padded so that these stay free of bank conflicts;
-// pixel coordinates are 32-bit (the host sends anything larger to the generic kernel).
+// NCHW: lane = pixel, warp w takes the w-th quarter of a chunk's channels, so a load instruction
+// reads one 128-byte line of a channel plane. NHWC: a pixel's channels are contiguous, TCC / 4
+// lanes read them with 16-byte loads and a warp's loads cover whole pixels; one thread per pixel
+// instead, which the first version had, reads with a stride of IC floats and took 42 us for
+// AlexNet conv4 on 64 images.
 //
-// TPER = channels per warp and chunk = loads per thread and chunk: 32 (chunks of 128 channels)
-// or 24 (chunks of 96), the latter for channel counts that are a multiple of 96 but not of 128
-// (AlexNet conv2), where a 128-channel chunk would leave a quarter of the threads without work.
+// The kernel is as much bound by instruction issue as by memory. Hence: the sign nibbles of eight
+// floats come from six byte permutes and two logic operations; both tiles are written and read
+// with wide shared-memory accesses, their rows padded so that these stay (nearly) free of bank
+// conflicts; pixel coordinates are 32-bit (the host sends anything larger to the generic kernel).
+//
+// TCC = 4 TPER channels per chunk: 128; 96 for channel counts that are a multiple of 96 but not
+// of 128 (AlexNet conv2), where a 128-channel chunk would leave a quarter of the threads without
+// work; 64 and 32 for layers that have no more channels than that.
 // Bytes past the last channel of a packed row are zero from allocation, and only zeros are
 // ever written there.
 constexpr int TPX = 32;    // pixels per block
 constexpr int TWARPS = 4;
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-
-// The +-1 bytes of four floats, the first in the lowest byte: sign bit set -> 0xFF, clear -> 0x01.
-// A selector nibble of 0xB / 0xF replicates the top bit of byte 3 of the first / second operand.
-__device__ __forceinline__ uint32_t sign_bytes(float a, float b, float c, float d) {
-    const uint32_t ab = prmt(__float_as_uint(a), __float_as_uint(b), 0xFBFBu);
-    const uint32_t cd = prmt(__float_as_uint(c), __float_as_uint(d), 0xFBFBu);
-    return (prmt(ab, cd, 0x5410u) & 0xFEFEFEFEu) ^ 0x01010101u;
-}
 
 // Element i of a column of floats whose rows are `pitch` bytes apart. The plain expression on
 // 64-bit element offsets compiled to seven integer instructions per load; 32-bit byte offsets to
@@ -174,11 +152,23 @@ __device__ __forceinline__ const float *row_ptr(const float *p, unsigned i, unsi
     return reinterpret_cast<const float *>(reinterpret_cast<const char *>(p) + (size_t)(i * pitch));
 }
 
-template <bool WITH_A, bool WITH_PACK, int TPER>
-__global__ void __launch_bounds__(TWARPS * 32) binarize_bytes_nchw_kernel(const BinArgs g) {
+__device__ __forceinline__ float4 ld_stream4(const float *p) {
+    float4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(p));
+    return v;
+}
+
+template <bool WITH_A, bool WITH_PACK, bool NHWC, int TPER>
+__global__ void __launch_bounds__(TWARPS * 32) binarize_nibbles_kernel(const BinArgs g) {
     constexpr int TCC = TPER * TWARPS;  // channels per chunk
     constexpr int FLD = TCC + 4;        // floats per pixel of the float tile
-    constexpr int TLD = TCC + 8;        // bytes per pixel of the byte tile
+    constexpr int TLD = TCC / 2 + (TPER == 32 ? 16 : 8);  // bytes per pixel of the nibble tile
+    constexpr int LPP = TCC / 4;        // NHWC: lanes per pixel,
+    constexpr int PPI = 32 / LPP;       // pixels per load instruction of a warp,
+    constexpr int LOADS = TPX / TWARPS / PPI;  // and 16-byte loads per thread and chunk
+    static_assert(!NHWC || 4 * LOADS == TPER, "a thread stages as many floats either way");
     __shared__ __align__(16) float f_s[WITH_A ? TPX * FLD : 4];
     __shared__ __align__(16) uint8_t b_s[WITH_PACK ? TPX * TLD : 8];
     __shared__ long row_s[TPX];  // a pixel's packed row, as an offset in units of 8 bytes
@@ -201,63 +191,87 @@ __global__ void __launch_bounds__(TWARPS * 32) binarize_bytes_nchw_kernel(const 
         row_s[lane] = live ? row * (g.words >> 1) : -1;
     }
 
-    // channel extent walked: the channels, rounded up to whole 32-bit words of the packed row
-    const int c_end = WITH_PACK ? min(g.words * 4, (g.ic + 3) & ~3) : g.ic;
+    const int c_end = g.ic;
     float acc = 0.f;
-    // Warp w owns the TPER consecutive channels [TPER w, TPER (w + 1)) of every chunk.
-    const int cw = TPER * warp;  // first channel of this warp inside a chunk
-    const float *pw = g.src + (long)n * g.img_stride + r + (long)cw * g.hw;
-    const unsigned pitch = (unsigned)g.hw * 4u;  // bytes between channels; the host checks the range
     float v[TPER];
-    if (live && TCC <= g.ic) {
+    // NCHW: warp w owns the TPER consecutive channels [TPER w, TPER (w + 1)) of every chunk.
+    // NHWC: load j of this thread is four channels of pixel p0 + j * PPI.
+    const int cw = NHWC ? 4 * (lane % LPP) : TPER * warp;
+    const int p0 = NHWC ? warp * (TPX / TWARPS) + lane / LPP : 0;
+    const float *pw = NHWC ? g.src + (long)(blockIdx.x * TPX + p0) * g.ic + cw
+                           : g.src + (long)n * g.img_stride + r + (long)cw * g.hw;
+    const unsigned pitch = (unsigned)g.hw * 4u;  // bytes between channels; the host checks the range
+    const bool vec = NHWC && (g.ic & 3) == 0 && (reinterpret_cast<uintptr_t>(g.src) & 15) == 0;
+    auto fetch = [&](int c0) {
+        if (NHWC) {
+            const float *p = pw + c0;
 #pragma unroll
-        for (int i = 0; i < TPER; i++) v[i] = ld_stream(row_ptr<TPER == 32>(pw, i, pitch));
-    } else {
+            for (int j = 0; j < LOADS; j++, p += (long)PPI * g.ic) {
+                const bool in = p0 + j * PPI < n_live;
+                if (vec) {
+                    const float4 t = in && c0 + cw < g.ic ? ld_stream4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
+                } else {
 #pragma unroll
-        for (int i = 0; i < TPER; i++)
-            v[i] = (live && cw + i < g.ic) ? ld_stream(row_ptr<TPER == 32>(pw, i, pitch)) : 0.f;
-    }
-    for (int c0 = 0; c0 < c_end; c0 += TCC) {
-        const bool full = c0 + TCC <= g.ic;  // no channel tail in this chunk
-        if (WITH_A) {
-            float4 *frow = reinterpret_cast<float4 *>(f_s + lane * FLD + cw);
-#pragma unroll
-            for (int j = 0; j < TPER / 4; j++)
-                frow[j] = make_float4(__fmul_rn(fabsf(v[4 * j]), g.inv_ic),
-                                      __fmul_rn(fabsf(v[4 * j + 1]), g.inv_ic),
-                                      __fmul_rn(fabsf(v[4 * j + 2]), g.inv_ic),
-                                      __fmul_rn(fabsf(v[4 * j + 3]), g.inv_ic));
-        }
-        if (WITH_PACK) {
-            uint2 *brow = reinterpret_cast<uint2 *>(b_s + lane * TLD + cw);
-#pragma unroll
-            for (int j = 0; j < TPER / 8; j++) {
-                uint32_t w2[2];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const int c = 8 * j + 4 * q;
-                    uint32_t word = sign_bytes(v[c], v[c + 1], v[c + 2], v[c + 3]);
-                    if (!full) {  // channels past the last one are zero bytes
-                        const int left = g.ic - (c0 + cw + c);
-                        word = left >= 4 ? word : left <= 0 ? 0u : (word & (0xFFFFFFFFu >> (8 * (4 - left))));
-                    }
-                    w2[q] = word;
+                    for (int i = 0; i < 4; i++)
+                        v[4 * j + i] = in && c0 + cw + i < g.ic ? __ldg(p + i) : 0.f;
                 }
-                brow[j] = make_uint2(w2[0], w2[1]);
             }
-        }
-        __syncthreads();
-        if (c0 + TCC < c_end) {  // next chunk's loads fly while this one is consumed
-            const float *pn = pw + (long)(c0 + TCC) * g.hw;
-            if (live && c0 + 2 * TCC <= g.ic) {
+        } else {
+            const float *pn = pw + (long)c0 * g.hw;
+            if (live && c0 + TCC <= g.ic) {
 #pragma unroll
                 for (int i = 0; i < TPER; i++) v[i] = ld_stream(row_ptr<TPER == 32>(pn, i, pitch));
             } else {
 #pragma unroll
                 for (int i = 0; i < TPER; i++)
-                    v[i] = (live && c0 + TCC + cw + i < g.ic) ? ld_stream(row_ptr<TPER == 32>(pn, i, pitch)) : 0.f;
+                    v[i] = (live && c0 + cw + i < g.ic) ? ld_stream(row_ptr<TPER == 32>(pn, i, pitch)) : 0.f;
             }
         }
+    };
+    fetch(0);
+    for (int c0 = 0; c0 < c_end; c0 += TCC) {
+        const int left = g.ic - (c0 + cw);  // channels from this thread's first one on
+        if (WITH_A) {
+#pragma unroll
+            for (int j = 0; j < TPER / 4; j++) {
+                float4 *f4 = reinterpret_cast<float4 *>(
+                    NHWC ? f_s + (p0 + j * PPI) * FLD + cw : f_s + lane * FLD + cw + 4 * j);
+                *f4 = make_float4(__fmul_rn(fabsf(v[4 * j]), g.inv_ic),
+                                  __fmul_rn(fabsf(v[4 * j + 1]), g.inv_ic),
+                                  __fmul_rn(fabsf(v[4 * j + 2]), g.inv_ic),
+                                  __fmul_rn(fabsf(v[4 * j + 3]), g.inv_ic));
+            }
+        }
+        if (WITH_PACK) {
+            const uint32_t *u = reinterpret_cast<const uint32_t *>(v);
+            if (NHWC) {
+#pragma unroll
+                for (int j = 0; j < LOADS; j++) {
+                    uint32_t w = ((u[4 * j] >> 28) & 0x8u) | ((u[4 * j + 1] >> 24) & 0x80u) |
+                                 ((u[4 * j + 2] >> 20) & 0x800u) | ((u[4 * j + 3] >> 16) & 0x8000u) |
+                                 0x2222u;
+                    w = first_nibbles(w, left >= 4 ? 8 : left);
+                    *reinterpret_cast<uint16_t *>(b_s + (p0 + j * PPI) * TLD + cw / 2) = (uint16_t)w;
+                }
+            } else {
+                uint32_t w[TPER / 8];
+#pragma unroll
+                for (int j = 0; j < TPER / 8; j++)  // channels past the last one are zero
+                    w[j] = first_nibbles(sign_nibbles(u + 8 * j), left - 8 * j);
+                uint8_t *b = b_s + lane * TLD + cw / 2;
+                if (TPER == 32) {
+                    *reinterpret_cast<uint4 *>(b) = make_uint4(w[0], w[1], w[TPER / 8 - 2], w[TPER / 8 - 1]);
+                } else if (TPER == 16) {
+                    *reinterpret_cast<uint2 *>(b) = make_uint2(w[0], w[TPER / 8 - 1]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < TPER / 8; j++) reinterpret_cast<uint32_t *>(b)[j] = w[j];
+                }
+            }
+        }
+        __syncthreads();
+        if (c0 + TCC < c_end) fetch(c0 + TCC);  // fly while this chunk is consumed
         if (WITH_A && warp == 0) {
             const int nc = min(TCC, g.ic - c0);
             const float *fr = f_s + lane * FLD;
@@ -284,14 +298,14 @@ __global__ void __launch_bounds__(TWARPS * 32) binarize_bytes_nchw_kernel(const 
                 for (; j < nc; j++) acc = __fadd_rn(acc, fr[j]);
             }
         } else if (WITH_PACK) {
-            // half a warp writes one pixel per pass: 16 (12) lanes x 8 bytes, one 128-byte line
+            // TCC / 16 lanes write a pixel's chunk, 8 bytes each
             const int first = WITH_A ? warp - 1 : warp, step = WITH_A ? TWARPS - 1 : TWARPS;
-            const int n8 = (min(TCC, c_end - c0) + 7) / 8;
-            constexpr int LPP = TCC / 8;   // lanes per pixel and chunk
-            constexpr int PPW = 32 / LPP;  // pixels a warp writes per pass
-            const int sub = lane / LPP, wl = lane % LPP;
+            const int n8 = (min(TCC, g.ic - c0) + 15) / 16;
+            constexpr int LPW = TCC / 16;  // lanes per pixel and chunk
+            constexpr int PPW = 32 / LPW;  // pixels a warp writes per pass
+            const int sub = lane / LPW, wl = lane % LPW;
             if (sub < PPW && wl < n8) {
-                uint2 *out = reinterpret_cast<uint2 *>(g.out) + (c0 >> 3) + wl;
+                uint2 *out = reinterpret_cast<uint2 *>(g.out) + (c0 >> 4) + wl;
                 const uint8_t *tile = b_s + 8 * wl;
                 for (int pi = PPW * first + sub; pi < n_live; pi += PPW * step)
                     out[row_s[pi]] = *reinterpret_cast<const uint2 *>(tile + pi * TLD);
@@ -348,53 +362,62 @@ BinArgs bin_args(const Plan &p, const float *src, void *out, float *a) {
 // tiled kernels: blocks per SM the carve-out is sized for (chunks of 128 and of 96 channels)
 constexpr int kResidentBlocks = 5, kResidentBlocks96 = 9;
 
+template <bool WITH_A, bool WITH_PACK, bool NHWC, int TPER>
+cudaError_t launch_tiled(const BinArgs &g, cudaStream_t s) {
+    // Shared-memory carve-out sized for a fixed number of blocks per SM, once per device. Left
+    // to itself the driver sizes it for as many blocks as the thread count allows, which
+    // leaves the L1 too small: the loads in flight occupy it although they do not allocate
+    // lines to keep, and a kernel that streams with 32 loads per thread outstanding does not
+    // need that many warps. Measured on conv4, minibatch 256, pass with the mean-|x| map:
+    // eight blocks (an L1 of 32 KB) 20.4 us, seven or six (64 KB) 16.9-17.3, five (96 KB)
+    // 17.0-17.1 with the whole step 0.5 us shorter, four or three (128 KB) 18.1. The
+    // 96-channel kernel on conv2: nine of its blocks (the same 64 KB of L1) 9.3 us, seven
+    // (96 KB) 9.7, five 11.2.
+    auto kernel = binarize_nibbles_kernel<WITH_A, WITH_PACK, NHWC, TPER>;
+    static std::atomic<bool> tuned[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!tuned[dev & 63].exchange(true, std::memory_order_acq_rel)) {
+        int smem_sm = 0;
+        cudaFuncAttributes fa;
+        cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+        if (smem_sm > 0 && cudaFuncGetAttributes(&fa, kernel) == cudaSuccess) {
+            const int resident = TPER == 32 ? kResidentBlocks : kResidentBlocks96;
+            long pct = (100L * resident * ((long)fa.sharedSizeBytes + 1024) + smem_sm - 1) / smem_sm;
+            if (pct > 100) pct = 100;
+            cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)pct);
+        }
+        (void)cudaGetLastError();
+    }
+    note_launch();
+    // Launched with programmatic stream serialisation like the convolution: behind one of
+    // this library's kernels (which trigger early) the blocks become resident while it
+    // drains and wait in dependency_wait(); behind anything else nothing changes.
+    return launch_overlapped(kernel, dim3((unsigned)((g.n_px + TPX - 1) / TPX)),
+                             dim3(TWARPS * 32), 0, s, 1, g);
+}
+
 template <bool WITH_A, bool WITH_PACK>
 cudaError_t launch_bin(const Plan &p, const BinArgs &g, cudaStream_t s) {
     const int threads = 128;
     const unsigned blocks = (unsigned)((g.n_px + threads - 1) / threads);
     if (blocks == 0) return cudaSuccess;
-    if (!p.src_nhwc && (p.family == kTcgen05 || !WITH_PACK) && g.n_px < (1L << 31) - TPX &&
+    if ((p.family == kTcgen05 || !WITH_PACK) && g.n_px < (1L << 31) - TPX &&
         (long)p.ih * p.iw < (1L << 24)) {
-        // Shared-memory carve-out sized for a fixed number of blocks per SM, once per device. Left
-        // to itself the driver sizes it for as many blocks as the thread count allows, which
-        // leaves the L1 too small: the loads in flight occupy it although they do not allocate
-        // lines to keep, and a kernel that streams with 32 loads per thread outstanding does not
-        // need that many warps. Measured on conv4, minibatch 256, pass with the mean-|x| map:
-        // eight blocks (an L1 of 32 KB) 20.4 us, seven or six (64 KB) 16.9-17.3, five (96 KB)
-        // 17.0-17.1 with the whole step 0.5 us shorter, four or three (128 KB) 18.1. The
-        // 96-channel kernel on conv2: nine of its blocks (the same 64 KB of L1) 9.3 us, seven
-        // (96 KB) 9.7, five 11.2.
-        static std::atomic<bool> tuned[64];
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (!tuned[dev & 63].exchange(true, std::memory_order_acq_rel)) {
-            int smem_sm = 0;
-            cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-            auto carve = [&](auto kernel, int resident) {
-                cudaFuncAttributes fa;
-                if (smem_sm <= 0 || cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return;
-                long pct = (100L * resident * ((long)fa.sharedSizeBytes + 1024) + smem_sm - 1) / smem_sm;
-                if (pct > 100) pct = 100;
-                cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)pct);
-            };
-            carve(binarize_bytes_nchw_kernel<WITH_A, WITH_PACK, 32>, kResidentBlocks);
-            carve(binarize_bytes_nchw_kernel<WITH_A, WITH_PACK, 24>, kResidentBlocks96);
-            (void)cudaGetLastError();
+        if (p.src_nhwc) {
+            if (g.ic <= 32) return launch_tiled<WITH_A, WITH_PACK, true, 8>(g, s);
+            if (g.ic <= 64) return launch_tiled<WITH_A, WITH_PACK, true, 16>(g, s);
+            return launch_tiled<WITH_A, WITH_PACK, true, 32>(g, s);
         }
-        note_launch();
-        // Launched with programmatic stream serialisation like the convolution: behind one of
-        // this library's kernels (which trigger early) the blocks become resident while it
-        // drains and wait in dependency_wait(); behind anything else nothing changes.
-        const dim3 grid((unsigned)((g.n_px + TPX - 1) / TPX)), block(TWARPS * 32);
+        if (g.ic <= 32) return launch_tiled<WITH_A, WITH_PACK, false, 8>(g, s);
+        if (g.ic <= 64) return launch_tiled<WITH_A, WITH_PACK, false, 16>(g, s);
         if (g.ic % 96 == 0 && g.ic % 128 != 0)
-            return launch_overlapped(binarize_bytes_nchw_kernel<WITH_A, WITH_PACK, 24>, grid, block,
-                                     0, s, 1, g);
-        return launch_overlapped(binarize_bytes_nchw_kernel<WITH_A, WITH_PACK, 32>, grid, block, 0,
-                                 s, 1, g);
+            return launch_tiled<WITH_A, WITH_PACK, false, 24>(g, s);
+        return launch_tiled<WITH_A, WITH_PACK, false, 32>(g, s);
     }
     switch (p.family) {
         case kPopc: binarize_kernel<kBitsDense, WITH_A, WITH_PACK><<<blocks, threads, 0, s>>>(g); break;
-        default: binarize_kernel<kBytesFramed, WITH_A, WITH_PACK><<<blocks, threads, 0, s>>>(g); break;
+        default: binarize_kernel<kNibblesFramed, WITH_A, WITH_PACK><<<blocks, threads, 0, s>>>(g); break;
     }
     note_launch();
     return cudaGetLastError();

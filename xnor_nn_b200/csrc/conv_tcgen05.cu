@@ -1,9 +1,11 @@
 // Binary convolution as an implicit GEMM on the 5th-generation tensor cores.
 //
-// Operands are +-1 bytes (0 where a channel, a filter or an image border does not exist), so the
-// int32 accumulator is the signed agreement count S of upstream's kernel
+// Operands are 4-bit floats, +-1 (0 where a channel, a filter or an image border does not exist),
+// and sums of them are exact in fp32 below 2^24 (plan.cpp sees to that), so the accumulator is the
+// signed agreement count S of upstream's kernel
 // (src/default/bcast_convolution_default.cpp:60-103) exactly: products of absent operands are 0,
-// which is upstream's "skip the tap" (:71-72) and its op_c correction (:102) in one.
+// which is upstream's "skip the tap" (:71-72) and its op_c correction (:102) in one. Against the
+// 8-bit integer kind the tensor pipe does twice the work per cycle on half the operand bytes.
 //
 //   D[position][filter] += A[position + shift(tap)][channel] * B[tap][filter][channel]
 //
@@ -15,8 +17,8 @@
 //   warp 0      one lane issues TMA loads (cp.async.bulk.tensor.2d, each CTA fetching its own
 //               tiles) into a ring of shared-memory buffers; completion is counted on an
 //               mbarrier per buffer
-//   warp 1      allocates tensor memory; one lane issues tcgen05.mma.kind::i8 (M=128, N<=256,
-//               K=32 per instruction) into one of two accumulators in tensor memory, and
+//   warp 1      allocates tensor memory; one lane issues tcgen05.mma.kind::mxf4 (M=128, N<=256,
+//               K=64 per instruction) into one of two accumulators in tensor memory, and
 //               tcgen05.commit hands buffers back / accumulators on
 //   warp 18     one lane is a second MMA issuer; the two take alternate ring buffers
 //   warps 2-17  epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
@@ -61,7 +63,13 @@ constexpr int kMaxStages = 8;       // ring buffers: as many as fit, at most thi
 constexpr int kEpiWarps = 16;       // epilogue warps: 4 TMEM lane quadrants x column groups
 constexpr int kIssuer2Warp = 2 + kEpiWarps;  // the second MMA-issuing thread lives in a warp of its own
 constexpr int kThreads = 64 + 32 * kEpiWarps + 32;
-constexpr uint32_t kTmemCols = 512;  // two accumulators of up to 256 columns
+// Tensor memory: two accumulators of n_tile columns and, in the last 16 columns, the block scales.
+// 2 x 256 + 16 is more than the 512 there are, so accumulators of 256 columns share 16 of them
+// (the last of the first = the first of the second): the epilogue empties those before anything
+// else and says so (Control::shared_free), and the next tile's first MMA waits for it.
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kScaleCol = 496;
+constexpr int kAccStep = 240;        // columns between the accumulators' starts, at most
 struct TcArgs {
     const float *alpha;
     const float *kmap;   // K per output pixel, or null: box-filter it from amap in the epilogue
@@ -81,7 +89,7 @@ struct TcArgs {
     uint32_t a_bytes, stage_bytes, tx_bytes;
     int dst_nhwc;
     // chained layers: instead of floats the epilogue writes the next layer's packed input
-    uint8_t *emit_bin;    // next layer's +-1 byte frame, or null
+    uint8_t *emit_bin;    // next layer's +-1 nibble frame, or null
     float *emit_a;        // next layer's mean-|x| map
     int e_wp, e_hp, e_lead, e_icp;  // the next layer's frame geometry
     float e_inv_ic;       // 1.f / (next layer's channels = this layer's filters)
@@ -96,8 +104,11 @@ struct TcArgs {
     int halo;             // 0, or rows of a halo tile (128 + 8)
     int n_a_slots;        // halo tiles in flight
     uint32_t a_slot_bytes, b_ring_off, b_slot_bytes, b_bytes;
-    int kk_last;          // MMAs of a tap's last channel chunk: its 32-channel slices that hold
-                          // channels at all (the chunk is padded with zero bytes to kchunk)
+    int kk_last;          // MMAs of a tap's last channel chunk: its 64-channel slices that hold
+                          // channels at all (the chunk is padded with zeros to kchunk bytes)
+    uint32_t acc_step;    // columns from the first accumulator to the second
+    int paced;            // NCHW floats: the column groups of a tile store one after the other
+    int shared_cols;      // the accumulators overlap (n_tile > kAccStep)
 };
 
 // ---- the kernel --------------------------------------------------------------------------------
@@ -114,6 +125,7 @@ struct __align__(16) Control {
     unsigned long long a_empty[4];
     unsigned long long started[2];  // two issuers: the tile's first MMA (which overwrites) is out
     unsigned long long drain[2];
+    unsigned long long shared_free;  // the columns both accumulators use have been read
     uint32_t tmem_base;
     int abort_flag;
     alignas(16) float alpha[kAlphaSmem];  // read with 16-byte loads
@@ -156,6 +168,11 @@ struct Deal {
     }
 };
 
+// (S * alpha) * K in upstream's order; the + 0 makes a sum of zero +0 whatever sign the adder gave it
+__device__ __forceinline__ float scaled(uint32_t s, float alpha, float k) {
+    return __fmul_rn(__fmaf_rn(__uint_as_float(s), alpha, 0.f), k);
+}
+
 // ---- epilogue role ---------------------------------------------------------------------------------
 // Warp w may touch TMEM lanes [32*(w%4), 32*(w%4)+32); several warps share a quadrant and split
 // its columns between them.
@@ -168,6 +185,8 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
     // a pair's accumulators are handed back on the leader's barriers
     const uint32_t acc_empty0 =
         PAIR ? mapa(smem_u32(&ctl->acc_empty[0]), 0) : smem_u32(&ctl->acc_empty[0]);
+    const uint32_t shared_free0 =
+        PAIR ? mapa(smem_u32(&ctl->shared_free), 0) : smem_u32(&ctl->shared_free);
     // Several warps share a quadrant and split its columns between them.
     const int quad = warp & 3;
     const int cgroup = (warp - 2) >> 2, cgroups = kEpiWarps / 4;
@@ -223,26 +242,42 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
             }
             // The NCHW float epilogue's column groups meet three times per tile (all tiles of a
             // CTA but its last): the same appointments are kept here.
-            if (!g.sums && !g.dst_nhwc && it + 1 < rounds && g.n_tile == 256) {
+            if (!g.sums && !g.dst_nhwc && g.paced && it + 1 < rounds) {
                 for (int w = 0; w < kEpiWarps / 4 - 1; w++) bar_sync(10, 32 * kEpiWarps);
                 continue;
             }
             break;
         }
         fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * g.n_tile);
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)b * g.acc_step;
+        // the warp that owns the columns shared with the other accumulator reads them first
+        const bool shared = g.shared_cols && cgroup == (b ? 0 : kEpiWarps / 4 - 1);
+        const bool reverse = shared && b == 0;
+        auto columns_read = [&](int step) {
+            if (!shared || step != 0) return;
+            fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_cluster(shared_free0);
+                else mbar_arrive(shared_free0);
+            }
+        };
         if (g.emit_bin) {
             // Chained layers: y = (S * alpha) * K is not stored. alpha and K are never negative,
             // so the sign bit of y is the sign bit of S: it goes straight into the next layer's
-            // byte frame (+1 = 0x01, -1 = 0xFF, filters past the last one 0). |y| summed over the
-            // filters and divided by their number is that layer's mean-|x| map; K is common to a
-            // pixel, so the sum runs over |S| * alpha and is scaled once at the end. A thread
-            // owns one pixel and 32 neighbouring filters = 32 contiguous bytes of the frame.
+            // frame (filters past the last one 0). |y| summed over the filters and divided by
+            // their number is that layer's mean-|x| map; K is common to a pixel, so the sum runs
+            // over |S| * alpha and is scaled once at the end. A thread owns one pixel and 32
+            // neighbouring filters = 16 contiguous bytes of the frame.
             const float *al = alpha_in_smem ? ctl->alpha + oc0 : g.alpha + oc0;
             uint8_t *row = g.emit_bin +
-                           ((long)g.e_lead + ((long)n * g.e_hp + oh) * g.e_wp + ow) * g.e_icp + oc0;
+                           ((long)g.e_lead + ((long)n * g.e_hp + oh) * g.e_wp + ow) * g.e_icp +
+                           oc0 / 2;
+            const int room = g.e_icp - oc0 / 2;  // bytes of the row from here on
             float part = 0.f;
-            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups) {
+            const int steps = (g.n_tile - 32 * cgroup + 32 * cgroups - 1) / (32 * cgroups);
+            for (int i = 0; i < steps; i++) {
+                const int c0 = 32 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
                 uint32_t v[32];
                 const int width = g.n_tile - c0 >= 32 ? 32 : 16;
                 if (width == 32) {
@@ -253,50 +288,40 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                     ld16(taddr + (uint32_t)c0, v);
                 }
                 wait_ld();
+                columns_read(i);
                 if (valid) {
                     const int lim = min(n_valid - c0, width);
-                    uint32_t w[8];
+                    uint32_t w[4];
+                    // a sum of zero counts as positive, whatever sign the adder gave it
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), 0.f));
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        w[j] = first_nibbles(sign_nibbles(v + 8 * j), lim - 8 * j);
                     if (alpha_in_smem && lim >= 32) {
                         const float4 *a4 = reinterpret_cast<const float4 *>(al + c0);
 #pragma unroll
                         for (int j = 0; j < 32; j += 4) {
                             const float4 a = a4[j >> 2];
-                            part = fmaf(fabsf((float)(int)v[j]), a.x, part);
-                            part = fmaf(fabsf((float)(int)v[j + 1]), a.y, part);
-                            part = fmaf(fabsf((float)(int)v[j + 2]), a.z, part);
-                            part = fmaf(fabsf((float)(int)v[j + 3]), a.w, part);
-                            // byte 3 of each count, sign-replicated: 0xFF where S < 0, else 0
-                            const uint32_t lo = __byte_perm(v[j], v[j + 1], 0x00FB);
-                            const uint32_t hi = __byte_perm(v[j + 2], v[j + 3], 0x00FB);
-                            w[j >> 2] = __byte_perm(lo, hi, 0x5410) | 0x01010101u;
+                            part = fmaf(fabsf(__uint_as_float(v[j])), a.x, part);
+                            part = fmaf(fabsf(__uint_as_float(v[j + 1])), a.y, part);
+                            part = fmaf(fabsf(__uint_as_float(v[j + 2])), a.z, part);
+                            part = fmaf(fabsf(__uint_as_float(v[j + 3])), a.w, part);
                         }
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            uint32_t word = 0;
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                if (j + i < lim) {
-                                    part = fmaf(fabsf((float)(int)v[j + i]), al[c0 + j + i], part);
-                                    word |= ((v[j + i] >> 31) ? 0xFFu : 0x01u) << (8 * i);
-                                }
-                            }
-                            w[j >> 2] = word;
-                        }
+                        for (int j = 0; j < 32; j++)
+                            if (j < lim) part = fmaf(fabsf(__uint_as_float(v[j])), al[c0 + j], part);
                     }
-                    if (width == 32 && oc0 + c0 + 32 <= g.e_icp && ((oc0 + c0) & 31) == 0) {
-                        // one whole 32-byte sector per thread in a single store
-                        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                                     ::"l"(row + c0), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                                       "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                                     : "memory");
+                    // n_tile is a multiple of 16: a thread's bytes start on 8, often on 16
+                    uint8_t *o = row + c0 / 2;
+                    if (width == 32 && c0 / 2 + 16 <= room && (oc0 & 31) == 0) {
+                        *reinterpret_cast<uint4 *>(o) = make_uint4(w[0], w[1], w[2], w[3]);
                     } else {
-                        if (oc0 + c0 + 16 <= g.e_icp)
-                            *reinterpret_cast<uint4 *>(row + c0) =
-                                make_uint4(w[0], w[1], w[2], w[3]);
-                        if (width == 32 && oc0 + c0 + 32 <= g.e_icp)
-                            *reinterpret_cast<uint4 *>(row + c0 + 16) =
-                                make_uint4(w[4], w[5], w[6], w[7]);
+                        if (c0 / 2 + 8 <= room) *reinterpret_cast<uint2 *>(o) = make_uint2(w[0], w[1]);
+                        if (width == 32 && c0 / 2 + 16 <= room)
+                            *reinterpret_cast<uint2 *>(o + 8) = make_uint2(w[2], w[3]);
                     }
                 }
             }
@@ -325,9 +350,11 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
             // loads (conv4 32.7 -> 31.6 us, VGG 78.6 -> 76.9). Only for tiles of 256 filters: with
             // narrower ones (conv3, N = 192) a tile's MMAs are over sooner than its epilogue
             // spread out like this, and the whole step got slower (55.1 -> 57.7 us).
-            const bool paced = it + 1 < rounds && g.n_tile == 256;
-            if (paced) for (int w = 0; w < cgroup; w++) bar_sync(10, 32 * kEpiWarps);
-            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups) {
+            const bool paced = g.paced && it + 1 < rounds;
+            const int steps = (g.n_tile - 32 * cgroup + 32 * cgroups - 1) / (32 * cgroups);
+            bool waited = !paced;
+            for (int i = 0; i < steps; i++) {
+                const int c0 = 32 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
                 uint32_t v[32];
                 if (c0 + 32 <= g.n_tile) {
                     ld32(taddr + (uint32_t)c0, v);
@@ -335,6 +362,11 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                     ld16(taddr + (uint32_t)c0, v);
                 }
                 wait_ld();
+                columns_read(i);
+                if (!waited) {
+                    waited = true;
+                    for (int w = 0; w < cgroup; w++) bar_sync(10, 32 * kEpiWarps);
+                }
                 if (valid) {
                     const int lim = n_valid - c0;
                     float *o = out + (long)c0 * ohw;
@@ -347,21 +379,20 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                             // streaming stores: the result is not read again by this library,
                             // and lines that leave L2 while this kernel runs (which needs little
                             // of HBM) do not have to leave it under the next, bandwidth-bound pass
-                            __stcs(o, __fmul_rn(__fmul_rn((float)(int)v[j], a.x), kk));
-                            __stcs(o + ohw, __fmul_rn(__fmul_rn((float)(int)v[j + 1], a.y), kk));
-                            __stcs(o + 2 * ohw, __fmul_rn(__fmul_rn((float)(int)v[j + 2], a.z), kk));
-                            __stcs(o + 3 * ohw, __fmul_rn(__fmul_rn((float)(int)v[j + 3], a.w), kk));
+                            __stcs(o, scaled(v[j], a.x, kk));
+                            __stcs(o + ohw, scaled(v[j + 1], a.y, kk));
+                            __stcs(o + 2 * ohw, scaled(v[j + 2], a.z, kk));
+                            __stcs(o + 3 * ohw, scaled(v[j + 3], a.w, kk));
                             o += 4 * ohw;
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; j++)
-                            if (j < lim)
-                                __stcs(o + (long)j * ohw,
-                                       __fmul_rn(__fmul_rn((float)(int)v[j], al[c0 + j]), kk));
+                            if (j < lim) __stcs(o + (long)j * ohw, scaled(v[j], al[c0 + j], kk));
                     }
                 }
             }
+            if (!waited) for (int w = 0; w < cgroup; w++) bar_sync(10, 32 * kEpiWarps);
             if (paced) for (int w = cgroup; w < kEpiWarps / 4 - 1; w++) bar_sync(10, 32 * kEpiWarps);
         } else if (!g.sums && g.dst_nhwc && (g.oc & 3) == 0) {
             // NHWC floats: a thread owns one pixel and 16 neighbouring filters at a time, which
@@ -371,16 +402,19 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
             // 256-bit stores need 32-byte alignment: rows and tiles that are multiples of 8
             // floats on a result buffer aligned likewise
             const bool wide = (g.oc & 7) == 0 && (oc0 & 7) == 0 && ((uintptr_t)g.dst & 31) == 0;
-            for (int c0 = 16 * cgroup; c0 < g.n_tile; c0 += 16 * cgroups) {
+            const int steps = (g.n_tile - 16 * cgroup + 16 * cgroups - 1) / (16 * cgroups);
+            for (int i = 0; i < steps; i++) {
+                const int c0 = 16 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
                 uint32_t v[16];
                 ld16(taddr + (uint32_t)c0, v);
                 wait_ld();
+                columns_read(i);
                 if (valid && wide && c0 + 16 <= n_valid) {
                     // 16 results = two whole 32-byte sectors, one 256-bit store each
                     float x[16];
 #pragma unroll
                     for (int j = 0; j < 16; j++)
-                        x[j] = __fmul_rn(__fmul_rn((float)(int)v[j], al[c0 + j]), kk);
+                        x[j] = scaled(v[j], al[c0 + j], kk);
 #pragma unroll
                     for (int h = 0; h < 16; h += 8)
                         asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -393,29 +427,31 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                     for (int j = 0; j < 16; j += 4) {
                         if (c0 + j >= n_valid) break;  // oc and n_valid are multiples of 4
                         float4 x;
-                        x.x = __fmul_rn(__fmul_rn((float)(int)v[j], al[c0 + j]), kk);
-                        x.y = __fmul_rn(__fmul_rn((float)(int)v[j + 1], al[c0 + j + 1]), kk);
-                        x.z = __fmul_rn(__fmul_rn((float)(int)v[j + 2], al[c0 + j + 2]), kk);
-                        x.w = __fmul_rn(__fmul_rn((float)(int)v[j + 3], al[c0 + j + 3]), kk);
+                        x.x = scaled(v[j], al[c0 + j], kk);
+                        x.y = scaled(v[j + 1], al[c0 + j + 1], kk);
+                        x.z = scaled(v[j + 2], al[c0 + j + 2], kk);
+                        x.w = scaled(v[j + 3], al[c0 + j + 3], kk);
                         *reinterpret_cast<float4 *>(out + c0 + j) = x;
                     }
                 }
             }
         } else {
-            for (int c0 = 16 * cgroup; c0 < g.n_tile; c0 += 16 * cgroups) {
+            const int steps = (g.n_tile - 16 * cgroup + 16 * cgroups - 1) / (16 * cgroups);
+            for (int i = 0; i < steps; i++) {
+                const int c0 = 16 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
                 uint32_t v[16];
                 ld16(taddr + (uint32_t)c0, v);
                 wait_ld();
+                columns_read(i);
                 if (valid) {
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
                         const int oc = oc0 + c0 + j;
                         if (oc >= g.oc) continue;
                         if (g.sums) {
-                            g.sums[((long)n * g.oc + oc) * ohw + r] = (int)v[j];
+                            g.sums[((long)n * g.oc + oc) * ohw + r] = (int)__uint_as_float(v[j]);
                         } else {
-                            const float x =
-                                __fmul_rn(__fmul_rn((float)(int)v[j], __ldg(g.alpha + oc)), kk);
+                            const float x = scaled(v[j], __ldg(g.alpha + oc), kk);
                             if (g.dst_nhwc) g.dst[pix * g.oc + oc] = x;
                             else g.dst[((long)n * g.oc + oc) * ohw + r] = x;
                         }
@@ -474,6 +510,9 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
             else if (n_iss > 1)
                 ok = mbar_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6,
                                g.wait_ns);
+            if (ok && ks == 0 && g.shared_cols && it > 0)
+                ok = mbar_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
+                               g.error, 7, g.wait_ns);
             if (!ok) break;
             fence_after();
             entered = true;
@@ -483,7 +522,7 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
             ok = mbar_wait(fbar, phase, abort_flag, g.error, 3, g.wait_ns);
             if (!ok) break;
         }
-        const uint32_t d_tmem = tmem_base + (uint32_t)(b * g.n_tile);
+        const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
         const uint32_t desc_off = (uint32_t)stage * stage_units;
         const uint64_t adesc = hi | (uint64_t)(a_lo0 + desc_off);
         const uint64_t bdesc = hi | (uint64_t)(b_lo0 + desc_off);
@@ -492,12 +531,8 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
 #pragma unroll
         for (int k = 0; k < KK; k++) {
             if (k < kk) {
-                if (PAIR)
-                    mma_i8_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
-                                g.idesc, (k == 0 && ks == 0) ? 0u : 1u);
-                else
-                    mma_i8(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), g.idesc,
-                           (k == 0 && ks == 0) ? 0u : 1u);
+                mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
+                               g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
             }
         }
         if (PAIR) commit_pair(empty0 + 8u * (uint32_t)stage);  // frees the stage in both CTAs
@@ -639,6 +674,9 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
             else if (n_iss > 1)
                 ok = mbar_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6,
                                g.wait_ns);
+            if (ok && ks == 0 && g.shared_cols && it > 0)
+                ok = mbar_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
+                               g.error, 7, g.wait_ns);
             if (!ok) break;
             fence_after();
             entered = true;
@@ -657,7 +695,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
             if (!ok) break;
         }
         fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(b * g.n_tile);
+        const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
         const uint64_t adesc =
             hi | (uint64_t)(a_lo0 + (uint32_t)sa * a_units + (uint32_t)kw * row_units);
         const uint64_t bdesc = hi | (uint64_t)(b_lo0 + (uint32_t)sb * b_units);
@@ -665,12 +703,8 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
 #pragma unroll
         for (int k = 0; k < KK; k++) {
             if (k < kk) {
-                if (PAIR)
-                    mma_i8_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
-                                g.idesc, (k == 0 && ks == 0) ? 0u : 1u);
-                else
-                    mma_i8(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), g.idesc,
-                           (k == 0 && ks == 0) ? 0u : 1u);
+                mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
+                               g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
             }
         }
         if (PAIR) commit_pair(empty0 + 8u * (uint32_t)sb);
@@ -749,6 +783,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             mbar_init(smem_u32(&ctl->started[b]), 1);
             mbar_init(smem_u32(&ctl->drain[b]), 1);
         }
+        mbar_init(smem_u32(&ctl->shared_free), PAIR ? 8 : 4);  // one arrival per lane quadrant
         ctl->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // the descriptors are launch parameters: fetch them while the predecessor still runs
@@ -760,6 +795,12 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         // address in both CTAs of a pair.
         tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
     }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem_base = ctl->tmem_base;
+    if (warp >= 2 && warp < 6)
+        fill_scales(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kScaleCol, 16);
     // Everything above touched only this CTA's own shared and tensor memory and the launch
     // parameters. What earlier kernels of the stream produced is read by the TMA producer and
     // the epilogue warps, each after its own dependency_wait(); the MMA issuer reads shared
@@ -776,7 +817,6 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     // soon as all of them have got here: its CTAs move in as these exit (SMs with one tile fewer
     // exit a round early) and set themselves up; they wait for this grid's results themselves.
     dependency_release();
-    const uint32_t tmem_base = ctl->tmem_base;
 
     const Deal<PAIR> deal(g);
     const int rounds = deal.rounds(g);
@@ -914,7 +954,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.m_tiles = m_tiles;
     g.n_tiles = p.ocp16 / p.n_tile;
     g.n_tile = p.n_tile;
-    g.kchunk = p.kchunk; g.chunks_per_tap = p.icp / p.kchunk; g.taps = p.kh * p.kw;
+    g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(p.icp, p.kchunk); g.taps = p.kh * p.kw;
     g.kw = p.kw; g.ph = p.ph; g.pw = p.pw; g.wp = p.wp; g.hp = p.hp; g.lead = p.lead;
     g.oh = p.oh; g.ow = p.ow; g.oc = p.oc; g.ocp16 = p.ocp16;
     g.dst_nhwc = p.dst_nhwc;
@@ -928,10 +968,11 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         g.e_inv_ic = next->inv_ic;
         g.n_inner = 1;
     }
-    // instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, N and M encoded
-    // (M = 256 for a pair: 128 rows in each CTA)
-    g.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.n_tile >> 3) << 17) |
-              ((uint32_t)((pair ? 2 * BM : BM) >> 4) << 24);
+    // M = 256 for a pair: 128 rows in each CTA
+    g.idesc = mxf4_idesc(pair ? 2 * BM : BM, (uint32_t)p.n_tile);
+    g.shared_cols = p.n_tile > kAccStep;
+    g.acc_step = (uint32_t)(p.n_tile < kAccStep ? p.n_tile : kAccStep);
+    g.paced = p.n_tile == 256;
     // matrix descriptor, upper half: stride between 8-row groups (8 * kchunk bytes, in 16-byte
     // units), descriptor version 1, swizzle mode
     const uint32_t sbo = (uint32_t)(8 * p.kchunk) >> 4;
@@ -941,12 +982,12 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.tx_bytes = g.a_bytes + (uint32_t)(b_rows * p.kchunk);  // per CTA
     g.stage_bytes = (g.tx_bytes + 1023u) & ~1023u;
     g.issuers = g.taps * g.chunks_per_tap < 2 ? 1 : 2;
-    g.kk_last = (p.ic - (g.chunks_per_tap - 1) * p.kchunk + 31) / 32;
+    g.kk_last = (p.ic - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
     g.halo = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
-    bool halo = pair && p.kchunk == 128 && p.kw >= 2 && p.kw <= 9 && g.issuers <= p.kw;
+    bool halo = pair && p.kw >= 2 && p.kw <= 9 && g.issuers <= p.kw;
     if (halo) {
         // three halo tiles of 136 positions, the rest of the room for filter tiles
         g.halo = BM + 8;

@@ -2,14 +2,15 @@
 //
 //   D[filter][position] += W[tap][filter][channel] * X[position + tap][channel]
 //
-// Operands are +-1 bytes (0 where a channel, a filter or an image border does not exist), so the
-// int32 accumulator is the signed agreement count S of upstream's kernel
+// Operands are 4-bit floats, +-1 (0 where a channel, a filter or an image border does not exist),
+// and sums of them are exact in fp32 below 2^24 (plan.cpp sees to that), so the accumulator is the
+// signed agreement count S of upstream's kernel
 // (src/default/bcast_convolution_default.cpp:60-103) exactly: products of absent operands are 0,
 // which is upstream's "skip the tap" (:71-72) and its op_c correction (:102) in one.
 //
 // A tile is 128 filters (UMMA M = the 128 lanes of tensor memory) by R whole output rows of one
-// image (UMMA N = R*OW rounded up to 16, at most 256). The activation operand of a filter tap is
-// then one 4-D TMA box {channels, OW columns, R rows, 1 image} of the byte tensor, shifted by
+// image (UMMA N = R*OW rounded up to 16, at most 240). The activation operand of a filter tap is
+// then one 4-D TMA box {channels, OW columns, R rows, 1 image} of the packed tensor, shifted by
 // the tap; whatever lies outside the image is filled with zeros by the copy engine, so no
 // position is computed that is not an output pixel and no im2col buffer exists. For the 13x13
 // AlexNet layers R = 13: a tile is a whole image, and what 32 filters produce for it is one
@@ -18,7 +19,7 @@
 // One CTA per SM, persistent over its tiles:
 //   warp 0      one lane issues the TMA loads of a pipeline stage (a weight tile and an
 //               activation box of one filter tap x one channel chunk) into a ring of buffers
-//   warp 1      allocates tensor memory; one lane issues tcgen05.mma.kind::i8 (M=128, K=32 per
+//   warp 1      allocates tensor memory; one lane issues tcgen05.mma.kind::mxf4 (M=128, K=64 per
 //               instruction) into one of two accumulators and hands buffers back with
 //               tcgen05.commit
 //   warps 2-5   epilogue, one warp per 32-lane quadrant of tensor memory = 32 filters: K of the
@@ -55,7 +56,8 @@ constexpr int kTeam = 2;            // epilogue warps per TMEM lane quadrant (th
 constexpr int kEpiWarps = 4 * kTeam;
 constexpr int kProducerW = 2 + kEpiWarps;  // the warp that loads the weight tiles
 constexpr int kThreads = 32 * (kProducerW + 1);
-constexpr uint32_t kTmemCols = 512;  // two accumulators of up to 256 columns
+constexpr uint32_t kTmemCols = 512;  // two accumulators of kImgColumns columns, block scales behind them
+constexpr uint32_t kScaleCol = 2 * kImgColumns;
 constexpr int kMaxStages = 8;
 constexpr int kControlBytes = 2304;
 
@@ -76,6 +78,7 @@ struct ImgArgs {
     int half_rows;                   // rows of the first half of a split tile
     // operands
     int kchunk, chunks_per_tap, taps, ocp16;
+    int kk_last;       // MMAs of a tap's last channel chunk: its 64-channel slices that hold channels
     uint32_t idesc_full, idesc_half;
     int n_full, n_half;
     uint32_t desc_hi;  // upper 32 bits of the shared-memory matrix descriptors
@@ -183,6 +186,12 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_xh) : "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem_base = ctl->tmem_base;
+    if (warp >= 2 && warp < 6)
+        fill_scales(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kScaleCol, 32);
     // Everything above touched only this CTA's own shared and tensor memory and the launch
     // parameters. What earlier kernels of the stream produced is read by the TMA producer and
     // the epilogue warps, each after its own dependency_wait(); the MMA issuer reads shared
@@ -194,7 +203,6 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
     // soon as all of them have got here: its CTAs move in as these exit and set themselves up;
     // they wait for this grid's results themselves.
     dependency_release();
-    const uint32_t tmem_base = ctl->tmem_base;
 
     const int rounds = rounds_of(g);
     const int ksteps = g.taps * g.chunks_per_tap;
@@ -290,8 +298,9 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                                g.wait_ns);
                 if (!ok) break;
                 fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(b * 256);
+                const uint32_t d_tmem = tmem_base + (uint32_t)(b * kImgColumns);
                 uint32_t accumulate = 0;
+                int chunk = 0;
                 for (int ks = 0; ks < ksteps; ks++) {
                     if (!ready) {
                         const uint32_t fbar = full0 + 8u * (uint32_t)stage;
@@ -305,10 +314,15 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                     ready = mbar_test(full0 + 8u * (uint32_t)next, next_phase);
                     const uint64_t adesc = hi | (uint64_t)(a_lo0 + desc_off);
                     const uint64_t bdesc = hi | (uint64_t)(b_lo0 + desc_off);
+                    // slices of zero padding behind the last channel are not multiplied
+                    const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+                    if (++chunk == g.chunks_per_tap) chunk = 0;
 #pragma unroll
                     for (int k = 0; k < KK; k++)
-                        mma_i8(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc,
-                               k == 0 ? accumulate : 1u);
+                        if (k < kk)
+                            mma_mxf4<false>(d_tmem, adesc + (uint64_t)(2 * k),
+                                            bdesc + (uint64_t)(2 * k), idesc,
+                                            tmem_base + kScaleCol, k == 0 ? accumulate : 1u);
                     accumulate = 1;
                     commit(empty0 + 8u * (uint32_t)stage);
                     desc_off = next == 0 ? 0u : desc_off + stage_units;
@@ -381,7 +395,7 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
             const int mis = (int)(((uintptr_t)run >> 2) & 3u);
             uint32_t *const srow_of_lane =
                 block_mode ? sbuf + (size_t)lane * ohw : sbuf + (size_t)lane * g.ldg + mis;
-            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 256);
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kImgColumns);
             if (live) {
                 fence_after();
                 const float *kk = ctl->kk[b];
@@ -407,13 +421,14 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                             const float4 k4 = *reinterpret_cast<const float4 *>(kk + c0 + j);
                             kv[j] = k4.x; kv[j + 1] = k4.y; kv[j + 2] = k4.z; kv[j + 3] = k4.w;
                         }
-                        // (float)S without the slow conversion pipe: |S| < 2^22, so the integer
-                        // lands exactly in the mantissa of 1.5 * 2^23 and one subtraction recovers it
+                        // S * alpha + 0: a sum of zero is +0 whatever the sign the adder gave it
 #pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            const float sf = __fsub_rn(__uint_as_float(0x4B400000u + v[j]), 12582912.f);
-                            v[j] = __float_as_uint(__fmul_rn(__fmul_rn(sf, al), kv[j]));
-                        }
+                        for (int j = 0; j < 32; j++)
+                            v[j] = __float_as_uint(
+                                __fmul_rn(__fmaf_rn(__uint_as_float(v[j]), al, 0.f), kv[j]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) v[j] = (uint32_t)(int)__uint_as_float(v[j]);
                     }
                     if (staged) {
                         if (c0 + 32 <= len) {
@@ -515,14 +530,13 @@ cudaError_t launch_conv_tcgen05_img(const Plan &p, const void *bin_src, const vo
     g.whole = p.img_whole;
     g.units = p.img_whole + 2 * (p.img_tiles - p.img_whole);
     g.half_rows = p.img_half_rows;
-    g.kchunk = p.kchunk; g.chunks_per_tap = p.icp / p.kchunk; g.taps = p.kh * p.kw;
+    g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(p.icp, p.kchunk); g.taps = p.kh * p.kw;
     g.ocp16 = p.ocp16;
+    g.kk_last = (p.ic - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     g.n_full = p.img_n;
     g.n_half = p.img_n_half ? p.img_n_half : p.img_n;
-    // instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, N and M encoded
-    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFilters >> 4) << 24);
-    g.idesc_full = idesc | ((uint32_t)(g.n_full >> 3) << 17);
-    g.idesc_half = idesc | ((uint32_t)(g.n_half >> 3) << 17);
+    g.idesc_full = mxf4_idesc(kFilters, (uint32_t)g.n_full);
+    g.idesc_half = mxf4_idesc(kFilters, (uint32_t)g.n_half);
     // matrix descriptor, upper half: stride between 8-row groups (8 * kchunk bytes, in 16-byte
     // units), descriptor version 1, swizzle mode
     const uint32_t sbo = (uint32_t)(8 * p.kchunk) >> 4;

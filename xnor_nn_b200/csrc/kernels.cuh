@@ -44,6 +44,25 @@ inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 b
 }
 
 #ifdef __CUDACC__
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+
+// The +-1 nibbles (e2m1: 0x2, and 0xA where the top bit of the word is set) of eight words, the
+// first in the lowest nibble. A selector nibble of 0xB / 0xF replicates the top bit of byte 3 of
+// the first / second operand, so eight words cost six byte permutes and two logic operations.
+__device__ __forceinline__ uint32_t sign_nibbles(const uint32_t *v) {
+    const uint32_t even = prmt(prmt(v[0], v[2], 0xFBFBu), prmt(v[4], v[6], 0xFBFBu), 0x5410u);
+    const uint32_t odd = prmt(prmt(v[1], v[3], 0xFBFBu), prmt(v[5], v[7], 0xFBFBu), 0x5410u);
+    return (((even & 0x0F0F0F0Fu) | (odd & 0xF0F0F0F0u)) & 0x88888888u) | 0x22222222u;
+}
+// The same with only the first `n` words present (n < 0 counts as none): the others are 0.
+__device__ __forceinline__ uint32_t first_nibbles(uint32_t word, int n) {
+    return n >= 8 ? word : n <= 0 ? 0u : word & (0xFFFFFFFFu >> (4 * (8 - n)));
+}
+
 // Lets the next kernel of the stream start its set-up now ...
 __device__ __forceinline__ void dependency_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -87,14 +106,14 @@ cudaError_t launch_conv_popc(const Plan &p, const uint32_t *bin_src, const uint3
                              const float *alpha, const float *k, const int32_t *op_c, float *dst,
                              int32_t *sums, cudaStream_t s);
 
-// The same contract on the tensor cores (tcgen05.mma kind::i8 over +-1 bytes, plan.hpp's framed
+// The same contract on the tensor cores (tcgen05.mma kind::mxf4 over +-1 nibbles, plan.hpp's framed
 // layout). `error_word` is a device int the kernel sets non-zero if one of its bounded waits
 // ran out; it is never cleared by the kernel. With k == nullptr the epilogue box-filters K from
 // the mean-|x| map `a` itself (same arithmetic as launch_box_filter) and records it in k_out,
 // which saves the separate stencil launch in the fused forward call.
 //
 // `next` chains two layers in the packed domain: instead of storing floats, the epilogue writes
-// the sign of every result into the following layer's byte frame and the mean |result| over the
+// the sign of every result into the following layer's frame and the mean |result| over the
 // filters into its mean-|x| map, which is what that layer's binarize_data and the first half of
 // its calculate_k would have produced from the stored floats (upstream
 // src/bcast_binarize_data.cpp:43-73, src/bcast_calculate_k.cpp:49-66). The signs are exact; the

@@ -42,11 +42,13 @@ static Family family_from_env() {
     return kAuto;
 }
 
-// Both tensor-core kernels read the zero-framed activation bytes and describe a unit-stride
-// convolution only.
+// Both tensor-core kernels read the zero-framed activation nibbles, describe a unit-stride
+// convolution only, and accumulate in fp32: exact while no sum can leave the 24-bit range in
+// which every integer is a float.
 static bool unit_stride(const Plan &p) {
     return p.sh == 1 && p.sw == 1 && p.oh > 0 && p.ow > 0 &&
-           (long)p.mb * (p.ih + p.ph) * (p.iw + p.pw) < (1L << 30);
+           (long)p.mb * (p.ih + p.ph) * (p.iw + p.pw) < (1L << 30) &&
+           (long)p.ic * p.kh * p.kw <= (1L << 24);
 }
 
 // The position-tile kernel walks the frame with one constant row shift per filter tap. That
@@ -62,8 +64,8 @@ static bool frame_walk_ok(const Plan &p) {
 
 // The image-row kernel addresses the frame as a 4-D tensor (channel, column, row, image) and lets
 // the copy engine fill whatever lies outside with zeros, so any padding and any output extent
-// work; a tile must hold at least one whole output row.
-static bool image_rows_ok(const Plan &p) { return unit_stride(p) && p.ow <= 256; }
+// work; a tile must hold at least one whole output row (an accumulator has kImgColumns columns).
+static bool image_rows_ok(const Plan &p) { return unit_stride(p) && p.ow <= kImgColumns; }
 
 // Relative duration of a tile whose UMMA N is n: an instruction occupies the tensor pipe for n/2
 // cycles, but the issuing thread needs about 45 cycles per tcgen05.mma and 275 per
@@ -90,7 +92,7 @@ void plan_image_rows(Plan *p) {
     const int m_blocks = div_up_i(p->oc, 128);
     long best = -1;
     int best_r = 0;
-    for (int r = 1; r <= p->oh && r * p->ow <= 256; r++) {
+    for (int r = 1; r <= p->oh && r * p->ow <= kImgColumns; r++) {
         const int n = div_up_i(r * p->ow, 16) * 16;
         const long tiles = (long)p->mb * div_up_i(p->oh, r) * m_blocks;
         const long rem = tiles % sms;
@@ -194,15 +196,13 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
         plan_popc();
         return;
     }
-    // K chunk = bytes of one channel group per pipeline stage = the swizzle span. Wide chunks
-    // mean few, fat stages (4 MMAs per barrier round trip at 128 B), which is worth some zero
-    // padding of the channels: 96 channels padded to 128 run the 5x5 AlexNet layer in 67 us, as
-    // three 32-byte chunks in 89 us. Take the widest chunk that pads the channels by no more
-    // than 35 %.
-    p->kchunk = 32;
-    for (int k = 128; k >= 64; k /= 2)
-        if (div_up_i(p->ic, k) * k <= p->ic * 1.35) { p->kchunk = k; break; }
-    p->icp = div_up_i(p->ic, p->kchunk) * p->kchunk;
+    // A position's channels are packed two to a byte, rows padded to the 16 bytes that a tensor
+    // map's stride has to be a multiple of. K chunk = bytes of a row per pipeline stage = the
+    // swizzle span: the widest one that a row fills by more than half. The copy engine fills what
+    // lies past the row with zeros, and slices of 64 channels that hold no channel are not
+    // multiplied, so the only cost of a chunk that is not full is shared memory.
+    p->icp = div_up_i(p->ic, 32) * 16;
+    p->kchunk = p->icp > 64 ? 128 : p->icp > 32 ? 64 : 32;
     // Filter tile of the position-tile kernel = its UMMA N: a multiple of 16, at most 256. The
     // filters are split into the fewest equal tiles and padded (with zero filters) to fill them,
     // so N stays as wide as possible: the kernel is bound by the instruction stream that issues

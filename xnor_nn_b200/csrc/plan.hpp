@@ -15,10 +15,14 @@ namespace xb200 {
 // so the choice is fixed at init and every executor of the descriptor follows it.
 enum Family : int {
     kPopc = 0,          // bits, LOP3 + POPC on the integer pipe; any stride, padding and format
-    kTcgen05 = 2,       // +-1 int8, tcgen05.mma kind::i8 into tensor memory; stride 1
+    kTcgen05 = 2,       // +-1 as 4-bit floats, tcgen05.mma kind::mxf4 into tensor memory; stride 1
     kTcgen05Rows = 3,   // request only: the same family, forced onto its image-row kernel
     kAuto = -1,
 };
+
+// Accumulator columns of the image-row kernel: two of them and 32 columns of block scales fill
+// the 512 columns of tensor memory.
+constexpr int kImgColumns = 240;
 
 struct Plan {
     // geometry (copied from the descriptor so kernels never chase the caller's struct)
@@ -41,15 +45,16 @@ struct Plan {
     int icw;  // 32-bit words per pixel
     int ocp;  // output channels rounded up to the kernel's channel tile
 
-    // ---- int8 layout (kTcgen05) ----------------------------------------------------------
-    // Activations are +-1 bytes on a zero frame so that a filter tap is a constant row shift:
-    // rows of (iw + pw) positions (the pw zeros after a row double as the left border of the
-    // next one), (ih + ph) rows per image (same sharing between images), lead rows of zeros in
-    // front. Position q of image n, row h, column w sits at row
+    // ---- 4-bit layout (kTcgen05) -----------------------------------------------------------
+    // A value is a 4-bit float (e2m1): +1 = 0x2, -1 = 0xA, 0 = 0x0, channel c in the low (c even)
+    // or high nibble of byte c/2. Activations are +-1 on a zero frame so that a filter tap is a
+    // constant row shift: rows of (iw + pw) positions (the pw zeros after a row double as the left
+    // border of the next one), (ih + ph) rows per image (same sharing between images), lead rows
+    // of zeros in front. Position q of image n, row h, column w sits at row
     //   lead + (n*(ih+ph) + h)*(iw+pw) + w
     // of a [rows][icp] byte matrix, and tap (kh,kw) of the output at q reads row
     //   q + (kh-ph)*(iw+pw) + (kw-pw).
-    int icp;        // channels rounded up to the K chunk (bytes per position)
+    int icp;        // bytes per position: two channels each, rounded up to 16
     int kchunk;     // bytes of K per pipeline stage: 128, 64 or 32 (= the swizzle span)
     int wp, hp;     // iw + pw, ih + ph
     int lead;       // zero rows in front of the first image

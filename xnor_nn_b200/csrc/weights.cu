@@ -1,117 +1,189 @@
 // Weight-side kernels: sign packing, alpha = mean |w| per output channel, and the per-pixel
-// count of contributing operands. They run once per weight change (a few hundred KB of
-// output), off the per-minibatch path, so they favour exactness over speed: alpha is summed by
-// one thread per output channel in upstream's (ic, kh, kw) order
-// (src/bcast_binarize_weights.cpp:99-114) and therefore rounds identically.
+// count of contributing operands, in one launch. A training step runs it once per pass.
+//
+// alpha is summed in upstream's (ic, kh, kw) order (src/bcast_binarize_weights.cpp:99-114) and
+// therefore rounds identically: a serial chain of IC*KH*KW additions per filter, four cycles each,
+// which is what bounds the launch (3456 additions: 7.3 us). So every filter gets a chain of its
+// own (OIHW: one warp per filter; HWIO: one lane, because 32 neighbouring filters share a line),
+// the loads of the next stretch are in flight while the current one is added up, and packing and
+// counting run in other blocks of the same launch meanwhile.
 #include "kernels.cuh"
 
 namespace xb200 {
 
 namespace {
 
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+constexpr int kStretch = 256;  // OIHW: elements a warp stages at a time
+constexpr int kSlab = 64;      // HWIO: elements of 32 filters a block stages at a time
+
 struct WArgs {
     const float *w;
     int oc, ic, kh, kw;
-    bool hwio;
+    float *alpha;
+    float inv_chw;
+    uint32_t *out;
+    int rows;   // filters per tap in the packed matrix (padded with zero filters)
+    int words;  // 32-bit words per packed row
+    int nibbles;  // 1: [tap][row][word of 8 channels]; 0: bits, [tap][word of 32 channels][row]
+    int32_t *op_c;
+    int ih, iw, oh, ow, sh, sw, ph, pw;
+    int alpha_blocks, pack_blocks;  // roles by block index: alpha, packing, then counting
 };
 
-__device__ __forceinline__ long w_index(const WArgs &g, int oc, int c, int kh, int kw) {
-    return g.hwio ? (((long)kh * g.kw + kw) * g.ic + c) * g.oc + oc
-                  : (((long)oc * g.ic + c) * g.kh + kh) * g.kw + kw;
+template <bool HWIO>
+__device__ __forceinline__ long w_index(const WArgs &g, int oc, int c, int tap) {
+    return HWIO ? ((long)tap * g.ic + c) * g.oc + oc : ((long)oc * g.ic + c) * (g.kh * g.kw) + tap;
 }
 
 __device__ __forceinline__ unsigned sign_clear(float x) { return (~__float_as_uint(x)) >> 31; }
 
-// bits: uint32 [tap][word][ocp]
-__global__ void pack_weight_bits_kernel(const WArgs g, uint32_t *out, int icw, int ocp) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long total = (long)g.kh * g.kw * icw * ocp;
-    if (i >= total) return;
-    const int oc = (int)(i % ocp);
-    const int word = (int)((i / ocp) % icw);
-    const int tap = (int)(i / ((long)ocp * icw));
-    const int kh = tap / g.kw, kw = tap - kh * g.kw;
-    uint32_t v = 0;
-    for (int b = 0; b < 32; b++) {
-        const int c = word * 32 + b;
-        unsigned bit = 0;
-        if (oc < g.oc && c < g.ic) bit = sign_clear(__ldg(g.w + w_index(g, oc, c, kh, kw)));
-        v = (v << 1) | bit;
+// alpha, OIHW: a warp walks its filter's contiguous run, lane 0 adds.
+__device__ __forceinline__ void alpha_oihw(const WArgs &g, float (*stage)[kStretch]) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int oc = blockIdx.x * kWarps + warp;
+    if (oc >= g.oc) return;
+    const int n = g.ic * g.kh * g.kw;
+    const float *p = g.w + (long)oc * n;
+    float *t = stage[warp];
+    float acc = 0.f, v[kStretch / 32];
+#pragma unroll
+    for (int i = 0; i < kStretch / 32; i++) {
+        const int e = i * 32 + lane;
+        v[i] = e < n ? __ldg(p + e) : 0.f;
     }
-    out[i] = v;
+    for (int e0 = 0; e0 < n; e0 += kStretch) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kStretch / 32; i++) t[i * 32 + lane] = __fmul_rn(fabsf(v[i]), g.inv_chw);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kStretch / 32; i++) {
+            const int e = e0 + kStretch + i * 32 + lane;
+            v[i] = e < n ? __ldg(p + e) : 0.f;
+        }
+        if (lane == 0) {
+            const int m = min(kStretch, n - e0);
+            int e = 0;
+            for (; e + 32 <= m; e += 32) {
+                float4 q[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) q[j] = *reinterpret_cast<const float4 *>(t + e + 4 * j);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    acc = __fadd_rn(acc, q[j].x);
+                    acc = __fadd_rn(acc, q[j].y);
+                    acc = __fadd_rn(acc, q[j].z);
+                    acc = __fadd_rn(acc, q[j].w);
+                }
+            }
+            for (; e < m; e++) acc = __fadd_rn(acc, t[e]);
+        }
+    }
+    if (lane == 0) g.alpha[oc] = acc;
 }
 
-// bytes: int8 [tap][ocp16][icp], +1 / -1, zero where the channel or the filter does not exist
-__global__ void pack_weight_bytes_kernel(const WArgs g, uint32_t *out, int icp, int ocp16) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int groups = icp / 4;
-    const long total = (long)g.kh * g.kw * ocp16 * groups;
-    if (i >= total) return;
-    const int grp = (int)(i % groups);
-    const int oc = (int)((i / groups) % ocp16);
-    const int tap = (int)(i / ((long)groups * ocp16));
-    const int kh = tap / g.kw, kw = tap - kh * g.kw;
-    uint32_t v = 0;
-    for (int b = 0; b < 4; b++) {
-        const int c = grp * 4 + b;
-        if (oc < g.oc && c < g.ic)
-            v |= (sign_clear(__ldg(g.w + w_index(g, oc, c, kh, kw))) ? 0x01u : 0xFFu) << (8 * b);
-    }
-    out[i] = v;
-}
-
-// alpha[oc] = sum over (ic, kh, kw) ascending of |w| * (1/(IC*KH*KW)), one thread per filter so
-// that the additions happen in upstream's order. A block owns 32 filters; the weights are staged
-// through shared memory in chunks so that the global reads are coalesced (OIHW: each filter's
-// weights are one contiguous run; HWIO: 32 neighbouring filters are contiguous for each (tap, ic)).
-constexpr int ACH = 128;  // elements of the (ic, kh, kw) walk per chunk
-
-__global__ void __launch_bounds__(256) alpha_kernel(const WArgs g, float *alpha, float inv_chw) {
-    __shared__ float t[32][ACH + 1];
-    const int oc0 = blockIdx.x * 32;
-    const int n = g.ic * g.kh * g.kw, khw = g.kh * g.kw;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float acc = 0.f;
-    for (int e0 = 0; e0 < n; e0 += ACH) {
-        const int ne = min(ACH, n - e0);
-        if (!g.hwio) {
-            // warp w stages filters w, w+8, ...: lanes walk the contiguous run of one filter
-            for (int f = warp; f < 32; f += 8)
-                for (int e = lane; e < ne; e += 32)
-                    t[f][e] = oc0 + f < g.oc ? fabsf(__ldg(g.w + (long)(oc0 + f) * n + e0 + e)) : 0.f;
-        } else {
-            // lanes walk 32 neighbouring filters of one (ic, kh, kw) element
-            for (int e = warp; e < ne; e += 8) {
-                const int idx = e0 + e;  // position in upstream's (ic, kh, kw) walk
-                const int c = idx / khw, tap = idx - c * khw;
-                t[lane][e] = oc0 + lane < g.oc
-                                 ? fabsf(__ldg(g.w + ((long)tap * g.ic + c) * g.oc + oc0 + lane))
-                                 : 0.f;
+// alpha, HWIO: 32 neighbouring filters are one line of every (tap, channel); the block stages
+// kSlab elements of them, warp 0 adds, one lane per filter.
+__device__ __forceinline__ void alpha_hwio(const WArgs &g, float (*stage)[kSlab][32]) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int oc = blockIdx.x * 32 + lane;
+    const int khw = g.kh * g.kw, n = g.ic * khw;
+    float acc = 0.f, v[kSlab / kWarps];
+    auto fetch = [&](int e0) {
+#pragma unroll
+        for (int i = 0; i < kSlab / kWarps; i++) {
+            const int e = e0 + i * kWarps + warp;  // position in upstream's (ic, kh, kw) walk
+            const int c = e / khw, tap = e - c * khw;
+            v[i] = e < n && oc < g.oc ? __ldg(g.w + w_index<true>(g, oc, c, tap)) : 0.f;
+        }
+    };
+    fetch(0);
+    int b = 0;
+    for (int e0 = 0; e0 < n; e0 += kSlab, b ^= 1) {
+#pragma unroll
+        for (int i = 0; i < kSlab / kWarps; i++)
+            stage[b][i * kWarps + warp][lane] = __fmul_rn(fabsf(v[i]), g.inv_chw);
+        __syncthreads();  // slab b is complete; the other one has been added up
+        fetch(e0 + kSlab);
+        if (warp == 0) {
+            const int m = min(kSlab, n - e0);
+            if (m == kSlab) {
+#pragma unroll
+                for (int e = 0; e < kSlab; e++) acc = __fadd_rn(acc, stage[b][e][lane]);
+            } else {
+                for (int e = 0; e < m; e++) acc = __fadd_rn(acc, stage[b][e][lane]);
             }
         }
-        __syncthreads();
-        if (warp == 0)
-            for (int e = 0; e < ne; e++) acc = __fadd_rn(acc, __fmul_rn(t[lane][e], inv_chw));
-        __syncthreads();
     }
-    if (warp == 0 && oc0 + lane < g.oc) alpha[oc0 + lane] = acc;
+    if (warp == 0 && oc < g.oc) g.alpha[oc] = acc;
 }
 
-__global__ void op_count_kernel(int32_t *op_c, int ic, int ih, int iw, int oh, int ow, int kh,
-                                int kw, int sh, int sw, int ph, int pw) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= oh * ow) return;
-    const int y = o / ow, x = o - y * ow;
-    int taps = 0;
-    for (int i = 0; i < kh; i++) {
-        const int h = y * sh - ph + i;
-        if (h < 0 || h >= ih) continue;
-        for (int j = 0; j < kw; j++) {
-            const int w = x * sw - pw + j;
-            taps += (w >= 0 && w < iw);
+// One 32-bit word of the packed matrix per thread; channels and filters that do not exist are 0.
+// OIHW: the items of a filter are neighbours, so that its run stays in the L1 while its taps are
+// read with a stride; HWIO: neighbouring threads take neighbouring filters.
+template <bool HWIO>
+__device__ __forceinline__ void pack(const WArgs &g) {
+    const int taps = g.kh * g.kw, span = g.nibbles ? 8 : 32;
+    const long total = (long)taps * g.rows * g.words;
+    const long i = (long)(blockIdx.x - g.alpha_blocks) * kThreads + threadIdx.x;
+    if (i >= total) return;
+    int f, tap, word;
+    if (HWIO) {
+        f = (int)(i % g.rows);
+        word = (int)(i / g.rows % g.words);
+        tap = (int)(i / ((long)g.rows * g.words));
+    } else {
+        word = (int)(i % g.words);
+        tap = (int)(i / g.words % taps);
+        f = (int)(i / ((long)g.words * taps));
+    }
+    uint32_t v = 0;
+    if (f < g.oc) {
+        const int c0 = word * span, n = min(span, g.ic - c0);
+        if (g.nibbles) {
+#pragma unroll
+            for (int b = 0; b < 8; b++)
+                if (b < n)
+                    v |= (sign_clear(__ldg(g.w + w_index<HWIO>(g, f, c0 + b, tap))) ? 0x2u : 0xAu)
+                         << (4 * b);
+        } else {
+            for (int b = 0; b < n; b++)
+                v |= sign_clear(__ldg(g.w + w_index<HWIO>(g, f, c0 + b, tap))) << (31 - b);
         }
     }
-    op_c[o] = taps * ic;
+    g.out[g.nibbles ? ((long)tap * g.rows + f) * g.words + word
+                    : ((long)tap * g.words + word) * g.rows + f] = v;
+}
+
+__device__ __forceinline__ void count_operands(const WArgs &g) {
+    const int o = (int)(blockIdx.x - g.alpha_blocks - g.pack_blocks) * kThreads + threadIdx.x;
+    if (o >= g.oh * g.ow) return;
+    const int y = o / g.ow, x = o - y * g.ow;
+    int rows = 0, cols = 0;
+    for (int i = 0; i < g.kh; i++) {
+        const int h = y * g.sh - g.ph + i;
+        rows += h >= 0 && h < g.ih;
+    }
+    for (int j = 0; j < g.kw; j++) {
+        const int w = x * g.sw - g.pw + j;
+        cols += w >= 0 && w < g.iw;
+    }
+    g.op_c[o] = rows * cols * g.ic;
+}
+
+template <bool HWIO>
+__global__ void __launch_bounds__(kThreads) weights_kernel(const WArgs g) {
+    __shared__ __align__(16) float stage[HWIO ? 2 * kSlab * 32 : kWarps * kStretch];
+    if ((int)blockIdx.x < g.alpha_blocks) {
+        if (HWIO) alpha_hwio(g, reinterpret_cast<float (*)[kSlab][32]>(stage));
+        else alpha_oihw(g, reinterpret_cast<float (*)[kStretch]>(stage));
+    } else if ((int)blockIdx.x < g.alpha_blocks + g.pack_blocks) {
+        pack<HWIO>(g);
+    } else {
+        count_operands(g);
+    }
 }
 
 }  // namespace
@@ -119,26 +191,22 @@ __global__ void op_count_kernel(int32_t *op_c, int ic, int ih, int iw, int oh, i
 cudaError_t launch_binarize_weights(const Plan &p, const float *w, void *bin_w, float *alpha,
                                     int32_t *op_c, cudaStream_t s) {
     WArgs g;
-    g.w = w; g.oc = p.oc; g.ic = p.ic; g.kh = p.kh; g.kw = p.kw; g.hwio = p.w_hwio;
-    const int threads = 128;
-    if (p.family == kTcgen05) {
-        const long total = (long)p.kh * p.kw * p.ocp16 * (p.icp / 4);
-        pack_weight_bytes_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, s>>>(
-            g, (uint32_t *)bin_w, p.icp, p.ocp16);
-    } else {
-        const long total = (long)p.kh * p.kw * p.icw * p.ocp;
-        pack_weight_bits_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, s>>>(
-            g, (uint32_t *)bin_w, p.icw, p.ocp);
-    }
-    note_launch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    alpha_kernel<<<(p.oc + 31) / 32, 256, 0, s>>>(g, alpha, p.inv_chw);
-    note_launch();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    op_count_kernel<<<(p.oh * p.ow + threads - 1) / threads, threads, 0, s>>>(
-        op_c, p.ic, p.ih, p.iw, p.oh, p.ow, p.kh, p.kw, p.sh, p.sw, p.ph, p.pw);
+    g.w = w; g.oc = p.oc; g.ic = p.ic; g.kh = p.kh; g.kw = p.kw;
+    g.alpha = alpha; g.inv_chw = p.inv_chw;
+    g.out = (uint32_t *)bin_w;
+    g.nibbles = p.family == kTcgen05;
+    g.rows = g.nibbles ? p.ocp16 : p.ocp;
+    g.words = g.nibbles ? p.icp / 4 : p.icw;
+    g.op_c = op_c;
+    g.ih = p.ih; g.iw = p.iw; g.oh = p.oh; g.ow = p.ow;
+    g.sh = p.sh; g.sw = p.sw; g.ph = p.ph; g.pw = p.pw;
+    const int per_block = p.w_hwio ? 32 : kWarps;  // filters an alpha block sums
+    g.alpha_blocks = (p.oc + per_block - 1) / per_block;
+    g.pack_blocks = (int)(((long)p.kh * p.kw * g.rows * g.words + kThreads - 1) / kThreads);
+    const int count_blocks = (p.oh * p.ow + kThreads - 1) / kThreads;
+    const unsigned grid = (unsigned)(g.alpha_blocks + g.pack_blocks + count_blocks);
+    if (p.w_hwio) weights_kernel<true><<<grid, kThreads, 0, s>>>(g);
+    else weights_kernel<false><<<grid, kThreads, 0, s>>>(g);
     note_launch();
     return cudaGetLastError();
 }
