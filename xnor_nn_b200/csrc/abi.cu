@@ -312,7 +312,7 @@ xnor_nn_status_t run_conv(const Plan &p, ResCtx *x, xnor_nn_resources_t res, flo
                                            x->error_word, x->stream));
                 return xnor_nn_success;
             }
-            CU(launch_conv_tcgen05(p, res[xnor_nn_resource_bin_src],
+            CU(launch_conv_tcgen05(conv_view(p), res[xnor_nn_resource_bin_src],
                                    res[xnor_nn_resource_bin_weights],
                                    (const float *)res[xnor_nn_resource_alpha],
                                    fuse_k ? nullptr : (const float *)res[xnor_nn_resource_k],
@@ -571,7 +571,7 @@ Slice slice_of(const Plan &p, int first, int count) {
     s.p = p;
     s.p.mb = count;
     s.p.q_total = (long)count * p.hp * p.wp;
-    s.p.rows = p.lead + s.p.q_total + 256 + (long)p.kh * p.wp + p.kw;
+    s.p.rows = p.lead + s.p.q_total + frame_slack(p);
     if (count != p.mb) plan_image_rows(&s.p);  // the tiling depends on the image count
     s.src = (size_t)first * p.ic * p.ih * p.iw * sizeof(float);
     s.a = (size_t)first * p.ih * p.iw * sizeof(float);
@@ -593,7 +593,7 @@ xnor_nn_status_t enqueue_forward(const Slice &sl, ResCtx *x, xnor_nn_resources_t
     sub[xnor_nn_resource_k] = (char *)res[xnor_nn_resource_k] + sl.k;
     CU(launch_binarize_data(sl.p, src, sub[xnor_nn_resource_bin_src],
                             (float *)sub[xnor_nn_resource_a], x->stream));
-    const bool fuse_k = sl.p.family == kTcgen05;
+    const bool fuse_k = sl.p.family == kTcgen05 && !sl.p.fold;
     if (!fuse_k)
         CU(launch_box_filter(sl.p, (const float *)sub[xnor_nn_resource_a],
                              (float *)sub[xnor_nn_resource_k], x->stream));
@@ -758,7 +758,7 @@ xnor_nn_status_t xnor_nn_b200_forward_chain(int layers, const xnor_nn_convolutio
         const Plan &a = *plan[i], &b = *plan[i + 1];
         if (a.mb != b.mb || a.oc != b.ic || a.oh != b.ih || a.ow != b.iw)
             return xnor_nn_error_invalid_input;
-        if (a.family != kTcgen05 || b.family != kTcgen05) {
+        if (a.family != kTcgen05 || b.family != kTcgen05 || a.fold || b.fold) {
             snprintf(t_last_error, sizeof t_last_error,
                      "layers %d and %d cannot be chained: both must run on the %s kernels", i,
                      i + 1, family_name(kTcgen05));
@@ -959,7 +959,7 @@ xnor_nn_status_t xnor_nn_b200_forward_sharded(const xnor_nn_convolution_t *c,
             xnor_nn_status_t st = init_common(
                 &sh.c, c->algorithm, c->src_format, c->weights_format, c->dst_format, sh.count,
                 c->oc, c->ic, c->ih, c->iw, c->kh, c->kw, c->sh, c->sw, c->ph, c->pw,
-                p->family == kTcgen05 && p->img ? kTcgen05Rows : p->family);
+                p->fold ? kAuto : p->family == kTcgen05 && p->img ? kTcgen05Rows : p->family);
             if (st == xnor_nn_success) st = xnor_nn_allocate_resources(&sh.c, sh.res);
             if (st == xnor_nn_success) {
                 sh.res[xnor_nn_resource_user_weights] = res[xnor_nn_resource_user_weights];
@@ -1023,7 +1023,7 @@ xnor_nn_status_t xnor_nn_b200_selftest_lost_commit(const xnor_nn_convolution_t *
                                    (const float *)res[xnor_nn_resource_k], nullptr, nullptr, dst,
                                    nullptr, x->error_word, x->stream, &t));
     else
-        CU(launch_conv_tcgen05(*p, res[xnor_nn_resource_bin_src],
+        CU(launch_conv_tcgen05(conv_view(*p), res[xnor_nn_resource_bin_src],
                                res[xnor_nn_resource_bin_weights],
                                (const float *)res[xnor_nn_resource_alpha],
                                (const float *)res[xnor_nn_resource_k], nullptr, nullptr, dst,

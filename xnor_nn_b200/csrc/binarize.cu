@@ -316,30 +316,83 @@ __global__ void __launch_bounds__(TWARPS * 32) binarize_nibbles_kernel(const Bin
     if (WITH_A && warp == 0 && live) g.a[px] = acc;
 }
 
+// ---- K: box filter of A ------------------------------------------------------------------------
+// A block takes a few output rows of one image: what they read of A goes to shared memory, already
+// multiplied by 1/(KH*KW) (each term of upstream's sum is that product) and with zeros where the
+// window leaves the image (adding +0 to a sum of non-negative terms changes nothing), and a thread
+// adds up an output's terms in upstream's order. A staged row has its columns sorted by their
+// remainder modulo the stride, so that neighbouring outputs read neighbouring words, and tap j is a
+// fixed distance from the output's first word: three instructions per term for the filter widths
+// that are compiled in (KW). AlexNet conv1 on 64 images, 121 taps: 18.8 us with the terms read from
+// global memory one after the other.
 struct BoxArgs {
     const float *a;
     float *k;
-    long n_out;
     int ih, iw, oh, ow, kh, kw, sh, sw, ph, pw;
     float inv_khw;
+    int rows, row_blocks;  // output rows per block, blocks per image
+    int span, phase;       // columns of A an output row reads; words per remainder
+    int lines;             // rows of A staged
+    FastDiv by_span, by_sw, by_ow;
+    int tap[11];           // word of tap j, from the output's first
 };
 
-__global__ void __launch_bounds__(256) box_filter_kernel(const BoxArgs g) {
-    const long o = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= g.n_out) return;
-    const int ohw = g.oh * g.ow;
-    const int n = (int)(o / ohw);
-    const int r = (int)(o - (long)n * ohw);
-    const int oh = r / g.ow, ow = r - oh * g.ow;
+constexpr int kBoxThreads = 256;
+constexpr int kBoxSmem = 40 * 1024;
+
+template <int KW>
+__global__ void __launch_bounds__(kBoxThreads) box_filter_kernel(const BoxArgs g) {
+    extern __shared__ __align__(16) float tile[];
+    const int n = blockIdx.x / g.row_blocks;
+    const int oy0 = (blockIdx.x - n * g.row_blocks) * g.rows;
+    const int n_out = min(g.rows, g.oh - oy0) * g.ow;
+    const int y0 = oy0 * g.sh - g.ph, pitch = g.phase * g.sw;
     const float *img = g.a + (long)n * g.ih * g.iw;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < g.lines * g.span; i += kBoxThreads) {
+        const int line = (int)g.by_span((uint32_t)i), xx = i - line * g.span;
+        const int y = y0 + line, x = xx - g.pw, xs = (int)g.by_sw((uint32_t)xx);
+        float v = 0.f;
+        if (y >= 0 && y < g.ih && x >= 0 && x < g.iw)
+            v = __fmul_rn(__ldg(img + y * g.iw + x), g.inv_khw);
+        tile[line * pitch + (xx - xs * g.sw) * g.phase + xs] = v;
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < n_out; o += kBoxThreads) {
+        const int r = (int)g.by_ow((uint32_t)o), x = o - r * g.ow;
+        const float *row = tile + r * g.sh * pitch + x;
+        float acc = 0.f;
+        for (int i = 0; i < g.kh; i++, row += pitch) {
+            if (KW > 0) {
+#pragma unroll
+                for (int j = 0; j < KW; j++) acc = __fadd_rn(acc, row[g.tap[j]]);
+            } else {
+                for (int j = 0, at = 0, rem = 0; j < g.kw; j++) {
+                    acc = __fadd_rn(acc, row[rem * g.phase + at]);
+                    if (++rem == g.sw) { rem = 0; at++; }
+                }
+            }
+        }
+        g.k[((long)n * g.oh + oy0 + r) * g.ow + x] = acc;
+    }
+}
+
+// Windows that do not fit shared memory: one thread per output, straight from A.
+__global__ void __launch_bounds__(kBoxThreads) box_filter_wide_kernel(const BoxArgs g) {
+    const long o = (long)blockIdx.x * kBoxThreads + threadIdx.x;
+    const long plane = (long)g.oh * g.ow;
+    const long n = o / plane;
+    const int r = (int)(o - n * plane), y = r / g.ow, x = r - y * g.ow;
+    if (y >= g.oh || n >= g.row_blocks) return;  // row_blocks: images here
+    const float *img = g.a + n * g.ih * g.iw;
     float acc = 0.f;
-    for (int kh = 0; kh < g.kh; kh++) {
-        const int ih = oh * g.sh - g.ph + kh;
-        if (ih < 0 || ih >= g.ih) continue;
-        for (int kw = 0; kw < g.kw; kw++) {
-            const int iw = ow * g.sw - g.pw + kw;
-            if (iw < 0 || iw >= g.iw) continue;
-            acc = __fadd_rn(acc, __fmul_rn(__ldg(img + ih * g.iw + iw), g.inv_khw));
+    for (int i = 0; i < g.kh; i++) {
+        const int h = y * g.sh - g.ph + i;
+        if (h < 0 || h >= g.ih) continue;
+        for (int j = 0; j < g.kw; j++) {
+            const int w = x * g.sw - g.pw + j;
+            if (w < 0 || w >= g.iw) continue;
+            acc = __fadd_rn(acc, __fmul_rn(__ldg(img + h * g.iw + w), g.inv_khw));
         }
     }
     g.k[o] = acc;
@@ -427,6 +480,7 @@ cudaError_t launch_bin(const Plan &p, const BinArgs &g, cudaStream_t s) {
 
 cudaError_t launch_binarize_data(const Plan &p, const float *src, void *bin_src, float *a,
                                  cudaStream_t s) {
+    if (p.fold) return launch_fold(p, src, bin_src, a, s);
     const BinArgs g = bin_args(p, src, bin_src, a);
     return a ? launch_bin<true, true>(p, g, s) : launch_bin<false, true>(p, g, s);
 }
@@ -439,15 +493,40 @@ cudaError_t launch_mean_abs(const Plan &p, const float *src, float *a, cudaStrea
 cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStream_t s) {
     BoxArgs g;
     g.a = a; g.k = k;
-    g.n_out = (long)p.mb * p.oh * p.ow;
     g.ih = p.ih; g.iw = p.iw; g.oh = p.oh; g.ow = p.ow; g.kh = p.kh; g.kw = p.kw;
     g.sh = p.sh; g.sw = p.sw; g.ph = p.ph; g.pw = p.pw;
     g.inv_khw = p.inv_khw;
-    const int threads = 256;
-    const unsigned blocks = (unsigned)((g.n_out + threads - 1) / threads);
-    if (blocks == 0) return cudaSuccess;
-    box_filter_kernel<<<blocks, threads, 0, s>>>(g);
+    if (p.mb < 1 || p.oh < 1 || p.ow < 1) return cudaSuccess;
+    g.span = (p.ow - 1) * p.sw + p.kw;
+    g.phase = div_up_i(g.span, p.sw);
+    g.by_span = FastDiv((uint32_t)g.span); g.by_sw = FastDiv((uint32_t)p.sw);
+    g.by_ow = FastDiv((uint32_t)p.ow);
+    for (int j = 0; j < 11; j++) g.tap[j] = j % p.sw * g.phase + j / p.sw;
+    // about one output per thread, if the rows that takes fit shared memory
+    g.rows = kBoxThreads / p.ow;
+    if (g.rows < 1) g.rows = 1;
+    if (g.rows > p.oh) g.rows = p.oh;
+    auto lines = [&](int rows) { return (long)(rows - 1) * p.sh + p.kh; };
+    auto bytes = [&](int rows) { return 4L * lines(rows) * g.phase * p.sw; };
+    while (g.rows > 1 && bytes(g.rows) > kBoxSmem) g.rows--;
     note_launch();
+    if (bytes(g.rows) > kBoxSmem) {
+        g.row_blocks = p.mb;
+        const long n_out = (long)p.mb * p.oh * p.ow;
+        box_filter_wide_kernel<<<(unsigned)((n_out + kBoxThreads - 1) / kBoxThreads), kBoxThreads,
+                                 0, s>>>(g);
+        return cudaGetLastError();
+    }
+    g.row_blocks = div_up_i(p.oh, g.rows);
+    g.lines = (int)lines(g.rows);
+    const unsigned blocks = (unsigned)(p.mb * g.row_blocks);
+    auto kernel = p.kw == 1    ? box_filter_kernel<1>
+                  : p.kw == 3  ? box_filter_kernel<3>
+                  : p.kw == 5  ? box_filter_kernel<5>
+                  : p.kw == 7  ? box_filter_kernel<7>
+                  : p.kw == 11 ? box_filter_kernel<11>
+                               : box_filter_kernel<0>;
+    kernel<<<blocks, kBoxThreads, (size_t)bytes(g.rows), s>>>(g);
     return cudaGetLastError();
 }
 

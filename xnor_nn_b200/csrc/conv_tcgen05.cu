@@ -63,13 +63,14 @@ constexpr int kMaxStages = 8;       // ring buffers: as many as fit, at most thi
 constexpr int kEpiWarps = 16;       // epilogue warps: 4 TMEM lane quadrants x column groups
 constexpr int kIssuer2Warp = 2 + kEpiWarps;  // the second MMA-issuing thread lives in a warp of its own
 constexpr int kThreads = 64 + 32 * kEpiWarps + 32;
-// Tensor memory: two accumulators of n_tile columns and, in the last 16 columns, the block scales.
-// 2 x 256 + 16 is more than the 512 there are, so accumulators of 256 columns share 16 of them
+// Tensor memory: two to four accumulators of n_tile columns and, in the last 16 columns, the block
+// scales. 2 x 256 + 16 is more than the 512 there are, so accumulators of 256 columns share 16 of them
 // (the last of the first = the first of the second): the epilogue empties those before anything
 // else and says so (Control::shared_free), and the next tile's first MMA waits for it.
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kScaleCol = 496;
 constexpr int kAccStep = 240;        // columns between the accumulators' starts, at most
+constexpr int kMaxAcc = 4;
 struct TcArgs {
     const float *alpha;
     const float *kmap;   // K per output pixel, or null: box-filter it from amap in the epilogue
@@ -82,7 +83,9 @@ struct TcArgs {
     int *error;
     long q_total;
     int m_tiles, n_tiles, n_tile;
-    int kchunk, chunks_per_tap, taps, kw, ph, pw;
+    FastDiv by_frame, by_wp;  // position -> image, row (q_total < 2^30)
+    int kchunk, chunks_per_tap, kw, ph, pw;
+    int taps, tap_kw;  // filter taps as the operands see them, columns among them (see Plan::cat)
     int wp, hp, lead, oh, ow, oc, ocp16;
     uint32_t idesc;
     uint32_t desc_hi;  // upper 32 bits of the shared-memory matrix descriptors
@@ -107,7 +110,9 @@ struct TcArgs {
     int kk_last;          // MMAs of a tap's last channel chunk: its 64-channel slices that hold
                           // channels at all (the chunk is padded with zeros to kchunk bytes)
     uint32_t acc_step;    // columns from the first accumulator to the second
-    int paced;            // NCHW floats: the column groups of a tile store one after the other
+    int n_acc;            // accumulators in tensor memory
+    int teams;            // epilogue teams that take the tiles in turn: 1, 2 or 4
+    FastDiv by_acc;       // tile -> round of the accumulators
     int shared_cols;      // the accumulators overlap (n_tile > kAccStep)
 };
 
@@ -119,11 +124,11 @@ constexpr int kAlphaSmem = 2048;  // filters whose alpha is staged in shared mem
 struct __align__(16) Control {
     unsigned long long full[kMaxStages];
     unsigned long long empty[kMaxStages];
-    unsigned long long acc_full[2];
-    unsigned long long acc_empty[2];
+    unsigned long long acc_full[kMaxAcc];
+    unsigned long long acc_empty[kMaxAcc];
     unsigned long long a_full[4];   // halo mode: a halo tile has landed / has been used up
     unsigned long long a_empty[4];
-    unsigned long long started[2];  // two issuers: the tile's first MMA (which overwrites) is out
+    unsigned long long started[kMaxAcc];  // two issuers: the tile's first MMA (which overwrites) is out
     unsigned long long drain[2];
     unsigned long long shared_free;  // the columns both accumulators use have been read
     uint32_t tmem_base;
@@ -187,23 +192,27 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
         PAIR ? mapa(smem_u32(&ctl->acc_empty[0]), 0) : smem_u32(&ctl->acc_empty[0]);
     const uint32_t shared_free0 =
         PAIR ? mapa(smem_u32(&ctl->shared_free), 0) : smem_u32(&ctl->shared_free);
-    // Several warps share a quadrant and split its columns between them.
+    // Several warps share a quadrant and split its columns between them. The warps form
+    // one, two or four teams that take the tiles in turn: what a tile costs an epilogue warp is
+    // mostly latency (its pixel's K, the accumulator's barrier, the loads from tensor memory, the
+    // stores going out), and tiles of different teams overlap it.
     const int quad = warp & 3;
-    const int cgroup = (warp - 2) >> 2, cgroups = kEpiWarps / 4;
+    const int cgroups = kEpiWarps / 4 / g.teams, team = (warp - 2) / (4 * cgroups);
+    const int cgroup = ((warp - 2) >> 2) - team * cgroups;
     const int frame = g.hp * g.wp;
     const long ohw = (long)g.oh * g.ow;
     bool ok = true;   // false once a wait ran out somewhere in the CTA
     float run = 0.f;  // chained layers: running sum of |y| over the filter tiles of a pixel
-    for (int it = 0; it < rounds; it++) {
+    for (int it = team; it < rounds; it += g.teams) {
         int mt, nt;
         deal.at(g, it, mt, nt);
-        const int b = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        const long q = (long)mt * BM + quad * 32 + lane;
-        const int n = (int)(q / frame);
-        const int rem = (int)(q - (long)n * frame);
-        const int oh = rem / g.wp, ow = rem - oh * g.wp;
-        const bool valid = q < g.q_total && oh < g.oh && ow < g.ow;
+        const int use = (int)g.by_acc((uint32_t)it), b = it - use * g.n_acc;
+        const uint32_t acc_phase = use & 1;
+        const uint32_t q = (uint32_t)mt * BM + quad * 32 + lane;
+        const int n = (int)g.by_frame(q);
+        const uint32_t rem = q - (uint32_t)n * (uint32_t)frame;
+        const int oh = (int)g.by_wp(rem), ow = (int)rem - oh * g.wp;
+        const bool valid = q < (uint32_t)g.q_total && oh < g.oh && ow < g.ow;
         const int r = oh * g.ow + ow;
         const long pix = (long)n * ohw + r;
         float kk = 0.f;
@@ -240,18 +249,12 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                 bar_sync(1 + quad, 32 * (kEpiWarps / 4));
                 continue;
             }
-            // The NCHW float epilogue's column groups meet three times per tile (all tiles of a
-            // CTA but its last): the same appointments are kept here.
-            if (!g.sums && !g.dst_nhwc && g.paced && it + 1 < rounds) {
-                for (int w = 0; w < kEpiWarps / 4 - 1; w++) bar_sync(10, 32 * kEpiWarps);
-                continue;
-            }
             break;
         }
         fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)b * g.acc_step;
         // the warp that owns the columns shared with the other accumulator reads them first
-        const bool shared = g.shared_cols && cgroup == (b ? 0 : kEpiWarps / 4 - 1);
+        const bool shared = g.shared_cols && cgroup == (b ? 0 : cgroups - 1);
         const bool reverse = shared && b == 0;
         auto columns_read = [&](int step) {
             if (!shared || step != 0) return;
@@ -343,16 +346,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
             // store instruction writes one contiguous run.
             float *out = g.dst + ((long)n * g.oc + oc0) * ohw + r;
             const float *al = alpha_in_smem ? ctl->alpha + oc0 : g.alpha + oc0;
-            // Except for a CTA's last tile the four column groups store one after the other
-            // (three meetings of all epilogue warps per tile, column group c stores between the
-            // c-th and the next): the stores of a tile then leave the SM over about twice the
-            // time, which leaves the SM's request port more room for the next tile's operand
-            // loads (conv4 32.7 -> 31.6 us, VGG 78.6 -> 76.9). Only for tiles of 256 filters: with
-            // narrower ones (conv3, N = 192) a tile's MMAs are over sooner than its epilogue
-            // spread out like this, and the whole step got slower (55.1 -> 57.7 us).
-            const bool paced = g.paced && it + 1 < rounds;
             const int steps = (g.n_tile - 32 * cgroup + 32 * cgroups - 1) / (32 * cgroups);
-            bool waited = !paced;
             for (int i = 0; i < steps; i++) {
                 const int c0 = 32 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
                 uint32_t v[32];
@@ -363,10 +357,6 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                 }
                 wait_ld();
                 columns_read(i);
-                if (!waited) {
-                    waited = true;
-                    for (int w = 0; w < cgroup; w++) bar_sync(10, 32 * kEpiWarps);
-                }
                 if (valid) {
                     const int lim = n_valid - c0;
                     float *o = out + (long)c0 * ohw;
@@ -392,8 +382,6 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                     }
                 }
             }
-            if (!waited) for (int w = 0; w < cgroup; w++) bar_sync(10, 32 * kEpiWarps);
-            if (paced) for (int w = cgroup; w < kEpiWarps / 4 - 1; w++) bar_sync(10, 32 * kEpiWarps);
         } else if (!g.sums && g.dst_nhwc && (g.oc & 3) == 0) {
             // NHWC floats: a thread owns one pixel and 16 neighbouring filters at a time, which
             // are contiguous in the result: four 16-byte stores.
@@ -500,9 +488,9 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
     const int chunk_step = n_iss % g.chunks_per_tap;
     uint32_t phase = 0;
     bool ok = true, entered = false;
+    int b = 0;  // the tile's accumulator and how often it has come round
+    uint32_t acc_phase = 0;
     for (;;) {
-        const int b = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
         if (!entered) {
             if (ks == 0)
                 ok = mbar_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
@@ -554,6 +542,7 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
             }
             entered = false;
             if (++it >= rounds) break;
+            if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
         }
     }
     if (!ok) {
@@ -610,8 +599,8 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                 armed_a |= 1u << sa;
                 parity_a = (parity_a & ~(1u << sa)) | (pa << sa);
                 if (++sa == g.n_a_slots) { sa = 0; pa ^= 1; }
-                int brow = brow0 + kh * g.kw * g.ocp16;
-                for (int kw = 0; kw < g.kw; kw++, brow += g.ocp16) {
+                int brow = brow0 + kh * g.tap_kw * g.ocp16;
+                for (int kw = 0; kw < g.tap_kw; kw++, brow += g.ocp16) {
                     const uint32_t ebar = empty0 + 8u * (uint32_t)sb;
                     if (!mbar_try_wait(ebar, pb ^ 1)) {
                         ok = mbar_wait(ebar, pb ^ 1, abort_flag, g.error, 1, g.wait_ns);
@@ -647,8 +636,8 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     volatile int *abort_flag = &ctl->abort_flag;
     const int rounds = Deal<PAIR>(g).rounds(g);
     if (rounds == 0) return;
-    const int ksteps = g.taps * g.chunks_per_tap;  // >= g.issuers; a multiple of g.kw
-    const int n_iss = g.issuers, kwn = g.kw;
+    const int ksteps = g.taps * g.chunks_per_tap;  // >= g.issuers; a multiple of g.tap_kw
+    const int n_iss = g.issuers, kwn = g.tap_kw;
     const uint64_t hi = (uint64_t)g.desc_hi << 32;
     const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (1u << 16);
     const uint32_t b_lo0 = (((stage0 + g.b_ring_off) >> 4) & 0x3FFF) | (1u << 16);
@@ -664,9 +653,9 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     uint32_t pa = ((who / kwn) / g.n_a_slots) & 1u;
     int chunk = (who / kwn) % g.chunks_per_tap;  // groups walk the chunks, then the filter rows
     bool ok = true, entered = false, a_seen = false;
+    int b = 0;  // the tile's accumulator and how often it has come round
+    uint32_t acc_phase = 0;
     for (;;) {
-        const int b = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
         if (!entered) {
             if (ks == 0)
                 ok = mbar_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
@@ -737,6 +726,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
             }
             entered = false;
             if (++it >= rounds) break;
+            if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
         }
     }
     if (!ok) {
@@ -776,13 +766,13 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             mbar_init(smem_u32(&ctl->a_full[a]), 1);
             mbar_init(smem_u32(&ctl->a_empty[a]), (uint32_t)g.issuers);
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < g.n_acc; b++) {
             mbar_init(smem_u32(&ctl->acc_full[b]), (uint32_t)g.issuers);
             // single CTA: one arrival per epilogue thread; pair: one per epilogue warp of both
-            mbar_init(smem_u32(&ctl->acc_empty[b]), PAIR ? 2 * kEpiWarps : 32 * kEpiWarps);
+            mbar_init(smem_u32(&ctl->acc_empty[b]), (uint32_t)((PAIR ? 2 : 32) * kEpiWarps / g.teams));
             mbar_init(smem_u32(&ctl->started[b]), 1);
-            mbar_init(smem_u32(&ctl->drain[b]), 1);
         }
+        for (int i = 0; i < 2; i++) mbar_init(smem_u32(&ctl->drain[i]), 1);
         mbar_init(smem_u32(&ctl->shared_free), PAIR ? 8 : 4);  // one arrival per lane quadrant
         ctl->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -869,7 +859,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     if (++chunk == g.chunks_per_tap) {  // next filter tap
                         chunk = 0;
                         brow += g.ocp16;
-                        if (++kw == g.kw) { kw = 0; row += g.wp - (g.kw - 1); }
+                        if (++kw == g.tap_kw) { kw = 0; row += g.wp - (g.tap_kw - 1); }
                         else row += 1;
                     }
                 }
@@ -954,9 +944,15 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.m_tiles = m_tiles;
     g.n_tiles = p.ocp16 / p.n_tile;
     g.n_tile = p.n_tile;
-    g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(p.icp, p.kchunk); g.taps = p.kh * p.kw;
+    // channels-wise: a tap, or the kw taps of a filter row one after the other
+    const int tap_bytes = p.cat ? p.kw * p.icp : p.icp;
+    const int tap_values = p.cat ? 2 * (p.kw - 1) * p.icp + p.ic : p.ic;
+    g.tap_kw = p.cat ? 1 : p.kw;
+    g.taps = p.kh * g.tap_kw;
+    g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(tap_bytes, p.kchunk);
     g.kw = p.kw; g.ph = p.ph; g.pw = p.pw; g.wp = p.wp; g.hp = p.hp; g.lead = p.lead;
     g.oh = p.oh; g.ow = p.ow; g.oc = p.oc; g.ocp16 = p.ocp16;
+    g.by_frame = FastDiv((uint32_t)(p.hp * p.wp)); g.by_wp = FastDiv((uint32_t)p.wp);
     g.dst_nhwc = p.dst_nhwc;
     g.emit_bin = nullptr; g.emit_a = nullptr; g.n_inner = 0;
     g.wait_ns = test && test->wait_ns ? test->wait_ns : 2000000000ull;
@@ -972,7 +968,6 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.idesc = mxf4_idesc(pair ? 2 * BM : BM, (uint32_t)p.n_tile);
     g.shared_cols = p.n_tile > kAccStep;
     g.acc_step = (uint32_t)(p.n_tile < kAccStep ? p.n_tile : kAccStep);
-    g.paced = p.n_tile == 256;
     // matrix descriptor, upper half: stride between 8-row groups (8 * kchunk bytes, in 16-byte
     // units), descriptor version 1, swizzle mode
     const uint32_t sbo = (uint32_t)(8 * p.kchunk) >> 4;
@@ -982,12 +977,12 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.tx_bytes = g.a_bytes + (uint32_t)(b_rows * p.kchunk);  // per CTA
     g.stage_bytes = (g.tx_bytes + 1023u) & ~1023u;
     g.issuers = g.taps * g.chunks_per_tap < 2 ? 1 : 2;
-    g.kk_last = (p.ic - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
+    g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
     g.halo = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
-    bool halo = pair && p.kw >= 2 && p.kw <= 9 && g.issuers <= p.kw;
+    bool halo = pair && g.tap_kw >= 2 && g.tap_kw <= 9 && g.issuers <= g.tap_kw;
     if (halo) {
         // three halo tiles of 136 positions, the rest of the room for filter tiles
         g.halo = BM + 8;
@@ -1005,10 +1000,12 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     }
     if (g.n_stages < 2) return cudaErrorNotSupported;
     CUtensorMap map_a, map_b;
-    if (!encode_bytes_2d(&map_a, bin_src, (uint64_t)p.rows, (uint64_t)p.icp, (uint32_t)p.kchunk,
+    // a position's row is tap_bytes long but only icp further than the one before it
+    if (!encode_bytes_2d(&map_a, bin_src, (uint64_t)(p.rows - (p.cat ? p.kw - 1 : 0)),
+                         (uint64_t)tap_bytes, (uint64_t)p.icp, (uint32_t)p.kchunk,
                          (uint32_t)(halo ? g.halo : BM)) ||
-        !encode_bytes_2d(&map_b, bin_w, (uint64_t)p.kh * p.kw * p.ocp16, (uint64_t)p.icp,
-                         (uint32_t)p.kchunk, (uint32_t)b_rows))
+        !encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
+                         (uint64_t)tap_bytes, (uint32_t)p.kchunk, (uint32_t)b_rows))
         return cudaErrorNotSupported;
 
     const int kk = p.kchunk / 32;
@@ -1034,10 +1031,11 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         if (e != cudaSuccess) return e;
         done.store(true, std::memory_order_release);
     }
-    note_launch();
+    int units = g.n_inner ? m_tiles : m_tiles * g.n_tiles, slots = sms;
     if (pair) {
-        int pairs = pair_count[d].load(std::memory_order_relaxed);
-        if (!pairs) {
+        units = ((m_tiles + 1) / 2) * g.n_tiles;
+        slots = pair_count[d].load(std::memory_order_relaxed);
+        if (!slots) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(2 * (sms / 2));
             cfg.blockDim = dim3(kThreads);
@@ -1047,19 +1045,26 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
             attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&pairs, kernel, &cfg) != cudaSuccess || pairs <= 0) {
+            if (cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg) != cudaSuccess || slots <= 0) {
                 (void)cudaGetLastError();
-                pairs = sms / 2;
+                slots = sms / 2;
             }
-            pair_count[d].store(pairs, std::memory_order_relaxed);
+            pair_count[d].store(slots, std::memory_order_relaxed);
         }
-        const int tiles = ((m_tiles + 1) / 2) * g.n_tiles;
-        const int clusters = tiles < pairs ? tiles : pairs;
-        return launch_overlapped(kernel, dim3(2 * clusters), dim3(kThreads), smem, s, 2, map_a, map_b, g);
     }
-    const int tiles = g.n_inner ? g.m_tiles : g.m_tiles * g.n_tiles;
-    const int grid = tiles < sms ? tiles : sms;
-    return launch_overlapped(kernel, dim3(grid), dim3(kThreads), smem, s, 1, map_a, map_b, g);
+    const int grid = units < slots ? units : slots;
+    // As many accumulators as fit (at most four), and one epilogue team for each of two or four of
+    // them if a CTA has that many tiles. With all 16 warps on every tile AlexNet conv3 (256
+    // images) took 41.3 us per pass, conv1 (64 images) 86, with two teams 37.7 and 79. The chained
+    // epilogue carries per-pixel state from one filter tile to the next: one team.
+    const int rounds = g.n_inner ? 1 : div_up_i(units, grid);
+    g.n_acc = g.shared_cols || g.n_inner ? 2 : (int)kScaleCol / p.n_tile;
+    if (g.n_acc > kMaxAcc) g.n_acc = kMaxAcc;
+    g.teams = g.n_acc == 4 && rounds >= 4 ? 4 : rounds >= 2 ? 2 : 1;
+    g.by_acc = FastDiv((uint32_t)g.n_acc);
+    note_launch();
+    return launch_overlapped(kernel, dim3((pair ? 2 : 1) * grid), dim3(kThreads), smem, s,
+                             pair ? 2 : 1, map_a, map_b, g);
 }
 
 }  // namespace xb200

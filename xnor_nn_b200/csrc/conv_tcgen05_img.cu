@@ -509,7 +509,7 @@ cudaError_t launch_conv_tcgen05_img(const Plan &p, const void *bin_src, const vo
     CUtensorMap map_w, map_x, map_xh;
     const uint64_t row = (uint64_t)p.icp;
     const uint32_t half_rows = p.img_half_rows ? (uint32_t)p.img_half_rows : (uint32_t)p.img_rows;
-    if (!encode_bytes_2d(&map_w, bin_w, (uint64_t)p.kh * p.kw * p.ocp16, row, (uint32_t)p.kchunk,
+    if (!encode_bytes_2d(&map_w, bin_w, (uint64_t)p.kh * p.kw * p.ocp16, row, row, (uint32_t)p.kchunk,
                          kFilters) ||
         !encode_bytes_4d(&map_x, x0, row, (uint64_t)p.wp, (uint64_t)p.hp, (uint64_t)p.mb, row,
                          row * p.wp, row * p.wp * p.hp, (uint32_t)p.kchunk, (uint32_t)p.ow,

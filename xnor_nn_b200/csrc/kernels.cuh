@@ -43,6 +43,23 @@ inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// n / d for n < 2^31 by a multiplication and a shift (the round-up method: Granlund and
+// Montgomery, "Division by invariant integers using multiplication", 1994).
+struct FastDiv {
+    uint32_t mul, shift;
+    FastDiv() = default;
+    explicit FastDiv(uint32_t d) {
+        shift = 0;
+        while ((1ull << shift) < d) shift++;
+        mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+        return (__umulhi(n, mul) + n) >> shift;
+    }
+#endif
+};
+
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t d;
@@ -80,6 +97,8 @@ __device__ __forceinline__ void dependency_wait() {
 // first loop of src/bcast_calculate_k.cpp:49-66.
 cudaError_t launch_binarize_data(const Plan &p, const float *src, void *bin_src, float *a,
                                  cudaStream_t s);
+// The same for a folded layer (Plan::fold); launch_binarize_data sends those here.
+cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a, cudaStream_t s);
 // The mean |x| map alone (calculate_k called on its own).
 cudaError_t launch_mean_abs(const Plan &p, const float *src, float *a, cudaStream_t s);
 // K = box filter of A over the filter window / (KH*KW), zero outside the image.

@@ -42,13 +42,32 @@ static Family family_from_env() {
     return kAuto;
 }
 
-// Both tensor-core kernels read the zero-framed activation nibbles, describe a unit-stride
-// convolution only, and accumulate in fp32: exact while no sum can leave the 24-bit range in
+// The tensor-core kernels accumulate in fp32: exact while no sum can leave the 24-bit range in
 // which every integer is a float.
+static bool sums_exact(const Plan &p) { return (long)p.ic * p.kh * p.kw <= (1L << 24); }
+
+// Both of them read the zero-framed activation nibbles and describe a unit-stride convolution.
 static bool unit_stride(const Plan &p) {
     return p.sh == 1 && p.sw == 1 && p.oh > 0 && p.ow > 0 &&
-           (long)p.mb * (p.ih + p.ph) * (p.iw + p.pw) < (1L << 30) &&
-           (long)p.ic * p.kh * p.kw <= (1L << 24);
+           (long)p.mb * (p.ih + p.ph) * (p.iw + p.pw) < (1L << 30) && sums_exact(p);
+}
+
+// A strided layer is folded when its packer's working set (a row block of some channels, a byte
+// per value, and the mean-|x| sums of the block's pixels) fits shared memory. The popcount kernel
+// it would otherwise run on needs 870 us for AlexNet conv1 on 64 images.
+constexpr long kFoldStage = 48 * 1024, kFoldSums = 48 * 1024, kFoldWords = 4096;
+static bool fold_ok(const Plan &p) {
+    if ((p.sh == 1 && p.sw == 1) || p.sh < 1 || p.sw < 1 || p.oh < 1 || p.ow < 1 || p.mb < 1)
+        return false;
+    const int rows = p.kh < p.sh ? p.kh : p.sh, taps = div_up_i(p.kh, p.sh);
+    const long span = (long)(p.ow - 1) * p.sw + p.kw;
+    // bytes staged at least, and words of a column they become: all of fewer than eight channels
+    // as bytes, or eight channels as nibbles
+    const long least = p.ic < 8 ? p.ic * rows * (span + 16) : 4 * rows * span;
+    const long words = p.ic < 8 ? (long)p.ic * rows * div_up_i(p.kw, 8) : (long)rows * p.kw;
+    return sums_exact(p) && least <= kFoldStage && 4L * p.sh * p.iw <= kFoldSums &&
+           words <= kFoldWords && (long)p.mb * (p.oh + taps - 1) * p.ow < (1L << 30) &&
+           (long)p.mb * (p.oh + taps + (p.ih + p.ph) / p.sh) < (1L << 30);
 }
 
 // The position-tile kernel walks the frame with one constant row shift per filter tap. That
@@ -140,6 +159,21 @@ void plan_image_rows(Plan *p) {
     p->img = true;
 }
 
+long frame_slack(const Plan &p) {
+    return 256 + (p.fold ? (long)p.fold_taps * p.wp : (long)p.kh * p.wp + p.kw);
+}
+
+Plan conv_view(const Plan &p) {
+    Plan v = p;
+    if (!p.fold) return v;
+    v.ic = p.fold_ic;
+    v.ih = p.hp; v.iw = p.wp;
+    v.kh = p.fold_taps; v.kw = 1;
+    v.sh = v.sw = 1;
+    v.ph = v.pw = 0;
+    return v;
+}
+
 void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
     memset(p, 0, sizeof(*p));
     p->mb = c->mb; p->ic = c->ic; p->ih = c->ih; p->iw = c->iw;
@@ -166,10 +200,11 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
     Family f = requested;
     if (f != kPopc && f != kTcgen05 && f != kTcgen05Rows) f = family_from_env();
     const bool frame = frame_walk_ok(*p), rows = image_rows_ok(*p);
-    if (f == kAuto) f = (frame || rows) ? kTcgen05 : kPopc;
+    const bool fold = f == kAuto && fold_ok(*p);
+    if (f == kAuto) f = (frame || rows || fold) ? kTcgen05 : kPopc;
     const bool force_rows = f == kTcgen05Rows;
     if (force_rows) f = rows ? kTcgen05 : kPopc;
-    if (f == kTcgen05 && !frame && !rows) f = kPopc;
+    if (f == kTcgen05 && !frame && !rows && !fold) f = kPopc;
     p->family = f;
 
     const size_t px_in = (size_t)p->mb * p->ih * p->iw;
@@ -201,7 +236,29 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
     // swizzle span: the widest one that a row fills by more than half. The copy engine fills what
     // lies past the row with zeros, and slices of 64 channels that hold no channel are not
     // multiplied, so the only cost of a chunk that is not full is shared memory.
-    p->icp = div_up_i(p->ic, 32) * 16;
+    int channels = p->ic, taps = p->kh * p->kw;
+    if (fold) {
+        p->fold = true;
+        p->fold_rows = p->kh < p->sh ? p->kh : p->sh;
+        p->fold_taps = taps = div_up_i(p->kh, p->sh);
+        p->fold_span = (p->ow - 1) * p->sw + p->kw;
+        if (p->ic < 8) {
+            p->fold_field = div_up_i(p->kw, 8) * 8;
+            p->fold_ic = p->ic * p->fold_rows * p->fold_field;
+            p->fold_channels = p->ic;
+        } else {
+            p->fold_field = 0;
+            p->fold_ic = div_up_i(p->ic, 8) * 8 * p->fold_rows * p->kw;
+            long fit = kFoldStage / (4L * p->fold_rows * p->fold_span);  // groups of eight
+            if (fit * p->fold_rows * p->kw > kFoldWords) fit = kFoldWords / (p->fold_rows * p->kw);
+            p->fold_channels = 8 * fit >= p->ic ? p->ic : 8 * (int)fit;
+        }
+        channels = p->fold_ic;
+        p->wp = p->ow;
+        p->hp = p->oh + taps - 1;
+        p->q_total = (long)p->mb * p->hp * p->wp;
+    }
+    p->icp = div_up_i(channels, 32) * 16;
     p->kchunk = p->icp > 64 ? 128 : p->icp > 32 ? 64 : 32;
     // Filter tile of the position-tile kernel = its UMMA N: a multiple of 16, at most 256. The
     // filters are split into the fewest equal tiles and padded (with zero filters) to fill them,
@@ -218,12 +275,19 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
         n_tiles *= 2;
     p->n_tile = div_up_i(div_up_i(p->oc, n_tiles), 16) * 16;
     p->ocp16 = p->n_tile * n_tiles;
-    p->lead = p->ph * p->wp + p->pw;
-    p->rows = p->lead + p->q_total + 256 + (long)p->kh * p->wp + p->kw;
+    p->lead = fold ? 0 : p->ph * p->wp + p->pw;
+    p->rows = p->lead + p->q_total + frame_slack(*p);
     p->bytes[xnor_nn_resource_bin_src] = (size_t)p->rows * p->icp;
-    p->bytes[xnor_nn_resource_bin_weights] = (size_t)p->kh * p->kw * p->ocp16 * p->icp;
+    p->bytes[xnor_nn_resource_bin_weights] = (size_t)taps * p->ocp16 * p->icp;
+    if (fold) return;
     p->img_forced = force_rows || !frame;
     plan_image_rows(p);
+    // Above 224 channels the taps fill 128-byte rows well enough by themselves, and a position
+    // tile can serve all taps of a row (conv_tcgen05.cu, halo tiles).
+    if (!p->img && frame && p->kw >= 2 && p->icp < 128) {
+        p->cat = true;
+        p->kchunk = p->kw * p->icp > 64 ? 128 : p->kw * p->icp > 32 ? 64 : 32;
+    }
     if (!p->img && !frame) plan_popc();  // neither tensor-core kernel can serve the shape
 }
 

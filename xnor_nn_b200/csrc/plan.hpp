@@ -63,6 +63,28 @@ struct Plan {
     int ocp16;      // output channels rounded up to 16 (UMMA N granularity)
     int n_tile;     // UMMA N per accumulator (<= 256, multiple of 16)
 
+    // Layers of few channels: the kw taps of a filter row read neighbouring positions, and
+    // positions are contiguous, so the operand row of position q can simply run on into the next
+    // kw - 1 positions: one tap per filter row, kw*icp bytes deep, from the same activations (a
+    // tensor map whose rows overlap). Weights are then [kh][ocp16][kw*icp]. The copy engine moves
+    // full 128-byte rows instead of kw short ones, and 64-channel slices are not cut off at every tap.
+    bool cat;
+
+    // ---- folded layers (kTcgen05, strides) -------------------------------------------------
+    // A strided layer becomes a unit-stride one for the same kernel: a position of the frame is an
+    // output column ow and a block hb of sh input rows, and its channels are the values
+    //   x[c][hb*sh - ph + i][ow*sw - pw + j],  i < fold_rows = min(kh, sh), j < kw, c < ic,
+    // in the order (i, j, c) with the channels rounded up to eight or, with fewer than eight
+    // channels, (c, i, j) with the columns rounded up to eight (fold_field; else 0): fold_ic in
+    // all. Output row oh then reads the fold_taps = ceil(kh/sh) blocks oh, oh+1, ...: a
+    // fold_taps x 1 filter whose rows past kh are zero weights. The frame has no border (what lies
+    // outside the image is stored as zeros): wp = ow, hp = oh + fold_taps - 1, lead = 0, and icp,
+    // kchunk describe fold_ic channels.
+    bool fold;
+    int fold_rows, fold_taps, fold_ic, fold_field;
+    int fold_span;      // input columns an output row reads: (ow-1)*sw + kw
+    int fold_channels;  // channels the packer stages at a time (all of them, or a multiple of 8)
+
     // ---- tiling of the image-row kernel (kTcgen05, conv_tcgen05_img.cu) ---------------------
     // That kernel puts 128 filters on the UMMA M side and, on the N side, `img_rows` whole output
     // rows of one image (img_rows * ow <= 256 positions, rounded up to 16 for the instruction).
@@ -84,6 +106,12 @@ struct Plan {
 
     size_t bytes[xnor_nn_resource_number];
 };
+
+// The layer the tensor-core kernel is launched on: the plan itself, or the unit-stride layer a
+// strided one was folded into. (The box filter K is the original layer's and computed apart.)
+Plan conv_view(const Plan &p);
+// Rows behind the last position that tile loads may reach.
+long frame_slack(const Plan &p);
 
 int div_up_i(int a, int b);
 

@@ -283,9 +283,10 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
 }  // namespace tc
 
 // ---- host side: tensor-map encoding (shared by the convolution launchers) ------------------------
-// A [rows][row_bytes] byte matrix, boxes of box_rows x box_bytes, swizzle span = box_bytes.
+// A byte matrix of `rows` rows of row_bytes, `pitch` bytes apart (rows may overlap), boxes of
+// box_rows x box_bytes, swizzle span = box_bytes.
 bool encode_bytes_2d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t row_bytes,
-                     uint32_t box_bytes, uint32_t box_rows);
+                     uint64_t pitch, uint32_t box_bytes, uint32_t box_rows);
 // A [d3][d2][d1][row_bytes] byte tensor (strides in bytes for d1, d2, d3), boxes of
 // 1 x box2 x box1 x box_bytes, swizzle span = box_bytes; out-of-range elements read as zero.
 bool encode_bytes_4d(CUtensorMap *map, const void *ptr, uint64_t row_bytes, uint64_t d1,

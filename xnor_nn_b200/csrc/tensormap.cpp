@@ -71,12 +71,12 @@ bool encode_cached(CUtensorMap *map, const Key &k) {
 }  // namespace
 
 bool encode_bytes_2d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t row_bytes,
-                     uint32_t box_bytes, uint32_t box_rows) {
+                     uint64_t pitch, uint32_t box_bytes, uint32_t box_rows) {
     Key k;
     memset(&k, 0, sizeof k);
     k.ptr = ptr; k.rank = 2;
     k.dim[0] = row_bytes; k.dim[1] = rows;
-    k.stride[0] = row_bytes;
+    k.stride[0] = pitch;
     k.box[0] = box_bytes; k.box[1] = box_rows;
     return encode_cached(map, k);
 }

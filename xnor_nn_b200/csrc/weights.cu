@@ -27,6 +27,9 @@ struct WArgs {
     int rows;   // filters per tap in the packed matrix (padded with zero filters)
     int words;  // 32-bit words per packed row
     int nibbles;  // 1: [tap][row][word of 8 channels]; 0: bits, [tap][word of 32 channels][row]
+    int fold_rows, fold_field;  // folded layers (plan.hpp): a tap is sh filter rows
+    int taps;
+    int cat_words;  // rows that hold all columns of a filter row (Plan::cat): words per column, or 0
     int32_t *op_c;
     int ih, iw, oh, ow, sh, sw, ph, pw;
     int alpha_blocks, pack_blocks;  // roles by block index: alpha, packing, then counting
@@ -125,7 +128,7 @@ __device__ __forceinline__ void alpha_hwio(const WArgs &g, float (*stage)[kSlab]
 // read with a stride; HWIO: neighbouring threads take neighbouring filters.
 template <bool HWIO>
 __device__ __forceinline__ void pack(const WArgs &g) {
-    const int taps = g.kh * g.kw, span = g.nibbles ? 8 : 32;
+    const int taps = g.taps, span = g.nibbles ? 8 : 32;
     const long total = (long)taps * g.rows * g.words;
     const long i = (long)(blockIdx.x - g.alpha_blocks) * kThreads + threadIdx.x;
     if (i >= total) return;
@@ -141,14 +144,39 @@ __device__ __forceinline__ void pack(const WArgs &g) {
     }
     uint32_t v = 0;
     if (f < g.oc) {
-        const int c0 = word * span, n = min(span, g.ic - c0);
-        if (g.nibbles) {
+        int c0 = word * span, from = tap;
+        if (g.cat_words) {
+            const int j = word / g.cat_words;
+            c0 -= j * g.cat_words * span;
+            from = tap * g.kw + j;
+        }
+        if (g.fold_rows) {
+            const int ic8 = (g.ic + 7) / 8 * 8;
+            for (int b = 0; b < 8; b++) {
+                int c, i, j;
+                if (g.fold_field) {
+                    j = (c0 + b) % g.fold_field;
+                    i = (c0 + b) / g.fold_field % g.fold_rows;
+                    c = (c0 + b) / (g.fold_field * g.fold_rows);
+                } else {
+                    c = (c0 + b) % ic8;
+                    j = (c0 + b) / ic8 % g.kw;
+                    i = (c0 + b) / (ic8 * g.kw);
+                }
+                const int kh = tap * g.sh + i;
+                if (c < g.ic && i < g.fold_rows && j < g.kw && kh < g.kh)
+                    v |= (sign_clear(__ldg(g.w + w_index<HWIO>(g, f, c, kh * g.kw + j))) ? 0x2u : 0xAu)
+                         << (4 * b);
+            }
+        } else if (g.nibbles) {
+            const int n = min(span, g.ic - c0);
 #pragma unroll
             for (int b = 0; b < 8; b++)
                 if (b < n)
-                    v |= (sign_clear(__ldg(g.w + w_index<HWIO>(g, f, c0 + b, tap))) ? 0x2u : 0xAu)
+                    v |= (sign_clear(__ldg(g.w + w_index<HWIO>(g, f, c0 + b, from))) ? 0x2u : 0xAu)
                          << (4 * b);
         } else {
+            const int n = min(span, g.ic - c0);
             for (int b = 0; b < n; b++)
                 v |= sign_clear(__ldg(g.w + w_index<HWIO>(g, f, c0 + b, tap))) << (31 - b);
         }
@@ -197,12 +225,20 @@ cudaError_t launch_binarize_weights(const Plan &p, const float *w, void *bin_w, 
     g.nibbles = p.family == kTcgen05;
     g.rows = g.nibbles ? p.ocp16 : p.ocp;
     g.words = g.nibbles ? p.icp / 4 : p.icw;
+    g.cat_words = 0;
+    if (p.cat) {
+        g.cat_words = g.words;
+        g.words *= p.kw;
+    }
+    g.fold_rows = p.fold ? p.fold_rows : 0;
+    g.fold_field = p.fold_field;
+    g.taps = p.fold ? p.fold_taps : p.cat ? p.kh : p.kh * p.kw;
     g.op_c = op_c;
     g.ih = p.ih; g.iw = p.iw; g.oh = p.oh; g.ow = p.ow;
     g.sh = p.sh; g.sw = p.sw; g.ph = p.ph; g.pw = p.pw;
     const int per_block = p.w_hwio ? 32 : kWarps;  // filters an alpha block sums
     g.alpha_blocks = (p.oc + per_block - 1) / per_block;
-    g.pack_blocks = (int)(((long)p.kh * p.kw * g.rows * g.words + kThreads - 1) / kThreads);
+    g.pack_blocks = (int)(((long)g.taps * g.rows * g.words + kThreads - 1) / kThreads);
     const int count_blocks = (p.oh * p.ow + kThreads - 1) / kThreads;
     const unsigned grid = (unsigned)(g.alpha_blocks + g.pack_blocks + count_blocks);
     if (p.w_hwio) weights_kernel<true><<<grid, kThreads, 0, s>>>(g);
