@@ -472,6 +472,7 @@ template <int KK, bool PAIR>
 __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                          uint32_t stage0, int who) {
     volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
     const int rounds = Deal<PAIR>(g).rounds(g);
     if (rounds == 0) return;
     const int ksteps = g.taps * g.chunks_per_tap;  // >= g.issuers (the launcher sees to it)
@@ -493,42 +494,43 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
     for (;;) {
         if (!entered) {
             if (ks == 0)
-                ok = mbar_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
+                ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
                                g.wait_ns);
             else if (n_iss > 1)
-                ok = mbar_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6,
+                ok = warp_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6,
                                g.wait_ns);
             if (ok && ks == 0 && g.shared_cols && it > 0)
-                ok = mbar_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
+                ok = warp_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
                                g.error, 7, g.wait_ns);
             if (!ok) break;
             fence_after();
             entered = true;
         }
         const uint32_t fbar = full0 + 8u * (uint32_t)stage;
-        if (!mbar_try_wait(fbar, phase)) {
-            ok = mbar_wait(fbar, phase, abort_flag, g.error, 3, g.wait_ns);
-            if (!ok) break;
-        }
+        ok = warp_wait(fbar, phase, abort_flag, g.error, 3, g.wait_ns);
+        if (!ok) break;
         const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
         const uint32_t desc_off = (uint32_t)stage * stage_units;
         const uint64_t adesc = hi | (uint64_t)(a_lo0 + desc_off);
         const uint64_t bdesc = hi | (uint64_t)(b_lo0 + desc_off);
         // slices of zero padding behind the last channel are not multiplied
         const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < KK; k++) {
-            if (k < kk) {
-                mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
-                               g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
+            for (int k = 0; k < KK; k++) {
+                if (k < kk) {
+                    mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
+                                   g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
+                }
+            }
+            if (PAIR) commit_pair(empty0 + 8u * (uint32_t)stage);  // frees the stage in both CTAs
+            else commit(empty0 + 8u * (uint32_t)stage);
+            if (n_iss > 1 && ks == 0) {
+                fence_before();
+                mbar_arrive(smem_u32(&ctl->started[b]));
             }
         }
-        if (PAIR) commit_pair(empty0 + 8u * (uint32_t)stage);  // frees the stage in both CTAs
-        else commit(empty0 + 8u * (uint32_t)stage);
-        if (n_iss > 1 && ks == 0) {
-            fence_before();
-            mbar_arrive(smem_u32(&ctl->started[b]));
-        }
+        __syncwarp();
         stage += n_iss;
         if (stage >= n_stages) { stage -= n_stages; phase ^= 1u; }
         chunk += chunk_step;
@@ -536,7 +538,7 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
         ks += n_iss;
         if (ks >= ksteps) {  // this thread's share of the tile is issued
             ks -= ksteps;
-            if (!(g.drop_commit && it == 0 && blockIdx.x == 0)) {
+            if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
                 if (PAIR) commit_pair(smem_u32(&ctl->acc_full[b]));
                 else commit(smem_u32(&ctl->acc_full[b]));
             }
@@ -547,8 +549,10 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
     }
     if (!ok) {
         // Let every MMA this thread has issued finish before tensor memory is released.
-        if (PAIR) commit_pair(smem_u32(&ctl->drain[who]));
-        else commit(smem_u32(&ctl->drain[who]));
+        if (leader) {
+            if (PAIR) commit_pair(smem_u32(&ctl->drain[who]));
+            else commit(smem_u32(&ctl->drain[who]));
+        }
         mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
     }
 }
@@ -565,6 +569,7 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                                               const CUtensorMap *map_a, const CUtensorMap *map_b,
                                               uint32_t stage0, uint32_t rank) {
     volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
     const Deal<PAIR> deal(g);
     const int rounds = deal.rounds(g);
     const uint32_t full_l = smem_u32(&ctl->full[0]), afull_l = smem_u32(&ctl->a_full[0]);
@@ -587,30 +592,30 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
         for (int kh = 0; ok && kh < g.kh; kh++) {
             for (int chunk = 0; ok && chunk < g.chunks_per_tap; chunk++) {
                 const uint32_t aebar = aempty0 + 8u * (uint32_t)sa;
-                if (!mbar_try_wait(aebar, pa ^ 1)) {
-                    ok = mbar_wait(aebar, pa ^ 1, abort_flag, g.error, 8, g.wait_ns);
-                    if (!ok) break;
-                }
+                ok = warp_wait(aebar, pa ^ 1, abort_flag, g.error, 8, g.wait_ns);
+                if (!ok) break;
                 const uint32_t abar = afull0 + 8u * (uint32_t)sa;
-                if (!PAIR || rank == 0) mbar_expect_tx(abar, mult * a_bytes);  // abar is local here
                 const uint32_t adst = stage0 + (uint32_t)sa * g.a_slot_bytes;
-                if (PAIR) tma_load_2d_pair(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
-                else tma_load_2d(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
+                if (leader) {
+                    if (!PAIR || rank == 0) mbar_expect_tx(abar, mult * a_bytes);  // abar is local here
+                    if (PAIR) tma_load_2d_pair(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
+                    else tma_load_2d(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
+                }
                 armed_a |= 1u << sa;
                 parity_a = (parity_a & ~(1u << sa)) | (pa << sa);
                 if (++sa == g.n_a_slots) { sa = 0; pa ^= 1; }
                 int brow = brow0 + kh * g.tap_kw * g.ocp16;
                 for (int kw = 0; kw < g.tap_kw; kw++, brow += g.ocp16) {
                     const uint32_t ebar = empty0 + 8u * (uint32_t)sb;
-                    if (!mbar_try_wait(ebar, pb ^ 1)) {
-                        ok = mbar_wait(ebar, pb ^ 1, abort_flag, g.error, 1, g.wait_ns);
-                        if (!ok) break;
-                    }
+                    ok = warp_wait(ebar, pb ^ 1, abort_flag, g.error, 1, g.wait_ns);
+                    if (!ok) break;
                     const uint32_t bar = full0 + 8u * (uint32_t)sb;
-                    if (!PAIR || rank == 0) mbar_expect_tx(bar, mult * g.b_bytes);
                     const uint32_t bdst = stage0 + g.b_ring_off + (uint32_t)sb * g.b_slot_bytes;
-                    if (PAIR) tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, bar);
-                    else tma_load_2d(bdst, map_b, chunk * g.kchunk, brow, bar);
+                    if (leader) {
+                        if (!PAIR || rank == 0) mbar_expect_tx(bar, mult * g.b_bytes);
+                        if (PAIR) tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, bar);
+                        else tma_load_2d(bdst, map_b, chunk * g.kchunk, brow, bar);
+                    }
                     armed_b |= 1u << sb;
                     parity_b = (parity_b & ~(1u << sb)) | (pb << sb);
                     if (++sb == g.n_stages) { sb = 0; pb ^= 1; }
@@ -634,6 +639,7 @@ template <int KK, bool PAIR>
 __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                               uint32_t stage0, int who) {
     volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
     const int rounds = Deal<PAIR>(g).rounds(g);
     if (rounds == 0) return;
     const int ksteps = g.taps * g.chunks_per_tap;  // >= g.issuers; a multiple of g.tap_kw
@@ -658,13 +664,13 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     for (;;) {
         if (!entered) {
             if (ks == 0)
-                ok = mbar_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
+                ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
                                g.wait_ns);
             else if (n_iss > 1)
-                ok = mbar_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6,
+                ok = warp_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6,
                                g.wait_ns);
             if (ok && ks == 0 && g.shared_cols && it > 0)
-                ok = mbar_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
+                ok = warp_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
                                g.error, 7, g.wait_ns);
             if (!ok) break;
             fence_after();
@@ -672,44 +678,45 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
         }
         if (!a_seen) {  // first step of this thread in the group: the halo tile must have landed
             const uint32_t abar = afull0 + 8u * (uint32_t)sa;
-            if (!mbar_try_wait(abar, pa)) {
-                ok = mbar_wait(abar, pa, abort_flag, g.error, 9, g.wait_ns);
-                if (!ok) break;
-            }
+            ok = warp_wait(abar, pa, abort_flag, g.error, 9, g.wait_ns);
+            if (!ok) break;
             a_seen = true;
         }
         const uint32_t fbar = full0 + 8u * (uint32_t)sb;
-        if (!mbar_try_wait(fbar, pb)) {
-            ok = mbar_wait(fbar, pb, abort_flag, g.error, 3, g.wait_ns);
-            if (!ok) break;
-        }
+        ok = warp_wait(fbar, pb, abort_flag, g.error, 3, g.wait_ns);
+        if (!ok) break;
         fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
         const uint64_t adesc =
             hi | (uint64_t)(a_lo0 + (uint32_t)sa * a_units + (uint32_t)kw * row_units);
         const uint64_t bdesc = hi | (uint64_t)(b_lo0 + (uint32_t)sb * b_units);
         const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < KK; k++) {
-            if (k < kk) {
-                mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
-                               g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
+            for (int k = 0; k < KK; k++) {
+                if (k < kk) {
+                    mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
+                                   g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
+                }
+            }
+            if (PAIR) commit_pair(empty0 + 8u * (uint32_t)sb);
+            else commit(empty0 + 8u * (uint32_t)sb);
+            if (n_iss > 1 && ks == 0) {
+                fence_before();
+                mbar_arrive(smem_u32(&ctl->started[b]));
             }
         }
-        if (PAIR) commit_pair(empty0 + 8u * (uint32_t)sb);
-        else commit(empty0 + 8u * (uint32_t)sb);
-        if (n_iss > 1 && ks == 0) {
-            fence_before();
-            mbar_arrive(smem_u32(&ctl->started[b]));
-        }
+        __syncwarp();
         sb += n_iss;
         if (sb >= g.n_stages) { sb -= g.n_stages; pb ^= 1u; }
         kw += n_iss;
         if (kw >= kwn) {
             // this thread's last step of the group is issued: its reads of the halo tile are
             // covered by this commit (both issuers commit: the barrier counts them)
-            if (PAIR) commit_pair(aempty0 + 8u * (uint32_t)sa);
-            else commit(aempty0 + 8u * (uint32_t)sa);
+            if (leader) {
+                if (PAIR) commit_pair(aempty0 + 8u * (uint32_t)sa);
+                else commit(aempty0 + 8u * (uint32_t)sa);
+            }
             do {
                 kw -= kwn;
                 if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
@@ -720,7 +727,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
         ks += n_iss;
         if (ks >= ksteps) {  // this thread's share of the tile is issued
             ks -= ksteps;
-            if (!(g.drop_commit && it == 0 && blockIdx.x == 0)) {
+            if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
                 if (PAIR) commit_pair(smem_u32(&ctl->acc_full[b]));
                 else commit(smem_u32(&ctl->acc_full[b]));
             }
@@ -730,8 +737,10 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
         }
     }
     if (!ok) {
-        if (PAIR) commit_pair(smem_u32(&ctl->drain[who]));
-        else commit(smem_u32(&ctl->drain[who]));
+        if (leader) {
+            if (PAIR) commit_pair(smem_u32(&ctl->drain[who]));
+            else commit(smem_u32(&ctl->drain[who]));
+        }
         mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
     }
 }
@@ -753,7 +762,8 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     Control *ctl = (Control *)base;
     uint8_t *stages = base + kControlBytes;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // warp-uniform, and known to be: the roles below run on whole warps
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     volatile int *abort_flag = &ctl->abort_flag;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
 
@@ -814,72 +824,69 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     const uint32_t stage0 = smem_u32(stages);
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- TMA producer ----
-            dependency_wait();
-            if (g.halo) {
-                producer_halo<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
-            } else {
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t armed = 0;  // bit s: stage s holds a load nobody is known to have consumed
-            uint32_t armed_parity = 0;
-            bool ok = true;
-            // a pair counts both CTAs' bytes on the leader's barrier
-            const uint32_t full_local = smem_u32(&ctl->full[0]);
-            const uint32_t full0 = PAIR && rank != 0 ? mapa(full_local, 0) : full_local;
-            const int b_rows = PAIR ? g.n_tile >> 1 : g.n_tile;  // filter rows this CTA loads
-            for (int it = 0; ok && it < rounds; it++) {
-                int mt, nt;
-                deal.at(g, it, mt, nt);
-                int row = g.lead + mt * BM - g.ph * g.wp - g.pw;  // tap (0,0)
-                int brow = nt * g.n_tile + (int)rank * b_rows;
-                int kw = 0, chunk = 0;
-                for (int ks = 0; ks < ksteps; ks++) {
-                    const uint32_t ebar = smem_u32(&ctl->empty[stage]);
-                    if (!mbar_try_wait(ebar, phase ^ 1)) {
-                        ok = mbar_wait(ebar, phase ^ 1, abort_flag, g.error, 1, g.wait_ns);
-                        if (!ok) break;
-                    }
-                    armed &= ~(1u << stage);
-                    const uint32_t bar = full0 + 8u * (uint32_t)stage;
-                    const uint32_t sa = stage0 + (uint32_t)stage * g.stage_bytes;
-                    if (PAIR) {
-                        if (rank == 0) mbar_expect_tx(bar, 2u * g.tx_bytes);  // bar is local here
-                        tma_load_2d_pair(sa, &map_a, chunk * g.kchunk, row, bar);
-                        tma_load_2d_pair(sa + g.a_bytes, &map_b, chunk * g.kchunk, brow, bar);
-                    } else {
-                        mbar_expect_tx(bar, g.tx_bytes);
-                        tma_load_2d(sa, &map_a, chunk * g.kchunk, row, bar);
-                        tma_load_2d(sa + g.a_bytes, &map_b, chunk * g.kchunk, brow, bar);
-                    }
-                    armed |= 1u << stage;
-                    armed_parity = (armed_parity & ~(1u << stage)) | (phase << stage);
-                    if (++stage == g.n_stages) { stage = 0; phase ^= 1; }
-                    if (++chunk == g.chunks_per_tap) {  // next filter tap
-                        chunk = 0;
-                        brow += g.ocp16;
-                        if (++kw == g.tap_kw) { kw = 0; row += g.wp - (g.tap_kw - 1); }
-                        else row += 1;
-                    }
+        // ---- TMA producer ----
+        dependency_wait();
+        const bool leader = elect_one();
+        if (g.halo) {
+            producer_halo<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
+        } else {
+        int stage = 0;
+        uint32_t phase = 0;
+        uint32_t armed = 0;  // bit s: stage s holds a load nobody is known to have consumed
+        uint32_t armed_parity = 0;
+        bool ok = true;
+        // a pair counts both CTAs' bytes on the leader's barrier
+        const uint32_t full_local = smem_u32(&ctl->full[0]);
+        const uint32_t full0 = PAIR && rank != 0 ? mapa(full_local, 0) : full_local;
+        const int b_rows = PAIR ? g.n_tile >> 1 : g.n_tile;  // filter rows this CTA loads
+        for (int it = 0; ok && it < rounds; it++) {
+            int mt, nt;
+            deal.at(g, it, mt, nt);
+            int row = g.lead + mt * BM - g.ph * g.wp - g.pw;  // tap (0,0)
+            int brow = nt * g.n_tile + (int)rank * b_rows;
+            int kw = 0, chunk = 0;
+            for (int ks = 0; ks < ksteps; ks++) {
+                const uint32_t ebar = smem_u32(&ctl->empty[stage]);
+                ok = warp_wait(ebar, phase ^ 1, abort_flag, g.error, 1, g.wait_ns);
+                if (!ok) break;
+                armed &= ~(1u << stage);
+                const uint32_t bar = full0 + 8u * (uint32_t)stage;
+                const uint32_t sa = stage0 + (uint32_t)stage * g.stage_bytes;
+                if (leader && PAIR) {
+                    if (rank == 0) mbar_expect_tx(bar, 2u * g.tx_bytes);  // bar is local here
+                    tma_load_2d_pair(sa, &map_a, chunk * g.kchunk, row, bar);
+                    tma_load_2d_pair(sa + g.a_bytes, &map_b, chunk * g.kchunk, brow, bar);
+                } else if (leader) {
+                    mbar_expect_tx(bar, g.tx_bytes);
+                    tma_load_2d(sa, &map_a, chunk * g.kchunk, row, bar);
+                    tma_load_2d(sa + g.a_bytes, &map_b, chunk * g.kchunk, brow, bar);
+                }
+                armed |= 1u << stage;
+                armed_parity = (armed_parity & ~(1u << stage)) | (phase << stage);
+                if (++stage == g.n_stages) { stage = 0; phase ^= 1; }
+                if (++chunk == g.chunks_per_tap) {  // next filter tap
+                    chunk = 0;
+                    brow += g.ocp16;
+                    if (++kw == g.tap_kw) { kw = 0; row += g.wp - (g.tap_kw - 1); }
+                    else row += 1;
                 }
             }
-            if (!ok && rank == 0) {
-                // Something gave up. Loads already issued still land in this CTA's shared
-                // memory: wait for them (bounded) before the CTA may exit. (The partner of a
-                // pair cannot wait on the leader's barrier; it stays until the leader has got
-                // through this and both have met at the cluster barrier below.)
-                for (int s = 0; s < g.n_stages; s++)
-                    if (armed & (1u << s)) {
-                        mbar_wait_quiet(smem_u32(&ctl->full[s]), (armed_parity >> s) & 1u,
-                                        g.wait_ns);
-                    }
-            }
-            }
+        }
+        if (!ok && rank == 0) {
+            // Something gave up. Loads already issued still land in this CTA's shared
+            // memory: wait for them (bounded) before the CTA may exit. (The partner of a
+            // pair cannot wait on the leader's barrier; it stays until the leader has got
+            // through this and both have met at the cluster barrier below.)
+            for (int s = 0; s < g.n_stages; s++)
+                if (armed & (1u << s)) {
+                    mbar_wait_quiet(smem_u32(&ctl->full[s]), (armed_parity >> s) & 1u,
+                                    g.wait_ns);
+                }
+        }
         }
     } else if (warp == 1 || warp == kIssuer2Warp) {
         const int who = warp == 1 ? 0 : 1;
-        if (lane == 0 && who < g.issuers && rank == 0) {
+        if (who < g.issuers && rank == 0) {
             if (g.halo) mma_role_halo<KK, PAIR>(g, ctl, tmem_base, stage0, who);
             else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
         }
