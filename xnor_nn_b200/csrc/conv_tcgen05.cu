@@ -128,7 +128,7 @@ struct __align__(16) Control {
     unsigned long long acc_empty[kMaxAcc];
     unsigned long long a_full[4];   // halo mode: a halo tile has landed / has been used up
     unsigned long long a_empty[4];
-    unsigned long long started[kMaxAcc];  // two issuers: the tile's first MMA (which overwrites) is out
+    unsigned long long started[kMaxAcc];  // two issuers: the tile's first MMAs (one overwrites) are done
     unsigned long long drain[2];
     unsigned long long shared_free;  // the columns both accumulators use have been read
     uint32_t tmem_base;
@@ -467,7 +467,10 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
 // tile: a commit covers the MMAs of the committing thread only. The sum is over integers, so the
 // order in which the two threads' MMAs reach the pipe does not matter, except for the tile's
 // first instruction, which overwrites the accumulator: its issuer waits for the epilogue to have
-// drained the accumulator, and the other issuer waits for it (started[]).
+// drained the accumulator, and the other issuer waits until it has been executed (started[], a
+// commit: nothing orders the MMAs of two threads that have only been issued). The ring has an even
+// number of buffers then, so that a buffer always has the same issuer, which sees every phase of
+// its barrier: to one that skips a phase, a buffer whose previous load has not landed looks full.
 template <int KK, bool PAIR>
 __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                          uint32_t stage0, int who) {
@@ -526,8 +529,8 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
             if (PAIR) commit_pair(empty0 + 8u * (uint32_t)stage);  // frees the stage in both CTAs
             else commit(empty0 + 8u * (uint32_t)stage);
             if (n_iss > 1 && ks == 0) {
-                fence_before();
-                mbar_arrive(smem_u32(&ctl->started[b]));
+                if (PAIR) commit_pair(smem_u32(&ctl->started[b]));
+                else commit(smem_u32(&ctl->started[b]));
             }
         }
         __syncwarp();
@@ -702,8 +705,8 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
             if (PAIR) commit_pair(empty0 + 8u * (uint32_t)sb);
             else commit(empty0 + 8u * (uint32_t)sb);
             if (n_iss > 1 && ks == 0) {
-                fence_before();
-                mbar_arrive(smem_u32(&ctl->started[b]));
+                if (PAIR) commit_pair(smem_u32(&ctl->started[b]));
+                else commit(smem_u32(&ctl->started[b]));
             }
         }
         __syncwarp();
@@ -1005,6 +1008,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         g.n_stages = (int)(room / g.stage_bytes);
         if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
     }
+    if (g.issuers == 2 && g.n_stages > 2) g.n_stages &= ~1;
     if (g.n_stages < 2) return cudaErrorNotSupported;
     CUtensorMap map_a, map_b;
     // a position's row is tap_bytes long but only icp further than the one before it

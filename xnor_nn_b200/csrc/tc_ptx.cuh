@@ -148,7 +148,7 @@ __device__ __forceinline__ void cluster_wait() {
 // memory: the reads before it are complete (tcgen05.wait::ld) and ordered by fence_before(), so the
 // arrival is relaxed. As a release at cluster scope it also waited until the thread's earlier
 // result stores had reached L2, 2500 to 3500 cycles during which the next tile's MMAs stood still
-// (a tile of AlexNet conv4 takes 8500): conv4 with 256 images 27.4 -> 24.6 us.
+// (a tile of AlexNet conv4 takes 8500): the kernel on conv4 with 256 images 27.4 -> 25.6 us.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                  : "memory");
