@@ -71,6 +71,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kScaleCol = 496;
 constexpr int kAccStep = 240;        // columns between the accumulators' starts, at most
 constexpr int kMaxAcc = 4;
+constexpr int kMaxASlots = 8;        // halo tiles in flight
 struct TcArgs {
     const float *alpha;
     const float *kmap;   // K per output pixel, or null: box-filter it from amap in the epilogue
@@ -107,6 +108,11 @@ struct TcArgs {
     int halo;             // 0, or rows of a halo tile (128 + 8)
     int n_a_slots;        // halo tiles in flight
     uint32_t a_slot_bytes, b_ring_off, b_slot_bytes, b_bytes;
+    // Resident filters (pairs whose tiles all have the same filter tile, if its operands of all
+    // taps fit shared memory beside three position tiles): halo mode with filter tiles that are
+    // loaded once, together with the first round's position tiles, and stay. halo is 128 then if
+    // there is one tap per filter row.
+    int resident;
     int kk_last;          // MMAs of a tap's last channel chunk: its 64-channel slices that hold
                           // channels at all (the chunk is padded with zeros to kchunk bytes)
     uint32_t acc_step;    // columns from the first accumulator to the second
@@ -126,8 +132,8 @@ struct __align__(16) Control {
     unsigned long long empty[kMaxStages];
     unsigned long long acc_full[kMaxAcc];
     unsigned long long acc_empty[kMaxAcc];
-    unsigned long long a_full[4];   // halo mode: a halo tile has landed / has been used up
-    unsigned long long a_empty[4];
+    unsigned long long a_full[kMaxASlots];  // halo mode: a halo tile has landed / has been used up
+    unsigned long long a_empty[kMaxASlots];
     unsigned long long started[kMaxAcc];  // two issuers: the tile's first MMAs (one overwrites) are done
     unsigned long long drain[2];
     unsigned long long shared_free;  // the columns both accumulators use have been read
@@ -599,8 +605,12 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                 if (!ok) break;
                 const uint32_t abar = afull0 + 8u * (uint32_t)sa;
                 const uint32_t adst = stage0 + (uint32_t)sa * g.a_slot_bytes;
+                // resident filters travel with the first round's position tiles
+                const bool with_b = g.resident && it == 0;
+                const uint32_t bytes =
+                    mult * (a_bytes + (with_b ? (uint32_t)g.tap_kw * g.b_bytes : 0u));
                 if (leader) {
-                    if (!PAIR || rank == 0) mbar_expect_tx(abar, mult * a_bytes);  // abar is local here
+                    if (!PAIR || rank == 0) mbar_expect_tx(abar, bytes);  // abar is local here
                     if (PAIR) tma_load_2d_pair(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
                     else tma_load_2d(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
                 }
@@ -608,6 +618,21 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                 parity_a = (parity_a & ~(1u << sa)) | (pa << sa);
                 if (++sa == g.n_a_slots) { sa = 0; pa ^= 1; }
                 int brow = brow0 + kh * g.tap_kw * g.ocp16;
+                if (g.resident) {
+                    if (with_b && leader) {
+                        uint32_t bdst = stage0 + g.b_ring_off +
+                                        (uint32_t)((kh * g.chunks_per_tap + chunk) * g.tap_kw) *
+                                            g.b_slot_bytes;
+                        for (int kw = 0; kw < g.tap_kw; kw++) {
+                            if (PAIR) tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, abar);
+                            else tma_load_2d(bdst, map_b, chunk * g.kchunk, brow, abar);
+                            brow += g.ocp16;
+                            bdst += g.b_slot_bytes;
+                        }
+                    }
+                    __syncwarp();
+                    continue;
+                }
                 for (int kw = 0; kw < g.tap_kw; kw++, brow += g.ocp16) {
                     const uint32_t ebar = empty0 + 8u * (uint32_t)sb;
                     ok = warp_wait(ebar, pb ^ 1, abort_flag, g.error, 1, g.wait_ns);
@@ -748,6 +773,76 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     }
 }
 
+// Resident filters: the only thing that arrives is position tiles, so a group (the taps of a filter
+// row on one channel chunk) is one wait, kw * KK MMAs and one commit, which one issuer keeps up
+// with. With the filters streamed a pair moved 320 KB per CTA and tile of AlexNet conv2 through L2,
+// which took 11400 cycles under the result stores of another tile (tensor pipe: 5100).
+template <int KK, bool PAIR>
+__device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl, uint32_t tmem_base,
+                                                  uint32_t stage0) {
+    volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
+    const int rounds = Deal<PAIR>(g).rounds(g);
+    if (rounds == 0) return;
+    const int groups = g.kh * g.chunks_per_tap;
+    const uint64_t hi = (uint64_t)g.desc_hi << 32;
+    const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (1u << 16);
+    const uint32_t b_lo0 = (((stage0 + g.b_ring_off) >> 4) & 0x3FFF) | (1u << 16);
+    const uint32_t a_units = g.a_slot_bytes >> 4, b_units = g.b_slot_bytes >> 4;
+    const uint32_t row_units = (uint32_t)g.kchunk >> 4;  // one position further
+    const uint32_t afull0 = smem_u32(&ctl->a_full[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
+    int sa = 0, b = 0;
+    uint32_t pa = 0, acc_phase = 0;
+    bool ok = true;
+    for (int it = 0; it < rounds; it++) {
+        const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
+        ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2, g.wait_ns);
+        if (ok && g.shared_cols && it > 0)
+            ok = warp_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag, g.error,
+                           7, g.wait_ns);
+        if (!ok) break;
+        for (int gr = 0, chunk = 0; gr < groups; gr++) {
+            ok = warp_wait(afull0 + 8u * (uint32_t)sa, pa, abort_flag, g.error, 9, g.wait_ns);
+            if (!ok) break;
+            fence_after();
+            const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+            if (leader) {
+                uint64_t adesc = hi | (uint64_t)(a_lo0 + (uint32_t)sa * a_units);
+                uint64_t bdesc = hi | (uint64_t)(b_lo0 + (uint32_t)(gr * g.tap_kw) * b_units);
+                for (int kw = 0; kw < g.tap_kw; kw++, adesc += row_units, bdesc += b_units) {
+#pragma unroll
+                    for (int k = 0; k < KK; k++) {
+                        if (k < kk) {
+                            mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k),
+                                           bdesc + (uint64_t)(2 * k), g.idesc,
+                                           tmem_base + kScaleCol, (gr | kw | k) == 0 ? 0u : 1u);
+                        }
+                    }
+                }
+                if (PAIR) commit_pair(aempty0 + 8u * (uint32_t)sa);
+                else commit(aempty0 + 8u * (uint32_t)sa);
+            }
+            __syncwarp();
+            if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
+            if (++chunk == g.chunks_per_tap) chunk = 0;
+        }
+        if (!ok) break;
+        if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
+            if (PAIR) commit_pair(smem_u32(&ctl->acc_full[b]));
+            else commit(smem_u32(&ctl->acc_full[b]));
+        }
+        __syncwarp();
+        if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
+    }
+    if (!ok) {
+        if (leader) {
+            if (PAIR) commit_pair(smem_u32(&ctl->drain[0]));
+            else commit(smem_u32(&ctl->drain[0]));
+        }
+        mbar_wait_quiet(smem_u32(&ctl->drain[0]), 0, g.wait_ns);
+    }
+}
+
 // KK = tcgen05.mma instructions per pipeline stage (kchunk / 32).
 // PAIR: the grid is made of clusters of two CTAs that share tiles of 256 positions x N filters
 // (tcgen05 cta_group::2). Each CTA loads its own 128 positions and its half of the filter tile,
@@ -775,7 +870,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             mbar_init(smem_u32(&ctl->full[s]), 1);
             mbar_init(smem_u32(&ctl->empty[s]), 1);
         }
-        for (int a = 0; a < 4; a++) {
+        for (int a = 0; a < g.n_a_slots; a++) {
             mbar_init(smem_u32(&ctl->a_full[a]), 1);
             mbar_init(smem_u32(&ctl->a_empty[a]), (uint32_t)g.issuers);
         }
@@ -890,7 +985,8 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     } else if (warp == 1 || warp == kIssuer2Warp) {
         const int who = warp == 1 ? 0 : 1;
         if (who < g.issuers && rank == 0) {
-            if (g.halo) mma_role_halo<KK, PAIR>(g, ctl, tmem_base, stage0, who);
+            if (PAIR && g.resident) mma_role_resident<KK, PAIR>(g, ctl, tmem_base, stage0);
+            else if (g.halo) mma_role_halo<KK, PAIR>(g, ctl, tmem_base, stage0, who);
             else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
         }
         __syncwarp();
@@ -988,37 +1084,6 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.stage_bytes = (g.tx_bytes + 1023u) & ~1023u;
     g.issuers = g.taps * g.chunks_per_tap < 2 ? 1 : 2;
     g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
-    // as many ring buffers as fit beside the control block
-    const size_t room = 227 * 1024 - 1024 - kControlBytes;
-    g.halo = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
-    g.b_bytes = (uint32_t)(b_rows * p.kchunk);
-    bool halo = pair && g.tap_kw >= 2 && g.tap_kw <= 9 && g.issuers <= g.tap_kw;
-    if (halo) {
-        // three halo tiles of 136 positions, the rest of the room for filter tiles
-        g.halo = BM + 8;
-        g.n_a_slots = 3;
-        g.a_slot_bytes = (uint32_t)(g.halo * p.kchunk + 1023) & ~1023u;
-        g.b_slot_bytes = (g.b_bytes + 1023u) & ~1023u;
-        g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
-        g.n_stages = (int)((room - g.b_ring_off) / g.b_slot_bytes);
-        if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
-        if (g.n_stages < 4) { g.halo = 0; halo = false; }
-    }
-    if (!halo) {
-        g.n_stages = (int)(room / g.stage_bytes);
-        if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
-    }
-    if (g.issuers == 2 && g.n_stages > 2) g.n_stages &= ~1;
-    if (g.n_stages < 2) return cudaErrorNotSupported;
-    CUtensorMap map_a, map_b;
-    // a position's row is tap_bytes long but only icp further than the one before it
-    if (!encode_bytes_2d(&map_a, bin_src, (uint64_t)(p.rows - (p.cat ? p.kw - 1 : 0)),
-                         (uint64_t)tap_bytes, (uint64_t)p.icp, (uint32_t)p.kchunk,
-                         (uint32_t)(halo ? g.halo : BM)) ||
-        !encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
-                         (uint64_t)tap_bytes, (uint32_t)p.kchunk, (uint32_t)b_rows))
-        return cudaErrorNotSupported;
-
     const int kk = p.kchunk / 32;
     void (*kernel)(CUtensorMap, CUtensorMap, TcArgs) =
         pair ? (kk == 4   ? conv_tcgen05_kernel<4, true>
@@ -1027,11 +1092,6 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
              : (kk == 4   ? conv_tcgen05_kernel<4, false>
                 : kk == 2 ? conv_tcgen05_kernel<2, false>
                           : conv_tcgen05_kernel<1, false>);
-    size_t smem = 1024 + kControlBytes +
-                  (halo ? (size_t)g.b_ring_off + (size_t)g.n_stages * g.b_slot_bytes
-                        : (size_t)g.n_stages * g.stage_bytes);
-    // At least 120 KB of shared memory so that one CTA owns the SM and all 512 TMEM columns.
-    if (smem < 120 * 1024) smem = 120 * 1024;
     // per device and kernel, once: the opt-in to large dynamic shared memory, the SM count and
     // the number of CTA pairs that can be resident together
     static std::atomic<bool> opted_in[64][3][2];
@@ -1063,7 +1123,68 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
             pair_count[d].store(slots, std::memory_order_relaxed);
         }
     }
-    const int grid = units < slots ? units : slots;
+    int grid = units < slots ? units : slots;
+    // Fewer pairs, if that costs no further round, so that each keeps to one filter tile.
+    const int one_nt = grid - grid % g.n_tiles;
+    const bool same_nt = pair && one_nt > 0 && div_up_i(units, one_nt) == div_up_i(units, grid);
+    // as many ring buffers as fit beside the control block
+    const size_t room = 227 * 1024 - 1024 - kControlBytes;
+    g.halo = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
+    g.b_bytes = (uint32_t)(b_rows * p.kchunk);
+    bool halo = pair && g.tap_kw >= 2 && g.tap_kw <= 9 && g.issuers <= g.tap_kw;
+    // Filters stay in shared memory if a pair works on several tiles of the same ones and their
+    // operands leave room for three position tiles (kernel alone: conv2 mb128 48.8 -> 43.8 us, conv3
+    // mb256 25.4 -> 23.0, conv1 mb64 26.1 -> 25.5; three is what conv2 needs the room for).
+    const int groups = g.kh * g.chunks_per_tap;
+    if (same_nt && div_up_i(units, one_nt) > 1 && g.tap_kw <= 9) {
+        const uint32_t rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
+        const uint32_t a_slot = (rows * p.kchunk + 1023) & ~1023u, b_slot = (g.b_bytes + 1023u) & ~1023u;
+        const size_t all_b = (size_t)groups * g.tap_kw * b_slot;
+        if (all_b + 3 * (size_t)a_slot <= room) {
+            g.resident = 1;
+            g.issuers = 1;
+            g.halo = (int)rows;
+            g.a_slot_bytes = a_slot; g.b_slot_bytes = b_slot;
+            g.n_a_slots = (int)((room - all_b) / a_slot);
+            if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
+            g.b_ring_off = (uint32_t)g.n_a_slots * a_slot;
+            g.n_stages = 2;
+            grid = one_nt;
+            halo = true;
+        }
+    }
+    if (halo && !g.resident) {
+        // three halo tiles of 136 positions, the rest of the room for filter tiles
+        g.halo = BM + 8;
+        g.n_a_slots = 3;
+        g.a_slot_bytes = (uint32_t)(g.halo * p.kchunk + 1023) & ~1023u;
+        g.b_slot_bytes = (g.b_bytes + 1023u) & ~1023u;
+        g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
+        g.n_stages = (int)((room - g.b_ring_off) / g.b_slot_bytes);
+        if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
+        if (g.n_stages < 4) { g.halo = 0; halo = false; }
+    }
+    if (!halo) {
+        g.n_stages = (int)(room / g.stage_bytes);
+        if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
+    }
+    if (g.issuers == 2 && g.n_stages > 2) g.n_stages &= ~1;
+    if (g.n_stages < 2) return cudaErrorNotSupported;
+    CUtensorMap map_a, map_b;
+    // a position's row is tap_bytes long but only icp further than the one before it
+    if (!encode_bytes_2d(&map_a, bin_src, (uint64_t)(p.rows - (p.cat ? p.kw - 1 : 0)),
+                         (uint64_t)tap_bytes, (uint64_t)p.icp, (uint32_t)p.kchunk,
+                         (uint32_t)(halo ? g.halo : BM)) ||
+        !encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
+                         (uint64_t)tap_bytes, (uint32_t)p.kchunk, (uint32_t)b_rows))
+        return cudaErrorNotSupported;
+
+    size_t smem = 1024 + kControlBytes +
+                  (g.resident ? (size_t)g.b_ring_off + (size_t)groups * g.tap_kw * g.b_slot_bytes
+                   : halo ? (size_t)g.b_ring_off + (size_t)g.n_stages * g.b_slot_bytes
+                        : (size_t)g.n_stages * g.stage_bytes);
+    // At least 120 KB of shared memory so that one CTA owns the SM and all 512 TMEM columns.
+    if (smem < 120 * 1024) smem = 120 * 1024;
     // As many accumulators as fit (at most four), and one epilogue team for each of two or four of
     // them if a CTA has that many tiles. With all 16 warps on every tile AlexNet conv3 (256
     // images) took 41.3 us per pass, conv1 (64 images) 86, with two teams 37.7 and 79. The chained
