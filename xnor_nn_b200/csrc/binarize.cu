@@ -343,6 +343,8 @@ constexpr int kBoxSmem = 40 * 1024;
 template <int KW>
 __global__ void __launch_bounds__(kBoxThreads) box_filter_kernel(const BoxArgs g) {
     extern __shared__ __align__(16) float tile[];
+    dependency_release();
+    dependency_wait();
     const int n = blockIdx.x / g.row_blocks;
     const int oy0 = (blockIdx.x - n * g.row_blocks) * g.rows;
     const int n_out = min(g.rows, g.oh - oy0) * g.ow;
@@ -379,6 +381,8 @@ __global__ void __launch_bounds__(kBoxThreads) box_filter_kernel(const BoxArgs g
 
 // Windows that do not fit shared memory: one thread per output, straight from A.
 __global__ void __launch_bounds__(kBoxThreads) box_filter_wide_kernel(const BoxArgs g) {
+    dependency_release();
+    dependency_wait();
     const long o = (long)blockIdx.x * kBoxThreads + threadIdx.x;
     const long plane = (long)g.oh * g.ow;
     const long n = o / plane;
@@ -513,9 +517,9 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
     if (bytes(g.rows) > kBoxSmem) {
         g.row_blocks = p.mb;
         const long n_out = (long)p.mb * p.oh * p.ow;
-        box_filter_wide_kernel<<<(unsigned)((n_out + kBoxThreads - 1) / kBoxThreads), kBoxThreads,
-                                 0, s>>>(g);
-        return cudaGetLastError();
+        return launch_overlapped(box_filter_wide_kernel,
+                                 dim3((unsigned)((n_out + kBoxThreads - 1) / kBoxThreads)),
+                                 dim3(kBoxThreads), 0, s, 1, g);
     }
     g.row_blocks = div_up_i(p.oh, g.rows);
     g.lines = (int)lines(g.rows);
@@ -526,8 +530,9 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
                   : p.kw == 7  ? box_filter_kernel<7>
                   : p.kw == 11 ? box_filter_kernel<11>
                                : box_filter_kernel<0>;
-    kernel<<<blocks, kBoxThreads, (size_t)bytes(g.rows), s>>>(g);
-    return cudaGetLastError();
+    // Launched under the tail of the packer, as the convolution is under its own: conv1 mb64 63.7 ->
+    // 60.7 us a pass, the three upstream calls of an odd layer 20.6 -> 19.4.
+    return launch_overlapped(kernel, dim3(blocks), dim3(kBoxThreads), (size_t)bytes(g.rows), s, 1, g);
 }
 
 }  // namespace xb200

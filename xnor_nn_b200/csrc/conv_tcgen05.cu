@@ -14,26 +14,27 @@
 // Positions on the frame border are computed and dropped by the epilogue.
 //
 // One CTA per SM, persistent over (position tile, filter tile) pairs:
-//   warp 0      one lane issues TMA loads (cp.async.bulk.tensor.2d, each CTA fetching its own
+//   warp 0      an elected lane issues TMA loads (cp.async.bulk.tensor.2d, each CTA fetching its own
 //               tiles) into a ring of shared-memory buffers; completion is counted on an
 //               mbarrier per buffer
-//   warp 1      allocates tensor memory; one lane issues tcgen05.mma.kind::mxf4 (M=128, N<=256,
-//               K=64 per instruction) into one of two accumulators in tensor memory, and
-//               tcgen05.commit hands buffers back / accumulators on
-//   warp 18     one lane is a second MMA issuer; the two take alternate ring buffers
+//   warp 1      allocates tensor memory; an elected lane issues tcgen05.mma.kind::mxf4 (M=128,
+//               N<=256, K=64 per instruction) into one of two to four accumulators in tensor
+//               memory, and tcgen05.commit hands buffers back / accumulators on
+//   warp 18     a second MMA issuer; the two take alternate ring buffers
 //   warps 2-17  epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
 //               and a share of the columns), scale by alpha[filter] * K[position] in upstream's
-//               order and store; runs under the next tile's MMAs thanks to the second
-//               accumulator
+//               order and store; runs under the next tiles' MMAs thanks to the other
+//               accumulators
 //
 // Layers of more than one round of tiles run as clusters of two CTAs on tcgen05 cta_group::2:
 // the pair shares a tile of 256 positions x N filters, each CTA loads its own 128 positions and
 // half of the filter tile, the leader issues M = 256 instructions for both, and each CTA's
-// epilogue drains its own tensor memory. With 128-byte channel chunks a pair loads a position
-// tile only once per filter row and chunk, with a halo of the positions that follow it, and the
-// taps of the row read that tile at row offsets (producer_halo / mma_role_halo): what bounds the
-// kernel is the number of requests an SM can send towards L2, operand reads and result stores
-// together.
+// epilogue drains its own tensor memory. A pair loads a position tile only once per filter row and
+// channel chunk, with a halo of the positions that follow it, and the taps of the row read that
+// tile at row offsets (producer_halo / mma_role_halo); filters that fit are loaded once and stay
+// (mma_role_resident). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters) or,
+// when its loads share the way to L2 with the stores of the tile before it, those: AlexNet conv4 on
+// 256 images takes 8200 cycles a tile without the other's stores and 10500 with them (pipe: 6900).
 //
 // The epilogue has three forms: floats in NCHW (a warp store is one contiguous run of a filter
 // plane), floats in NHWC (a thread owns whole 32-byte sectors and writes them with 256-bit
@@ -102,7 +103,7 @@ struct TcArgs {
     int drop_commit;      // self-test: CTA 0 leaves out the commit that publishes its first tile
     int issuers;          // threads that issue MMAs: 1, or 2 taking alternate pipeline stages
     int n_stages;         // ring buffers in use
-    // Halo mode (pairs, 128-byte chunks, filters at least two taps wide): the position tile of a
+    // Halo mode (pairs, filters at least two taps wide): the position tile of a
     // filter row is loaded once, with the kw - 1 positions that follow it, and serves all kw taps
     // of the row (a tap is a row offset into the tile); the ring then holds filter tiles only.
     int halo;             // 0, or rows of a halo tile (128 + 8)
