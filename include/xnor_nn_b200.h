@@ -76,7 +76,8 @@ xnor_nn_status_t xnor_nn_b200_binarize(const xnor_nn_convolution_t *c, xnor_nn_r
  *   source: res[0][user_src]; result: res[layers-1][user_dst] (host or device memory);
  *   layer i+1 must take what layer i produces: same mb, ic = oc, ih = oh, iw = ow, else
  *   xnor_nn_error_invalid_input; every chained layer must run on the tensor-core kernels (unit
- *   stride), else xnor_nn_unimplemented.
+ *   stride), else xnor_nn_unimplemented. A layer in the middle whose paddings differ or are as
+ *   large as its filter does pass floats on, through a buffer that the first call allocates.
  * The packed signs, hence every integer sum, equal those of calling the layers one after another;
  * the mean-|x| maps of layers 1.. are summed in a fixed but not strictly sequential order, so the
  * floats agree with the layer-by-layer result to rounding (about 1e-6 relative), reproducibly.

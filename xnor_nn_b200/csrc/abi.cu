@@ -760,8 +760,8 @@ xnor_nn_status_t xnor_nn_b200_forward_chain(int layers, const xnor_nn_convolutio
             return xnor_nn_error_invalid_input;
         if (a.family != kTcgen05 || b.family != kTcgen05 || a.fold || b.fold) {
             snprintf(t_last_error, sizeof t_last_error,
-                     "layers %d and %d cannot be chained: both must run on the %s kernels", i,
-                     i + 1, family_name(kTcgen05));
+                     "layers %d and %d cannot be chained: both must have unit strides and run on "
+                     "the %s kernels", i, i + 1, family_name(kTcgen05));
             return xnor_nn_unimplemented;
         }
     }
@@ -797,6 +797,24 @@ xnor_nn_status_t xnor_nn_b200_forward_chain(int layers, const xnor_nn_convolutio
         void **r = res[i];
         ChainTarget next;
         const bool emit = i + 1 < layers;
+        if (!plan[i]->frame_walk) {
+            // Paddings that only the image-row kernel can serve, which has no chained epilogue:
+            // its floats go to the next layer's packer, laid out as that layer reads them.
+            Plan alone = *plan[i];
+            float *out = dst;
+            if (emit) {
+                st = ensure_stage(ctx[i + 1], 0, dst_elems(alone) * sizeof(float));
+                if (st != xnor_nn_success) return st;
+                out = (float *)ctx[i + 1]->stage[0];
+                alone.dst_nhwc = plan[i + 1]->src_nhwc;
+            }
+            st = run_conv(alone, x, r, out, nullptr, true);
+            if (st != xnor_nn_success) return st;
+            if (emit)
+                CU(launch_binarize_data(*plan[i + 1], out, res[i + 1][xnor_nn_resource_bin_src],
+                                        (float *)res[i + 1][xnor_nn_resource_a], x->stream));
+            continue;
+        }
         if (emit) {
             const Plan &n = *plan[i + 1];
             next.bin_src = res[i + 1][xnor_nn_resource_bin_src];

@@ -201,6 +201,7 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
     if (f != kPopc && f != kTcgen05 && f != kTcgen05Rows) f = family_from_env();
     const bool frame = frame_walk_ok(*p), rows = image_rows_ok(*p);
     const bool fold = f == kAuto && fold_ok(*p);
+    p->frame_walk = frame;
     if (f == kAuto) f = (frame || rows || fold) ? kTcgen05 : kPopc;
     const bool force_rows = f == kTcgen05Rows;
     if (force_rows) f = rows ? kTcgen05 : kPopc;

@@ -90,6 +90,7 @@ struct Plan {
     // rows of one image (img_rows * ow <= 256 positions, rounded up to 16 for the instruction).
     // Tiles are dealt round-robin to one CTA per SM; the tiles of a last, partly filled round are
     // cut in two row halves so that they spread over twice as many SMs.
+    bool frame_walk;     // the position-tile kernel can serve the shape
     bool img;            // the forward pass launches the image-row kernel (else the position-tile one)
     bool img_forced;     // asked for by name, or the position-tile kernel cannot serve the shape
     int img_rows;        // output rows per tile
