@@ -137,6 +137,7 @@ def test_full_size_chain_conv3_conv4_matches_the_layers_run_separately():
     mid = torch.empty(mb * 384 * 169, device="cuda")
     want = torch.empty(mb * 256 * 169, device="cuda")
     convs[0].forward(src, mid)
+    convs[0].synchronize()  # the layers issue on streams of their own
     convs[1].forward(mid, want)
     convs[1].synchronize()
     sums_want = convs[1].forward_sums()
