@@ -1,5 +1,6 @@
 """Chains over layers that the position-tile kernel cannot serve (paddings that differ or are as
-large as the filter: the image-row kernel's). Reference: the oracle, layer by layer."""
+large as the filter: the image-row kernel's), and the order in which a chained layer sums |result|.
+Reference: the oracle, layer by layer."""
 import numpy as np
 import pytest
 
@@ -65,5 +66,24 @@ def test_chain_over_image_row_layers(oracle, name):
     a = convs[-1].read(xb.SLOT_A, np.float32)
     assert np.all(np.abs(a - want["a"]) <= A_REL_TOL * np.abs(want["a"]))
     assert np.all(np.abs(got - want["dst"]) <= REL_TOL * np.abs(want["dst"]))
+    for cv in convs:
+        cv.close()
+
+def test_same_image_gives_the_same_bits_anywhere_in_a_batch():
+    """256 filters (accumulators that overlap), three rounds of tiles per thread block: an image's
+    A, K and results do not depend on which round its positions fall into."""
+    torch = pytest.importorskip("torch")
+    mb = 256
+    layers = [_layer(mb, 64, 256, 13, 13, 3, 1, 1), _layer(mb, 256, 32, 13, 13, 3, 1, 1)]
+    convs, _, _ = _build(layers, 4000)
+    src = torch.from_numpy(synth.normal(5, 64 * 169)).cuda().repeat(mb)
+    dst = torch.empty(mb * 32 * 169, device="cuda")
+    torch.cuda.synchronize()
+    xb.forward_chain(convs, src, dst)
+    convs[0].synchronize()
+    for what in (convs[1].read(xb.SLOT_A, np.float32), convs[1].read(xb.SLOT_K, np.float32),
+                 dst.cpu().numpy()):
+        bits = what.view(np.uint32).reshape(mb, -1)
+        assert np.array_equal(bits, np.broadcast_to(bits[0], bits.shape))
     for cv in convs:
         cv.close()

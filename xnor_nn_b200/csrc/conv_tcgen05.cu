@@ -210,6 +210,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
     const int cgroup = ((warp - 2) >> 2) - team * cgroups;
     const int frame = g.hp * g.wp;
     const long ohw = (long)g.oh * g.ow;
+    const bool emits = !PAIR && g.emit_bin;  // chained layers do not run on pairs
     bool ok = true;   // false once a wait ran out somewhere in the CTA
     float run = 0.f;  // chained layers: running sum of |y| over the filter tiles of a pixel
     for (int it = team; it < rounds; it += g.teams) {
@@ -254,7 +255,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
             // Given up: touch nothing any more. The chained epilogue's warps of a quadrant meet
             // on a named barrier once per tile; a warp that has given up keeps that appointment
             // so that one that has not (yet) cannot be left waiting there.
-            if (g.emit_bin) {
+            if (emits) {
                 bar_sync(1 + quad, 32 * (kEpiWarps / 4));
                 continue;
             }
@@ -274,7 +275,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                 else mbar_arrive(shared_free0);
             }
         };
-        if (g.emit_bin) {
+        if (emits) {
             // Chained layers: y = (S * alpha) * K is not stored. alpha and K are never negative,
             // so the sign bit of y is the sign bit of S: it goes straight into the next layer's
             // frame (filters past the last one 0). |y| summed over the filters and divided by
@@ -287,12 +288,22 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                            oc0 / 2;
             const int room = g.e_icp - oc0 / 2;  // bytes of the row from here on
             float part = 0.f;
-            const int steps = (g.n_tile - 32 * cgroup + 32 * cgroups - 1) / (32 * cgroups);
-            for (int i = 0; i < steps; i++) {
-                const int c0 = 32 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
+            // The partial sum is added up in ascending order whichever accumulator the tile is in:
+            // shared columns at the end (the last 16 of 256) are fetched first and kept.
+            uint32_t kept[16];
+            if (reverse) {
+                ld16(taddr + (uint32_t)g.n_tile - 16u, kept);
+                wait_ld();
+                columns_read(0);
+            }
+            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups) {
                 uint32_t v[32];
                 const int width = g.n_tile - c0 >= 32 ? 32 : 16;
-                if (width == 32) {
+                if (reverse && c0 + 32 == g.n_tile) {
+                    ld16(taddr + (uint32_t)c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[16 + j] = kept[j];
+                } else if (width == 32) {
                     ld32(taddr + (uint32_t)c0, v);
                 } else {
 #pragma unroll
@@ -300,7 +311,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                     ld16(taddr + (uint32_t)c0, v);
                 }
                 wait_ld();
-                columns_read(i);
+                if (!reverse) columns_read(c0 == 32 * cgroup ? 0 : 1);
                 if (valid) {
                     const int lim = min(n_valid - c0, width);
                     uint32_t w[4];
