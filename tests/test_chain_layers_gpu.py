@@ -40,6 +40,12 @@ CHAINS = {
                           _layer(2, 40, 16, 7, 8, 3, 1, 1)],
     "all_uneven": [_layer(2, 20, 40, 9, 9, 3, 0, 1), _layer(2, 40, 260, 9, 9, 3, 0, 1),
                    _layer(2, 260, 24, 9, 9, 3, 0, 1)],
+    # a last layer asked onto the image-row kernel runs on position tiles in a chain: more tiles than
+    # SMs, rows of 32 and of 64 bytes
+    "last_asked_onto_rows_32": [_layer(2140, 24, 40, 2, 2, 3, 1, 1),
+                                _layer(2140, 40, 32, 2, 2, 3, 1, 1, kernel=xb.KERNEL_TCGEN05_I8_ROWS)],
+    "last_asked_onto_rows_64": [_layer(2140, 24, 100, 2, 2, 3, 1, 1),
+                                _layer(2140, 100, 32, 2, 2, 3, 1, 1, kernel=xb.KERNEL_TCGEN05_I8_ROWS)],
     # what a layer between two others was declared to store or to read does not matter in a chain
     "layouts_differ": [_layer(2, 20, 40, 9, 9, 3, 0, 1, dst=xb.NHWC),
                        _layer(2, 40, 48, 9, 9, 3, 0, 1, dst=xb.NCHW),

@@ -1145,12 +1145,16 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
     g.halo = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
-    bool halo = pair && g.tap_kw >= 2 && g.tap_kw <= 9 && g.issuers <= g.tap_kw;
+    // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
+    // (issue_probe checks that one). Narrower rows come with several taps a filter row when a layer
+    // that was asked onto the image-row kernel ends a chain; it takes the plain ring.
+    const bool row_offsets_ok = g.tap_kw == 1 || (g.tap_kw <= 9 && p.kchunk == 128);
+    bool halo = pair && g.tap_kw >= 2 && row_offsets_ok && g.issuers <= g.tap_kw;
     // Filters stay in shared memory if a pair works on several tiles of the same ones and their
     // operands leave room for three position tiles (kernel alone: conv2 mb128 48.8 -> 43.8 us, conv3
     // mb256 25.4 -> 23.0, conv1 mb64 26.1 -> 25.5; three is what conv2 needs the room for).
     const int groups = g.kh * g.chunks_per_tap;
-    if (same_nt && div_up_i(units, one_nt) > 1 && g.tap_kw <= 9) {
+    if (same_nt && div_up_i(units, one_nt) > 1 && row_offsets_ok) {
         const uint32_t rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
         const uint32_t a_slot = (rows * p.kchunk + 1023) & ~1023u, b_slot = (g.b_bytes + 1023u) & ~1023u;
         const size_t all_b = (size_t)groups * g.tap_kw * b_slot;
