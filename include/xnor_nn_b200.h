@@ -34,7 +34,7 @@ typedef enum {
                                                 serve go to the rows kernel, then to popc. */
     xnor_nn_b200_kernel_tcgen05_i8_rows = 3  /* tcgen05.mma kind::mxf4, tiles of 128 filters
                                                 x whole output rows of one image; unit stride,
-                                                rows of at most 240 pixels, any padding */
+                                                rows of at most 256 pixels, any padding */
 } xnor_nn_b200_kernel_t;
 
 /* xnor_nn_init_convolution (src/common_convolution.cpp:9-63) with the kernel family stated.

@@ -9,7 +9,7 @@
 // which is upstream's "skip the tap" (:71-72) and its op_c correction (:102) in one.
 //
 // A tile is 128 filters (UMMA M = the 128 lanes of tensor memory) by R whole output rows of one
-// image (UMMA N = R*OW rounded up to 16, at most 240). The activation operand of a filter tap is
+// image (UMMA N = R*OW rounded up to 16, at most 240; one row, at most 256). The activation operand of a filter tap is
 // then one 4-D TMA box {channels, OW columns, R rows, 1 image} of the packed tensor, shifted by
 // the tap; whatever lies outside the image is filled with zeros by the copy engine, so no
 // position is computed that is not an output pixel and no im2col buffer exists. For the 13x13
@@ -56,7 +56,10 @@ constexpr int kTeam = 2;            // epilogue warps per TMEM lane quadrant (th
 constexpr int kEpiWarps = 4 * kTeam;
 constexpr int kProducerW = 2 + kEpiWarps;  // the warp that loads the weight tiles
 constexpr int kThreads = 32 * (kProducerW + 1);
-constexpr uint32_t kTmemCols = 512;  // two accumulators of kImgColumns columns, block scales behind them
+// Two accumulators of kImgColumns columns and the block scales behind them; tiles of a row of more
+// pixels have one accumulator (n_acc), since two of 256 columns leave no room for the scales. Rows
+// of 254 pixels, 64 channels and filters, 8 images: 75 us a pass, 129 on the popcount kernel.
+constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kScaleCol = 2 * kImgColumns;
 constexpr int kMaxStages = 8;
 constexpr int kControlBytes = 2304;
@@ -81,6 +84,7 @@ struct ImgArgs {
     int kk_last;       // MMAs of a tap's last channel chunk: its 64-channel slices that hold channels
     uint32_t idesc_full, idesc_half;
     int n_full, n_half;
+    int n_acc;         // accumulators: 2, or 1
     uint32_t desc_hi;  // upper 32 bits of the shared-memory matrix descriptors
     uint32_t a_bytes, stage_bytes, tx_full, tx_half;
     int stages;
@@ -100,7 +104,7 @@ struct __align__(16) Control {
     unsigned long long drain;
     uint32_t tmem_base;
     int abort_flag;
-    float kk[2][256];  // K of the tile's pixels, per accumulator
+    float kk[2][256];  // K of the tile's pixels, for tiles in turn
 };
 static_assert(sizeof(Control) <= kControlBytes, "control block");
 
@@ -292,8 +296,8 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
             for (int it = 0; ok && it < rounds; it++) {
                 const int unit = (int)blockIdx.x + it * (int)gridDim.x;
                 const uint32_t idesc = unit >= g.whole ? g.idesc_half : g.idesc_full;
-                const int b = it & 1;
-                const uint32_t acc_phase = (it >> 1) & 1;
+                const int b = g.n_acc == 2 ? it & 1 : 0;
+                const uint32_t acc_phase = (g.n_acc == 2 ? it >> 1 : it) & 1;
                 ok = mbar_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2,
                                g.wait_ns);
                 if (!ok) break;
@@ -353,8 +357,8 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
         bool live = true;  // false once something gave up: keep the barriers, touch nothing
         for (int it = 0; it < rounds; it++) {
             const Tile t = tile_of(g, (int)blockIdx.x + it * (int)gridDim.x);
-            const int b = it & 1;
-            const uint32_t acc_phase = (it >> 1) & 1;
+            const int b = g.n_acc == 2 ? it & 1 : 0;
+            const uint32_t acc_phase = (g.n_acc == 2 ? it >> 1 : it) & 1;
             const int n_cols = t.half >= 0 ? g.n_half : g.n_full;
             const int rows_in = min(t.rows, g.oh - t.r0);
             const int len = rows_in > 0 ? rows_in * g.ow : 0;  // output pixels of the tile
@@ -369,7 +373,7 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                         kk = box_k(g, t.n, t.r0 + r, p - r * g.ow);
                         if (g.kmap_out && t.mt == 0) g.kmap_out[pix0 + p] = kk;
                     }
-                    ctl->kk[b][p] = kk;
+                    ctl->kk[it & 1][p] = kk;
                 }
             }
             bar_sync(1, 32 * kEpiWarps);
@@ -398,7 +402,7 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kImgColumns);
             if (live) {
                 fence_after();
-                const float *kk = ctl->kk[b];
+                const float *kk = ctl->kk[it & 1];
                 uint32_t *const srow = srow_of_lane;
                 for (int c0 = 32 * cg; c0 < n_cols; c0 += 32 * kTeam) {
                     uint32_t v[32];
@@ -536,6 +540,7 @@ cudaError_t launch_conv_tcgen05_img(const Plan &p, const void *bin_src, const vo
     g.kk_last = (p.ic - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     g.n_full = p.img_n;
     g.n_half = p.img_n_half ? p.img_n_half : p.img_n;
+    g.n_acc = p.img_n > kImgColumns ? 1 : 2;
     g.idesc_full = mxf4_idesc(kFilters, (uint32_t)g.n_full);
     g.idesc_half = mxf4_idesc(kFilters, (uint32_t)g.n_half);
     // matrix descriptor, upper half: stride between 8-row groups (8 * kchunk bytes, in 16-byte

@@ -83,8 +83,8 @@ static bool frame_walk_ok(const Plan &p) {
 
 // The image-row kernel addresses the frame as a 4-D tensor (channel, column, row, image) and lets
 // the copy engine fill whatever lies outside with zeros, so any padding and any output extent
-// work; a tile must hold at least one whole output row (an accumulator has kImgColumns columns).
-static bool image_rows_ok(const Plan &p) { return unit_stride(p) && p.ow <= kImgColumns; }
+// work; a tile must hold at least one whole output row.
+static bool image_rows_ok(const Plan &p) { return unit_stride(p) && p.ow <= kImgWideColumns; }
 
 // Relative duration of a tile whose UMMA N is n: an instruction occupies the tensor pipe for n/2
 // cycles, but the issuing thread needs about 45 cycles per tcgen05.mma and 275 per
@@ -111,7 +111,7 @@ void plan_image_rows(Plan *p) {
     const int m_blocks = div_up_i(p->oc, 128);
     long best = -1;
     int best_r = 0;
-    for (int r = 1; r <= p->oh && r * p->ow <= kImgColumns; r++) {
+    for (int r = 1; r <= p->oh && (r == 1 || r * p->ow <= kImgColumns); r++) {
         const int n = div_up_i(r * p->ow, 16) * 16;
         const long tiles = (long)p->mb * div_up_i(p->oh, r) * m_blocks;
         const long rem = tiles % sms;

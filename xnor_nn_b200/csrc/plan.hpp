@@ -21,8 +21,10 @@ enum Family : int {
 };
 
 // Accumulator columns of the image-row kernel: two of them and 32 columns of block scales fill
-// the 512 columns of tensor memory.
+// the 512 columns of tensor memory. Rows of more pixels, up to kImgWideColumns, have a single
+// accumulator, which the next tile waits for.
 constexpr int kImgColumns = 240;
+constexpr int kImgWideColumns = 256;
 
 struct Plan {
     // geometry (copied from the descriptor so kernels never chase the caller's struct)
@@ -87,7 +89,8 @@ struct Plan {
 
     // ---- tiling of the image-row kernel (kTcgen05, conv_tcgen05_img.cu) ---------------------
     // That kernel puts 128 filters on the UMMA M side and, on the N side, `img_rows` whole output
-    // rows of one image (img_rows * ow <= 256 positions, rounded up to 16 for the instruction).
+    // rows of one image (img_rows * ow <= 240 positions, or one row of up to 256, rounded up to 16
+    // for the instruction).
     // Tiles are dealt round-robin to one CTA per SM; the tiles of a last, partly filled round are
     // cut in two row halves so that they spread over twice as many SMs.
     bool frame_walk;     // the position-tile kernel can serve the shape
