@@ -33,6 +33,9 @@ FOLDED = [
     _c("two_channels_one_word_a_row", 3, 24, 2, 31, 70, 7, 7, sh=2, sw=2, ph=3, pw=3),
     _c("four_channels_two_words_a_row", 3, 24, 4, 33, 34, 10, 10, sh=3, sw=2, ph=9, pw=9),
     _c("three_channels_three_words_a_row", 2, 24, 3, 40, 71, 18, 18, sh=5, sw=5, ph=2, pw=2),
+    # seven channels: rows of 1000 values, and the largest stage there is (48048 bytes of bits)
+    _c("seven_channels_wide", 1, 8, 7, 17, 1000, 8, 8, sh=8, sw=8),
+    _c("seven_channels_wide_border", 1, 8, 7, 11, 1117, 11, 11, sh=11, sw=11, ph=1900, pw=1900),
     _c("channels_last", 3, 40, 37, 16, 17, 3, 3, sh=2, sw=2, ph=1, pw=1, fmt=(1, 1, 1)),
     _c("channels_last_conv1", 2, 36, 3, 47, 51, 11, 11, sh=4, sw=4, fmt=(1, 1, 0)),
     _c("many_tiles", 70, 48, 3, 61, 61, 3, 3, sh=2, sw=2, ph=1, pw=1),

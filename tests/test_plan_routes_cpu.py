@@ -50,3 +50,13 @@ def test_rows_that_only_the_image_row_kernel_serves(ow):
 def test_rows_beyond_an_accumulator_run_on_popc():
     assert _kernel(2, 24, 20, 9, 253, 3, 3, ph=3, pw=3) == xb.KERNEL_POPC
     assert _kernel(2, 24, 20, 9, 257, 3, 3, ph=1, pw=1) == xb.KERNEL_TCGEN05_I8
+
+
+def test_strided_layers_of_few_channels_fold_while_their_bits_fit():
+    """The packer stages a bit per value, in 48 KB. Borders count in a row's pitch even where a wide
+    stride skips most of them."""
+    assert _kernel(1, 8, 7, 16, 1000, 8, 8, sh=8, sw=8) == xb.KERNEL_TCGEN05_I8
+    assert _kernel(1, 8, 7, 11, 1117, 11, 11, sh=11, sw=11, ph=1900, pw=1900) == xb.KERNEL_TCGEN05_I8
+    assert _kernel(1, 8, 7, 11, 1117, 11, 11, sh=11, sw=11, ph=2000, pw=2000) == xb.KERNEL_POPC
+    # one output column: it reads 11 columns, 4000 columns of border in front of it
+    assert _kernel(1, 8, 7, 11, 1100, 11, 11, sh=11, sw=9400, ph=4, pw=4100) == xb.KERNEL_POPC

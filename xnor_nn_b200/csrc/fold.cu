@@ -268,12 +268,10 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
     g.px_stride = p.src_nhwc ? p.ic : 1;
     g.inv_ic = p.inv_ic;
     g.by_iw = FastDiv((uint32_t)p.iw);
-    // few channels: the word after the one that a row's last eight columns start in is read too
     g.chunks = div_up_i(p.iw + p.pw, 32);
     g.by_chunks = FastDiv((uint32_t)g.chunks);
-    const int bit_words = p.fold_span / 32 + 3;
     const bool two = few && p.fold_field == 16;
-    g.pitch = !few ? p.fold_span : bit_words > g.chunks ? bit_words : g.chunks;
+    g.pitch = few ? fold_bit_pitch(p) : p.fold_span;
     const int n8 = div_up_i(p.fold_channels, 8);
     g.nw = few ? p.ic * p.fold_rows * (two ? 1 : p.fold_field / 8) : p.fold_rows * p.kw * n8;
     g.by_nw = FastDiv((uint32_t)g.nw);
@@ -287,7 +285,7 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
     int dev = 0;
     cudaGetDevice(&dev);
     std::atomic<bool> &done = opted_in[dev & 63][a ? 1 : 0];
-    // few channels: bits take less shared memory than the 48 KB that need no opt-in (fold_ok)
+    // few channels: the bits fit the 48 KB that need no opt-in (fold_ok)
     if (!few && !done.load(std::memory_order_acquire)) {
         const cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);

@@ -52,9 +52,17 @@ static bool unit_stride(const Plan &p) {
            (long)p.mb * (p.ih + p.ph) * (p.iw + p.pw) < (1L << 30) && sums_exact(p);
 }
 
-// A strided layer is folded when its packer's working set (a row block of some channels, a byte
-// per value, and the mean-|x| sums of the block's pixels) fits shared memory. The popcount kernel
-// it would otherwise run on needs 870 us for AlexNet conv1 on 64 images.
+int fold_bit_pitch(const Plan &p) {
+    // the word after the one that a row's last eight columns start in is read too
+    const long span = ((long)(p.ow - 1) * p.sw + p.kw) / 32 + 3, row = ((long)p.iw + p.pw + 31) / 32;
+    const long pitch = span > row ? span : row;
+    return pitch < (1L << 30) ? (int)pitch : 1 << 30;
+}
+
+// A strided layer is folded when its packer's working set (a row block of some channels, a bit per
+// value with fewer than eight of them, else half a byte, and the mean-|x| sums of the block's
+// pixels) fits shared memory. The popcount kernel it would otherwise run on needs 870 us for
+// AlexNet conv1 on 64 images.
 constexpr long kFoldStage = 48 * 1024, kFoldSums = 48 * 1024, kFoldWords = 4096;
 static bool fold_ok(const Plan &p) {
     if ((p.sh == 1 && p.sw == 1) || p.sh < 1 || p.sw < 1 || p.oh < 1 || p.ow < 1 || p.mb < 1)
@@ -62,8 +70,8 @@ static bool fold_ok(const Plan &p) {
     const int rows = p.kh < p.sh ? p.kh : p.sh, taps = div_up_i(p.kh, p.sh);
     const long span = (long)(p.ow - 1) * p.sw + p.kw;
     // bytes staged at least, and words of a column they become: all of fewer than eight channels
-    // as bytes, or eight channels as nibbles
-    const long least = p.ic < 8 ? p.ic * rows * (span + 16) : 4 * rows * span;
+    // as bits, or eight channels as nibbles
+    const long least = p.ic < 8 ? 4L * p.ic * rows * fold_bit_pitch(p) : 4 * rows * span;
     const long words = p.ic < 8 ? (long)p.ic * rows * div_up_i(p.kw, 8) : (long)rows * p.kw;
     return sums_exact(p) && least <= kFoldStage && 4L * p.sh * p.iw <= kFoldSums &&
            words <= kFoldWords && (long)p.mb * (p.oh + taps - 1) * p.ow < (1L << 30) &&
