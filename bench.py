@@ -88,7 +88,8 @@ def binary_ops(L, mb):
 
 def pipe_probe():
     """Live ceilings of the candidate instruction paths (xnor_nn_b200/pipe_probe, built with the
-    library): binary TOPS of the LOP3+POPC tile, of mma.sync b1 and of tcgen05.mma kind::i8."""
+    library): binary TOPS of the LOP3+POPC tile, of mma.sync b1 and of tcgen05.mma kind::i8 and
+    kind::mxf4."""
     exe = os.path.join(ROOT, "xnor_nn_b200", "pipe_probe")
     if not os.path.exists(exe):
         return None
@@ -499,21 +500,21 @@ def measure_layer(xb, torch, args, cfg_name, kernel, rank, world, dist, probe, b
         dist.all_gather_object(names, lay.kernel_name)
         lay.kernel_name = next(n for n in names if n)
     n_src_max = lay.n_src if mb == mb_max else mb_max * L.ic * L.ih * L.iw
-    # compulsory bytes of the packing pass: 4 B per source element in, 1 B (tensor-core family)
-    # or 1 bit (integer-pipe family) per element out, plus the mean-|x| map
+    # compulsory bytes of the packing pass: 4 B per source element in, half a byte (tensor-core
+    # family) or 1 bit (integer-pipe family) per element out, plus the mean-|x| map
     tc = (lay.kernel_name or "tcgen05").startswith("tcgen05")
-    bin_bytes = 4.0 * n_src_max + (n_src_max if tc else n_src_max / 8.0) + 4.0 * mb_max * L.ih * L.iw
+    bin_bytes = 4.0 * n_src_max + n_src_max / (2.0 if tc else 8.0) + 4.0 * mb_max * L.ih * L.iw
     pk, pk_kind = peaks()
     conv_tops = binary_ops(L, mb_max) / (conv_ms * 1e-3) / 1e12
     if tc:
-        peak = probe.get("tcgen05_i8_tops") if probe else None
-        peak_note = "tcgen05.mma kind::i8 ceiling measured in this run (pipe_probe)"
+        peak = probe.get("tcgen05_mxf4_tops") if probe else None
+        peak_note = "tcgen05.mma kind::mxf4 ceiling measured in this run (pipe_probe)"
         bound = "tensor"
     else:
         peak = probe.get("popc_binary_tops") if probe else None
         peak_note = "LOP3+POPC ceiling measured in this run (pipe_probe)"
         bound = "int_pipe"
-    alt_peak = 2.0 * pk["bf16_tflops"] if tc else None
+    alt_peak = 4.0 * pk["bf16_tflops"] if tc else None  # dense 4-bit floats: four times bf16
     traffic = captured_traffic(cfg_name, lay.kernel_name) if world == 1 else None
     roofline = {"kernel": "conv_" + lay.kernel_name, "bound": bound, "achieved": conv_tops,
                 "peak": peak, "unit": "TFLOP/s", "frac": (conv_tops / peak) if peak else None,
@@ -522,7 +523,7 @@ def measure_layer(xb, torch, args, cfg_name, kernel, rank, world, dist, probe, b
                 "peak_source": peak_note, "ms": conv_ms,
                 "timing": "launches issued back to back on one stream, CUDA events around the "
                           "sequence, milliseconds per launch (includes what lies between launches)",
-                "frac_of_2x_bf16_%s" % pk_kind: (conv_tops / alt_peak) if alt_peak else None,
+                "frac_of_4x_bf16_%s" % pk_kind: (conv_tops / alt_peak) if alt_peak else None,
                 "binarize": {"kernel": "sign-pack with the mean-|x| map (the pass the step runs)",
                              "bound": "hbm", "achieved": bin_bytes / (bin_ms * 1e-3) / 1e9,
                              "peak": pk["hbm_gbs"], "unit": "GB/s",
@@ -577,7 +578,7 @@ def measure_layer(xb, torch, args, cfg_name, kernel, rank, world, dist, probe, b
         "ms_per_step_min": float(np.min(regions)), "ms_per_step_max": float(np.max(regions)),
         "timed_regions": len(regions), "timed_ms": total,
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "s8" if tc else "u32", "data": "synthetic",
+        "dtype": "e2m1" if tc else "u32", "data": "synthetic",
         "config": {"workload": L.name, "minibatch": L.mb, "images_per_gpu": mb_max,
                    "kernel": lay.kernel_name, "parallelism": "minibatch slices x%d" % world,
                    "l2": ("inputs larger than L2: %d rotating tensor sets of %.1f MB"

@@ -66,7 +66,7 @@ def build(force=False, verbose=False):
                                "-o", LIB] + objs
         subprocess.check_call(cmd)
     # The pipe-rate probe is a stand-alone program (measured ceilings for the benchmark).
-    if force or _stale(PROBE, [PROBE_SRC, os.path.abspath(__file__)]):
+    if force or _stale(PROBE, [PROBE_SRC, os.path.join(CSRC, "tc_ptx.cuh"), os.path.abspath(__file__)]):
         subprocess.check_call([NVCC] + ARCH + ["-O3", "-std=c++17", "-lineinfo", "-ccbin",
                                                "/usr/bin/g++", "-o", PROBE, PROBE_SRC])
     # ... and so is the probe of instruction issue costs (profiles/ quotes its output).

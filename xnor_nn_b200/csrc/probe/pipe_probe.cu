@@ -1,17 +1,22 @@
 // Pipe-rate probe: the measured ceilings the convolution kernels are judged against.
 //
-// Runs register- and shared-memory-resident loops (no global traffic) of the three candidate
+// Runs register- and shared-memory-resident loops (no global traffic) of the four candidate
 // formulations of the bit contraction and prints one JSON object with binary TOPS
 // (2 ops per bit pair):
 //   popc        LOP3 + POPC + IADD in the 4x8 register tile of the integer-pipe kernel
 //   mma_b1      mma.sync.m16n8k256 xor.popc, the legacy binary tensor path
-//   tcgen05_i8  tcgen05.mma.kind::i8 M=128 N=256 K=32 on +-1 bytes, issued by one thread per SM
-//               with a commit every four instructions, as the convolution's issue loop does
+//   tcgen05_mxf4  tcgen05.mma.kind::mxf4 M=128 N=256 K=64 on 4-bit floats, issued by one thread per
+//               SM with a commit every four instructions: what the convolution runs on
+//   tcgen05_i8  the same with kind::i8, K=32, on bytes: half the rate on twice the operand bytes
 // Every wait is bounded; on a timeout the status field says so.
 #include <cstdint>
 #include <cstdio>
 
 #include <cuda_runtime.h>
+
+#include "../tc_ptx.cuh"
+
+using namespace xb200::tc;
 
 namespace {
 
@@ -58,72 +63,58 @@ __global__ void mma_b1(int *out, const uint32_t *in, int iters) {
     out[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok;
-}
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
+// MMAs of one kind into one accumulator of 256 columns. The block scales of the 4-bit kind sit in
+// the last 16 columns of tensor memory, as in the convolution.
+constexpr uint32_t kScaleCol = 496;
 
-__global__ void __launch_bounds__(128, 1) tcgen05_i8(int iters, int *err) {
+template <bool MXF4>
+__global__ void __launch_bounds__(128, 1) tcgen05_rate(int iters, int *err) {
     extern __shared__ uint8_t raw[];
     uint8_t *base = (uint8_t *)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
     __shared__ unsigned long long done, sink;
     __shared__ uint32_t tbase;
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sink)) : "memory");
+        mbar_init(smem_u32(&done), 1);
+        mbar_init(smem_u32(&sink), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tbase)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (warp == 0) tmem_alloc(smem_u32(&tbase), 512);
+    fence_before();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    fence_after();
     const uint32_t tm = tbase;
+    if (MXF4) fill_scales(tm + ((uint32_t)(warp * 32) << 16) + kScaleCol, 16);
+    fence_before();
+    __syncthreads();
+    fence_after();
     if (threadIdx.x == 0) {
         // K-major 128-byte-swizzled tiles: A 128 x 128 B at base, B 256 x 128 B behind it
         const uint32_t sa = smem_u32(base), sb = sa + 16384;
         const uint64_t hi = (uint64_t)(64u | (1u << 14) | (2u << 29)) << 32;
         const uint64_t ad = hi | (uint64_t)(((sa >> 4) & 0x3FFF) | (1u << 16));
         const uint64_t bd = hi | (uint64_t)(((sb >> 4) & 0x3FFF) | (1u << 16));
-        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (32u << 17) | (8u << 24);
+        const uint32_t idesc =
+            MXF4 ? mxf4_idesc(128, 256)
+                 : (2u << 4) | (1u << 7) | (1u << 10) | (32u << 17) | (8u << 24);
         for (int i = 0; i < iters; i += 4) {
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                    ::"r"(tm), "l"(ad + 2 * k), "l"(bd + 2 * k), "r"(idesc), "r"(1u) : "memory");
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(smem_u32(&sink)) : "memory");
+            for (int k = 0; k < 4; k++) {
+                if (MXF4) mma_mxf4<false>(tm, ad + 2 * k, bd + 2 * k, idesc, tm + kScaleCol, 1u);
+                else mma_i8(tm, ad + 2 * k, bd + 2 * k, idesc, 1u);
+            }
+            commit(smem_u32(&sink));
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                     ::"r"(smem_u32(&done)) : "memory");
+        commit(smem_u32(&done));
         const unsigned long long t0 = global_ns();
-        while (!try_wait(smem_u32(&done), 0))
+        while (!mbar_try_wait(smem_u32(&done), 0))
             if (global_ns() - t0 > 2000000000ull) { *err = 1; break; }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    fence_before();
     __syncthreads();
     if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(512u)
-                     : "memory");
+        fence_after();
+        tmem_free(tm, 512);
     }
 }
 
@@ -171,17 +162,20 @@ int main() {
     const double b1_tops = (double)blocks * (threads / 32) * (iters / 4) * 8 * (2.0 * 16 * 8 * 256) /
                            (ms * 1e-3) / 1e12;
 
-    cudaFuncSetAttribute(tcgen05_i8, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(tcgen05_rate<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(tcgen05_rate<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     const int mmas = 8192;
-    ms = best_ms([&] { tcgen05_i8<<<sms, 128, 130 * 1024>>>(mmas, err); });
+    ms = best_ms([&] { tcgen05_rate<false><<<sms, 128, 130 * 1024>>>(mmas, err); });
     const double i8_tops = (double)sms * mmas * 2.0 * 128 * 256 * 32 / (ms * 1e-3) / 1e12;
+    ms = best_ms([&] { tcgen05_rate<true><<<sms, 128, 130 * 1024>>>(mmas, err); });
+    const double mxf4_tops = (double)sms * mmas * 2.0 * 128 * 256 * 64 / (ms * 1e-3) / 1e12;
 
     int timed_out = 0;
     cudaMemcpy(&timed_out, err, 4, cudaMemcpyDeviceToHost);
     const cudaError_t e = cudaDeviceSynchronize();
     printf("{\"popc_binary_tops\": %.1f, \"mma_b1_binary_tops\": %.1f, \"tcgen05_i8_tops\": %.1f, "
-           "\"sms\": %d, \"status\": \"%s\"}\n",
-           popc_tops, b1_tops, i8_tops, sms,
+           "\"tcgen05_mxf4_tops\": %.1f, \"sms\": %d, \"status\": \"%s\"}\n",
+           popc_tops, b1_tops, i8_tops, mxf4_tops, sms,
            e != cudaSuccess ? cudaGetErrorString(e) : (timed_out ? "tcgen05 wait timed out" : "ok"));
     return e != cudaSuccess || timed_out;
 }
