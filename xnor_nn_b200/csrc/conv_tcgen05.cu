@@ -478,6 +478,70 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
     }
 }
 
+// ---- TMA producer role: position and filter tiles of a step in one ring buffer ---------------------
+template <bool PAIR>
+__device__ __forceinline__ void producer_ring(const TcArgs &g, Control *ctl,
+                                              const CUtensorMap *map_a, const CUtensorMap *map_b,
+                                              uint32_t stage0, uint32_t rank) {
+    volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
+    const Deal<PAIR> deal(g);
+    const int rounds = deal.rounds(g), ksteps = g.taps * g.chunks_per_tap;
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t armed = 0;  // bit s: stage s holds a load nobody is known to have consumed
+    uint32_t armed_parity = 0;
+    bool ok = true;
+    // a pair counts both CTAs' bytes on the leader's barrier
+    const uint32_t full_local = smem_u32(&ctl->full[0]);
+    const uint32_t full0 = PAIR && rank != 0 ? mapa(full_local, 0) : full_local;
+    const int b_rows = PAIR ? g.n_tile >> 1 : g.n_tile;  // filter rows this CTA loads
+    for (int it = 0; ok && it < rounds; it++) {
+        int mt, nt;
+        deal.at(g, it, mt, nt);
+        int row = g.lead + mt * BM - g.ph * g.wp - g.pw;  // tap (0,0)
+        int brow = nt * g.n_tile + (int)rank * b_rows;
+        int kw = 0, chunk = 0;
+        for (int ks = 0; ks < ksteps; ks++) {
+            const uint32_t ebar = smem_u32(&ctl->empty[stage]);
+            ok = warp_wait(ebar, phase ^ 1, abort_flag, g.error, 1, g.wait_ns);
+            if (!ok) break;
+            armed &= ~(1u << stage);
+            const uint32_t bar = full0 + 8u * (uint32_t)stage;
+            const uint32_t sa = stage0 + (uint32_t)stage * g.stage_bytes;
+            if (leader && PAIR) {
+                if (rank == 0) mbar_expect_tx(bar, 2u * g.tx_bytes);  // bar is local here
+                tma_load_2d_pair(sa, map_a, chunk * g.kchunk, row, bar);
+                tma_load_2d_pair(sa + g.a_bytes, map_b, chunk * g.kchunk, brow, bar);
+            } else if (leader) {
+                mbar_expect_tx(bar, g.tx_bytes);
+                tma_load_2d(sa, map_a, chunk * g.kchunk, row, bar);
+                tma_load_2d(sa + g.a_bytes, map_b, chunk * g.kchunk, brow, bar);
+            }
+            armed |= 1u << stage;
+            armed_parity = (armed_parity & ~(1u << stage)) | (phase << stage);
+            if (++stage == g.n_stages) { stage = 0; phase ^= 1; }
+            if (++chunk == g.chunks_per_tap) {  // next filter tap
+                chunk = 0;
+                brow += g.ocp16;
+                if (++kw == g.tap_kw) { kw = 0; row += g.wp - (g.tap_kw - 1); }
+                else row += 1;
+            }
+        }
+    }
+    if (!ok && rank == 0) {
+        // Something gave up. Loads already issued still land in this CTA's shared
+        // memory: wait for them (bounded) before the CTA may exit. (The partner of a
+        // pair cannot wait on the leader's barrier; it stays until the leader has got
+        // through this and both have met at the cluster barrier at the end.)
+        for (int s = 0; s < g.n_stages; s++)
+            if (armed & (1u << s)) {
+                mbar_wait_quiet(smem_u32(&ctl->full[s]), (armed_parity >> s) & 1u,
+                                g.wait_ns);
+            }
+    }
+}
+
 // ---- MMA issuer role -----------------------------------------------------------------------------
 // One thread feeds the tensor pipe; the instructions of a pipeline stage (KK tcgen05.mma and the
 // tcgen05.commit that hands the stage back) cost that thread more cycles than the pipe needs for
@@ -580,28 +644,26 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
     }
 }
 
-// ---- halo mode: producer and MMA issuers -----------------------------------------------------------
+// ---- halo mode (pairs only): producer and MMA issuers ----------------------------------------------
 // Step order inside a tile: filter row kh, channel chunk, filter column kw (the sums are integers:
 // any order gives the same result). A group = the kw steps of one (kh, chunk): one halo tile of
 // g.halo positions in slot G % n_a_slots (G counts groups across tiles), kw filter tiles in
 // consecutive slots of the filter ring. A descriptor that starts r rows into a 128-byte-swizzled
 // tile reads rows r .. r + 127 of it (the swizzle is a function of the shared-memory address), so
 // tap kw of the group is the halo tile's descriptor advanced by kw rows.
-template <bool PAIR>
 __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                                               const CUtensorMap *map_a, const CUtensorMap *map_b,
                                               uint32_t stage0, uint32_t rank) {
     volatile int *abort_flag = &ctl->abort_flag;
     const bool leader = elect_one();
-    const Deal<PAIR> deal(g);
+    const Deal<true> deal(g);
     const int rounds = deal.rounds(g);
     const uint32_t full_l = smem_u32(&ctl->full[0]), afull_l = smem_u32(&ctl->a_full[0]);
     // a pair counts both CTAs' bytes on the leader's barriers
-    const uint32_t full0 = PAIR && rank != 0 ? mapa(full_l, 0) : full_l;
-    const uint32_t afull0 = PAIR && rank != 0 ? mapa(afull_l, 0) : afull_l;
+    const uint32_t full0 = rank != 0 ? mapa(full_l, 0) : full_l;
+    const uint32_t afull0 = rank != 0 ? mapa(afull_l, 0) : afull_l;
     const uint32_t empty0 = smem_u32(&ctl->empty[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
-    const int b_rows = PAIR ? g.n_tile >> 1 : g.n_tile;
-    const uint32_t mult = PAIR ? 2u : 1u;
+    const int b_rows = g.n_tile >> 1;
     const uint32_t a_bytes = (uint32_t)g.halo * (uint32_t)g.kchunk;
     int sb = 0, sa = 0;
     uint32_t pb = 0, pa = 0;
@@ -622,11 +684,10 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                 // resident filters travel with the first round's position tiles
                 const bool with_b = g.resident && it == 0;
                 const uint32_t bytes =
-                    mult * (a_bytes + (with_b ? (uint32_t)g.tap_kw * g.b_bytes : 0u));
+                    2u * (a_bytes + (with_b ? (uint32_t)g.tap_kw * g.b_bytes : 0u));
                 if (leader) {
-                    if (!PAIR || rank == 0) mbar_expect_tx(abar, bytes);  // abar is local here
-                    if (PAIR) tma_load_2d_pair(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
-                    else tma_load_2d(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
+                    if (rank == 0) mbar_expect_tx(abar, bytes);  // abar is local here
+                    tma_load_2d_pair(adst, map_a, chunk * g.kchunk, row0 + kh * g.wp, abar);
                 }
                 armed_a |= 1u << sa;
                 parity_a = (parity_a & ~(1u << sa)) | (pa << sa);
@@ -638,8 +699,7 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                                         (uint32_t)((kh * g.chunks_per_tap + chunk) * g.tap_kw) *
                                             g.b_slot_bytes;
                         for (int kw = 0; kw < g.tap_kw; kw++) {
-                            if (PAIR) tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, abar);
-                            else tma_load_2d(bdst, map_b, chunk * g.kchunk, brow, abar);
+                            tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, abar);
                             brow += g.ocp16;
                             bdst += g.b_slot_bytes;
                         }
@@ -654,9 +714,8 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                     const uint32_t bar = full0 + 8u * (uint32_t)sb;
                     const uint32_t bdst = stage0 + g.b_ring_off + (uint32_t)sb * g.b_slot_bytes;
                     if (leader) {
-                        if (!PAIR || rank == 0) mbar_expect_tx(bar, mult * g.b_bytes);
-                        if (PAIR) tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, bar);
-                        else tma_load_2d(bdst, map_b, chunk * g.kchunk, brow, bar);
+                        if (rank == 0) mbar_expect_tx(bar, 2u * g.b_bytes);
+                        tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, bar);
                     }
                     armed_b |= 1u << sb;
                     parity_b = (parity_b & ~(1u << sb)) | (pb << sb);
@@ -677,12 +736,12 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
     }
 }
 
-template <int KK, bool PAIR>
+template <int KK>
 __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                               uint32_t stage0, int who) {
     volatile int *abort_flag = &ctl->abort_flag;
     const bool leader = elect_one();
-    const int rounds = Deal<PAIR>(g).rounds(g);
+    const int rounds = Deal<true>(g).rounds(g);
     if (rounds == 0) return;
     const int ksteps = g.taps * g.chunks_per_tap;  // >= g.issuers; a multiple of g.tap_kw
     const int n_iss = g.issuers, kwn = g.tap_kw;
@@ -737,15 +796,13 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
 #pragma unroll
             for (int k = 0; k < KK; k++) {
                 if (k < kk) {
-                    mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
+                    mma_mxf4<true>(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
                                    g.idesc, tmem_base + kScaleCol, (k == 0 && ks == 0) ? 0u : 1u);
                 }
             }
-            if (PAIR) commit_pair(empty0 + 8u * (uint32_t)sb);
-            else commit(empty0 + 8u * (uint32_t)sb);
+            commit_pair(empty0 + 8u * (uint32_t)sb);
             if (n_iss > 1 && ks == 0) {
-                if (PAIR) commit_pair(smem_u32(&ctl->started[b]));
-                else commit(smem_u32(&ctl->started[b]));
+                commit_pair(smem_u32(&ctl->started[b]));
             }
         }
         __syncwarp();
@@ -756,8 +813,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
             // this thread's last step of the group is issued: its reads of the halo tile are
             // covered by this commit (both issuers commit: the barrier counts them)
             if (leader) {
-                if (PAIR) commit_pair(aempty0 + 8u * (uint32_t)sa);
-                else commit(aempty0 + 8u * (uint32_t)sa);
+                commit_pair(aempty0 + 8u * (uint32_t)sa);
             }
             do {
                 kw -= kwn;
@@ -770,8 +826,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
         if (ks >= ksteps) {  // this thread's share of the tile is issued
             ks -= ksteps;
             if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
-                if (PAIR) commit_pair(smem_u32(&ctl->acc_full[b]));
-                else commit(smem_u32(&ctl->acc_full[b]));
+                commit_pair(smem_u32(&ctl->acc_full[b]));
             }
             entered = false;
             if (++it >= rounds) break;
@@ -780,8 +835,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     }
     if (!ok) {
         if (leader) {
-            if (PAIR) commit_pair(smem_u32(&ctl->drain[who]));
-            else commit(smem_u32(&ctl->drain[who]));
+            commit_pair(smem_u32(&ctl->drain[who]));
         }
         mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
     }
@@ -791,12 +845,12 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
 // row on one channel chunk) is one wait, kw * KK MMAs and one commit, which one issuer keeps up
 // with. With the filters streamed a pair moved 320 KB per CTA and tile of AlexNet conv2 through L2,
 // which took 11400 cycles under the result stores of another tile (tensor pipe: 5100).
-template <int KK, bool PAIR>
+template <int KK>
 __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                                   uint32_t stage0) {
     volatile int *abort_flag = &ctl->abort_flag;
     const bool leader = elect_one();
-    const int rounds = Deal<PAIR>(g).rounds(g);
+    const int rounds = Deal<true>(g).rounds(g);
     if (rounds == 0) return;
     const int groups = g.kh * g.chunks_per_tap;
     const uint64_t hi = (uint64_t)g.desc_hi << 32;
@@ -827,14 +881,13 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
 #pragma unroll
                     for (int k = 0; k < KK; k++) {
                         if (k < kk) {
-                            mma_mxf4<PAIR>(d_tmem, adesc + (uint64_t)(2 * k),
+                            mma_mxf4<true>(d_tmem, adesc + (uint64_t)(2 * k),
                                            bdesc + (uint64_t)(2 * k), g.idesc,
                                            tmem_base + kScaleCol, (gr | kw | k) == 0 ? 0u : 1u);
                         }
                     }
                 }
-                if (PAIR) commit_pair(aempty0 + 8u * (uint32_t)sa);
-                else commit(aempty0 + 8u * (uint32_t)sa);
+                commit_pair(aempty0 + 8u * (uint32_t)sa);
             }
             __syncwarp();
             if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
@@ -842,16 +895,14 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
         }
         if (!ok) break;
         if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
-            if (PAIR) commit_pair(smem_u32(&ctl->acc_full[b]));
-            else commit(smem_u32(&ctl->acc_full[b]));
+            commit_pair(smem_u32(&ctl->acc_full[b]));
         }
         __syncwarp();
         if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
     }
     if (!ok) {
         if (leader) {
-            if (PAIR) commit_pair(smem_u32(&ctl->drain[0]));
-            else commit(smem_u32(&ctl->drain[0]));
+            commit_pair(smem_u32(&ctl->drain[0]));
         }
         mbar_wait_quiet(smem_u32(&ctl->drain[0]), 0, g.wait_ns);
     }
@@ -876,7 +927,6 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 
     // warp-uniform, and known to be: the roles below run on whole warps
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    volatile int *abort_flag = &ctl->abort_flag;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
 
     if (threadIdx.x == 0) {
@@ -930,78 +980,27 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     // exit a round early) and set themselves up; they wait for this grid's results themselves.
     dependency_release();
 
-    const Deal<PAIR> deal(g);
-    const int rounds = deal.rounds(g);
-    const int ksteps = g.taps * g.chunks_per_tap;
     const uint32_t stage0 = smem_u32(stages);
 
     if (warp == 0) {
         // ---- TMA producer ----
         dependency_wait();
-        const bool leader = elect_one();
-        if (g.halo) {
-            producer_halo<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
+        if constexpr (PAIR) {
+            if (g.halo) producer_halo(g, ctl, &map_a, &map_b, stage0, rank);
+            else producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
         } else {
-        int stage = 0;
-        uint32_t phase = 0;
-        uint32_t armed = 0;  // bit s: stage s holds a load nobody is known to have consumed
-        uint32_t armed_parity = 0;
-        bool ok = true;
-        // a pair counts both CTAs' bytes on the leader's barrier
-        const uint32_t full_local = smem_u32(&ctl->full[0]);
-        const uint32_t full0 = PAIR && rank != 0 ? mapa(full_local, 0) : full_local;
-        const int b_rows = PAIR ? g.n_tile >> 1 : g.n_tile;  // filter rows this CTA loads
-        for (int it = 0; ok && it < rounds; it++) {
-            int mt, nt;
-            deal.at(g, it, mt, nt);
-            int row = g.lead + mt * BM - g.ph * g.wp - g.pw;  // tap (0,0)
-            int brow = nt * g.n_tile + (int)rank * b_rows;
-            int kw = 0, chunk = 0;
-            for (int ks = 0; ks < ksteps; ks++) {
-                const uint32_t ebar = smem_u32(&ctl->empty[stage]);
-                ok = warp_wait(ebar, phase ^ 1, abort_flag, g.error, 1, g.wait_ns);
-                if (!ok) break;
-                armed &= ~(1u << stage);
-                const uint32_t bar = full0 + 8u * (uint32_t)stage;
-                const uint32_t sa = stage0 + (uint32_t)stage * g.stage_bytes;
-                if (leader && PAIR) {
-                    if (rank == 0) mbar_expect_tx(bar, 2u * g.tx_bytes);  // bar is local here
-                    tma_load_2d_pair(sa, &map_a, chunk * g.kchunk, row, bar);
-                    tma_load_2d_pair(sa + g.a_bytes, &map_b, chunk * g.kchunk, brow, bar);
-                } else if (leader) {
-                    mbar_expect_tx(bar, g.tx_bytes);
-                    tma_load_2d(sa, &map_a, chunk * g.kchunk, row, bar);
-                    tma_load_2d(sa + g.a_bytes, &map_b, chunk * g.kchunk, brow, bar);
-                }
-                armed |= 1u << stage;
-                armed_parity = (armed_parity & ~(1u << stage)) | (phase << stage);
-                if (++stage == g.n_stages) { stage = 0; phase ^= 1; }
-                if (++chunk == g.chunks_per_tap) {  // next filter tap
-                    chunk = 0;
-                    brow += g.ocp16;
-                    if (++kw == g.tap_kw) { kw = 0; row += g.wp - (g.tap_kw - 1); }
-                    else row += 1;
-                }
-            }
-        }
-        if (!ok && rank == 0) {
-            // Something gave up. Loads already issued still land in this CTA's shared
-            // memory: wait for them (bounded) before the CTA may exit. (The partner of a
-            // pair cannot wait on the leader's barrier; it stays until the leader has got
-            // through this and both have met at the cluster barrier below.)
-            for (int s = 0; s < g.n_stages; s++)
-                if (armed & (1u << s)) {
-                    mbar_wait_quiet(smem_u32(&ctl->full[s]), (armed_parity >> s) & 1u,
-                                    g.wait_ns);
-                }
-        }
+            producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
         }
     } else if (warp == 1 || warp == kIssuer2Warp) {
         const int who = warp == 1 ? 0 : 1;
         if (who < g.issuers && rank == 0) {
-            if (PAIR && g.resident) mma_role_resident<KK, PAIR>(g, ctl, tmem_base, stage0);
-            else if (g.halo) mma_role_halo<KK, PAIR>(g, ctl, tmem_base, stage0, who);
-            else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
+            if constexpr (PAIR) {
+                if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
+                else if (g.halo) mma_role_halo<KK>(g, ctl, tmem_base, stage0, who);
+                else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
+            } else {
+                mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
+            }
         }
         __syncwarp();
     } else {
