@@ -30,15 +30,17 @@ typedef enum {
     xnor_nn_b200_kernel_popc = 0,            /* LOP3+POPC integer pipe; every shape and format */
     xnor_nn_b200_kernel_tcgen05_i8 = 2,      /* tcgen05.mma kind::mxf4, tiles of 128 frame
                                                 positions x up to 256 filters; unit stride,
-                                                padding smaller than the filter. Shapes it cannot
-                                                serve go to the rows kernel, then to popc. */
+                                                padding smaller than the filter. Asked for, shapes
+                                                it cannot serve go to the rows kernel, then to
+                                                popc; `auto` also folds strided layers into it
+                                                (and reports this value for them). */
     xnor_nn_b200_kernel_tcgen05_i8_rows = 3  /* tcgen05.mma kind::mxf4, tiles of 128 filters
                                                 x whole output rows of one image; unit stride,
                                                 rows of at most 256 pixels, any padding */
 } xnor_nn_b200_kernel_t;
 
 /* xnor_nn_init_convolution (src/common_convolution.cpp:9-63) with the kernel family stated.
- * A family that cannot serve the shape (strided convolutions on the tensor-core families)
+ * A family that cannot serve the shape (strided convolutions on a tensor-core family by name)
  * degrades to popc, the way an upstream bcast request degrades to the reference algorithm
  * when oc is not a multiple of the vector width (src/bcast_convolution.cpp:45-56). */
 xnor_nn_status_t xnor_nn_b200_init_convolution(xnor_nn_convolution_t *c,
@@ -75,9 +77,9 @@ xnor_nn_status_t xnor_nn_b200_binarize(const xnor_nn_convolution_t *c, xnor_nn_r
  *   c[i], res[i]: the layers in order, each initialised, allocated and with binarize_weights done;
  *   source: res[0][user_src]; result: res[layers-1][user_dst] (host or device memory);
  *   layer i+1 must take what layer i produces: same mb, ic = oc, ih = oh, iw = ow, else
- *   xnor_nn_error_invalid_input; every chained layer must run on the tensor-core kernels (unit
- *   stride), else xnor_nn_unimplemented. A layer in the middle whose paddings differ or are as
- *   large as its filter does pass floats on, through a buffer that the first call allocates.
+ *   xnor_nn_error_invalid_input; every chained layer must run on the tensor-core kernels with unit
+ *   strides, else xnor_nn_unimplemented. A layer whose paddings differ or are as large as its
+ *   filter does pass floats on to the next, through a buffer that the first call allocates.
  * The packed signs, hence every integer sum, equal those of calling the layers one after another;
  * the mean-|x| maps of layers 1.. are summed in a fixed but not strictly sequential order, so the
  * floats agree with the layer-by-layer result to rounding (about 1e-6 relative), reproducibly.

@@ -38,8 +38,8 @@
 //
 // The epilogue has three forms: floats in NCHW (a warp store is one contiguous run of a filter
 // plane), floats in NHWC (a thread owns whole 32-byte sectors and writes them with 256-bit
-// stores), and, for chained layers, no floats at all: the sign byte of every result goes into the
-// next layer's frame and sum |result| into its mean-|x| map (ChainTarget in kernels.cuh).
+// stores), and, for chained layers, no floats at all: the sign of every result goes into the next
+// layer's frame and sum |result| into its mean-|x| map (ChainTarget in kernels.cuh).
 //
 // Every wait on an mbarrier is bounded in time: when the bound is hit the kernel records where
 // in *error, every role winds down, copies in flight are waited for (again bounded), tensor
@@ -106,7 +106,7 @@ struct TcArgs {
     // Halo mode (pairs, filters at least two taps wide): the position tile of a
     // filter row is loaded once, with the kw - 1 positions that follow it, and serves all kw taps
     // of the row (a tap is a row offset into the tile); the ring then holds filter tiles only.
-    int halo;             // 0, or rows of a halo tile (128 + 8)
+    int halo;             // 0, or rows of a halo tile (128 + 8; 128 with a single tap per row)
     int n_a_slots;        // halo tiles in flight
     uint32_t a_slot_bytes, b_ring_off, b_slot_bytes, b_bytes;
     // Resident filters (pairs whose tiles all have the same filter tile, if its operands of all
@@ -543,7 +543,7 @@ __device__ __forceinline__ void producer_ring(const TcArgs &g, Control *ctl,
 }
 
 // ---- MMA issuer role -----------------------------------------------------------------------------
-// One thread feeds the tensor pipe; the instructions of a pipeline stage (KK tcgen05.mma and the
+// One lane feeds the tensor pipe; the instructions of a pipeline stage (KK tcgen05.mma and the
 // tcgen05.commit that hands the stage back) cost that thread more cycles than the pipe needs for
 // them unless N is 256. With two issuers the stages are dealt alternately (issuer i takes stages
 // i, i+2, ... of the running stage sequence, which continues across tiles), each commits its own
@@ -1047,10 +1047,10 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         sm_count[d].store(sms, std::memory_order_relaxed);
     }
-    // CTA pairs when the layer is more than one round of tiles (measured on AlexNet conv4: 35.0
-    // against 36.9 us at 256 images, 24.3 against 24.9 at 128; with a single round the pair's
-    // longer hand-shakes cost more than its lighter loads save: 15.6 against 14.7 us at 64
-    // images). Floats or sums out only (the chained epilogue carries per-pixel state across the
+    // CTA pairs when the layer is more than one round of tiles (measured with 8-bit operands on
+    // AlexNet conv4: 35.0 against 36.9 us at 256 images, 24.3 against 24.9 at 128). With a single
+    // round the pair's longer hand-shakes cost more than its lighter loads save: a pass on one image
+    // 13.5 against 12.4 us with the present operands, on 32 images 17.5 against 16.6. Floats or sums out only (the chained epilogue carries per-pixel state across the
     // filter tiles of one CTA), and a filter tile that splits into two UMMA-sized halves.
     const bool pair = !next && p.n_tile % 32 == 0 && m_tiles >= 2 &&
                       (long)m_tiles * (p.ocp16 / p.n_tile) > sms;
@@ -1151,7 +1151,8 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     bool halo = pair && g.tap_kw >= 2 && row_offsets_ok && g.issuers <= g.tap_kw;
     // Filters stay in shared memory if a pair works on several tiles of the same ones and their
     // operands leave room for three position tiles (kernel alone: conv2 mb128 48.8 -> 43.8 us, conv3
-    // mb256 25.4 -> 23.0, conv1 mb64 26.1 -> 25.5; three is what conv2 needs the room for).
+    // mb256 25.4 -> 23.0, conv1 mb64 26.1 -> 25.5). Three is the least that was measured: conv2
+    // leaves no room for more, the other two have six and eight.
     const int groups = g.kh * g.chunks_per_tap;
     if (same_nt && div_up_i(units, one_nt) > 1 && row_offsets_ok) {
         const uint32_t rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);

@@ -202,8 +202,8 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
 
     // The position-tile kernel serves every shape it can: with one tcgen05.commit per four
     // instructions a tile costs the same whatever its N, so the shape with the fewest tiles wins,
-    // and that kernel's tiles are always 128 x 256 (measured on the five benchmark layers: 36 /
-    // 44 / 68 / 95 us against 45 / 49 / 74 / 109 us). The image-row kernel takes what is left:
+    // and that kernel's tiles are always 128 x 256 (measured, with 8-bit operands, on conv4, conv3,
+    // conv2 and VGG: 36 / 44 / 68 / 95 us against 45 / 49 / 74 / 109 us). The image-row kernel takes what is left:
     // paddings as large as the filter, output extents that do not follow from the padding.
     Family f = requested;
     if (f != kPopc && f != kTcgen05 && f != kTcgen05Rows) f = family_from_env();
