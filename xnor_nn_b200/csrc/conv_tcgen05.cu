@@ -32,9 +32,10 @@
 // epilogue drains its own tensor memory. A pair loads a position tile only once per filter row and
 // channel chunk, with a halo of the positions that follow it, and the taps of the row read that
 // tile at row offsets (producer_halo / mma_role_halo); filters that fit are loaded once and stay
-// (mma_role_resident). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters) or,
-// when its loads share the way to L2 with the stores of the tile before it, those: AlexNet conv4 on
-// 256 images takes 8200 cycles a tile without the other's stores and 10500 with them (pipe: 6900).
+// (mma_role_resident), in layers of few channels beside position tiles that serve all taps of the
+// filter (mma_role_planes). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters)
+// or, when its loads share the way to L2 with the stores of the tile before it, those: AlexNet conv4
+// on 256 images takes 8200 cycles a tile without the other's stores and 10500 with them (pipe: 6900).
 //
 // The epilogue has three forms: floats in NCHW (a warp store is one contiguous run of a filter
 // plane), floats in NHWC (a thread owns whole 32-byte sectors and writes them with 256-bit
@@ -114,6 +115,10 @@ struct TcArgs {
     // loaded once, together with the first round's position tiles, and stay. halo is 128 then if
     // there is one tap per filter row.
     int resident;
+    // Resident filters with position tiles of 16-byte channel columns (producer_planes): columns of a
+    // tile, positions of it, bytes per position and the upper half of its matrix descriptors. 0: not so.
+    int planes, plane_rows, pos_bytes;
+    uint32_t plane_desc_hi;
     int kk_last;          // MMAs of a tap's last channel chunk: its 64-channel slices that hold
                           // channels at all (the chunk is padded with zeros to kchunk bytes)
     uint32_t acc_step;    // columns from the first accumulator to the second
@@ -908,6 +913,157 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
     }
 }
 
+// Position tiles of 16-byte columns (resident filters): the packed bytes of all positions that any tap
+// of a tile reads, 128 + (kh-1) wp + kw-1 of them, are loaded once, as [column][position][16 bytes].
+// That is the tensor core's unswizzled K-major form (eight positions of a column are a core matrix of
+// 128 contiguous bytes, the next eight follow, the next column is plane_rows * 16 further on), in
+// which a tap is a start address: 16 bytes per position. A filter row's taps read neighbouring
+// positions, so byte 32 s of its operand (what the s-th instruction starts at) is column
+// 32 s % pos_bytes / 16 of position 32 s / pos_bytes, and the column after a position's last one is
+// the next position's first, which the tensor map delivers like any other.
+__device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
+                                                const CUtensorMap *map_a, const CUtensorMap *map_b,
+                                                uint32_t stage0, uint32_t rank) {
+    volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
+    const Deal<true> deal(g);
+    const int rounds = deal.rounds(g);
+    const uint32_t full_l = smem_u32(&ctl->full[0]), afull_l = smem_u32(&ctl->a_full[0]);
+    // a pair counts both CTAs' bytes on the leader's barriers
+    const uint32_t full0 = rank != 0 ? mapa(full_l, 0) : full_l;
+    const uint32_t afull0 = rank != 0 ? mapa(afull_l, 0) : afull_l;
+    const uint32_t aempty0 = smem_u32(&ctl->a_empty[0]);
+    const uint32_t a_bytes = (uint32_t)(g.planes * g.plane_rows) * 16u;
+    int sa = 0;
+    uint32_t pa = 0, armed = 0, parity = 0;
+    int b_sent = 0;
+    bool ok = true;
+    for (int it = 0; it < rounds; it++) {
+        int mt, nt;
+        deal.at(g, it, mt, nt);
+        ok = warp_wait(aempty0 + 8u * (uint32_t)sa, pa ^ 1, abort_flag, g.error, 8, g.wait_ns);
+        if (!ok) break;
+        const uint32_t abar = afull0 + 8u * (uint32_t)sa;
+        if (leader) {
+            if (rank == 0) mbar_expect_tx(abar, 2u * a_bytes);  // abar is local here
+            tma_load_3d_pair(stage0 + (uint32_t)sa * g.a_slot_bytes, map_a, 0,
+                             g.lead + mt * BM - g.ph * g.wp - g.pw, 0, abar);
+        }
+        armed |= 1u << sa;
+        parity = (parity & ~(1u << sa)) | (pa << sa);
+        if (++sa == g.n_a_slots) { sa = 0; pa ^= 1; }
+        if (it == 0) {  // the filters, a barrier for each share of the groups
+            const int brow0 = nt * g.n_tile + (int)rank * (g.n_tile >> 1);
+            const int groups = g.kh * g.chunks_per_tap;
+            for (int part = 0, gr = 0; part < g.n_stages; part++) {
+                const int end = groups * (part + 1) / g.n_stages;
+                const uint32_t bar = full0 + 8u * (uint32_t)part;
+                if (leader && rank == 0) mbar_expect_tx(bar, 2u * (uint32_t)(end - gr) * g.b_bytes);
+                for (; gr < end; gr++) {
+                    const int row = gr / g.chunks_per_tap, chunk = gr - row * g.chunks_per_tap;
+                    if (leader)
+                        tma_load_2d_pair(stage0 + g.b_ring_off + (uint32_t)gr * g.b_slot_bytes, map_b,
+                                         chunk * g.kchunk, brow0 + row * g.ocp16, bar);
+                }
+            }
+            b_sent = g.n_stages;
+        }
+        __syncwarp();
+    }
+    if (!ok && rank == 0) {
+        // Something gave up. Loads already issued still land in this CTA's shared memory: wait
+        // for them (bounded) before the CTA may exit.
+        for (int i = 0; i < b_sent; i++) mbar_wait_quiet(full_l + 8u * (uint32_t)i, 0, g.wait_ns);
+        for (int i = 0; i < g.n_a_slots; i++)
+            if (armed & (1u << i))
+                mbar_wait_quiet(afull_l + 8u * (uint32_t)i, (parity >> i) & 1u, g.wait_ns);
+    }
+}
+
+// Two issuers take alternate groups (a chunk of a filter row). Nothing but a tile's first instruction
+// and the barriers around the tile ties them to each other: both see every position tile and every
+// accumulator, and of a filter barrier there is only one phase. One issuer needed 240 cycles per
+// instruction of 256 filters, the tensor pipe 128.
+template <int KK>
+__device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, uint32_t tmem_base,
+                                                uint32_t stage0, int who) {
+    volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
+    const int rounds = Deal<true>(g).rounds(g);
+    if (rounds == 0) return;
+    const int groups = g.kh * g.chunks_per_tap, columns = g.pos_bytes >> 4, n_iss = g.issuers;
+    const uint64_t a_hi = (uint64_t)g.plane_desc_hi << 32, b_hi = (uint64_t)g.desc_hi << 32;
+    const uint32_t lbo = (uint32_t)g.plane_rows;  // from a column to the next, in 16 bytes
+    const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (lbo << 16);
+    const uint32_t b_lo0 = (((stage0 + g.b_ring_off) >> 4) & 0x3FFF) | (1u << 16);
+    const uint32_t a_units = g.a_slot_bytes >> 4, b_units = g.b_slot_bytes >> 4;
+    const uint32_t full0 = smem_u32(&ctl->full[0]);
+    const uint32_t afull0 = smem_u32(&ctl->a_full[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
+    int sa = 0, b = 0;
+    uint32_t pa = 0, acc_phase = 0;
+    bool ok = true;
+    for (int it = 0; it < rounds; it++) {
+        const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
+        if (who == 0) {
+            ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2, g.wait_ns);
+            if (ok && g.shared_cols && it > 0)
+                ok = warp_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag,
+                               g.error, 7, g.wait_ns);
+        } else {  // the instruction that overwrites the accumulator has been executed
+            ok = warp_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6, g.wait_ns);
+        }
+        if (ok) ok = warp_wait(afull0 + 8u * (uint32_t)sa, pa, abort_flag, g.error, 9, g.wait_ns);
+        if (!ok) break;
+        fence_after();
+        const uint32_t tile = a_lo0 + (uint32_t)sa * a_units;
+        for (int gr = who; gr < groups; gr += n_iss) {
+            if (it == 0) {  // the share of the filters that the group belongs to
+                int part = 0;
+                while (groups * (part + 1) / g.n_stages <= gr) part++;
+                ok = warp_wait(full0 + 8u * (uint32_t)part, 0, abort_flag, g.error, 3, g.wait_ns);
+                if (!ok) break;
+                fence_after();
+            }
+            const int row = gr / g.chunks_per_tap, chunk = gr - row * g.chunks_per_tap;
+            const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+            // position and column that the chunk's bytes start at, from the filter row's first
+            const int byte = chunk * g.kchunk, pos = byte / g.pos_bytes;
+            int c = (byte - pos * g.pos_bytes) >> 4, at = row * g.wp + pos;
+            if (leader) {
+                const uint64_t bdesc = b_hi | (uint64_t)(b_lo0 + (uint32_t)gr * b_units);
+#pragma unroll
+                for (int k = 0; k < KK; k++) {
+                    if (k < kk) {
+                        mma_mxf4<true>(d_tmem, a_hi | (uint64_t)(tile + (uint32_t)c * lbo + (uint32_t)at),
+                                       bdesc + (uint64_t)(2 * k), g.idesc, tmem_base + kScaleCol,
+                                       (gr | k) == 0 ? 0u : 1u);
+                        // two columns further: the next position's, or the one's after it
+                        c += 2;
+                        if (c >= columns) { c -= columns; at++; }
+                        if (c >= columns) { c -= columns; at++; }
+                    }
+                }
+                if (gr == 0 && n_iss > 1) commit_pair(smem_u32(&ctl->started[b]));
+            }
+            __syncwarp();
+        }
+        if (!ok) break;
+        if (leader) {
+            commit_pair(aempty0 + 8u * (uint32_t)sa);
+            if (!(g.drop_commit && it == 0 && blockIdx.x == 0)) commit_pair(smem_u32(&ctl->acc_full[b]));
+        }
+        __syncwarp();
+        if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
+        if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
+    }
+    if (!ok) {
+        if (leader) {
+            commit_pair(smem_u32(&ctl->drain[who]));
+        }
+        mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
+    }
+}
+
 // KK = tcgen05.mma instructions per pipeline stage (kchunk / 32).
 // PAIR: the grid is made of clusters of two CTAs that share tiles of 256 positions x N filters
 // (tcgen05 cta_group::2). Each CTA loads its own 128 positions and its half of the filter tile,
@@ -986,7 +1142,8 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         // ---- TMA producer ----
         dependency_wait();
         if constexpr (PAIR) {
-            if (g.halo) producer_halo(g, ctl, &map_a, &map_b, stage0, rank);
+            if (g.planes) producer_planes(g, ctl, &map_a, &map_b, stage0, rank);
+            else if (g.halo) producer_halo(g, ctl, &map_a, &map_b, stage0, rank);
             else producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
         } else {
             producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
@@ -995,7 +1152,8 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         const int who = warp == 1 ? 0 : 1;
         if (who < g.issuers && rank == 0) {
             if constexpr (PAIR) {
-                if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
+                if (g.planes) mma_role_planes<KK>(g, ctl, tmem_base, stage0, who);
+                else if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
                 else if (g.halo) mma_role_halo<KK>(g, ctl, tmem_base, stage0, who);
                 else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
             } else {
@@ -1142,6 +1300,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const bool same_nt = pair && one_nt > 0 && div_up_i(units, one_nt) == div_up_i(units, grid);
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
+    g.planes = 0; g.plane_rows = 0; g.pos_bytes = p.icp; g.plane_desc_hi = 0;
     g.halo = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
     // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
@@ -1154,7 +1313,33 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // mb256 25.4 -> 23.0, conv1 mb64 26.1 -> 25.5). Three is the least that was measured: conv2
     // leaves no room for more, the other two have six and eight.
     const int groups = g.kh * g.chunks_per_tap;
-    if (same_nt && div_up_i(units, one_nt) > 1 && row_offsets_ok) {
+    // Layers whose filter rows are one operand row (Plan::cat): the position tile as 16-byte columns, if
+    // the positions of all taps are one box (256 rows) and two tiles fit beside the filters. AlexNet
+    // conv2, 128 images, kernel alone: 42.6 -> 40.3 us from loading 16 KB a tile instead of 160, 33.8
+    // with two issuers, which nothing keeps from taking alternate groups here. Wider positions and
+    // folded layers keep rows of 128 bytes, eight times fewer requests: with columns a pass of conv3
+    // (256 images) took 39.6 us instead of 38.3, of conv1 (64 images) 62.0 instead of 59.4.
+    if (same_nt && div_up_i(units, one_nt) > 1 && p.cat) {
+        const int columns = p.icp / 16, planes = columns + (columns & 1);
+        const int rows = BM + (g.kh - 1) * p.wp + p.kw - 1;
+        const uint32_t a_slot = (uint32_t)(planes * rows * 16 + 1023) & ~1023u;
+        const uint32_t b_slot = (g.b_bytes + 1023u) & ~1023u;
+        const size_t all_b = (size_t)groups * b_slot;
+        if (rows <= 256 && all_b + 2 * (size_t)a_slot <= room) {
+            g.resident = 1;
+            g.issuers = groups > 1 ? 2 : 1;
+            g.planes = planes; g.plane_rows = rows;
+            g.plane_desc_hi = 8u | (1u << 14);  // 128 bytes from eight positions to the next, no swizzle
+            g.a_slot_bytes = a_slot; g.b_slot_bytes = b_slot;
+            g.n_a_slots = (int)((room - all_b) / a_slot);
+            if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
+            g.b_ring_off = (uint32_t)g.n_a_slots * a_slot;
+            g.n_stages = groups < kMaxStages ? groups : kMaxStages;  // barriers of the filters
+            grid = one_nt;
+            halo = true;
+        }
+    }
+    if (!g.resident && same_nt && div_up_i(units, one_nt) > 1 && row_offsets_ok) {
         const uint32_t rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
         const uint32_t a_slot = (rows * p.kchunk + 1023) & ~1023u, b_slot = (g.b_bytes + 1023u) & ~1023u;
         const size_t all_b = (size_t)groups * g.tap_kw * b_slot;
@@ -1186,13 +1371,17 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         g.n_stages = (int)(room / g.stage_bytes);
         if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
     }
-    if (g.issuers == 2 && g.n_stages > 2) g.n_stages &= ~1;
-    if (g.n_stages < 2) return cudaErrorNotSupported;
+    if (g.issuers == 2 && g.n_stages > 2 && !g.planes) g.n_stages &= ~1;
+    if (g.n_stages < (g.planes ? 1 : 2)) return cudaErrorNotSupported;
     CUtensorMap map_a, map_b;
     // a position's row is tap_bytes long but only icp further than the one before it
-    if (!encode_bytes_2d(&map_a, bin_src, (uint64_t)(p.rows - (p.cat ? p.kw - 1 : 0)),
-                         (uint64_t)tap_bytes, (uint64_t)p.icp, (uint32_t)p.kchunk,
-                         (uint32_t)(halo ? g.halo : BM)) ||
+    const bool a_ok =
+        g.planes ? encode_planes_3d(&map_a, bin_src, (uint64_t)(p.rows - (g.planes * 16 > p.icp)),
+                                    (uint64_t)g.planes, (uint64_t)p.icp, (uint32_t)g.plane_rows)
+                 : encode_bytes_2d(&map_a, bin_src, (uint64_t)(p.rows - (p.cat ? p.kw - 1 : 0)),
+                                   (uint64_t)tap_bytes, (uint64_t)p.icp, (uint32_t)p.kchunk,
+                                   (uint32_t)(halo ? g.halo : BM));
+    if (!a_ok ||
         !encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
                          (uint64_t)tap_bytes, (uint32_t)p.kchunk, (uint32_t)b_rows))
         return cudaErrorNotSupported;

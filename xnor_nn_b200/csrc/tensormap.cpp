@@ -55,7 +55,8 @@ bool encode_cached(CUtensorMap *map, const Key &k) {
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUtensorMapSwizzle sw = k.box[0] == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
                                   : k.box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                   : CU_TENSOR_MAP_SWIZZLE_32B;
+                                  : k.box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                   : CU_TENSOR_MAP_SWIZZLE_NONE;
     if (fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, k.rank, const_cast<void *>(k.ptr), k.dim, k.stride,
            k.box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -78,6 +79,17 @@ bool encode_bytes_2d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t 
     k.dim[0] = row_bytes; k.dim[1] = rows;
     k.stride[0] = pitch;
     k.box[0] = box_bytes; k.box[1] = box_rows;
+    return encode_cached(map, k);
+}
+
+bool encode_planes_3d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t planes,
+                      uint64_t pitch, uint32_t box_rows) {
+    Key k;
+    memset(&k, 0, sizeof k);
+    k.ptr = ptr; k.rank = 3;
+    k.dim[0] = 16; k.dim[1] = rows; k.dim[2] = planes;
+    k.stride[0] = pitch; k.stride[1] = 16;
+    k.box[0] = 16; k.box[1] = box_rows; k.box[2] = (uint32_t)planes;
     return encode_cached(map, k);
 }
 
