@@ -1,0 +1,56 @@
+"""What the position-tile launcher asks of the driver (tests/cpp/tile_launch.cpp): addresses, extents,
+strides and boxes of every tensor map keep to what cuTensorMapEncodeTiled documents, each stride
+building on the one before it, and no box reaches past the frame. (Rows may overlap: filter rows that
+are one operand row run on into the next positions.) Host code only."""
+import json
+import os
+import subprocess
+
+import pytest
+
+import cases
+import test_folded_gpu
+import test_position_columns_gpu
+import test_resident_filters_gpu
+import test_streamed_filters_gpu
+from xnor_nn_b200 import build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+LAYERS = (test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.RESIDENT +
+          test_streamed_filters_gpu.STREAMED + test_folded_gpu.FOLDED + cases.SHAPE_CASES + [
+              cases._c("alexnet_conv2_mb128", 128, 256, 96, 27, 27, 5, 5, ph=2, pw=2),
+              cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
+              cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
+
+
+@pytest.fixture(scope="module")
+def launches(tmp_path_factory):
+    """What the launcher did with each of LAYERS, in order."""
+    build.build()
+    exe = str(tmp_path_factory.mktemp("tile_launch") / "tile_launch")
+    objs = [os.path.join(build.OBJ, n + ".o") for n in ("conv_tcgen05.cu", "plan.cpp", "tensormap.cpp")]
+    subprocess.check_call(
+        ["g++", "-std=c++17", "-O1", "-I", os.path.join(build.ROOT, "include"), "-I", build.CSRC, "-I",
+         "/usr/local/cuda/include", os.path.join(HERE, "cpp", "tile_launch.cpp")] + objs + ["-o", exe])
+    keys = ("mb", "oc", "ic", "ih", "iw", "kh", "kw", "sh", "sw", "ph", "pw")
+    env = {k: v for k, v in os.environ.items() if k != "XNOR_NN_B200_KERNEL"}
+    out = subprocess.check_output(
+        [exe] + [",".join(str(c[1][k]) for k in keys) for c in LAYERS], text=True, env=env).splitlines()
+    assert len(out) == len(LAYERS)
+    return [json.loads(line) for line in out]
+
+
+@pytest.mark.parametrize("i", range(len(LAYERS)), ids=[c[0] for c in LAYERS])
+def test_tensor_maps_keep_to_the_documented_rules(launches, i):
+    got = launches[i]
+    for m in got.get("maps", ()):
+        assert m["ptr"] % 16 == 0
+        assert all(0 < d <= 1 << 32 for d in m["dim"])
+        assert all(0 < b <= 256 for b in m["box"])
+        assert m["box"][0] % 16 == 0 and m["box"][0] <= (16, 32, 64, 128)[m["swizzle"]]
+        assert all(s % 16 == 0 and s < 1 << 40 for s in m["stride"])
+        for near, far in zip(m["stride"], m["stride"][1:]):
+            assert far % near == 0, m
+        if m["ptr"] == got["activations"]:
+            last = m["dim"][0] + sum((d - 1) * s for d, s in zip(m["dim"][1:], m["stride"]))
+            assert last <= got["rows"] * got["icp"], m

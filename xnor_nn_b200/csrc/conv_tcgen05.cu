@@ -116,8 +116,9 @@ struct TcArgs {
     // there is one tap per filter row.
     int resident;
     // Resident filters with position tiles of 16-byte channel columns (producer_planes): columns of a
-    // tile, positions of it, bytes per position and the upper half of its matrix descriptors. 0: not so.
-    int planes, plane_rows, pos_bytes;
+    // tile, positions of it and positions from one column to the next (a multiple of 8), bytes per
+    // position and the upper half of its matrix descriptors. 0: not so.
+    int planes, plane_rows, plane_pitch, pos_bytes;
     uint32_t plane_desc_hi;
     int kk_last;          // MMAs of a tap's last channel chunk: its 64-channel slices that hold
                           // channels at all (the chunk is padded with zeros to kchunk bytes)
@@ -914,13 +915,14 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
 }
 
 // Position tiles of 16-byte columns (resident filters): the packed bytes of all positions that any tap
-// of a tile reads, 128 + (kh-1) wp + kw-1 of them, are loaded once, as [column][position][16 bytes].
+// of a tile reads, 128 + (kh-1) wp + kw-1 of them, are loaded once, as [column][position][16 bytes]:
+// a box of 16 bytes by all positions for each column, from a plain map of the frame.
 // That is the tensor core's unswizzled K-major form (eight positions of a column are a core matrix of
-// 128 contiguous bytes, the next eight follow, the next column is plane_rows * 16 further on), in
+// 128 contiguous bytes, the next eight follow, the next column is plane_pitch * 16 further on), in
 // which a tap is a start address: 16 bytes per position. A filter row's taps read neighbouring
 // positions, so byte 32 s of its operand (what the s-th instruction starts at) is column
 // 32 s % pos_bytes / 16 of position 32 s / pos_bytes, and the column after a position's last one is
-// the next position's first, which the tensor map delivers like any other.
+// the next position's first: with an odd number of columns that one is loaded again, a position on.
 __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
                                                 const CUtensorMap *map_a, const CUtensorMap *map_b,
                                                 uint32_t stage0, uint32_t rank) {
@@ -934,6 +936,7 @@ __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
     const uint32_t afull0 = rank != 0 ? mapa(afull_l, 0) : afull_l;
     const uint32_t aempty0 = smem_u32(&ctl->a_empty[0]);
     const uint32_t a_bytes = (uint32_t)(g.planes * g.plane_rows) * 16u;
+    const int columns = g.pos_bytes >> 4;
     int sa = 0;
     uint32_t pa = 0, armed = 0, parity = 0;
     int b_sent = 0;
@@ -946,8 +949,12 @@ __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
         const uint32_t abar = afull0 + 8u * (uint32_t)sa;
         if (leader) {
             if (rank == 0) mbar_expect_tx(abar, 2u * a_bytes);  // abar is local here
-            tma_load_3d_pair(stage0 + (uint32_t)sa * g.a_slot_bytes, map_a, 0,
-                             g.lead + mt * BM - g.ph * g.wp - g.pw, 0, abar);
+            const int row = g.lead + mt * BM - g.ph * g.wp - g.pw;
+            uint32_t adst = stage0 + (uint32_t)sa * g.a_slot_bytes;
+            for (int c = 0; c < g.planes; c++, adst += (uint32_t)g.plane_pitch * 16u) {
+                const bool next = c == columns;
+                tma_load_2d_pair(adst, map_a, next ? 0 : 16 * c, next ? row + 1 : row, abar);
+            }
         }
         armed |= 1u << sa;
         parity = (parity & ~(1u << sa)) | (pa << sa);
@@ -993,7 +1000,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
     if (rounds == 0) return;
     const int groups = g.kh * g.chunks_per_tap, columns = g.pos_bytes >> 4, n_iss = g.issuers;
     const uint64_t a_hi = (uint64_t)g.plane_desc_hi << 32, b_hi = (uint64_t)g.desc_hi << 32;
-    const uint32_t lbo = (uint32_t)g.plane_rows;  // from a column to the next, in 16 bytes
+    const uint32_t lbo = (uint32_t)g.plane_pitch;  // from a column to the next, in 16 bytes
     const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (lbo << 16);
     const uint32_t b_lo0 = (((stage0 + g.b_ring_off) >> 4) & 0x3FFF) | (1u << 16);
     const uint32_t a_units = g.a_slot_bytes >> 4, b_units = g.b_slot_bytes >> 4;
@@ -1300,7 +1307,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const bool same_nt = pair && one_nt > 0 && div_up_i(units, one_nt) == div_up_i(units, grid);
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
-    g.planes = 0; g.plane_rows = 0; g.pos_bytes = p.icp; g.plane_desc_hi = 0;
+    g.planes = 0; g.plane_rows = 0; g.plane_pitch = 0; g.pos_bytes = p.icp; g.plane_desc_hi = 0;
     g.halo = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
     // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
@@ -1322,13 +1329,14 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     if (same_nt && div_up_i(units, one_nt) > 1 && p.cat) {
         const int columns = p.icp / 16, planes = columns + (columns & 1);
         const int rows = BM + (g.kh - 1) * p.wp + p.kw - 1;
-        const uint32_t a_slot = (uint32_t)(planes * rows * 16 + 1023) & ~1023u;
+        const int pitch = (rows + 7) & ~7;  // a load lands on a multiple of 128 bytes
+        const uint32_t a_slot = (uint32_t)(planes * pitch * 16 + 1023) & ~1023u;
         const uint32_t b_slot = (g.b_bytes + 1023u) & ~1023u;
         const size_t all_b = (size_t)groups * b_slot;
         if (rows <= 256 && all_b + 2 * (size_t)a_slot <= room) {
             g.resident = 1;
             g.issuers = groups > 1 ? 2 : 1;
-            g.planes = planes; g.plane_rows = rows;
+            g.planes = planes; g.plane_rows = rows; g.plane_pitch = pitch;
             g.plane_desc_hi = 8u | (1u << 14);  // 128 bytes from eight positions to the next, no swizzle
             g.a_slot_bytes = a_slot; g.b_slot_bytes = b_slot;
             g.n_a_slots = (int)((room - all_b) / a_slot);
@@ -1376,8 +1384,8 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     CUtensorMap map_a, map_b;
     // a position's row is tap_bytes long but only icp further than the one before it
     const bool a_ok =
-        g.planes ? encode_planes_3d(&map_a, bin_src, (uint64_t)(p.rows - (g.planes * 16 > p.icp)),
-                                    (uint64_t)g.planes, (uint64_t)p.icp, (uint32_t)g.plane_rows)
+        g.planes ? encode_bytes_2d(&map_a, bin_src, (uint64_t)p.rows, (uint64_t)p.icp,
+                                   (uint64_t)p.icp, 16, (uint32_t)g.plane_rows)
                  : encode_bytes_2d(&map_a, bin_src, (uint64_t)(p.rows - (p.cat ? p.kw - 1 : 0)),
                                    (uint64_t)tap_bytes, (uint64_t)p.icp, (uint32_t)p.kchunk,
                                    (uint32_t)(halo ? g.halo : BM));

@@ -163,14 +163,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, int c0, int c1,
-                                                 int c2, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
 // Arrives on the barrier at this offset in both CTAs of the pair once every tcgen05.mma issued
 // so far by this thread has completed.
 __device__ __forceinline__ void commit_pair(uint32_t bar) {
@@ -318,14 +310,9 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
 
 // ---- host side: tensor-map encoding (shared by the convolution launchers) ------------------------
 // A byte matrix of `rows` rows of row_bytes, `pitch` bytes apart (rows may overlap), boxes of
-// box_rows x box_bytes, swizzle span = box_bytes.
+// box_rows x box_bytes, swizzle span = box_bytes (boxes of 16 bytes are not swizzled).
 bool encode_bytes_2d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t row_bytes,
                      uint64_t pitch, uint32_t box_bytes, uint32_t box_rows);
-// A byte matrix of `rows` rows, `pitch` bytes apart, as 16-byte columns: boxes of box_rows rows and all
-// `planes` columns land as [column][row][16 bytes]. Column c of a row is its bytes 16 c ... 16 c + 15,
-// also where they belong to the row after it (planes * 16 > pitch).
-bool encode_planes_3d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t planes,
-                      uint64_t pitch, uint32_t box_rows);
 // A [d3][d2][d1][row_bytes] byte tensor (strides in bytes for d1, d2, d3), boxes of
 // 1 x box2 x box1 x box_bytes, swizzle span = box_bytes; out-of-range elements read as zero.
 bool encode_bytes_4d(CUtensorMap *map, const void *ptr, uint64_t row_bytes, uint64_t d1,

@@ -82,17 +82,6 @@ bool encode_bytes_2d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t 
     return encode_cached(map, k);
 }
 
-bool encode_planes_3d(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t planes,
-                      uint64_t pitch, uint32_t box_rows) {
-    Key k;
-    memset(&k, 0, sizeof k);
-    k.ptr = ptr; k.rank = 3;
-    k.dim[0] = 16; k.dim[1] = rows; k.dim[2] = planes;
-    k.stride[0] = pitch; k.stride[1] = 16;
-    k.box[0] = 16; k.box[1] = box_rows; k.box[2] = (uint32_t)planes;
-    return encode_cached(map, k);
-}
-
 bool encode_bytes_4d(CUtensorMap *map, const void *ptr, uint64_t row_bytes, uint64_t d1,
                      uint64_t d2, uint64_t d3, uint64_t s1, uint64_t s2, uint64_t s3,
                      uint32_t box_bytes, uint32_t box1, uint32_t box2) {
