@@ -1,7 +1,8 @@
 """What the position-tile launcher asks of the driver (tests/cpp/tile_launch.cpp): addresses, extents,
 strides and boxes of every tensor map keep to what cuTensorMapEncodeTiled documents, each stride
 building on the one before it, and no box reaches past the frame. (Rows may overlap: filter rows that
-are one operand row run on into the next positions.) Host code only."""
+are one operand row run on into the next positions.) And which layers load their position tiles as
+16-byte columns, at the lines where that was measured to stop paying. Host code only."""
 import json
 import os
 import subprocess
@@ -16,9 +17,26 @@ import test_streamed_filters_gpu
 from xnor_nn_b200 import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-LAYERS = (test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.RESIDENT +
+# (name, mb, oc, ic, ih, iw, kh, kw): either side of each line of the rule
+FASTER_AS_COLUMNS = [
+    cases._c("conv2", 128, 256, 96, 27, 27, 5, 5, ph=2, pw=2),
+    cases._c("three_tiles_a_pair", 75, 256, 96, 27, 27, 3, 3, ph=1, pw=1),
+    cases._c("two_tiles_a_pair_32_channels", 71, 192, 32, 17, 17, 5, 5, ph=2, pw=2),
+    cases._c("33_channels_96_filters", 266, 96, 33, 14, 14, 3, 3, ph=1, pw=1),
+    cases._c("33_channels_64_filters_four_rows", 160, 64, 33, 17, 17, 4, 4, ph=2, pw=2),
+    cases._c("two_tiles_in_flight", 40, 256, 224, 56, 56, 3, 3, ph=1, pw=1),
+]
+FASTER_AS_ROWS = [
+    cases._c("two_filter_rows", 71, 384, 128, 28, 28, 2, 2, ph=1, pw=1),
+    cases._c("one_filter_row", 306, 384, 160, 14, 14, 1, 3),
+    cases._c("two_tiles_a_pair", 45, 256, 96, 27, 27, 3, 3, ph=1, pw=1),
+    cases._c("two_tiles_a_pair_33_channels", 90, 192, 33, 17, 17, 3, 3, ph=1, pw=1),
+    cases._c("33_channels_64_filters", 266, 64, 33, 14, 14, 3, 3, ph=1, pw=1),
+    cases._c("filters_not_resident_beside_rows", 1129, 192, 127, 8, 8, 5, 5, ph=2, pw=2),
+    cases._c("257_rows", 80, 256, 96, 3, 62, 3, 4, ph=1, pw=1),
+]
+LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.RESIDENT +
           test_streamed_filters_gpu.STREAMED + test_folded_gpu.FOLDED + cases.SHAPE_CASES + [
-              cases._c("alexnet_conv2_mb128", 128, 256, 96, 27, 27, 5, 5, ph=2, pw=2),
               cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
               cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
 
@@ -54,3 +72,11 @@ def test_tensor_maps_keep_to_the_documented_rules(launches, i):
         if m["ptr"] == got["activations"]:
             last = m["dim"][0] + sum((d - 1) * s for d, s in zip(m["dim"][1:], m["stride"]))
             assert last <= got["rows"] * got["icp"], m
+
+
+@pytest.mark.parametrize("i", range(len(FASTER_AS_COLUMNS + FASTER_AS_ROWS)),
+                         ids=[c[0] for c in FASTER_AS_COLUMNS + FASTER_AS_ROWS])
+def test_columns_where_they_are_faster(launches, i):
+    got = launches[i]
+    boxes = [m["box"][0] for m in got["maps"] if m["ptr"] == got["activations"]]
+    assert (boxes == [16]) == (i < len(FASTER_AS_COLUMNS)), boxes

@@ -998,7 +998,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
     const bool leader = elect_one();
     const int rounds = Deal<true>(g).rounds(g);
     if (rounds == 0) return;
-    const int groups = g.kh * g.chunks_per_tap, columns = g.pos_bytes >> 4, n_iss = g.issuers;
+    const int groups = g.kh * g.chunks_per_tap, columns = g.pos_bytes >> 4;
     const uint64_t a_hi = (uint64_t)g.plane_desc_hi << 32, b_hi = (uint64_t)g.desc_hi << 32;
     const uint32_t lbo = (uint32_t)g.plane_pitch;  // from a column to the next, in 16 bytes
     const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (lbo << 16);
@@ -1023,7 +1023,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
         if (!ok) break;
         fence_after();
         const uint32_t tile = a_lo0 + (uint32_t)sa * a_units;
-        for (int gr = who; gr < groups; gr += n_iss) {
+        for (int gr = who; gr < groups; gr += 2) {
             if (it == 0) {  // the share of the filters that the group belongs to
                 int part = 0;
                 while (groups * (part + 1) / g.n_stages <= gr) part++;
@@ -1050,7 +1050,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
                         if (c >= columns) { c -= columns; at++; }
                     }
                 }
-                if (gr == 0 && n_iss > 1) commit_pair(smem_u32(&ctl->started[b]));
+                if (gr == 0) commit_pair(smem_u32(&ctl->started[b]));
             }
             __syncwarp();
         }
@@ -1316,53 +1316,51 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const bool row_offsets_ok = g.tap_kw == 1 || (g.tap_kw <= 9 && p.kchunk == 128);
     bool halo = pair && g.tap_kw >= 2 && row_offsets_ok && g.issuers <= g.tap_kw;
     // Filters stay in shared memory if a pair works on several tiles of the same ones and their
-    // operands leave room for three position tiles (kernel alone: conv2 mb128 48.8 -> 43.8 us, conv3
-    // mb256 25.4 -> 23.0, conv1 mb64 26.1 -> 25.5). Three is the least that was measured: conv2
-    // leaves no room for more, the other two have six and eight.
+    // operands leave room for three position tiles of 128-byte rows. Kernel alone, conv3 on 256 images
+    // 25.4 -> 23.0 us (six such tiles in flight), conv1 on 64 images 26.1 -> 25.5 (eight).
     const int groups = g.kh * g.chunks_per_tap;
-    // Layers whose filter rows are one operand row (Plan::cat): the position tile as 16-byte columns, if
-    // the positions of all taps are one box (256 rows) and two tiles fit beside the filters. AlexNet
-    // conv2, 128 images, kernel alone: 42.6 -> 40.3 us from loading 16 KB a tile instead of 160, 33.8
-    // with two issuers, which nothing keeps from taking alternate groups here. Wider positions and
-    // folded layers keep rows of 128 bytes, eight times fewer requests: with columns a pass of conv3
-    // (256 images) took 39.6 us instead of 38.3, of conv1 (64 images) 62.0 instead of 59.4.
-    if (same_nt && div_up_i(units, one_nt) > 1 && p.cat) {
+    const int walk = same_nt ? div_up_i(units, one_nt) : 1;  // tiles of a pair
+    const uint32_t halo_rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
+    const uint32_t row_slot = (halo_rows * p.kchunk + 1023) & ~1023u, b_slot = (g.b_bytes + 1023u) & ~1023u;
+    const size_t all_b = (size_t)groups * g.tap_kw * b_slot;
+    if (walk > 1 && row_offsets_ok && all_b + 3 * (size_t)row_slot <= room) {
+        // Position tiles as 16-byte columns: layers whose filter rows are one operand row (Plan::cat), if
+        // the positions of all taps are one box (256 rows) and two tiles fit. AlexNet conv2 on 128
+        // images, kernel alone: 42.6 -> 40.3 us from loading 16 KB a tile instead of 160, 33.8 with two
+        // issuers. What pays for the columns is that a tile is loaded once for all filter rows and that
+        // two issuers share it; what they cost is requests of 16 bytes and a first tile that has to land
+        // whole. Columns against 128-byte rows, kernel alone, over 1756 layers of 3 to 224 channels, 16
+        // to 512 filters, 1 to 7 filter rows and up to 17 tiles a pair:
+        //   one or two filter rows                                      0.89 to 1.17, median 1.01
+        //   more, two tiles a pair and more than 32 channels            0.95 to 1.10, median 1.01
+        //   more, 33 to 64 channels, three operand rows, 64 filters     1.00 to 1.02, median 1.02
+        //   more, filters that would not be resident beside rows        0.94 to 1.10, median 1.00
+        //   the others                                                  0.73 to 1.04, median 0.94
+        // Only the last take columns; layers of the fourth kind stream their filters.
         const int columns = p.icp / 16, planes = columns + (columns & 1);
         const int rows = BM + (g.kh - 1) * p.wp + p.kw - 1;
         const int pitch = (rows + 7) & ~7;  // a load lands on a multiple of 128 bytes
-        const uint32_t a_slot = (uint32_t)(planes * pitch * 16 + 1023) & ~1023u;
-        const uint32_t b_slot = (g.b_bytes + 1023u) & ~1023u;
-        const size_t all_b = (size_t)groups * b_slot;
-        if (rows <= 256 && all_b + 2 * (size_t)a_slot <= room) {
-            g.resident = 1;
-            g.issuers = groups > 1 ? 2 : 1;
+        const uint32_t col_slot = (uint32_t)(planes * pitch * 16 + 1023) & ~1023u;
+        const bool as_columns = p.cat && g.kh >= 3 && (walk >= 3 || p.icp == 16) &&
+                                !(p.icp == 32 && groups == 3 && p.n_tile <= 64) && rows <= 256 &&
+                                all_b + 2 * (size_t)col_slot <= room;
+        g.resident = 1;
+        if (as_columns) {
+            g.issuers = 2;
             g.planes = planes; g.plane_rows = rows; g.plane_pitch = pitch;
             g.plane_desc_hi = 8u | (1u << 14);  // 128 bytes from eight positions to the next, no swizzle
-            g.a_slot_bytes = a_slot; g.b_slot_bytes = b_slot;
-            g.n_a_slots = (int)((room - all_b) / a_slot);
-            if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
-            g.b_ring_off = (uint32_t)g.n_a_slots * a_slot;
             g.n_stages = groups < kMaxStages ? groups : kMaxStages;  // barriers of the filters
-            grid = one_nt;
-            halo = true;
-        }
-    }
-    if (!g.resident && same_nt && div_up_i(units, one_nt) > 1 && row_offsets_ok) {
-        const uint32_t rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
-        const uint32_t a_slot = (rows * p.kchunk + 1023) & ~1023u, b_slot = (g.b_bytes + 1023u) & ~1023u;
-        const size_t all_b = (size_t)groups * g.tap_kw * b_slot;
-        if (all_b + 3 * (size_t)a_slot <= room) {
-            g.resident = 1;
+        } else {
             g.issuers = 1;
-            g.halo = (int)rows;
-            g.a_slot_bytes = a_slot; g.b_slot_bytes = b_slot;
-            g.n_a_slots = (int)((room - all_b) / a_slot);
-            if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
-            g.b_ring_off = (uint32_t)g.n_a_slots * a_slot;
+            g.halo = (int)halo_rows;
             g.n_stages = 2;
-            grid = one_nt;
-            halo = true;
         }
+        g.a_slot_bytes = as_columns ? col_slot : row_slot; g.b_slot_bytes = b_slot;
+        g.n_a_slots = (int)((room - all_b) / g.a_slot_bytes);
+        if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
+        g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
+        grid = one_nt;
+        halo = true;
     }
     if (halo && !g.resident) {
         // three halo tiles of 136 positions, the rest of the room for filter tiles
@@ -1380,7 +1378,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
     }
     if (g.issuers == 2 && g.n_stages > 2 && !g.planes) g.n_stages &= ~1;
-    if (g.n_stages < (g.planes ? 1 : 2)) return cudaErrorNotSupported;
+    if (g.n_stages < 2) return cudaErrorNotSupported;
     CUtensorMap map_a, map_b;
     // a position's row is tap_bytes long but only icp further than the one before it
     const bool a_ok =
