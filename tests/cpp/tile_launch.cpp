@@ -1,7 +1,7 @@
 // What the position-tile launcher hands the driver, without a GPU: its object files are linked against
 // stand-ins for the few CUDA runtime calls it makes (a device of 148 SMs and 74 pairs of them). For
-// each layer on the command line (mb,oc,ic,ih,iw,kh,kw,sh,sw,ph,pw) one line of JSON: the launch and
-// the tensor maps it asked for.
+// each layer on the command line (mb,oc,ic,ih,iw,kh,kw,sh,sw,ph,pw) one line of JSON: the tensor
+// maps it asked for, the launch, and the parameters that say which form of the kernel runs.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -10,6 +10,7 @@
 #include <cstring>
 #include <string>
 
+#include "conv_tile_args.cuh"
 #include "kernels.cuh"
 
 namespace xb200 {
@@ -57,9 +58,18 @@ cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *, const cudaLaunc
     *n = 74;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) {
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **args) {
+    const xb200::TcArgs &g = *(const xb200::TcArgs *)args[2];
+    const bool pair = c->numAttrs > 1 && c->attrs[1].val.clusterDim.x == 2;
     char text[512];
-    snprintf(text, sizeof text, "\"grid\": %u, \"smem\": %zu", c->gridDim.x, c->dynamicSmemBytes);
+    snprintf(text, sizeof text,
+             "\"grid\": %u, \"smem\": %zu, \"pair\": %s, \"planes\": %d, \"plane_rows\": %d, "
+             "\"resident\": %d, \"halo\": %d, \"a_slots\": %d, \"stages\": %d, \"issuers\": %d, "
+             "\"groups\": %d, \"kchunk\": %d, \"tap_kw\": %d, \"m_tiles\": %d, \"n_tiles\": %d, "
+             "\"shared_cols\": %d",
+             c->gridDim.x, c->dynamicSmemBytes, pair ? "true" : "false", g.planes, g.plane_rows,
+             g.resident, g.halo, g.n_a_slots, g.n_stages, g.issuers, g.kh * g.chunks_per_tap, g.kchunk,
+             g.tap_kw, g.m_tiles, g.n_tiles, g.shared_cols);
     g_launch = text;
     return cudaSuccess;
 }

@@ -19,12 +19,13 @@ pytestmark = pytest.mark.gpu
 # one image; 40 images: one tile per thread block on many SMs; 256 images: several tiles per block,
 # the position-tile kernel on CTA pairs (the block that loses its commit is a pair's leader, so
 # both blocks of the pair give up, keep the epilogue's meetings and leave through the cluster
-# barrier)
-@pytest.mark.parametrize("mb", [1, 40, 256])
-def test_lost_commit_times_out_and_the_resources_stay_usable(kernel, mb):
+# barrier). Layer D, 96 channels: the position-tile kernel with position tiles as columns beside
+# resident filters, two issuers on every tile of a pair
+@pytest.mark.parametrize("layer, mb", [("A", 1), ("A", 40), ("A", 256), ("D", 64)])
+def test_lost_commit_times_out_and_the_resources_stay_usable(kernel, layer, mb):
     torch = pytest.importorskip("torch")
-    L = synth.layer_shape("A", mb=mb)
-    src, w = synth.make_inputs("A", mb=mb)
+    L = synth.layer_shape(layer, mb=mb)
+    src, w = synth.make_inputs(layer, mb=mb)
     conv = xb.Convolution(xb.ALGORITHM_BCAST, xb.NCHW, xb.OIHW, xb.NCHW, L.mb, L.oc, L.ic, L.ih,
                           L.iw, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, w, kernel=kernel)
     assert conv.kernel == kernel
@@ -42,7 +43,7 @@ def test_lost_commit_times_out_and_the_resources_stay_usable(kernel, mb):
     # within microseconds of one another (the MMA issuers waiting for its accumulator to be handed
     # back, 2 and 6, the producer behind them, 1 and 8): whichever expires first is recorded.
     err = xb.last_error()
-    if mb == 256:
+    if mb == 256 or layer == "D":
         assert "gave up waiting (site " in err, err
     else:
         assert "gave up waiting (site 4)" in err, err

@@ -1,8 +1,9 @@
 """What the position-tile launcher asks of the driver (tests/cpp/tile_launch.cpp): addresses, extents,
 strides and boxes of every tensor map keep to what cuTensorMapEncodeTiled documents, each stride
 building on the one before it, and no box reaches past the frame. (Rows may overlap: filter rows that
-are one operand row run on into the next positions.) And which layers load their position tiles as
-16-byte columns, at the lines where that was measured to stop paying. Host code only."""
+are one operand row run on into the next positions.) Which layers load their position tiles as 16-byte
+columns, at the lines where that was measured to stop paying. And that the layers of the GPU tests take
+the forms of the kernel that they are there for. Host code only."""
 import json
 import os
 import subprocess
@@ -35,8 +36,11 @@ FASTER_AS_ROWS = [
     cases._c("filters_not_resident_beside_rows", 1129, 192, 127, 8, 8, 5, 5, ph=2, pw=2),
     cases._c("257_rows", 80, 256, 96, 3, 62, 3, 4, ph=1, pw=1),
 ]
-LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.RESIDENT +
-          test_streamed_filters_gpu.STREAMED + test_folded_gpu.FOLDED + cases.SHAPE_CASES + [
+GPU_COLUMNS = test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.COLUMNS
+LOST_COMMIT = cases._c("lost_commit", 64, 256, 96, 27, 27, 5, 5, ph=2, pw=2)
+LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + GPU_COLUMNS + test_position_columns_gpu.ROWS +
+          test_resident_filters_gpu.ROWS + [LOST_COMMIT] + test_streamed_filters_gpu.STREAMED +
+          test_folded_gpu.FOLDED + cases.SHAPE_CASES + [
               cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
               cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
 
@@ -56,6 +60,13 @@ def launches(tmp_path_factory):
         [exe] + [",".join(str(c[1][k]) for k in keys) for c in LAYERS], text=True, env=env).splitlines()
     assert len(out) == len(LAYERS)
     return [json.loads(line) for line in out]
+
+
+def _of(launches, layers):
+    """The launches of consecutive layers of LAYERS."""
+    at = LAYERS.index(layers[0])
+    assert LAYERS[at:at + len(layers)] == layers
+    return launches[at:at + len(layers)]
 
 
 @pytest.mark.parametrize("i", range(len(LAYERS)), ids=[c[0] for c in LAYERS])
@@ -80,3 +91,28 @@ def test_columns_where_they_are_faster(launches, i):
     got = launches[i]
     boxes = [m["box"][0] for m in got["maps"] if m["ptr"] == got["activations"]]
     assert (boxes == [16]) == (i < len(FASTER_AS_COLUMNS)), boxes
+
+
+def test_gpu_tests_of_position_columns_reach_them(launches):
+    got = _of(launches, GPU_COLUMNS)
+    assert all(g["planes"] and g["resident"] and g["issuers"] == 2 for g in got + _of(launches, [LOST_COMMIT]))
+    assert {g["icp"] // 16 for g in got} >= {1, 2, 3, 5, 7}
+    assert {g["a_slots"] for g in got} >= {2, 8} and 256 in {g["plane_rows"] for g in got}
+    assert {g["kchunk"] for g in got} == {32, 64, 128}
+    assert {g["m_tiles"] % 2 for g in got} == {0, 1} and {g["n_tiles"] for g in got} == {1, 2, 3}
+    assert min(g["groups"] for g in got) < 8 < max(g["groups"] for g in got)
+    assert 8 in {g["groups"] for g in got} and 1 in {g["shared_cols"] for g in got}
+    assert not any(g["planes"] for g in _of(launches, test_position_columns_gpu.ROWS))
+
+
+def test_gpu_tests_of_resident_rows_reach_them(launches):
+    got = _of(launches, test_resident_filters_gpu.ROWS)
+    assert all(g["resident"] and not g["planes"] and g["pair"] for g in got)
+    seen = {(g["tap_kw"], g["n_tiles"], g["shared_cols"]) for g in got}
+    assert seen >= {(t, n, c) for t in (1, 3) for n, c in ((1, 0), (1, 1), (2, 0))} | {(3, 3, 0)}
+    assert {g["kchunk"] for g in got} == {32, 64, 128} and {g["groups"] % 2 for g in got} == {0, 1}
+
+
+def test_gpu_tests_of_streamed_filters_reach_them(launches):
+    got = _of(launches, test_streamed_filters_gpu.STREAMED)
+    assert all(g["halo"] and not g["resident"] and g["issuers"] == 2 for g in got)
