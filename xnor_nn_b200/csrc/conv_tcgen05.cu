@@ -794,10 +794,14 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     }
 }
 
-// Resident filters: the only thing that arrives is position tiles, so a group (the taps of a filter
-// row on one channel chunk) is one wait, kw * KK MMAs and one commit, which one issuer keeps up
-// with. With the filters streamed a pair moved 320 KB per CTA and tile of AlexNet conv2 through L2,
-// which took 11400 cycles under the result stores of another tile (tensor pipe: 5100).
+// Resident filters beside position tiles of rows: layers of more than 224 channels, one tap a filter
+// row, folded layers, and those that columns are no gain for. The only thing that arrives is position
+// tiles, so a group (the taps of a filter row on one channel chunk) is one wait, kw * KK MMAs and one
+// commit, from one issuer: about 500 cycles a group and 30 an instruction (layers of 64 filters that
+// differ in nothing else), where the tensor pipe needs N / 2 an instruction. Wide tiles with several
+// taps a group hide that, narrow ones are bound by it. With the filters streamed a pair moved 320 KB
+// per CTA and tile of AlexNet conv2 (on rows then) through L2, which took 11400 cycles under the
+// result stores of another tile (tensor pipe: 5100).
 template <int KK>
 __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                                   uint32_t stage0) {
@@ -936,8 +940,9 @@ __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
 
 // Two issuers take alternate groups (a chunk of a filter row). Nothing but a tile's first instruction
 // and the barriers around the tile ties them to each other: both see every position tile and every
-// accumulator, and of a filter barrier there is only one phase. One issuer needed 240 cycles per
-// instruction of 256 filters, the tensor pipe 128.
+// accumulator, and of a filter barrier there is only one phase. Alone, an issuer needs about 750
+// cycles a group and 80 an instruction (layers of 64 filters, 9 to 33 instructions in 3 to 9 groups):
+// on AlexNet conv2, four instructions a group, 240 cycles for each, where the tensor pipe needs 128.
 template <int KK>
 __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                                 uint32_t stage0, int who) {

@@ -45,9 +45,9 @@ struct TcArgs {
     int n_a_slots;        // halo tiles in flight
     uint32_t a_slot_bytes, b_ring_off, b_slot_bytes, b_bytes;
     // Resident filters (pairs whose tiles all have the same filter tile, if its operands of all
-    // taps fit shared memory beside three position tiles): halo mode with filter tiles that are
-    // loaded once, together with the first round's position tiles, and stay. halo is 128 then if
-    // there is one tap per filter row.
+    // taps fit shared memory beside three position tiles of 128-byte rows): filter tiles are loaded
+    // once, together with the first round's position tiles, and stay. Position tiles as in halo mode
+    // (halo is 128 if there is one tap per filter row), or as columns:
     int resident;
     // Resident filters with position tiles of 16-byte channel columns (producer_planes): columns of a
     // tile, positions of it and positions from one column to the next (a multiple of 8), bytes per
