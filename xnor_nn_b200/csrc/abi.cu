@@ -583,7 +583,8 @@ Slice slice_of(const Plan &p, int first, int count) {
     return s;
 }
 
-// binarize + A, K, convolution of one slice, device pointers, on the context's stream.
+// binarize + A, K, convolution of one slice, device pointers, on the context's stream; one launch for
+// small layers.
 xnor_nn_status_t enqueue_forward(const Slice &sl, ResCtx *x, xnor_nn_resources_t res,
                                  const float *src, float *dst) {
     xnor_nn_resources_t sub;
@@ -591,6 +592,13 @@ xnor_nn_status_t enqueue_forward(const Slice &sl, ResCtx *x, xnor_nn_resources_t
     sub[xnor_nn_resource_bin_src] = (char *)res[xnor_nn_resource_bin_src] + sl.bin_src;
     sub[xnor_nn_resource_a] = (char *)res[xnor_nn_resource_a] + sl.a;
     sub[xnor_nn_resource_k] = (char *)res[xnor_nn_resource_k] + sl.k;
+    if (whole_ok(sl.p)) {
+        CU(launch_conv_whole(sl.p, src, sub[xnor_nn_resource_bin_src],
+                             res[xnor_nn_resource_bin_weights], (const float *)res[xnor_nn_resource_alpha],
+                             (float *)sub[xnor_nn_resource_a], (float *)sub[xnor_nn_resource_k], dst,
+                             x->error_word, x->stream));
+        return xnor_nn_success;
+    }
     CU(launch_binarize_data(sl.p, src, sub[xnor_nn_resource_bin_src],
                             (float *)sub[xnor_nn_resource_a], x->stream));
     const bool fuse_k = sl.p.family == kTcgen05 && !sl.p.fold;

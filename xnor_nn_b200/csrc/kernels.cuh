@@ -157,6 +157,14 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
                                 const ChainTarget *next = nullptr,
                                 const ConvSelfTest *test = nullptr);
 
+// A forward pass of a small layer in one launch (conv_whole.cu): packs the source, leaves frame and
+// maps as launch_binarize_data and the convolution would, and stores the result. For the layers that
+// whole_ok() names.
+bool whole_ok(const Plan &p);
+cudaError_t launch_conv_whole(const Plan &p, const float *src, void *bin_src, const void *bin_w,
+                              const float *alpha, float *a, float *k, float *dst, int *error_word,
+                              cudaStream_t s);
+
 // The same contract (without chaining) with the operand roles swapped: 128 filters on the UMMA M
 // side, whole output rows of one image on the N side (Plan::img_*, conv_tcgen05_img.cu). Reads
 // the same packed operands as launch_conv_tcgen05; the forward pass uses it when Plan::img is set.

@@ -243,14 +243,18 @@ __device__ __forceinline__ void mma_mxf4(uint32_t d_tmem, uint64_t adesc, uint64
             ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(scales), "r"(accumulate)
             : "memory");
 }
+// Writes one value to this warp's 32 lanes of `cols` columns (a multiple of 8).
+__device__ __forceinline__ void fill_columns(uint32_t taddr, int cols, uint32_t value) {
+    for (int c = 0; c < cols; c += 8)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};"
+                     ::"r"(taddr + (uint32_t)c), "r"(value)
+                     : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 // Writes the block scales: this warp's 32 lanes of `cols` columns (a multiple of 16). All four
 // quadrants of lanes have to be written before the first mma_mxf4.
 __device__ __forceinline__ void fill_scales(uint32_t taddr, int cols) {
-    for (int c = 0; c < cols; c += 8)
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};"
-                     ::"r"(taddr + (uint32_t)c), "r"(kScaleOne)
-                     : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    fill_columns(taddr, cols, kScaleOne);
 }
 
 // Arrives on the barrier once every tcgen05.mma issued so far by this thread has completed.
