@@ -321,10 +321,12 @@ __global__ void __launch_bounds__(TWARPS * 32) binarize_nibbles_kernel(const Bin
 // multiplied by 1/(KH*KW) (each term of upstream's sum is that product) and with zeros where the
 // window leaves the image (adding +0 to a sum of non-negative terms changes nothing), and a thread
 // adds up an output's terms in upstream's order. A staged row has its columns sorted by their
-// remainder modulo the stride, so that neighbouring outputs read neighbouring words, and tap j is a
-// fixed distance from the output's first word: three instructions per term for the filter widths
-// that are compiled in (KW). AlexNet conv1 on 64 images, 121 taps: 18.8 us with the terms read from
-// global memory one after the other.
+// remainder modulo the stride, so that neighbouring outputs read neighbouring words, and tap j is word
+// j / SW of remainder j % SW, both known to the compiler for the widths and strides in use. A thread
+// keeps its column while it stages, eight lines at a time, and all its loads go out before the first is
+// used. AlexNet conv1 on 64 images (121 taps), launched alone: 18.8 us with the terms read from global memory
+// one after the other, 16.4 with them staged one by one (8.8 M warp instructions), 13.8 now (5.5 M); the
+// pass on one stream, of which the packer's rewrite is 2 to 3 us, 59.9 -> 55.7.
 struct BoxArgs {
     const float *a;
     float *k;
@@ -333,49 +335,90 @@ struct BoxArgs {
     int rows, row_blocks;  // output rows per block, blocks per image
     int span, phase;       // columns of A an output row reads; words per remainder
     int lines;             // rows of A staged
-    FastDiv by_span, by_sw, by_ow;
-    int tap[11];           // word of tap j, from the output's first
+    int cols, line_step;   // threads side by side on a staged row; rows staged at a time
+    FastDiv by_cols, by_sw, by_ow;
 };
 
-constexpr int kBoxThreads = 256;
+constexpr int kBoxThreads = 256, kBoxAhead = 8;
 constexpr int kBoxSmem = 40 * 1024;
 
-template <int KW>
+// A line of the window of the thread's upper output (FIRST), of its lower one (SECOND), or of both.
+template <int KW, int SW, bool FIRST, bool SECOND>
+__device__ __forceinline__ void add_line(const BoxArgs &g, const float *row, float &first, float &second) {
+    if (KW > 0) {
+#pragma unroll
+        for (int j = 0; j < KW; j++) {
+            const float v = row[j % SW * g.phase + j / SW];
+            if (FIRST) first = __fadd_rn(first, v);
+            if (SECOND) second = __fadd_rn(second, v);
+        }
+    } else {
+        for (int j = 0, at = 0, rem = 0; j < g.kw; j++) {
+            const float v = row[rem * g.phase + at];
+            if (FIRST) first = __fadd_rn(first, v);
+            if (SECOND) second = __fadd_rn(second, v);
+            if (++rem == g.sw) { rem = 0; at++; }
+        }
+    }
+}
+
+// TWO: a thread adds up two outputs, one below the other, and reads what their windows share once.
+template <int KW, int SW, bool TWO>
 __global__ void __launch_bounds__(kBoxThreads) box_filter_kernel(const BoxArgs g) {
     extern __shared__ __align__(16) float tile[];
     dependency_release();
     dependency_wait();
     const int n = blockIdx.x / g.row_blocks;
     const int oy0 = (blockIdx.x - n * g.row_blocks) * g.rows;
-    const int n_out = min(g.rows, g.oh - oy0) * g.ow;
     const int y0 = oy0 * g.sh - g.ph, pitch = g.phase * g.sw;
     const float *img = g.a + (long)n * g.ih * g.iw;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < g.lines * g.span; i += kBoxThreads) {
-        const int line = (int)g.by_span((uint32_t)i), xx = i - line * g.span;
-        const int y = y0 + line, x = xx - g.pw, xs = (int)g.by_sw((uint32_t)xx);
-        float v = 0.f;
-        if (y >= 0 && y < g.ih && x >= 0 && x < g.iw)
-            v = __fmul_rn(__ldg(img + y * g.iw + x), g.inv_khw);
-        tile[line * pitch + (xx - xs * g.sw) * g.phase + xs] = v;
+    const int first = (int)g.by_cols(threadIdx.x);
+    // staged lines that the image has
+    const int lo = min(max(0, -y0), g.lines), hi = min(g.lines, g.ih - y0);
+    for (int c = threadIdx.x - first * g.cols; c < g.span && first < g.line_step; c += g.cols) {
+        const int xs = (int)g.by_sw((uint32_t)c), x = c - g.pw;
+        const bool in = x >= 0 && x < g.iw;
+        float *to = tile + (c - xs * g.sw) * g.phase + xs;
+        // every load is of an address that exists, so that none waits behind a branch of another
+        const float *from = img + y0 * g.iw + min(max(x, 0), g.iw - 1);
+        int line = lo + first;
+        if (hi - lo > 2 * g.line_step) {
+            for (; line < hi; line += kBoxAhead * g.line_step) {
+                float v[kBoxAhead];
+#pragma unroll
+                for (int i = 0; i < kBoxAhead; i++)
+                    v[i] = __ldg(from + min(line + i * g.line_step, hi - 1) * g.iw);
+#pragma unroll
+                for (int i = 0; i < kBoxAhead; i++)
+                    if (line + i * g.line_step < hi)
+                        to[(line + i * g.line_step) * pitch] = in ? __fmul_rn(v[i], g.inv_khw) : 0.f;
+            }
+        } else if (line < hi) {  // one line a thread, or two
+            const int other = min(line + g.line_step, hi - 1);
+            const float u = __ldg(from + line * g.iw), v = __ldg(from + other * g.iw);
+            to[line * pitch] = in ? __fmul_rn(u, g.inv_khw) : 0.f;
+            if (line + g.line_step < hi) to[other * pitch] = in ? __fmul_rn(v, g.inv_khw) : 0.f;
+        }
+        for (int line = first; line < lo; line += g.line_step) to[line * pitch] = 0.f;
+        for (int line = max(hi, 0) + first; line < g.lines; line += g.line_step) to[line * pitch] = 0.f;
     }
     __syncthreads();
+    const int n_out = (TWO ? g.rows >> 1 : g.rows) * g.ow;
     for (int o = threadIdx.x; o < n_out; o += kBoxThreads) {
-        const int r = (int)g.by_ow((uint32_t)o), x = o - r * g.ow;
+        const int q = (int)g.by_ow((uint32_t)o), x = o - q * g.ow, r = TWO ? 2 * q : q;
         const float *row = tile + r * g.sh * pitch + x;
-        float acc = 0.f;
-        for (int i = 0; i < g.kh; i++, row += pitch) {
-            if (KW > 0) {
-#pragma unroll
-                for (int j = 0; j < KW; j++) acc = __fadd_rn(acc, row[g.tap[j]]);
-            } else {
-                for (int j = 0, at = 0, rem = 0; j < g.kw; j++) {
-                    acc = __fadd_rn(acc, row[rem * g.phase + at]);
-                    if (++rem == g.sw) { rem = 0; at++; }
-                }
-            }
+        float upper = 0.f, lower = 0.f;
+        int i = 0;
+        if (TWO) {
+            for (; i < g.sh; i++, row += pitch) add_line<KW, SW, true, false>(g, row, upper, lower);
+            for (; i < g.kh; i++, row += pitch) add_line<KW, SW, true, true>(g, row, upper, lower);
+            for (; i < g.sh + g.kh; i++, row += pitch) add_line<KW, SW, false, true>(g, row, upper, lower);
+        } else {
+            for (; i < g.kh; i++, row += pitch) add_line<KW, SW, true, false>(g, row, upper, lower);
         }
-        g.k[((long)n * g.oh + oy0 + r) * g.ow + x] = acc;
+        float *to = g.k + ((long)n * g.oh + oy0 + r) * g.ow + x;
+        if (oy0 + r < g.oh) to[0] = upper;
+        if (TWO && oy0 + r + 1 < g.oh) to[g.ow] = lower;
     }
 }
 
@@ -400,6 +443,20 @@ __global__ void __launch_bounds__(kBoxThreads) box_filter_wide_kernel(const BoxA
         }
     }
     g.k[o] = acc;
+}
+
+using BoxFn = void (*)(BoxArgs);
+template <bool TWO>
+BoxFn box_kernel(int kw, int sw) {
+    if (sw == 1 && kw == 1) return box_filter_kernel<1, 1, TWO>;
+    if (sw == 1 && kw == 3) return box_filter_kernel<3, 1, TWO>;
+    if (sw == 1 && kw == 5) return box_filter_kernel<5, 1, TWO>;
+    if (sw == 1 && kw == 7) return box_filter_kernel<7, 1, TWO>;
+    if (sw == 2 && kw == 3) return box_filter_kernel<3, 2, TWO>;
+    if (sw == 2 && kw == 5) return box_filter_kernel<5, 2, TWO>;
+    if (sw == 2 && kw == 7) return box_filter_kernel<7, 2, TWO>;
+    if (sw == 4 && kw == 11) return box_filter_kernel<11, 4, TWO>;
+    return box_filter_kernel<0, 1, TWO>;
 }
 
 BinArgs bin_args(const Plan &p, const float *src, void *out, float *a) {
@@ -503,16 +560,17 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
     if (p.mb < 1 || p.oh < 1 || p.ow < 1) return cudaSuccess;
     g.span = (p.ow - 1) * p.sw + p.kw;
     g.phase = div_up_i(g.span, p.sw);
-    g.by_span = FastDiv((uint32_t)g.span); g.by_sw = FastDiv((uint32_t)p.sw);
-    g.by_ow = FastDiv((uint32_t)p.ow);
-    for (int j = 0; j < 11; j++) g.tap[j] = j % p.sw * g.phase + j / p.sw;
-    // about one output per thread, if the rows that takes fit shared memory
-    g.rows = kBoxThreads / p.ow;
-    if (g.rows < 1) g.rows = 1;
-    if (g.rows > p.oh) g.rows = p.oh;
+    g.by_sw = FastDiv((uint32_t)p.sw); g.by_ow = FastDiv((uint32_t)p.ow);
     auto lines = [&](int rows) { return (long)(rows - 1) * p.sh + p.kh; };
     auto bytes = [&](int rows) { return 4L * lines(rows) * g.phase * p.sw; };
-    while (g.rows > 1 && bytes(g.rows) > kBoxSmem) g.rows--;
+    // Two outputs a thread where their windows are large and share half of their lines at least (measured
+    // at 11 x 11 with stride 4: conv1 on 64 images 56.5 -> 55.7 us on one stream), else one; about one
+    // thread for each, if the rows that takes fit shared memory.
+    const int up = p.kh >= 2 * p.sh && p.kh * p.kw >= 49 && p.oh > 1 && bytes(2) <= kBoxSmem ? 2 : 1;
+    g.rows = up * (kBoxThreads / p.ow);
+    if (g.rows > div_up_i(p.oh, up) * up) g.rows = div_up_i(p.oh, up) * up;
+    if (g.rows < up) g.rows = up;
+    while (g.rows > up && bytes(g.rows) > kBoxSmem) g.rows -= up;
     note_launch();
     if (bytes(g.rows) > kBoxSmem) {
         g.row_blocks = p.mb;
@@ -524,12 +582,11 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
     g.row_blocks = div_up_i(p.oh, g.rows);
     g.lines = (int)lines(g.rows);
     const unsigned blocks = (unsigned)(p.mb * g.row_blocks);
-    auto kernel = p.kw == 1    ? box_filter_kernel<1>
-                  : p.kw == 3  ? box_filter_kernel<3>
-                  : p.kw == 5  ? box_filter_kernel<5>
-                  : p.kw == 7  ? box_filter_kernel<7>
-                  : p.kw == 11 ? box_filter_kernel<11>
-                               : box_filter_kernel<0>;
+    const int cols = div_up_i(g.span, 32) * 32;
+    g.cols = cols < kBoxThreads ? cols : kBoxThreads;
+    g.line_step = kBoxThreads / g.cols;
+    g.by_cols = FastDiv((uint32_t)g.cols);
+    auto kernel = up > 1 ? box_kernel<true>(p.kw, p.sw) : box_kernel<false>(p.kw, p.sw);
     // Launched under the tail of the packer, as the convolution is under its own: conv1 mb64 63.7 ->
     // 60.7 us a pass, the three upstream calls of an odd layer 20.6 -> 19.4.
     return launch_overlapped(kernel, dim3(blocks), dim3(kBoxThreads), (size_t)bytes(g.rows), s, 1, g);

@@ -13,11 +13,14 @@
 // their mean |x|, from blocks that pack nothing.
 //
 // Fewer than eight channels (fold_few_kernel): the eight nibbles of a word are neighbouring
-// columns. Both halves are bound by instruction issue, so a warp reads 32 neighbouring columns, a
-// vote turns their signs into one word of bits, and a thread, which keeps its place in the column,
-// takes eight bits from two words and spreads them to nibbles. AlexNet conv1 on 64 images (40 MB
-// in, 20 MB out): 22 us; 32 without the channels and the pair of words compiled in, 37-39 with a byte staged per value and a table lookup per word
-// (28 M warp instructions), 55 with every nibble fetched on its own.
+// columns. Bound by instruction issue, then by the loads in flight. A warp reads 32 neighbouring columns of
+// eight lines or column groups at once; a lane's eight signs are one word of nibbles, and a transposition
+// among eight lanes (three exchanges) makes it the word of eight neighbouring columns, zero where there is
+// no image. The second half then only shifts and masks pairs of words. AlexNet conv1 on 64 images (40 MB
+// in, 20 MB out), launched alone: 26.7 us and 21.3 M warp instructions with a vote per 32 signs, bits
+// spread to nibbles for every column that reads them; 20.8 us and 11.2 M now (a pass among others 55.0 ->
+// 50.6). Before that: 37-39 us with a byte staged per value and a table lookup per word, 55 with every nibble
+// fetched on its own.
 // Otherwise (fold_kernel) they are neighbouring channels of a pixel, put together once per pixel
 // and copied.
 #include "kernels.cuh"
@@ -28,8 +31,8 @@ namespace xb200 {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kTasks = 4;   // few channels: warp loads per channel before the first is used
+constexpr int kThreads = 256, kFewThreads = 128;
+constexpr int kTasks = 8;   // few channels: warp loads per channel before the first is used
 
 struct FoldArgs {
     const float *src;
@@ -38,85 +41,109 @@ struct FoldArgs {
     int ic, ih, iw, hw;
     int rows, sh, sw, ph, pw, kw;  // rows = Plan::fold_rows
     int hb, ow, span, words;       // packed row blocks and columns; words = 32-bit words per column
-    int pitch;                     // staged row: words (few channels: of 32 columns' bits)
+    int pitch;                     // staged row: words (few channels: of eight columns)
     int group;                     // channels staged at a time
     int row_blocks;                // blocks of sh rows that cover the image
     int nw;                        // words of a column per group of channels
     long img_stride, c_stride, px_stride;
     float inv_ic;
     int stage_off, table_off;      // bytes into dynamic shared memory
-    int chunks;                    // few channels: words of bits that hold a row's columns
+    int chunks;                    // few channels: 32 columns each, of a row
     FastDiv by_iw, by_nw, by_chunks;
 };
 
-// Eight bits to the low bits of eight nibbles.
-__device__ __forceinline__ uint32_t spread(uint32_t b) {
-    b = (b | (b << 12)) & 0x000F000Fu;
-    b = (b | (b << 6)) & 0x03030303u;
-    return (b | (b << 3)) & 0x11111111u;
-}
+// Eight lanes (numbered by `sub`) hold a word of eight nibbles each: nibble i of lane j becomes nibble j
+// of lane i. Three exchanges: halves, bytes, nibbles.
+struct NibbleTranspose {
+    uint32_t halves, bytes, keep;
+    int turn;
+    __device__ __forceinline__ explicit NibbleTranspose(int sub)
+        : halves(sub & 4 ? 0x3276u : 0x5410u), bytes(sub & 2 ? 0x3715u : 0x6240u),
+          keep(sub & 1 ? 0xF0F0F0F0u : 0x0F0F0F0Fu), turn(sub & 1 ? 28 : 4) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t w) const {
+        w = prmt(w, __shfl_xor_sync(0xffffffffu, w, 4), halves);
+        w = prmt(w, __shfl_xor_sync(0xffffffffu, w, 2), bytes);
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, w, 1);
+        return (w & keep) | (__funnelshift_l(other, other, turn) & ~keep);
+    }
+};
 
 // IC channels (0: up to seven, four at a time); TWO: a row of a filter is two words of a column,
 // which are put together and stored as one.
 template <bool WITH_A, int IC, bool TWO>
-__global__ void __launch_bounds__(kThreads) fold_few_kernel(const FoldArgs g) {
+__global__ void __launch_bounds__(kFewThreads) fold_few_kernel(const FoldArgs g) {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint32_t *bits = reinterpret_cast<uint32_t *>(smem);  // [channel][row][pitch], 1 = negative
+    uint32_t *nibbles = reinterpret_cast<uint32_t *>(smem);  // [channel][row][pitch], eight columns a word
+    constexpr int kWarps = kFewThreads / 32;
 
     const int n = blockIdx.x / g.row_blocks, hb = blockIdx.x - n * g.row_blocks;
     const int h0 = hb * g.sh - g.ph;  // input row of the block's first line
     const int lines = min(g.sh, g.ih - h0), first = h0 < 0 ? -h0 : 0;
     const bool packs = hb < g.hb;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // warp-uniform, and known to be: what depends on a task alone is computed once per warp
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     dependency_release();
+    // rows outside the image and what a column reaches past it are zeros
+    if (packs)
+        for (int i = threadIdx.x; i < g.ic * g.rows * g.pitch; i += kFewThreads) nibbles[i] = 0u;
+    __syncthreads();
     dependency_wait();
 
-    // a task is 32 neighbouring columns (borders included) of a line
+    // A task is 32 neighbouring columns (borders included) of a line; a warp has eight in flight. Their
+    // signs of a channel are a lane's eight nibbles, which transposed among eight lanes are the words of
+    // eight columns that are wanted: lane l gets columns 8 (l / 8) ... of task l % 8.
     const float *img = g.src + n * g.img_stride + (long)h0 * g.iw * g.px_stride;
     float *a = g.a + (long)n * g.hw + (long)h0 * g.iw;
     const int tasks = lines * g.chunks;
-    for (int t0 = first * g.chunks + warp; t0 < tasks; t0 += kTasks * kThreads / 32) {
+    const NibbleTranspose transpose(lane & 7);
+    for (int t0 = first * g.chunks + warp; t0 < tasks; t0 += kTasks * kWarps) {
         float acc[kTasks] = {};
-        int px[kTasks];  // pixel of this lane, or -1
+        unsigned px[kTasks];  // pixel of this lane, from the line h0 on
+        uint32_t exist = 0;   // nibble k: the lane's column of task k is in the image
 #pragma unroll
         for (int k = 0; k < kTasks; k++) {
-            const int t = t0 + k * kThreads / 32;
+            const int t = t0 + k * kWarps;
             const int line = (int)g.by_chunks((uint32_t)t);
             const int ix = 32 * (t - line * g.chunks) + lane - g.pw;
-            px[k] = t < tasks && ix >= 0 && ix < g.iw ? line * g.iw + ix : -1;
+            px[k] = (unsigned)(line * g.iw + ix);
+            if (t < tasks && (unsigned)ix < (unsigned)g.iw) exist |= 0xFu << (4 * k);
         }
+        // the task whose words this lane stores
+        const int mine = t0 + (lane & 7) * kWarps, my_line = (int)g.by_chunks((uint32_t)mine);
+        const bool keep = packs && mine < tasks && my_line < g.rows;
+        uint32_t *to = nibbles + my_line * g.pitch + 4 * (mine - my_line * g.chunks) + (lane >> 3);
         constexpr int NC = IC > 0 ? IC : 4;
         const int ic = IC > 0 ? IC : g.ic;
         for (int c = 0; c < ic; c += NC) {
-            float v[kTasks][NC];
+            float v[NC][kTasks];
 #pragma unroll
-            for (int k = 0; k < kTasks; k++) {
-                const float *s = img + px[k] * (int)g.px_stride + c * g.c_stride;
+            for (int i = 0; i < NC; i++) {
+                // a warp-uniform channel plane and a lane's 32-bit offset into the row block
+                const char *plane = reinterpret_cast<const char *>(img + (c + i) * g.c_stride);
+                const unsigned size = 4u * (unsigned)g.px_stride;
 #pragma unroll
-                for (int i = 0; i < NC; i++)
-                    v[k][i] = px[k] >= 0 && c + i < ic ? __ldg(s + i * g.c_stride) : 0.f;
+                for (int k = 0; k < kTasks; k++)
+                    v[i][k] = (exist >> (4 * k) & 1u) && c + i < ic
+                                  ? __ldg(reinterpret_cast<const float *>(plane + px[k] * size))
+                                  : 0.f;
             }
 #pragma unroll
-            for (int k = 0; k < kTasks; k++) {
-                const int t = t0 + k * kThreads / 32;
-                const int line = (int)g.by_chunks((uint32_t)t);
-                const bool keep = packs && t < tasks && line < g.rows;  // the same in all lanes
-                uint32_t *to = bits + (c * g.rows + line) * g.pitch + (t - line * g.chunks);
+            for (int i = 0; i < NC; i++) {
+                if (c + i >= ic) break;
+                const uint32_t w =
+                    transpose(sign_nibbles(reinterpret_cast<const uint32_t *>(v[i])) & exist);
+                if (keep) to[(c + i) * g.rows * g.pitch] = w;
+                if (WITH_A) {
 #pragma unroll
-                for (int i = 0; i < NC; i++) {
-                    if (c + i >= ic) break;
-                    if (WITH_A) acc[k] = __fadd_rn(acc[k], __fmul_rn(fabsf(v[k][i]), g.inv_ic));
-                    if (keep) {
-                        const uint32_t b = __ballot_sync(0xffffffffu, __float_as_int(v[k][i]) < 0);
-                        if (lane == 0) to[i * g.rows * g.pitch] = b;
-                    }
+                    for (int k = 0; k < kTasks; k++)
+                        acc[k] = __fadd_rn(acc[k], __fmul_rn(fabsf(v[i][k]), g.inv_ic));
                 }
             }
         }
         if (WITH_A) {
 #pragma unroll
             for (int k = 0; k < kTasks; k++)
-                if (px[k] >= 0) a[px[k]] = acc[k];
+                if (exist >> (4 * k) & 1u) a[px[k]] = acc[k];
         }
     }
     if (!packs) return;
@@ -124,35 +151,27 @@ __global__ void __launch_bounds__(kThreads) fold_few_kernel(const FoldArgs g) {
 
     // Item w of a column: a word, i.e. eight columns q of row i of channel c, or both of a row's two.
     // Threads are dealt whole columns' worth of items, so that a thread keeps its w.
-    constexpr int SPAN = TWO ? 16 : 8;
     const int per = TWO ? 1 : (g.kw + 7) / 8;
-    const int groups = g.nw < kThreads ? (int)g.by_nw(kThreads) : 1;
-    const int group = g.nw < kThreads ? (int)g.by_nw(threadIdx.x) : 0;
+    const int groups = g.nw < kFewThreads ? (int)g.by_nw(kFewThreads) : 1;
+    const int group = g.nw < kFewThreads ? (int)g.by_nw(threadIdx.x) : 0;
     if (group >= groups) return;
     uint32_t *out = g.out + ((long)n * g.hb + hb) * g.ow * g.words;
-    for (int w = threadIdx.x - group * g.nw; w < g.nw; w += kThreads) {
-        const int f = w / per, q = w - f * per, i = f % g.rows;
-        const bool row_in = h0 + i >= 0 && h0 + i < g.ih;
-        const int left = row_in ? g.kw - 8 * q : 0;
-        const uint32_t exist0 = first_nibbles(0xFFFFFFFFu, left);
-        const uint32_t exist1 = TWO ? first_nibbles(0xFFFFFFFFu, left - 8) : 0u;
-        const uint32_t *row = bits + f * g.pitch;
-        for (int col = group; col < g.ow; col += groups) {
-            const int x = col * g.sw + 8 * q;  // border columns in front included
-            uint32_t b = 0, mask0 = exist0, mask1 = exist1;
-            if (row_in) b = __funnelshift_r(row[x >> 5], row[(x >> 5) + 1], x & 31);
-            if (x < g.pw || x + SPAN > g.pw + g.iw) {  // columns outside the image
-                const int before = g.pw - x, inside = g.pw + g.iw - x;
-                mask0 = first_nibbles(mask0, inside) & ~first_nibbles(0xFFFFFFFFu, before);
-                if (TWO)
-                    mask1 = first_nibbles(mask1, inside - 8) & ~first_nibbles(0xFFFFFFFFu, before - 8);
-            }
-            const uint32_t w0 = ((spread(b & 0xFFu) << 3) | 0x22222222u) & mask0;
+    for (int w = threadIdx.x - group * g.nw; w < g.nw; w += kFewThreads) {
+        const int f = w / per, q = w - f * per;
+        const uint32_t mask0 = first_nibbles(0xFFFFFFFFu, g.kw - 8 * q);
+        const uint32_t mask1 = TWO ? first_nibbles(0xFFFFFFFFu, g.kw - 8) : 0u;
+        const uint32_t *row = nibbles + f * g.pitch;
+        uint32_t *o = out + group * g.words + (TWO ? 2 * w : w);
+        int x = group * g.sw + 8 * q;  // border columns in front included
+        for (int col = group; col < g.ow; col += groups, x += groups * g.sw, o += groups * g.words) {
+            const uint32_t *at = row + (x >> 3);
+            const uint32_t b0 = at[0], b1 = at[1];
+            const uint32_t w0 = __funnelshift_r(b0, b1, 4 * (x & 7)) & mask0;
             if (TWO) {
-                const uint32_t w1 = ((spread((b >> 8) & 0xFFu) << 3) | 0x22222222u) & mask1;
-                *reinterpret_cast<uint2 *>(out + col * g.words + 2 * w) = make_uint2(w0, w1);
+                const uint32_t w1 = __funnelshift_r(b1, at[2], 4 * (x & 7)) & mask1;
+                *reinterpret_cast<uint2 *>(o) = make_uint2(w0, w1);
             } else {
-                out[col * g.words + w] = w0;
+                *o = w0;
             }
         }
     }
@@ -271,7 +290,7 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
     g.chunks = div_up_i(p.iw + p.pw, 32);
     g.by_chunks = FastDiv((uint32_t)g.chunks);
     const bool two = few && p.fold_field == 16;
-    g.pitch = few ? fold_bit_pitch(p) : p.fold_span;
+    g.pitch = few ? 4 * fold_bit_pitch(p) : p.fold_span;
     const int n8 = div_up_i(p.fold_channels, 8);
     g.nw = few ? p.ic * p.fold_rows * (two ? 1 : p.fold_field / 8) : p.fold_rows * p.kw * n8;
     g.by_nw = FastDiv((uint32_t)g.nw);
@@ -285,7 +304,12 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
     int dev = 0;
     cudaGetDevice(&dev);
     std::atomic<bool> &done = opted_in[dev & 63][a ? 1 : 0];
-    // few channels: the bits fit the 48 KB that need no opt-in (fold_ok)
+    // Few channels: fold_ok counts a bit a value, four of which take 192 KB at most.
+    if (few && smem > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+    }
     if (!few && !done.load(std::memory_order_acquire)) {
         const cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
@@ -293,8 +317,8 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
         done.store(true, std::memory_order_release);
     }
     note_launch();
-    return launch_overlapped(kernel, dim3((unsigned)(p.mb * g.row_blocks)), dim3(kThreads), smem, s,
-                             1, g);
+    return launch_overlapped(kernel, dim3((unsigned)(p.mb * g.row_blocks)),
+                             dim3(few ? kFewThreads : kThreads), smem, s, 1, g);
 }
 
 }  // namespace xb200
