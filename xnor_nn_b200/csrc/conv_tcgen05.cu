@@ -20,8 +20,8 @@
 //   warp 1      allocates tensor memory; an elected lane issues tcgen05.mma.kind::mxf4 (M=128,
 //               N<=256, K=64 per instruction) into one of two to four accumulators in tensor
 //               memory, and tcgen05.commit hands buffers back / accumulators on
-//   warp 18     a second MMA issuer; the two take alternate ring buffers
-//   warps 2-17  epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
+//   warp 10     a second MMA issuer; the two take alternate ring buffers
+//   warps 2-9   epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
 //               and a share of the columns), scale by alpha[filter] * K[position] in upstream's
 //               order and store; runs under the next tiles' MMAs thanks to the other
 //               accumulators
@@ -63,7 +63,11 @@ using namespace tc;
 
 constexpr int BM = 128;            // positions per tile = UMMA M = TMEM lanes
 constexpr int kMaxStages = 8;       // ring buffers: as many as fit, at most this
-constexpr int kEpiWarps = 16;       // epilogue warps: 4 TMEM lane quadrants x column groups
+// Epilogue warps: 4 TMEM lane quadrants x column groups. With 16 instead of 8 every pass is a little slower
+// (among others, on one stream, us): conv2 on 128 images 45.1 and 47.9 against 44.1 and 45.6, conv3 on 256
+// 33.9 and 37.3 against 33.1 and 37.5, VGG 72.9 and 74.9 against 71.8 and 74.4, conv4 38.0 and 41.9 against
+// 37.1 and 41.6: the stores of a tile have the next tile's MMAs to hide behind either way.
+constexpr int kEpiWarps = 8;
 constexpr int kIssuer2Warp = 2 + kEpiWarps;  // the second MMA-issuing thread lives in a warp of its own
 constexpr int kThreads = 64 + 32 * kEpiWarps + 32;
 // Tensor memory: two to four accumulators of n_tile columns and, in the last 16 columns, the block
@@ -78,6 +82,7 @@ constexpr int kMaxASlots = 8;        // halo tiles in flight
 
 // ---- the kernel --------------------------------------------------------------------------------
 
+constexpr int kSums = 4;  // chained layers: sums of |y| per filter tile, every fourth 32 filters each
 constexpr int kAlphaSmem = 2048;  // filters whose alpha is staged in shared memory
 
 
@@ -94,7 +99,7 @@ struct __align__(16) Control {
     uint32_t tmem_base;
     int abort_flag;
     alignas(16) float alpha[kAlphaSmem];  // read with 16-byte loads
-    float fold[2][4][kEpiWarps / 4][32];  // chained layers: per-warp partial sums of |y|
+    float fold[2][4][kSums][32];  // chained layers: partial sums of |y|
 };
 constexpr int kControlBytes = (sizeof(Control) + 1023) / 1024 * 1024;
 static_assert(offsetof(Control, alpha) % 16 == 0, "alpha is read as float4");
@@ -155,7 +160,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
     const uint32_t shared_free0 =
         PAIR ? mapa(smem_u32(&ctl->shared_free), 0) : smem_u32(&ctl->shared_free);
     // Several warps share a quadrant and split its columns between them. The warps form
-    // one, two or four teams that take the tiles in turn: what a tile costs an epilogue warp is
+    // one or two teams that take the tiles in turn: what a tile costs an epilogue warp is
     // mostly latency (its pixel's K, the accumulator's barrier, the loads from tensor memory, the
     // stores going out), and tiles of different teams overlap it.
     const int quad = warp & 3;
@@ -240,7 +245,9 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                            ((long)g.e_lead + ((long)n * g.e_hp + oh) * g.e_wp + ow) * g.e_icp +
                            oc0 / 2;
             const int room = g.e_icp - oc0 / 2;  // bytes of the row from here on
-            float part = 0.f;
+            // two sums a warp, of alternate groups of 32 filters
+            float part = 0.f, other = 0.f;
+            int groups = 0;
             // The partial sum is added up in ascending order whichever accumulator the tile is in:
             // shared columns at the end (the last 16 of 256) are fetched first and kept.
             uint32_t kept[16];
@@ -249,7 +256,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                 wait_ld();
                 columns_read(0);
             }
-            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups) {
+            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups, groups++) {
                 uint32_t v[32];
                 const int width = g.n_tile - c0 >= 32 ? 32 : 16;
                 if (reverse && c0 + 32 == g.n_tile) {
@@ -300,16 +307,21 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                             *reinterpret_cast<uint2 *>(o + 8) = make_uint2(w[2], w[3]);
                     }
                 }
+                const float t = part;
+                part = other;
+                other = t;
             }
-            // Fold the column groups' partial sums in a fixed order (group 0, 1, 2, 3, then the
-            // next filter tile), so the map is reproducible; the four warps of a lane quadrant
-            // meet on a named barrier of their own.
-            ctl->fold[it & 1][quad][cgroup][lane] = part;
+            // Fold the partial sums in a fixed order (group 0, 1, 2, 3, then the next filter tile), so the
+            // map is reproducible; the warps of a lane quadrant meet on a named barrier of their own.
+            static_assert(kSums == 2 * (kEpiWarps / 4), "two sums a warp");
+            const bool even = !(groups & 1);
+            ctl->fold[it & 1][quad][cgroup][lane] = even ? part : other;
+            ctl->fold[it & 1][quad][cgroup + kEpiWarps / 4][lane] = even ? other : part;
             bar_sync(1 + quad, 32 * (kEpiWarps / 4));
             if (cgroup == 0) {
                 if (nt == 0) run = 0.f;
 #pragma unroll
-                for (int c = 0; c < kEpiWarps / 4; c++)
+                for (int c = 0; c < kSums; c++)
                     run = __fadd_rn(run, ctl->fold[it & 1][quad][c][lane]);
                 if (nt == g.n_tiles - 1 && valid)
                     g.emit_a[pix] = __fmul_rn(__fmul_rn(run, kk), g.e_inv_ic);
@@ -1350,14 +1362,13 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
                         : (size_t)g.n_stages * g.stage_bytes);
     // At least 120 KB of shared memory so that one CTA owns the SM and all 512 TMEM columns.
     if (smem < 120 * 1024) smem = 120 * 1024;
-    // As many accumulators as fit (at most four), and one epilogue team for each of two or four of
-    // them if a CTA has that many tiles. With all 16 warps on every tile AlexNet conv3 (256
-    // images) took 41.3 us per pass, conv1 (64 images) 86, with two teams 37.7 and 79. The chained
-    // epilogue carries per-pixel state from one filter tile to the next: one team.
+    // As many accumulators as fit (at most four), and two epilogue teams if a CTA has that many tiles. With
+    // all warps (16 then) on every tile AlexNet conv3 (256 images) took 41.3 us per pass, conv1 (64 images)
+    // 86, with two teams 37.7 and 79. The chained epilogue carries per-pixel state from one filter tile to the next: one team.
     const int rounds = g.n_inner ? 1 : div_up_i(units, grid);
     g.n_acc = g.shared_cols || g.n_inner ? 2 : (int)kScaleCol / p.n_tile;
     if (g.n_acc > kMaxAcc) g.n_acc = kMaxAcc;
-    g.teams = g.n_acc == 4 && rounds >= 4 ? 4 : rounds >= 2 ? 2 : 1;
+    g.teams = rounds >= 2 ? 2 : 1;
     g.by_acc = FastDiv((uint32_t)g.n_acc);
     note_launch();
     return launch_overlapped(kernel, dim3((pair ? 2 : 1) * grid), dim3(kThreads), smem, s,
