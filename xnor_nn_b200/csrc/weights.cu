@@ -279,32 +279,47 @@ __global__ void __launch_bounds__(kWfThreads) wf_partial_kernel(const float *fro
     if (threadIdx.x == 0) partial[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kWfThreads) wf_scale_kernel(const float *from, float *to,
+// Elements begin .. elems.
+__global__ void __launch_bounds__(kWfThreads) wf_scale_kernel(const float *from, float *to, long begin,
                                                               long elems, const float *partial,
                                                               float inv_elems) {
     __shared__ float sh[kWfThreads];
     const float mean = __fmul_rn(fold256(partial[threadIdx.x], sh), inv_elems);
-    for (long i = (long)blockIdx.x * kWfThreads + threadIdx.x; i < elems;
+    for (long i = begin + (long)blockIdx.x * kWfThreads + threadIdx.x; i < elems;
          i += (long)gridDim.x * kWfThreads)
         to[i] = __fmul_rn(from[i] >= .0f ? 1.f : -1.f, mean);
 }
 }  // namespace
 
+// The block sums need 1 KB of scratch. The result itself serves, where it has that much and is not also
+// the source: its first 256 elements hold the sums until everything behind them is written, then a block
+// that has read them overwrites them. Stream-ordered scratch, which the other cases take, costs the host
+// 20 us a call (a training step of one layer 258 -> 238 us), and where the stream is waited for between
+// calls, so that its memory goes back each time, 500 and more.
 cudaError_t launch_binarize_weights_float(long elems, const float *from, float *to,
                                           cudaStream_t s) {
-    float *partial = nullptr;
-    cudaError_t e = cudaMallocAsync(&partial, kWfBlocks * sizeof(float), s);
-    if (e != cudaSuccess) return e;
+    const bool in_result = elems >= 2 * kWfBlocks && (to + elems <= from || from + elems <= to);
+    float *partial = to;
+    if (!in_result) {
+        const cudaError_t e = cudaMallocAsync(&partial, kWfBlocks * sizeof(float), s);
+        if (e != cudaSuccess) return e;
+    }
     wf_partial_kernel<<<kWfBlocks, kWfThreads, 0, s>>>(from, elems, partial);
     note_launch();
-    long blocks = (elems + kWfThreads - 1) / kWfThreads;
+    const long begin = in_result ? kWfBlocks : 0;
+    const float inv = 1.f / (float)elems;
+    long blocks = (elems - begin + kWfThreads - 1) / kWfThreads;
     if (blocks > 1184) blocks = 1184;
     if (blocks < 1) blocks = 1;
-    wf_scale_kernel<<<(unsigned)blocks, kWfThreads, 0, s>>>(from, to, elems, partial,
-                                                            1.f / (float)elems);
+    wf_scale_kernel<<<(unsigned)blocks, kWfThreads, 0, s>>>(from, to, begin, elems, partial, inv);
     note_launch();
-    e = cudaGetLastError();
-    const cudaError_t f = cudaFreeAsync(partial, s);
+    if (in_result) {
+        static_assert(kWfBlocks == kWfThreads, "one block reads all sums before it writes");
+        wf_scale_kernel<<<1, kWfThreads, 0, s>>>(from, to, 0, begin, partial, inv);
+        note_launch();
+    }
+    const cudaError_t e = cudaGetLastError();
+    const cudaError_t f = in_result ? cudaSuccess : cudaFreeAsync(partial, s);
     return e != cudaSuccess ? e : f;
 }
 
