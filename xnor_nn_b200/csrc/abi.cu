@@ -281,6 +281,12 @@ xnor_nn_status_t exec_calculate_k(const xnor_nn_convolution_t *c, xnor_nn_resour
         xnor_nn_status_t st =
             stage_in(x, 0, res[xnor_nn_resource_user_src], src_bytes(*p), &src, &staged);
         if (st != xnor_nn_success) return st;
+        if (maps_ok(*p)) {
+            CU(launch_maps(*p, (const float *)src, (float *)res[xnor_nn_resource_a],
+                           (float *)res[xnor_nn_resource_k], x->error_word, x->stream));
+            if (staged) CU(cudaStreamSynchronize(x->stream));
+            return xnor_nn_success;
+        }
         CU(launch_mean_abs(*p, (const float *)src, (float *)res[xnor_nn_resource_a], x->stream));
     }
     CU(launch_box_filter(*p, (const float *)res[xnor_nn_resource_a],

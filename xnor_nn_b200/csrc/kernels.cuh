@@ -105,6 +105,12 @@ cudaError_t launch_mean_abs(const Plan &p, const float *src, float *a, cudaStrea
 // Replaces the second loop of upstream src/bcast_calculate_k.cpp:69-85.
 cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStream_t s);
 
+// Both in one launch, for the small layers that maps_ok() names (maps.cu). `error_word` as for the
+// convolutions below.
+bool maps_ok(const Plan &p);
+cudaError_t launch_maps(const Plan &p, const float *src, float *a, float *k, int *error_word,
+                        cudaStream_t s);
+
 // ---- weights ---------------------------------------------------------------------------------
 // Sign-pack into the family's layout, alpha[oc] = mean |w|, op_c[oh][ow] = IC * taps inside.
 // Replaces upstream src/bcast_binarize_weights.cpp:54-142.

@@ -1,0 +1,139 @@
+// Packing the source by tasks of 32 neighbouring pixels x 32 channels, a task a warp (conv_whole.cu,
+// maps.cu): loads, and the sum of |x| over the channels in upstream's order, which tasks of the same pixels
+// hand on from warp to warp.
+#pragma once
+
+#include "kernels.cuh"
+#include "tc_ptx.cuh"
+
+namespace xb200 {
+namespace tasks {
+
+// 32 channels of 32 pixels, channels-last: eight lanes read a pixel's channels with 16-byte loads, four
+// pixels at a time, and an 8 x 8 transposition of those quadruples leaves a lane with all channels of
+// pixel 4 (lane % 8) + lane / 8.
+__device__ __forceinline__ void transpose8(float *v, int sub) {
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) {
+        const bool up = sub & d;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (j & d) continue;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                // the quadruple that goes to the partner: j + d from the lower lane, j from the upper
+                const float send = up ? v[4 * j + i] : v[4 * (j + d) + i];
+                const float got = __shfl_xor_sync(0xffffffffu, send, d);
+                if (up) v[4 * j + i] = got;
+                else v[4 * (j + d) + i] = got;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void mul2(float &a, float &b, float by) {
+    asm("{\n\t.reg .b64 x, y;\n\t"
+        "mov.b64 x, {%0, %1};\n\t"
+        "mov.b64 y, {%2, %2};\n\t"
+        "mul.rn.f32x2 x, x, y;\n\t"
+        "mov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(a), "+f"(b)
+        : "f"(by));
+}
+
+// Whose turn it is to add: a counter, since a warp may wait for it from several columns ahead, where an
+// mbarrier's parity says nothing. Bounded like every wait.
+__device__ __forceinline__ int turn_of(const int *turn) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(tc::smem_u32(turn)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void turn_pass(int *turn, int next) {
+    asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(turn)), "r"(next) : "memory");
+}
+__device__ __forceinline__ bool turn_wait(const int *turn, int want, volatile int *abort_flag, int *error,
+                                          unsigned long long limit_ns) {
+    bool ok = turn_of(turn) == want;
+    if (!ok) {
+        const unsigned long long t0 = tc::global_ns();
+        for (;;) {
+            for (int i = 0; i < 64 && !ok; i++) ok = turn_of(turn) == want;
+            if (ok || *abort_flag) break;
+            if (tc::global_ns() - t0 > limit_ns) {
+                *abort_flag = 1;
+                atomicCAS(error, 0, 21);
+                break;
+            }
+        }
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+// `tile`: its pixels first .. last, in groups of 32; `g`: the source.
+template <bool NHWC, class Args, class Tile>
+__device__ __forceinline__ void load_task(const Args &g, const Tile &tile, int t, int lane, float *v) {
+    const int col = t / tile.groups, gr = t - col * tile.groups;
+    const int c0 = 32 * col, nc = min(32, g.ic - c0);
+    if (NHWC && g.vec) {
+        const int sub = lane & 7, px = tile.first + 32 * gr + (lane >> 3);
+        const float *p = g.src + (long)px * g.ic + c0 + 4 * sub;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (px + 4 * j < tile.last && 4 * sub < nc)
+                x = __ldg(reinterpret_cast<const float4 *>(p + (long)(4 * j) * g.ic));
+            v[4 * j] = x.x; v[4 * j + 1] = x.y; v[4 * j + 2] = x.z; v[4 * j + 3] = x.w;
+        }
+        return;
+    }
+    const int px = tile.first + 32 * gr + lane;
+    const bool live = px < tile.last;
+    if (NHWC) {
+        const float *p = g.src + (long)px * g.ic + c0;
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] = live && i < nc ? __ldg(p + i) : 0.f;
+        return;
+    }
+    // an address is a warp-uniform channel plane and a lane's 32-bit offset into it (the host checks
+    // the range)
+    const unsigned n = live ? g.by_hw((uint32_t)px) : 0, r = live ? px - n * g.hw : 0;
+    const unsigned at = 4u * (n * (unsigned)(g.ic * g.hw) + r);
+    const char *plane = reinterpret_cast<const char *>(g.src) + (size_t)c0 * g.hw * 4;
+    const size_t pitch = (size_t)g.hw * 4;
+    if (live && nc == 32) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] = __ldg(reinterpret_cast<const float *>(plane + i * pitch + at));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+            v[i] = live && i < nc ? __ldg(reinterpret_cast<const float *>(plane + i * pitch + at)) : 0.f;
+    }
+}
+
+// Adds the task's |x| / IC to the sum of the channels before it, once those have been added; v is used
+// up. The caller passes the turn on (or has the mean, after the last channels).
+__device__ __forceinline__ bool add_task(float *v, int nc, int col, float inv_ic, const int *turn,
+                                         const float *sum, volatile int *abort_flag, int *error,
+                                         unsigned long long limit_ns, float *out) {
+    // |x| / IC = |x / IC|: two products an instruction, the sign goes with the addition
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) mul2(v[i], v[i + 1], inv_ic);
+    float acc = 0.f;
+    if (col > 0) {
+        if (!turn_wait(turn, col, abort_flag, error, limit_ns)) return false;
+        acc = *(const volatile float *)sum;
+    }
+    if (nc == 32) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) acc = __fadd_rn(acc, fabsf(v[i]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+            if (i < nc) acc = __fadd_rn(acc, fabsf(v[i]));
+    }
+    *out = acc;
+    return true;
+}
+
+}  // namespace tasks
+}  // namespace xb200
