@@ -20,8 +20,8 @@
 //   warp 1      allocates tensor memory; an elected lane issues tcgen05.mma.kind::mxf4 (M=128,
 //               N<=256, K=64 per instruction) into one of two to four accumulators in tensor
 //               memory, and tcgen05.commit hands buffers back / accumulators on
-//   warp 10     a second MMA issuer; the two take alternate ring buffers
-//   warps 2-9   epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
+//   warp 18     a second MMA issuer; the two take alternate ring buffers
+//   warps 2-17  (in pairs with long tiles 2-9, and the second issuer 10) epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
 //               and a share of the columns), scale by alpha[filter] * K[position] in upstream's
 //               order and store; runs under the next tiles' MMAs thanks to the other
 //               accumulators
@@ -63,13 +63,8 @@ using namespace tc;
 
 constexpr int BM = 128;            // positions per tile = UMMA M = TMEM lanes
 constexpr int kMaxStages = 8;       // ring buffers: as many as fit, at most this
-// Epilogue warps: 4 TMEM lane quadrants x column groups. With 16 instead of 8 every pass is a little slower
-// (among others, on one stream, us): conv2 on 128 images 45.1 and 47.9 against 44.1 and 45.6, conv3 on 256
-// 33.9 and 37.3 against 33.1 and 37.5, VGG 72.9 and 74.9 against 71.8 and 74.4, conv4 38.0 and 41.9 against
-// 37.1 and 41.6: the stores of a tile have the next tile's MMAs to hide behind either way.
-constexpr int kEpiWarps = 8;
-constexpr int kIssuer2Warp = 2 + kEpiWarps;  // the second MMA-issuing thread lives in a warp of its own
-constexpr int kThreads = 64 + 32 * kEpiWarps + 32;
+constexpr int kEpiWarps = 16;       // epilogue warps: 4 TMEM lane quadrants x column groups;
+constexpr int kFewEpiWarps = 8;     // in pairs whose tiles are long (launch_conv_tcgen05)
 // Tensor memory: two to four accumulators of n_tile columns and, in the last 16 columns, the block
 // scales. 2 x 256 + 16 is more than the 512 there are, so accumulators of 256 columns share 16 of them
 // (the last of the first = the first of the second): the epilogue empties those before anything
@@ -80,9 +75,11 @@ constexpr int kAccStep = 240;        // columns between the accumulators' starts
 constexpr int kMaxAcc = 4;
 constexpr int kMaxASlots = 8;        // halo tiles in flight
 
+// The second MMA issuer is a warp of its own, behind the epilogue's.
+constexpr int threads_of(int epi_warps) { return 64 + 32 * epi_warps + 32; }
+
 // ---- the kernel --------------------------------------------------------------------------------
 
-constexpr int kSums = 4;  // chained layers: sums of |y| per filter tile, every fourth 32 filters each
 constexpr int kAlphaSmem = 2048;  // filters whose alpha is staged in shared memory
 
 
@@ -99,7 +96,7 @@ struct __align__(16) Control {
     uint32_t tmem_base;
     int abort_flag;
     alignas(16) float alpha[kAlphaSmem];  // read with 16-byte loads
-    float fold[2][4][kSums][32];  // chained layers: partial sums of |y|
+    float fold[2][4][kEpiWarps / 4][32];  // chained layers: per-warp partial sums of |y|
 };
 constexpr int kControlBytes = (sizeof(Control) + 1023) / 1024 * 1024;
 static_assert(offsetof(Control, alpha) % 16 == 0, "alpha is read as float4");
@@ -148,7 +145,7 @@ __device__ __forceinline__ float scaled(uint32_t s, float alpha, float k) {
 // ---- epilogue role ---------------------------------------------------------------------------------
 // Warp w may touch TMEM lanes [32*(w%4), 32*(w%4)+32); several warps share a quadrant and split
 // its columns between them.
-template <bool PAIR>
+template <bool PAIR, int EPI>
 __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                               int warp, int lane, bool alpha_in_smem) {
     volatile int *abort_flag = &ctl->abort_flag;
@@ -160,11 +157,11 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
     const uint32_t shared_free0 =
         PAIR ? mapa(smem_u32(&ctl->shared_free), 0) : smem_u32(&ctl->shared_free);
     // Several warps share a quadrant and split its columns between them. The warps form
-    // one or two teams that take the tiles in turn: what a tile costs an epilogue warp is
+    // one, two or four teams that take the tiles in turn: what a tile costs an epilogue warp is
     // mostly latency (its pixel's K, the accumulator's barrier, the loads from tensor memory, the
     // stores going out), and tiles of different teams overlap it.
     const int quad = warp & 3;
-    const int cgroups = kEpiWarps / 4 / g.teams, team = (warp - 2) / (4 * cgroups);
+    const int cgroups = EPI / 4 / g.teams, team = (warp - 2) / (4 * cgroups);
     const int cgroup = ((warp - 2) >> 2) - team * cgroups;
     const int frame = g.hp * g.wp;
     const long ohw = (long)g.oh * g.ow;
@@ -214,7 +211,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
             // on a named barrier once per tile; a warp that has given up keeps that appointment
             // so that one that has not (yet) cannot be left waiting there.
             if (emits) {
-                bar_sync(1 + quad, 32 * (kEpiWarps / 4));
+                bar_sync(1 + quad, 32 * (EPI / 4));
                 continue;
             }
             break;
@@ -245,9 +242,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                            ((long)g.e_lead + ((long)n * g.e_hp + oh) * g.e_wp + ow) * g.e_icp +
                            oc0 / 2;
             const int room = g.e_icp - oc0 / 2;  // bytes of the row from here on
-            // two sums a warp, of alternate groups of 32 filters
-            float part = 0.f, other = 0.f;
-            int groups = 0;
+            float part = 0.f;
             // The partial sum is added up in ascending order whichever accumulator the tile is in:
             // shared columns at the end (the last 16 of 256) are fetched first and kept.
             uint32_t kept[16];
@@ -256,7 +251,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                 wait_ld();
                 columns_read(0);
             }
-            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups, groups++) {
+            for (int c0 = 32 * cgroup; c0 < g.n_tile; c0 += 32 * cgroups) {
                 uint32_t v[32];
                 const int width = g.n_tile - c0 >= 32 ? 32 : 16;
                 if (reverse && c0 + 32 == g.n_tile) {
@@ -307,21 +302,16 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                             *reinterpret_cast<uint2 *>(o + 8) = make_uint2(w[2], w[3]);
                     }
                 }
-                const float t = part;
-                part = other;
-                other = t;
             }
-            // Fold the partial sums in a fixed order (group 0, 1, 2, 3, then the next filter tile), so the
-            // map is reproducible; the warps of a lane quadrant meet on a named barrier of their own.
-            static_assert(kSums == 2 * (kEpiWarps / 4), "two sums a warp");
-            const bool even = !(groups & 1);
-            ctl->fold[it & 1][quad][cgroup][lane] = even ? part : other;
-            ctl->fold[it & 1][quad][cgroup + kEpiWarps / 4][lane] = even ? other : part;
-            bar_sync(1 + quad, 32 * (kEpiWarps / 4));
+            // Fold the column groups' partial sums in a fixed order (group 0, 1, 2, 3, then the
+            // next filter tile), so the map is reproducible; the four warps of a lane quadrant
+            // meet on a named barrier of their own.
+            ctl->fold[it & 1][quad][cgroup][lane] = part;
+            bar_sync(1 + quad, 32 * (EPI / 4));
             if (cgroup == 0) {
                 if (nt == 0) run = 0.f;
 #pragma unroll
-                for (int c = 0; c < kSums; c++)
+                for (int c = 0; c < EPI / 4; c++)
                     run = __fadd_rn(run, ctl->fold[it & 1][quad][c][lane]);
                 if (nt == g.n_tiles - 1 && valid)
                     g.emit_a[pix] = __fmul_rn(__fmul_rn(run, kk), g.e_inv_ic);
@@ -1042,8 +1032,8 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
 // own tensor memory. A stage is a third smaller per CTA that way (32 KB instead of 48 KB at
 // N = 256), which is what the kernel is short of: at one stage per 512 cycles a single CTA pulls
 // 94 B/clk from L2, four fifths of what the SM's port delivers.
-template <int KK, bool PAIR>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int KK, bool PAIR, int EPI>
+__global__ void __launch_bounds__(threads_of(EPI), 1)
 conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const TcArgs g) {
     extern __shared__ uint8_t smem_raw[];
@@ -1068,7 +1058,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         for (int b = 0; b < g.n_acc; b++) {
             mbar_init(smem_u32(&ctl->acc_full[b]), (uint32_t)g.issuers);
             // single CTA: one arrival per epilogue thread; pair: one per epilogue warp of both
-            mbar_init(smem_u32(&ctl->acc_empty[b]), (uint32_t)((PAIR ? 2 : 32) * kEpiWarps / g.teams));
+            mbar_init(smem_u32(&ctl->acc_empty[b]), (uint32_t)((PAIR ? 2 : 32) * EPI / g.teams));
             mbar_init(smem_u32(&ctl->started[b]), 1);
         }
         for (int i = 0; i < 2; i++) mbar_init(smem_u32(&ctl->drain[i]), 1);
@@ -1119,7 +1109,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         } else {
             producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
         }
-    } else if (warp == 1 || warp == kIssuer2Warp) {
+    } else if (warp == 1 || warp == 2 + EPI) {
         const int who = warp == 1 ? 0 : 1;
         if (who < g.issuers && rank == 0) {
             if constexpr (PAIR) {
@@ -1136,11 +1126,11 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         // ---- epilogue warps: stage alpha among themselves, then drain accumulators ----
         dependency_wait();
         if (alpha_in_smem) {
-            for (int i = threadIdx.x - 64; i < g.ocp16; i += 32 * kEpiWarps)
+            for (int i = threadIdx.x - 64; i < g.ocp16; i += 32 * EPI)
                 ctl->alpha[i] = i < g.oc ? __ldg(g.alpha + i) : 0.f;
-            bar_sync(5, 32 * kEpiWarps);
+            bar_sync(5, 32 * EPI);
         }
-        epilogue_role<PAIR>(g, ctl, tmem_base, warp, lane, alpha_in_smem);
+        epilogue_role<PAIR, EPI>(g, ctl, tmem_base, warp, lane, alpha_in_smem);
     }
 
     fence_before();
@@ -1227,17 +1217,27 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.issuers = g.taps * g.chunks_per_tap < 2 ? 1 : 2;
     g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     const int kk = p.kchunk / 32;
+    // Eight epilogue warps instead of sixteen where a pair's tile keeps the tensor pipe busy for 4096 cycles
+    // or more: its stores have the next tile's MMAs to hide behind either way. A pass among others and on one
+    // stream, 16 and 8 warps, us: conv2 on 128 images (5120 cycles) 45.4 -> 44.2 and 47.9 -> 46.8, conv4 on 256
+    // (6912) on one stream 42.8 -> 42.1, VGG (9216) 73.0 -> 72.2 and 75.4 -> 73.8; but conv3 (3456) 33.9 -> 34.0,
+    // 48 channels and 368 filters (864) on one stream 18.2 -> 19.1, one tap of 51 channels (16) 23.0 -> 24.2.
+    const long tile_cycles =
+        (long)g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last) * p.n_tile / 2;
+    const bool few = pair && kk == 4 && tile_cycles >= 4096;
+    const int epi = few ? kFewEpiWarps : kEpiWarps;
     void (*kernel)(CUtensorMap, CUtensorMap, TcArgs) =
-        pair ? (kk == 4   ? conv_tcgen05_kernel<4, true>
-                : kk == 2 ? conv_tcgen05_kernel<2, true>
-                          : conv_tcgen05_kernel<1, true>)
-             : (kk == 4   ? conv_tcgen05_kernel<4, false>
-                : kk == 2 ? conv_tcgen05_kernel<2, false>
-                          : conv_tcgen05_kernel<1, false>);
+        few    ? conv_tcgen05_kernel<4, true, kFewEpiWarps>
+        : pair ? (kk == 4   ? conv_tcgen05_kernel<4, true, kEpiWarps>
+                  : kk == 2 ? conv_tcgen05_kernel<2, true, kEpiWarps>
+                            : conv_tcgen05_kernel<1, true, kEpiWarps>)
+               : (kk == 4   ? conv_tcgen05_kernel<4, false, kEpiWarps>
+                  : kk == 2 ? conv_tcgen05_kernel<2, false, kEpiWarps>
+                            : conv_tcgen05_kernel<1, false, kEpiWarps>);
     // per device and kernel, once: the opt-in to large dynamic shared memory, the SM count and
     // the number of CTA pairs that can be resident together
-    static std::atomic<bool> opted_in[64][3][2];
-    std::atomic<bool> &done = opted_in[d][kk == 4 ? 0 : kk == 2 ? 1 : 2][pair ? 1 : 0];
+    static std::atomic<bool> opted_in[64][3][3];
+    std::atomic<bool> &done = opted_in[d][kk == 4 ? 0 : kk == 2 ? 1 : 2][few ? 2 : pair ? 1 : 0];
     if (!done.load(std::memory_order_acquire)) {
         const cudaError_t e = cudaFuncSetAttribute(
             kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -1251,7 +1251,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         if (!slots) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(2 * (sms / 2));
-            cfg.blockDim = dim3(kThreads);
+            cfg.blockDim = dim3(threads_of(epi));
             cfg.dynamicSmemBytes = 227 * 1024 - 1024;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1362,16 +1362,17 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
                         : (size_t)g.n_stages * g.stage_bytes);
     // At least 120 KB of shared memory so that one CTA owns the SM and all 512 TMEM columns.
     if (smem < 120 * 1024) smem = 120 * 1024;
-    // As many accumulators as fit (at most four), and two epilogue teams if a CTA has that many tiles. With
-    // all warps (16 then) on every tile AlexNet conv3 (256 images) took 41.3 us per pass, conv1 (64 images)
-    // 86, with two teams 37.7 and 79. The chained epilogue carries per-pixel state from one filter tile to the next: one team.
+    // As many accumulators as fit (at most four), and one epilogue team for each of two or four of
+    // them if a CTA has that many tiles. With all 16 warps on every tile AlexNet conv3 (256
+    // images) took 41.3 us per pass, conv1 (64 images) 86, with two teams 37.7 and 79. The chained
+    // epilogue carries per-pixel state from one filter tile to the next: one team.
     const int rounds = g.n_inner ? 1 : div_up_i(units, grid);
     g.n_acc = g.shared_cols || g.n_inner ? 2 : (int)kScaleCol / p.n_tile;
     if (g.n_acc > kMaxAcc) g.n_acc = kMaxAcc;
-    g.teams = rounds >= 2 ? 2 : 1;
+    g.teams = g.n_acc == 4 && rounds >= 4 && !few ? 4 : rounds >= 2 ? 2 : 1;
     g.by_acc = FastDiv((uint32_t)g.n_acc);
     note_launch();
-    return launch_overlapped(kernel, dim3((pair ? 2 : 1) * grid), dim3(kThreads), smem, s,
+    return launch_overlapped(kernel, dim3((pair ? 2 : 1) * grid), dim3(threads_of(epi)), smem, s,
                              pair ? 2 : 1, map_a, map_b, g);
 }
 

@@ -58,7 +58,7 @@ struct TcArgs {
                           // channels at all (the chunk is padded with zeros to kchunk bytes)
     uint32_t acc_step;    // columns from the first accumulator to the second
     int n_acc;            // accumulators in tensor memory
-    int teams;            // epilogue teams that take the tiles in turn: 1 or 2
+    int teams;            // epilogue teams that take the tiles in turn: 1, 2 or 4
     FastDiv by_acc;       // tile -> round of the accumulators
     int shared_cols;      // the accumulators overlap (n_tile > kAccStep)
 };
