@@ -120,11 +120,10 @@ struct Tile {
 template <bool NHWC>
 __device__ __forceinline__ bool finish_task(const WholeArgs &g, Control *ctl, uint8_t *operand,
                                             const Tile &tile, bool owner, int t, int lane, float *v) {
-    const bool vec = NHWC && g.vec;
     const int col = t / tile.groups, gr = t - col * tile.groups;
     const int nc = min(32, g.ic - 32 * col);
-    if (vec) transpose8(v, lane & 7);
-    const int px = tile.first + 32 * gr + (vec ? 4 * (lane & 7) + (lane >> 3) : lane);
+    if (NHWC) transpose8(v, lane & 7);
+    const int px = tile.first + 32 * gr + (NHWC ? 4 * (lane & 7) + (lane >> 3) : lane);
     const bool live = px < tile.last;
     const int n = live ? (int)g.by_hw((uint32_t)px) : 0, r = live ? px - n * g.hw : 0;
     const int h = (int)g.by_iw((uint32_t)r), w = r - h * g.iw;

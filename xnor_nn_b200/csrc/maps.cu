@@ -62,19 +62,18 @@ __global__ void __launch_bounds__(kThreads) maps_kernel(const MapArgs g) {
     b.last = n * g.hw + max(hi, lo) * g.iw;
     b.groups = max(1, (b.last - b.first + 31) >> 5);
     b.tasks = b.groups * g.columns;
-    const bool vec = NHWC && g.vec;
     bool ok = true;
     for (int t = warp; ok && t < b.tasks; t += kWarps) {
         const int col = t / b.groups, gr = t - col * b.groups;
         const int nc = min(32, g.ic - 32 * col);
         float v[32];
         load_task<NHWC>(g, b, t, lane, v);
-        if (vec) transpose8(v, lane & 7);
+        if (NHWC) transpose8(v, lane & 7);
         float acc;
         ok = add_task(v, nc, col, g.inv_ic, &summed[gr], &sum[gr][lane], &abort_flag, g.error, g.wait_ns,
                       &acc);
         if (!ok) break;
-        const int px = b.first + 32 * gr + (vec ? 4 * (lane & 7) + (lane >> 3) : lane);
+        const int px = b.first + 32 * gr + (NHWC ? 4 * (lane & 7) + (lane >> 3) : lane);
         if (col + 1 < g.columns) {
             sum[gr][lane] = acc;
             __syncwarp();

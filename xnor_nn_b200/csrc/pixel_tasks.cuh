@@ -9,8 +9,8 @@
 namespace xb200 {
 namespace tasks {
 
-// 32 channels of 32 pixels, channels-last: eight lanes read a pixel's channels with 16-byte loads, four
-// pixels at a time, and an 8 x 8 transposition of those quadruples leaves a lane with all channels of
+// 32 channels of 32 pixels, channels-last: eight lanes read a pixel's channels, four each (with 16-byte
+// loads where they are aligned) and four pixels at a time, and an 8 x 8 transposition of those quadruples leaves a lane with all channels of
 // pixel 4 (lane % 8) + lane / 8.
 __device__ __forceinline__ void transpose8(float *v, int sub) {
 #pragma unroll
@@ -69,31 +69,31 @@ __device__ __forceinline__ bool turn_wait(const int *turn, int want, volatile in
     return __all_sync(0xffffffffu, ok);
 }
 
-// `tile`: its pixels first .. last, in groups of 32; `g`: the source.
+// `tile`: its pixels first .. last, in groups of 32; `g`: the source. Lane l has pixel l of the group,
+// channels-last after transpose8 pixel 4 (l % 8) + l / 8.
 template <bool NHWC, class Args, class Tile>
 __device__ __forceinline__ void load_task(const Args &g, const Tile &tile, int t, int lane, float *v) {
     const int col = t / tile.groups, gr = t - col * tile.groups;
     const int c0 = 32 * col, nc = min(32, g.ic - c0);
-    if (NHWC && g.vec) {
+    if (NHWC) {  // transpose8 puts it in order
         const int sub = lane & 7, px = tile.first + 32 * gr + (lane >> 3);
         const float *p = g.src + (long)px * g.ic + c0 + 4 * sub;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (px + 4 * j < tile.last && 4 * sub < nc)
-                x = __ldg(reinterpret_cast<const float4 *>(p + (long)(4 * j) * g.ic));
-            v[4 * j] = x.x; v[4 * j + 1] = x.y; v[4 * j + 2] = x.z; v[4 * j + 3] = x.w;
+        for (int j = 0; j < 8; j++, p += (long)4 * g.ic) {
+            const bool in = px + 4 * j < tile.last;
+            if (g.vec) {
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in && 4 * sub < nc) x = __ldg(reinterpret_cast<const float4 *>(p));
+                v[4 * j] = x.x; v[4 * j + 1] = x.y; v[4 * j + 2] = x.z; v[4 * j + 3] = x.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) v[4 * j + i] = in && 4 * sub + i < nc ? __ldg(p + i) : 0.f;
+            }
         }
         return;
     }
     const int px = tile.first + 32 * gr + lane;
     const bool live = px < tile.last;
-    if (NHWC) {
-        const float *p = g.src + (long)px * g.ic + c0;
-#pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = live && i < nc ? __ldg(p + i) : 0.f;
-        return;
-    }
     // an address is a warp-uniform channel plane and a lane's 32-bit offset into it (the host checks
     // the range)
     const unsigned n = live ? g.by_hw((uint32_t)px) : 0, r = live ? px - n * g.hw : 0;
