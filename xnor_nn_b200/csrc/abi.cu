@@ -706,12 +706,13 @@ xnor_nn_status_t xnor_nn_b200_forward(const xnor_nn_convolution_t *c, xnor_nn_re
     if (wd == kElsewhere) return wrong_device("the result tensor");
     if (ws == kHost && wd == kHost && src_bytes(*p) >= 2 * ResCtx::kSliceBytes)
         return forward_host_pipelined(*p, x, res);
-    const void *src = nullptr;
+    const void *src = res[xnor_nn_resource_user_src];
     bool staged = false;
-    xnor_nn_status_t st = stage_in(x, 0, res[xnor_nn_resource_user_src], src_bytes(*p), &src, &staged);
+    xnor_nn_status_t st = xnor_nn_success;
+    if (ws == kHost) st = stage_in(x, 0, src, src_bytes(*p), &src, &staged);
     if (st != xnor_nn_success) return st;
     void *user = res[xnor_nn_resource_user_dst];
-    const bool direct = on_device(user);
+    const bool direct = wd == kHere;
     float *dst = (float *)user;
     if (!direct) {
         st = ensure_stage(x, 2, dst_elems(*p) * sizeof(float));

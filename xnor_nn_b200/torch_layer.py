@@ -12,11 +12,15 @@ already live on the GPU.
 * backward (xnor_nn_conv_layer.cpp:88-125): a plain float convolution backward. The gradient
   of the weights uses the real input and the output gradient; the gradient of the input uses
   `binarize_weights_float(weight)` = sign(w) * mean(w) in place of the weights; afterwards the
-  weights count as changed. The float gradients are library calls (`torch.nn.grad`), as they
-  are GEMM calls upstream; the binary forward pass is the part this library accelerates.
+  weights count as changed. The float gradients are library calls (the operator behind
+  `torch.nn.grad.conv2d_weight` and `conv2d_input`, which would each make a tensor to stand for the one
+  that the gradient does not depend on), as they are GEMM calls upstream; the binary forward pass is
+  the part this library accelerates.
 
 torch is imported here only; the rest of the package does not need it.
 """
+import contextlib
+
 import torch
 
 import xnor_nn_b200 as xb
@@ -42,15 +46,13 @@ class _XnorConvFunction(torch.autograd.Function):
         if ctx.has_bias and ctx.needs_input_grad[2]:
             grad_b = grad_y.sum(dim=(0, 2, 3))
         if ctx.needs_input_grad[1]:
-            grad_w = torch.nn.grad.conv2d_weight(x, weight.shape, grad_y, stride=layer.stride,
-                                                 padding=layer.padding)
+            grad_w = layer._float_backward(grad_y, x, weight, (False, True, False))[1]
             layer._weights_changed = True
         if ctx.needs_input_grad[0]:
             bweight = torch.empty_like(weight)
             layer._conv_for(x).binarize_weights_float(
                 weight.detach(), bweight, stream=torch.cuda.current_stream().cuda_stream)
-            grad_x = torch.nn.grad.conv2d_input(x.shape, bweight, grad_y, stride=layer.stride,
-                                                padding=layer.padding)
+            grad_x = layer._float_backward(grad_y, x, bweight, (True, False, False))[0]
         return grad_x, grad_w, grad_b, None
 
 
@@ -98,6 +100,10 @@ class XnorConv2d(torch.nn.Module):
             self._convs[key] = conv
         return conv
 
+    def _float_backward(self, grad_y, x, weight, wanted):
+        return torch.ops.aten.convolution_backward(
+            grad_y, x, weight.contiguous(), None, self.stride, self.padding, (1, 1), False, (0, 0), 1, wanted)
+
     def _forward_device(self, x):
         if not x.is_cuda or x.dtype != torch.float32 or x.dim() != 4:
             raise ValueError("XnorConv2d takes a float32 CUDA tensor of shape (mb, ic, ih, iw); "
@@ -109,7 +115,8 @@ class XnorConv2d(torch.nn.Module):
         x = x.contiguous()
         conv = self._conv_for(x)
         key = self._key(x)
-        with torch.cuda.device(x.device):
+        here = torch.cuda.current_device() == x.device.index
+        with contextlib.nullcontext() if here else torch.cuda.device(x.device):
             conv.set_stream(torch.cuda.current_stream().cuda_stream)
             w = self.weight.detach()
             stamp = (w.data_ptr(), w._version)
