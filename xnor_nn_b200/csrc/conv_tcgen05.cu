@@ -942,9 +942,11 @@ __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
 
 // Two issuers take alternate groups (a chunk of a filter row). Nothing but a tile's first instruction
 // and the barriers around the tile ties them to each other: both see every position tile and every
-// accumulator, and of a filter barrier there is only one phase. Alone, an issuer needs about 750
-// cycles a group and 80 an instruction (layers of 64 filters, 9 to 33 instructions in 3 to 9 groups):
-// on AlexNet conv2, four instructions a group, 240 cycles for each, where the tensor pipe needs 128.
+// accumulator, and of a filter barrier there is only one phase. What a group costs an issuer is mostly the
+// chain of scalar instructions around its MMAs (750 cycles and 80 for each instruction, alone, on layers of 64
+// filters; the tensor pipe needs 128 an instruction on AlexNet conv2): working the starts out once instead of
+// dividing in every group took conv2 on 128 images from 42.9 to 42.0 us a pass among others, 96 channels on
+// 75 images from 27.7 to 27.1 and on one stream from 33.3 to 32.3. A table of 32 starts is one a lane.
 template <int KK>
 __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                                 uint32_t stage0, int who) {
@@ -952,7 +954,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
     const bool leader = elect_one();
     const int rounds = Deal<true>(g).rounds(g);
     if (rounds == 0) return;
-    const int groups = g.kh * g.chunks_per_tap, columns = g.pos_bytes >> 4;
+    const int groups = g.kh * g.chunks_per_tap;
     const uint64_t a_hi = (uint64_t)g.plane_desc_hi << 32, b_hi = (uint64_t)g.desc_hi << 32;
     const uint32_t lbo = (uint32_t)g.plane_pitch;  // from a column to the next, in 16 bytes
     const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (lbo << 16);
@@ -960,6 +962,14 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
     const uint32_t a_units = g.a_slot_bytes >> 4, b_units = g.b_slot_bytes >> 4;
     const uint32_t full0 = smem_u32(&ctl->full[0]);
     const uint32_t afull0 = smem_u32(&ctl->a_full[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
+    // where a chunk's instructions start, from the filter row's first position and column: a lane works
+    // one out, so that no group has to divide
+    uint32_t start_of = 0;
+    {
+        const int byte = (threadIdx.x & 31) / KK * g.kchunk + (threadIdx.x & 31) % KK * 32;
+        const int pos = byte / g.pos_bytes;
+        start_of = (uint32_t)((byte - pos * g.pos_bytes) >> 4) * lbo + (uint32_t)pos;
+    }
     int sa = 0, b = 0;
     uint32_t pa = 0, acc_phase = 0;
     bool ok = true;
@@ -977,6 +987,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
         if (!ok) break;
         fence_after();
         const uint32_t tile = a_lo0 + (uint32_t)sa * a_units;
+        int row = who / g.chunks_per_tap, chunk = who - row * g.chunks_per_tap;
         for (int gr = who; gr < groups; gr += 2) {
             if (it == 0) {  // the share of the filters that the group belongs to
                 int part = 0;
@@ -985,28 +996,24 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
                 if (!ok) break;
                 fence_after();
             }
-            const int row = gr / g.chunks_per_tap, chunk = gr - row * g.chunks_per_tap;
             const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
-            // position and column that the chunk's bytes start at, from the filter row's first
-            const int byte = chunk * g.kchunk, pos = byte / g.pos_bytes;
-            int c = (byte - pos * g.pos_bytes) >> 4, at = row * g.wp + pos;
+            uint32_t start[KK];
+#pragma unroll
+            for (int k = 0; k < KK; k++) start[k] = __shfl_sync(0xffffffffu, start_of, chunk * KK + k);
             if (leader) {
+                const uint32_t at = tile + (uint32_t)(row * g.wp);
                 const uint64_t bdesc = b_hi | (uint64_t)(b_lo0 + (uint32_t)gr * b_units);
 #pragma unroll
                 for (int k = 0; k < KK; k++) {
-                    if (k < kk) {
-                        mma_mxf4<true>(d_tmem, a_hi | (uint64_t)(tile + (uint32_t)c * lbo + (uint32_t)at),
-                                       bdesc + (uint64_t)(2 * k), g.idesc, tmem_base + kScaleCol,
-                                       (gr | k) == 0 ? 0u : 1u);
-                        // two columns further: the next position's, or the one's after it
-                        c += 2;
-                        if (c >= columns) { c -= columns; at++; }
-                        if (c >= columns) { c -= columns; at++; }
-                    }
+                    if (k < kk)
+                        mma_mxf4<true>(d_tmem, a_hi | (uint64_t)(at + start[k]), bdesc + (uint64_t)(2 * k),
+                                       g.idesc, tmem_base + kScaleCol, (gr | k) == 0 ? 0u : 1u);
                 }
                 if (gr == 0) commit_pair(smem_u32(&ctl->started[b]));
             }
             __syncwarp();
+            chunk += 2;
+            while (chunk >= g.chunks_per_tap) { chunk -= g.chunks_per_tap; row++; }
         }
         if (!ok) break;
         if (leader) {
@@ -1305,7 +1312,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         const int rows = BM + (g.kh - 1) * p.wp + p.kw - 1;
         const int pitch = (rows + 7) & ~7;  // a load lands on a multiple of 128 bytes
         const uint32_t col_slot = (uint32_t)(planes * pitch * 16 + 1023) & ~1023u;
-        const bool as_columns = p.cat && g.kh >= 3 && (walk >= 3 || p.icp == 16) &&
+        const bool as_columns = p.cat && g.kh >= 3 && g.chunks_per_tap * kk <= 32 && (walk >= 3 || p.icp == 16) &&
                                 !(p.icp == 32 && groups == 3 && p.n_tile <= 64) && rows <= 256 &&
                                 all_b + 2 * (size_t)col_slot <= room;
         g.resident = 1;
