@@ -1224,14 +1224,17 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.issuers = g.taps * g.chunks_per_tap < 2 ? 1 : 2;
     g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     const int kk = p.kchunk / 32;
-    // Eight epilogue warps instead of sixteen where a pair's tile keeps the tensor pipe busy for 4096 cycles
-    // or more: its stores have the next tile's MMAs to hide behind either way. A pass among others and on one
-    // stream, 16 and 8 warps, us: conv2 on 128 images (5120 cycles) 45.4 -> 44.2 and 47.9 -> 46.8, conv4 on 256
-    // (6912) on one stream 42.8 -> 42.1, VGG (9216) 73.0 -> 72.2 and 75.4 -> 73.8; but conv3 (3456) 33.9 -> 34.0,
-    // 48 channels and 368 filters (864) on one stream 18.2 -> 19.1, one tap of 51 channels (16) 23.0 -> 24.2.
+    // Eight epilogue warps instead of sixteen where a pair has four tiles or more and each keeps the tensor
+    // pipe busy for 4096 cycles or more: the stores have the next tile's MMAs to hide behind either way, all
+    // but the last tile's. A pass among others and on one stream, 16 and 8 warps, us: conv2 on 128 images (5120
+    // cycles, six tiles) 45.4 -> 44.2 and 47.9 -> 46.8, VGG (9216, six) 73.0 -> 72.2 and 75.4 -> 73.8. conv4 on
+    // 256 images (6912, three) 38.3 -> 38.8 in one set of runs, 37.6 -> 37.2 in another, chained layers that end
+    // in two such tiles 43.5 -> 43.8; conv3 (3456) 33.9 -> 34.0, 48 channels and 368 filters (864) on one stream
+    // 18.2 -> 19.1, one tap of 51 channels (16) 23.0 -> 24.2.
     const long tile_cycles =
         (long)g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last) * p.n_tile / 2;
-    const bool few = pair && kk == 4 && tile_cycles >= 4096;
+    const int pair_tiles = div_up_i(((m_tiles + 1) / 2) * g.n_tiles, sms / 2);
+    const bool few = pair && kk == 4 && tile_cycles >= 4096 && pair_tiles >= 4;
     const int epi = few ? kFewEpiWarps : kEpiWarps;
     void (*kernel)(CUtensorMap, CUtensorMap, TcArgs) =
         few    ? conv_tcgen05_kernel<4, true, kFewEpiWarps>
