@@ -26,7 +26,8 @@
 //
 // What bounds it, in cycles of a tile of AlexNet conv4 (136 pixels of 384 channels, 384 KB of filters per
 // 256, 1.9 GHz): 1200 until the first loads go out, 12000 of packing (three tasks a worker: 1300 to 2500 for
-// a task's loads, 1300 to 1900 of instructions), which the filter loads share the way from L2 with, then the
+// a task's loads, 1300 to 1900 of instructions; an SM takes floats in at 20 to 25 bytes a cycle, and 12, 16 or
+// 24 workers, or loads a task ahead, do not change that), which the filter loads share the way with, then the
 // MMAs (5300 with narrow filter tiles, all of which are in shared memory by then; 9500 with 256 filters,
 // which come through the ring meanwhile), then 1000 to 5600 for the stores. One issuer needs about 500 cycles a
 // filter tile, mostly the chain of scalar instructions around its MMAs, hence four (MMAs of one image:
