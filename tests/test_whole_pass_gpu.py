@@ -70,3 +70,30 @@ def test_one_launch(oracle, case):
 @pytest.mark.parametrize("case", TWO_LAUNCHES, ids=[c[0] for c in TWO_LAUNCHES])
 def test_beyond_its_limits(oracle, case):
     _run(oracle, case, 2)
+
+
+def test_result_over_the_source():
+    """A pass whose result overlaps its source packs all of it before it stores anything: two launches."""
+    torch = pytest.importorskip("torch")
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(12, 64, 14, 14, generator=gen, device="cuda")
+    w = torch.randn(64, 64, 3, 3, generator=gen, device="cuda")
+    conv = xb.Convolution(xb.ALGORITHM_BCAST, xb.NCHW, xb.OIHW, xb.NCHW, 12, 64, 64, 14, 14, 3, 3, 1, 1, 1,
+                          1, w)
+    want = torch.empty_like(x)
+    counts = []
+    shifted = torch.empty(x.numel() + 5, device="cuda")
+    torch.cuda.synchronize()
+    for src, dst in ((x, want), (x.clone(), None), (shifted[:-5].view_as(x), shifted[5:].view_as(x))):
+        if dst is None:
+            dst = src
+        elif dst is not want:
+            src.copy_(x)
+        torch.cuda.synchronize()
+        before = xb.kernel_launches()
+        conv.forward(src, dst)
+        counts.append(xb.kernel_launches() - before)
+        conv.synchronize()
+        assert torch.equal(dst, want)
+    assert counts == [1, 2, 2]
+    conv.close()

@@ -598,7 +598,12 @@ xnor_nn_status_t enqueue_forward(const Slice &sl, ResCtx *x, xnor_nn_resources_t
     sub[xnor_nn_resource_bin_src] = (char *)res[xnor_nn_resource_bin_src] + sl.bin_src;
     sub[xnor_nn_resource_a] = (char *)res[xnor_nn_resource_a] + sl.a;
     sub[xnor_nn_resource_k] = (char *)res[xnor_nn_resource_k] + sl.k;
-    if (whole_ok(sl.p)) {
+    // One launch stores results of some tiles while others still read the source; a caller may pass one
+    // tensor for both.
+    const uintptr_t s0 = (uintptr_t)src, d0 = (uintptr_t)dst;
+    const bool apart =
+        s0 + src_bytes(sl.p) <= d0 || d0 + dst_elems(sl.p) * sizeof(float) <= s0;
+    if (apart && whole_ok(sl.p)) {
         CU(launch_conv_whole(sl.p, src, sub[xnor_nn_resource_bin_src],
                              res[xnor_nn_resource_bin_weights], (const float *)res[xnor_nn_resource_alpha],
                              (float *)sub[xnor_nn_resource_a], (float *)sub[xnor_nn_resource_k], dst,
