@@ -74,8 +74,8 @@ __device__ __forceinline__ void store_nchw(const StoreAt &s, const float *al, bo
     }
 }
 
-// NHWC, a number of filters that is a multiple of four: a thread owns one pixel and 16 neighbouring
-// filters at a time, which are contiguous in the result.
+// NHWC, a number of filters that is a multiple of four and a result that starts on 16 bytes: a thread
+// owns one pixel and 16 neighbouring filters at a time, which are contiguous in the result.
 template <class F>
 __device__ __forceinline__ void store_nhwc(const StoreAt &s, const float *al, int n_tile, uint32_t taddr,
                                            int cgroup, int cgroups, bool reverse, F columns_read) {
@@ -118,7 +118,7 @@ __device__ __forceinline__ void store_nhwc(const StoreAt &s, const float *al, in
     }
 }
 
-// NHWC, any number of filters.
+// NHWC, any number of filters and any start of the result.
 template <class F>
 __device__ __forceinline__ void store_nhwc_odd(const StoreAt &s, const float *al, int n_tile,
                                                uint32_t taddr, int cgroup, int cgroups, bool reverse,

@@ -357,9 +357,10 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                     }
                 }
             }
-        } else if (!g.sums && g.dst_nhwc && (g.oc & 3) == 0) {
+        } else if (!g.sums && g.dst_nhwc && (g.oc & 3) == 0 && ((uintptr_t)g.dst & 15) == 0) {
             // NHWC floats: a thread owns one pixel and 16 neighbouring filters at a time, which
-            // are contiguous in the result: four 16-byte stores.
+            // are contiguous in the result: four 16-byte stores. (A result that starts between two
+            // 16-byte boundaries, such as a view into a buffer, is stored float by float below.)
             float *out = g.dst + pix * g.oc + oc0;
             const float *al = alpha_in_smem ? ctl->alpha + oc0 : g.alpha + oc0;
             // 256-bit stores need 32-byte alignment: rows and tiles that are multiples of 8

@@ -355,7 +355,7 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
             auto nothing = [](int) {};
             if (!g.dst_nhwc)
                 store_nchw(to, ctl->alpha, true, g.n_tile, taddr, cgroup, cgroups, false, nothing);
-            else if ((g.oc & 3) == 0)
+            else if ((g.oc & 3) == 0 && ((uintptr_t)g.dst & 15) == 0)
                 store_nhwc(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups, false, nothing);
             else
                 store_nhwc_odd(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups, false, nothing);
