@@ -182,6 +182,20 @@ xnor_nn_status_t xnor_nn_b200_forward_sharded(const xnor_nn_convolution_t *c,
 xnor_nn_status_t xnor_nn_b200_selftest_lost_commit(const xnor_nn_convolution_t *c,
                                                    xnor_nn_resources_t res, unsigned wait_ms);
 
+/* The same for the kernel that runs a small layer's pass in one launch (xnor_nn_b200_forward, layers
+ * of at most one tile per SM; xnor_nn_error_invalid_input for others). What is lost: as above, an
+ * arrival of the first block's packed operand, or, in every block, the turns in which a pixel's
+ * running sum of |x| is handed from one group of 32 channels to the next. res[user_src] and
+ * res[user_dst] device memory. */
+typedef enum {
+    xnor_nn_b200_lost_commit = 0,
+    xnor_nn_b200_lost_operand = 1,
+    xnor_nn_b200_lost_turn = 2
+} xnor_nn_b200_lost_t;
+xnor_nn_status_t xnor_nn_b200_selftest_small_layer(const xnor_nn_convolution_t *c,
+                                                   xnor_nn_resources_t res, unsigned wait_ms,
+                                                   xnor_nn_b200_lost_t lost);
+
 /* Number of kernels this library has launched in this process, for benchmark accounting. */
 long xnor_nn_b200_kernel_launches(void);
 

@@ -92,6 +92,7 @@ def lib():
         L.xnor_nn_b200_kernel_launches.restype = C.c_long
         L.xnor_nn_b200_forward_sharded.argtypes = [dp, rp, C.POINTER(C.c_int), C.c_int]
         L.xnor_nn_b200_selftest_lost_commit.argtypes = [dp, rp, C.c_uint]
+        L.xnor_nn_b200_selftest_small_layer.argtypes = [dp, rp, C.c_uint, C.c_int]
         L.xnor_nn_b200_calculate_k_noalloc.argtypes = [dp, C.c_void_p, C.c_void_p, C.c_void_p]
         L.xnor_nn_b200_noalloc_max_pixels.restype = C.c_long
         L.xnor_nn_b200_noalloc_last_error.restype = C.c_char_p

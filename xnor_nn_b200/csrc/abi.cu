@@ -1050,7 +1050,7 @@ xnor_nn_status_t xnor_nn_b200_selftest_lost_commit(const xnor_nn_convolution_t *
         where_is(res[xnor_nn_resource_user_dst], x->device) != kHere)
         return xnor_nn_error_invalid_input;
     DeviceGuard dg(x->device);
-    ConvSelfTest t;
+    ConvSelfTest t = {};
     t.wait_ns = (unsigned long long)wait_ms * 1000000ull;
     t.drop_commit = 1;
     float *dst = (float *)res[xnor_nn_resource_user_dst];
@@ -1066,6 +1066,37 @@ xnor_nn_status_t xnor_nn_b200_selftest_lost_commit(const xnor_nn_convolution_t *
                                (const float *)res[xnor_nn_resource_alpha],
                                (const float *)res[xnor_nn_resource_k], nullptr, nullptr, dst,
                                nullptr, x->error_word, x->stream, nullptr, &t));
+    return sync_and_check(x);
+}
+
+xnor_nn_status_t xnor_nn_b200_selftest_small_layer(const xnor_nn_convolution_t *c,
+                                                   xnor_nn_resources_t res, unsigned wait_ms,
+                                                   xnor_nn_b200_lost_t lost) {
+    if (!c || !res || !res[xnor_nn_resource_user_src] || !res[xnor_nn_resource_user_dst] ||
+        !res[xnor_nn_resource_bin_src] || !res[xnor_nn_resource_bin_weights] ||
+        !res[xnor_nn_resource_a] || !res[xnor_nn_resource_k] || !res[xnor_nn_resource_alpha])
+        return xnor_nn_error_invalid_input;
+    const Plan *p = plan_of(c);
+    ResCtx *x = find_ctx(res);
+    if (!p || !x || wait_ms == 0 || wait_ms > 1000 ||
+        where_is(res[xnor_nn_resource_user_src], x->device) != kHere ||
+        where_is(res[xnor_nn_resource_user_dst], x->device) != kHere)
+        return xnor_nn_error_invalid_input;
+    DeviceGuard dg(x->device);
+    ConvSelfTest t = {};
+    t.wait_ns = (unsigned long long)wait_ms * 1000000ull;
+    t.drop_commit = lost == xnor_nn_b200_lost_commit;
+    t.drop_operand = lost == xnor_nn_b200_lost_operand;
+    t.drop_turn = lost == xnor_nn_b200_lost_turn;
+    if (!p->formats_ok || !whole_ok(*p) || !(t.drop_commit || t.drop_operand || t.drop_turn) ||
+        (t.drop_turn && p->ic <= 32))  // the channels of one task: nothing is handed on
+        return xnor_nn_error_invalid_input;
+    x->staged_a_valid = false;
+    CU(launch_conv_whole(*p, (const float *)res[xnor_nn_resource_user_src],
+                         res[xnor_nn_resource_bin_src], res[xnor_nn_resource_bin_weights],
+                         (const float *)res[xnor_nn_resource_alpha],
+                         (float *)res[xnor_nn_resource_a], (float *)res[xnor_nn_resource_k],
+                         (float *)res[xnor_nn_resource_user_dst], x->error_word, x->stream, &t));
     return sync_and_check(x);
 }
 

@@ -485,11 +485,12 @@ __device__ __forceinline__ void producer_ring(const TcArgs &g, Control *ctl,
             }
         }
     }
-    if (!ok && rank == 0) {
-        // Something gave up. Loads already issued still land in this CTA's shared
-        // memory: wait for them (bounded) before the CTA may exit. (The partner of a
-        // pair cannot wait on the leader's barrier; it stays until the leader has got
-        // through this and both have met at the cluster barrier at the end.)
+    if (rank == 0) {
+        // Loads already issued land in this CTA's shared memory: wait for them (bounded) before
+        // the CTA may exit. Whoever consumes them waits for them too, unless something gives up,
+        // be it after this role is through. (The partner of a pair cannot wait on the leader's
+        // barrier; it stays until the leader has got through this and both have met at the
+        // cluster barrier at the end.)
         for (int s = 0; s < g.n_stages; s++)
             if (armed & (1u << s)) {
                 mbar_wait_quiet(smem_u32(&ctl->full[s]), (armed_parity >> s) & 1u,
@@ -590,14 +591,13 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
             if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
         }
     }
-    if (!ok) {
-        // Let every MMA this thread has issued finish before tensor memory is released.
-        if (leader) {
-            if (PAIR) commit_pair(smem_u32(&ctl->drain[who]));
-            else commit(smem_u32(&ctl->drain[who]));
-        }
-        mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
+    // Every MMA this thread has issued finishes before tensor memory is released. (The epilogue waits
+    // for that as well, unless something gives up, be it after this role is through.)
+    if (leader) {
+        if (PAIR) commit_pair_here(smem_u32(&ctl->drain[who]));
+        else commit(smem_u32(&ctl->drain[who]));
     }
+    mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
 }
 
 // ---- halo mode (pairs only): producer and MMA issuers ----------------------------------------------
@@ -680,9 +680,8 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
             }
         }
     }
-    if (!ok && rank == 0) {
-        // Something gave up. Loads already issued still land in this CTA's shared memory: wait
-        // for them (bounded) before the CTA may exit.
+    if (rank == 0) {
+        // as in producer_ring: loads already issued land before the CTA may exit
         for (int s = 0; s < g.n_stages; s++)
             if (armed_b & (1u << s))
                 mbar_wait_quiet(full_l + 8u * (uint32_t)s, (parity_b >> s) & 1u, g.wait_ns);
@@ -789,12 +788,8 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
             if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
         }
     }
-    if (!ok) {
-        if (leader) {
-            commit_pair(smem_u32(&ctl->drain[who]));
-        }
-        mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
-    }
+    if (leader) commit_pair_here(smem_u32(&ctl->drain[who]));
+    mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
 }
 
 // Resident filters beside position tiles of rows: layers of more than 224 channels, one tap a filter
@@ -860,12 +855,8 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
         __syncwarp();
         if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
     }
-    if (!ok) {
-        if (leader) {
-            commit_pair(smem_u32(&ctl->drain[0]));
-        }
-        mbar_wait_quiet(smem_u32(&ctl->drain[0]), 0, g.wait_ns);
-    }
+    if (leader) commit_pair_here(smem_u32(&ctl->drain[0]));
+    mbar_wait_quiet(smem_u32(&ctl->drain[0]), 0, g.wait_ns);
 }
 
 // Position tiles of 16-byte columns (resident filters): the packed bytes of all positions that any tap
@@ -931,9 +922,8 @@ __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
         }
         __syncwarp();
     }
-    if (!ok && rank == 0) {
-        // Something gave up. Loads already issued still land in this CTA's shared memory: wait
-        // for them (bounded) before the CTA may exit.
+    if (rank == 0) {
+        // as in producer_ring: loads already issued land before the CTA may exit
         for (int i = 0; i < b_sent; i++) mbar_wait_quiet(full_l + 8u * (uint32_t)i, 0, g.wait_ns);
         for (int i = 0; i < g.n_a_slots; i++)
             if (armed & (1u << i))
@@ -1025,12 +1015,8 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
         if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
         if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
     }
-    if (!ok) {
-        if (leader) {
-            commit_pair(smem_u32(&ctl->drain[who]));
-        }
-        mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
-    }
+    if (leader) commit_pair_here(smem_u32(&ctl->drain[who]));
+    mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
 }
 
 // KK = tcgen05.mma instructions per pipeline stage (kchunk / 32).

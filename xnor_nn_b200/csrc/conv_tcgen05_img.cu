@@ -266,14 +266,13 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                     }
                 }
             }
-            if (!ok) {
-                // Something gave up. Loads already issued still land in this CTA's shared
-                // memory: wait for them (bounded) before the CTA may exit.
-                for (long j = 0; j < g.stages && j < issued; j++) {
-                    const long gi = issued - 1 - j;
-                    mbar_wait_quiet(full0 + 8u * (uint32_t)(gi % g.stages),
-                                    (uint32_t)((gi / g.stages) & 1), g.wait_ns);
-                }
+            // Loads already issued land in this CTA's shared memory: wait for them (bounded) before
+            // the CTA may exit. The MMA issuer waits for them too, unless something gives up, be it
+            // after this role is through.
+            for (long j = 0; j < g.stages && j < issued; j++) {
+                const long gi = issued - 1 - j;
+                mbar_wait_quiet(full0 + 8u * (uint32_t)(gi % g.stages),
+                                (uint32_t)((gi / g.stages) & 1), g.wait_ns);
             }
         }
     } else if (warp == 1) {
@@ -336,11 +335,9 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                 if (ok && !(g.drop_commit && it == 0 && blockIdx.x == 0))
                     commit(smem_u32(&ctl->acc_full[b]));
             }
-            if (!ok) {
-                // Let every MMA already issued finish before tensor memory is released.
-                commit(smem_u32(&ctl->drain));
-                mbar_wait_quiet(smem_u32(&ctl->drain), 0, g.wait_ns);
-            }
+            // every MMA already issued finishes before tensor memory is released
+            commit(smem_u32(&ctl->drain));
+            mbar_wait_quiet(smem_u32(&ctl->drain), 0, g.wait_ns);
         }
         __syncwarp();
     } else {

@@ -81,6 +81,8 @@ struct WholeArgs {
     uint32_t b_bytes, stage_bytes, b_off;
     uint32_t idesc, a_desc_hi, b_desc_hi, tmem_cols;
     unsigned long long wait_ns;
+    int turn_step;                      // 1; these three are otherwise in self-tests only (ConvSelfTest)
+    int more_commits, more_operand;     // arrivals that CTA 0 waits for in vain
     FastDiv by_frame, by_wp, by_hw, by_iw;
 };
 
@@ -154,7 +156,7 @@ __device__ __forceinline__ bool finish_task(const WholeArgs &g, Control *ctl, ui
     if (col + 1 < g.columns) {
         ctl->sum[gr][lane] = acc;
         __syncwarp();
-        if (lane == 0) turn_pass(&ctl->summed[gr], col + 1);
+        if (lane == 0) turn_pass(&ctl->summed[gr], col + g.turn_step);
     } else if (live) {
         ctl->a[row] = acc;
         if (mine) g.a[px] = acc;
@@ -218,13 +220,13 @@ __device__ __forceinline__ void issue(const WholeArgs &g, Control *ctl, const ui
             if (stage >= g.n_stages) { stage -= g.n_stages; phase ^= 1u; }
         }
     }
-    if (ok) {
-        if (leader) commit(smem_u32(&ctl->acc_full));
-    } else {
-        // MMAs already issued finish before tensor memory is released
-        if (leader) commit(smem_u32(&ctl->drain[WHO]));
-        mbar_wait_quiet(smem_u32(&ctl->drain[WHO]), 0, g.wait_ns);
+    if (leader) {
+        if (ok) commit(smem_u32(&ctl->acc_full));
+        commit(smem_u32(&ctl->drain[WHO]));
     }
+    // MMAs already issued finish before tensor memory is released: the epilogue's wait says so, unless
+    // some role gave up, be it after this one is through
+    mbar_wait_quiet(smem_u32(&ctl->drain[WHO]), 0, g.wait_ns);
     __syncwarp();
 }
 
@@ -247,9 +249,10 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
         }
         for (int i = 0; i < g.parts; i++)
             mbar_init(smem_u32(&ctl->packed[i]),
-                      (uint32_t)(tile.groups * min(g.part_columns, g.columns - i * g.part_columns)));
+                      (uint32_t)(tile.groups * min(g.part_columns, g.columns - i * g.part_columns) +
+                                 (blockIdx.x == 0 ? g.more_operand : 0)));
         for (int i = 0; i < tile.groups; i++) ctl->summed[i] = 0;
-        mbar_init(smem_u32(&ctl->acc_full), kIssuers);
+        mbar_init(smem_u32(&ctl->acc_full), (uint32_t)(kIssuers + (blockIdx.x == 0 ? g.more_commits : 0)));
         mbar_init(smem_u32(&ctl->cleared), 4);
         for (int i = 0; i < kIssuers; i++) mbar_init(smem_u32(&ctl->drain[i]), 1);
         ctl->abort_flag = 0;
@@ -298,10 +301,10 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
             if (++stage == g.n_stages) { stage = 0; phase ^= 1; }
             if (++tap == g.taps) { tap = 0; chunk++; }
         }
-        if (!ok)  // loads in flight still land in this CTA's shared memory
-            for (int i = max(0, sent - g.n_stages); i < sent; i++)
-                mbar_wait_quiet(smem_u32(&ctl->full[i % g.n_stages]), (uint32_t)(i / g.n_stages) & 1u,
-                                g.wait_ns);
+        // Loads in flight land in this CTA's shared memory, which it may not leave before, whoever gave up
+        // and when.
+        for (int i = max(0, sent - g.n_stages); i < sent; i++)
+            mbar_wait_quiet(smem_u32(&ctl->full[i % g.n_stages]), (uint32_t)(i / g.n_stages) & 1u, g.wait_ns);
     } else if (warp == kFirstIssuer) {
         issue<0>(g, ctl, operand, b0, tmem_base, scales);
     } else if (warp == kFirstIssuer + 1) {
@@ -434,7 +437,7 @@ bool whole_ok(const Plan &p) {
 
 cudaError_t launch_conv_whole(const Plan &p, const float *src, void *bin_src, const void *bin_w,
                               const float *alpha, float *a, float *k, float *dst, int *error_word,
-                              cudaStream_t s) {
+                              cudaStream_t s, const ConvSelfTest *test) {
     WholeArgs g;
     size_t smem;
     if (!whole_shape(p, &g, &smem)) return cudaErrorNotSupported;
@@ -453,7 +456,10 @@ cudaError_t launch_conv_whole(const Plan &p, const float *src, void *bin_src, co
     g.a_desc_hi = g.swizzled ? g.b_desc_hi : 8u | (1u << 14);
     g.tmem_cols = 32;
     while (g.tmem_cols < (uint32_t)g.n_tile + 16) g.tmem_cols *= 2;
-    g.wait_ns = 2000000000ull;
+    g.wait_ns = test && test->wait_ns ? test->wait_ns : 2000000000ull;
+    g.turn_step = test && test->drop_turn ? 0 : 1;
+    g.more_commits = test ? test->drop_commit : 0;
+    g.more_operand = test ? test->drop_operand : 0;
     g.by_frame = FastDiv((uint32_t)(p.hp * p.wp)); g.by_wp = FastDiv((uint32_t)p.wp);
     g.by_hw = FastDiv((uint32_t)g.hw); g.by_iw = FastDiv((uint32_t)p.iw);
     CUtensorMap map_b;

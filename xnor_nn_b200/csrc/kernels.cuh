@@ -150,12 +150,14 @@ struct ChainTarget {
     int wp, hp, lead, icp;  // its frame geometry (Plan)
     float inv_ic;         // its Plan::inv_ic
 };
-// `test` (normally null) shortens a tensor-core kernel's wait limit and makes one CTA lose the
-// commit that publishes its first accumulator, so that a test can watch a bounded wait run out:
-// the kernel returns by itself with *error_word set and the results of the call invalid.
+// `test` (normally null) shortens a kernel's wait limit and makes one CTA lose the commit that
+// publishes its first accumulator, so that a test can watch a bounded wait run out: the kernel returns
+// by itself with *error_word set and the results of the call invalid. The one-launch pass can lose an
+// arrival of its packed operand instead, or the turns at which running sums are handed on.
 struct ConvSelfTest {
     unsigned long long wait_ns;  // 0: the normal limit (2 s)
     int drop_commit;
+    int drop_operand, drop_turn;
 };
 cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *bin_w,
                                 const float *alpha, const float *k, const float *a, float *k_out,
@@ -169,7 +171,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
 bool whole_ok(const Plan &p);
 cudaError_t launch_conv_whole(const Plan &p, const float *src, void *bin_src, const void *bin_w,
                               const float *alpha, float *a, float *k, float *dst, int *error_word,
-                              cudaStream_t s);
+                              cudaStream_t s, const ConvSelfTest *test = nullptr);
 
 // The same contract (without chaining) with the operand roles swapped: 128 filters on the UMMA M
 // side, whole output rows of one image on the N side (Plan::img_*, conv_tcgen05_img.cu). Reads

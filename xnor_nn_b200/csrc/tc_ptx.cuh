@@ -173,6 +173,13 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
         ::"r"(bar), "h"(both)
         : "memory");
 }
+// The same on this CTA's barrier alone: for a wait that the other CTA, which may leave meanwhile, has
+// no part in.
+__device__ __forceinline__ void commit_pair_here(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                 ::"r"(bar)
+                 : "memory");
+}
 
 // Shared memory -> global memory, `bytes` a multiple of 16, both addresses 16-byte aligned.
 // Completion is tracked per thread in bulk groups.
