@@ -12,6 +12,7 @@ import pytest
 
 import cases
 import test_folded_gpu
+import test_long_filter_rows_gpu
 import test_position_columns_gpu
 import test_resident_filters_gpu
 import test_streamed_filters_gpu
@@ -40,7 +41,7 @@ GPU_COLUMNS = test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.COLU
 LOST_COMMIT = cases._c("lost_commit", 64, 256, 96, 27, 27, 5, 5, ph=2, pw=2)
 LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + GPU_COLUMNS + test_position_columns_gpu.ROWS +
           test_resident_filters_gpu.ROWS + [LOST_COMMIT] + test_streamed_filters_gpu.STREAMED +
-          test_folded_gpu.FOLDED + cases.SHAPE_CASES + [
+          test_folded_gpu.FOLDED + test_long_filter_rows_gpu.LONG_ROWS + cases.SHAPE_CASES + [
               cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
               cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
 
@@ -103,6 +104,14 @@ def test_gpu_tests_of_position_columns_reach_them(launches):
     assert min(g["groups"] for g in got) < 8 < max(g["groups"] for g in got)
     assert 8 in {g["groups"] for g in got} and 1 in {g["shared_cols"] for g in got}
     assert not any(g["planes"] for g in _of(launches, test_position_columns_gpu.ROWS))
+
+
+def test_gpu_tests_of_long_filter_rows_reach_columns(launches):
+    layers = test_long_filter_rows_gpu.LONG_ROWS
+    got = _of(launches, layers)
+    assert all(g["planes"] and g["resident"] and g["issuers"] == 2 for g in got)
+    starts = [g["groups"] // c[1]["kh"] * g["kchunk"] // 32 for g, c in zip(got, layers)]
+    assert starts == [32, 36, 36, 40, 88]
 
 
 def test_gpu_tests_of_resident_rows_reach_them(launches):

@@ -953,14 +953,16 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
     const uint32_t a_units = g.a_slot_bytes >> 4, b_units = g.b_slot_bytes >> 4;
     const uint32_t full0 = smem_u32(&ctl->full[0]);
     const uint32_t afull0 = smem_u32(&ctl->a_full[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
-    // where a chunk's instructions start, from the filter row's first position and column: a lane works
-    // one out, so that no group has to divide
-    uint32_t start_of = 0;
-    {
-        const int byte = (threadIdx.x & 31) / KK * g.kchunk + (threadIdx.x & 31) % KK * 32;
+    // Where the instructions of a filter row's chunks start, from its first position and column: a lane
+    // works one out, so that no group has to divide. Rows of more than 32 instructions (over 1 KB) have
+    // the chunk's worked out by KK lanes in every group.
+    auto start_at = [&](int byte) {
         const int pos = byte / g.pos_bytes;
-        start_of = (uint32_t)((byte - pos * g.pos_bytes) >> 4) * lbo + (uint32_t)pos;
-    }
+        return (uint32_t)((byte - pos * g.pos_bytes) >> 4) * lbo + (uint32_t)pos;
+    };
+    const int lane = threadIdx.x & 31;
+    const bool long_rows = g.chunks_per_tap * KK > 32;
+    uint32_t start_of = start_at(lane / KK * g.kchunk + lane % KK * 32);
     int sa = 0, b = 0;
     uint32_t pa = 0, acc_phase = 0;
     bool ok = true;
@@ -988,9 +990,11 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
                 fence_after();
             }
             const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+            if (long_rows) start_of = start_at(chunk * g.kchunk + lane % KK * 32);
             uint32_t start[KK];
 #pragma unroll
-            for (int k = 0; k < KK; k++) start[k] = __shfl_sync(0xffffffffu, start_of, chunk * KK + k);
+            for (int k = 0; k < KK; k++)
+                start[k] = __shfl_sync(0xffffffffu, start_of, (long_rows ? 0 : chunk * KK) + k);
             if (leader) {
                 const uint32_t at = tile + (uint32_t)(row * g.wp);
                 const uint64_t bdesc = b_hi | (uint64_t)(b_lo0 + (uint32_t)gr * b_units);
@@ -1297,12 +1301,14 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         //   more, 33 to 64 channels, three operand rows, 64 filters     1.00 to 1.02, median 1.02
         //   more, filters that would not be resident beside rows        0.94 to 1.10, median 1.00
         //   the others                                                  0.73 to 1.04, median 0.94
-        // Only the last take columns; layers of the fourth kind stream their filters.
+        // Only the last take columns; layers of the fourth kind stream their filters. Filters of ten and more
+        // columns, whose rows may be more than 1 KB, gain more, not less: 13 x 6 on 167 channels 241 us a
+        // pass, 315 as rows; 33 x 3 on 39 62 and 73; 25 x 3 on 214 142 and 174.
         const int columns = p.icp / 16, planes = columns + (columns & 1);
         const int rows = BM + (g.kh - 1) * p.wp + p.kw - 1;
         const int pitch = (rows + 7) & ~7;  // a load lands on a multiple of 128 bytes
         const uint32_t col_slot = (uint32_t)(planes * pitch * 16 + 1023) & ~1023u;
-        const bool as_columns = p.cat && g.kh >= 3 && g.chunks_per_tap * kk <= 32 && (walk >= 3 || p.icp == 16) &&
+        const bool as_columns = p.cat && g.kh >= 3 && (walk >= 3 || p.icp == 16) &&
                                 !(p.icp == 32 && groups == 3 && p.n_tile <= 64) && rows <= 256 &&
                                 all_b + 2 * (size_t)col_slot <= room;
         g.resident = 1;
