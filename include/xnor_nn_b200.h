@@ -190,7 +190,8 @@ xnor_nn_status_t xnor_nn_b200_selftest_lost_commit(const xnor_nn_convolution_t *
 typedef enum {
     xnor_nn_b200_lost_commit = 0,
     xnor_nn_b200_lost_operand = 1,
-    xnor_nn_b200_lost_turn = 2
+    xnor_nn_b200_lost_turn = 2,
+    xnor_nn_b200_lost_turn_of_k = 3 /* of the kernel that runs calculate_k of small layers instead */
 } xnor_nn_b200_lost_t;
 xnor_nn_status_t xnor_nn_b200_selftest_small_layer(const xnor_nn_convolution_t *c,
                                                    xnor_nn_resources_t res, unsigned wait_ms,

@@ -1,4 +1,4 @@
-"""Bounded waits of the one-launch pass (conv_whole.cu) that run out, in the form that leaves the GPU
+"""Bounded waits of the one-launch pass (conv_whole.cu) and of calculate_k in one launch (maps.cu) that run out, in the form that leaves the GPU
 healthy: the test hook shortens the limit and loses a commit, an arrival of the packed operand or the
 hand-over of running sums. Every role winds down, loads and MMAs in flight are waited for, the host turns
 the error word into a status, and the next pass on the same resources is right, bit for bit."""
@@ -13,7 +13,7 @@ from xnor_nn_b200 import synth
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-COMMIT, OPERAND, TURN = 0, 1, 2
+COMMIT, OPERAND, TURN, TURN_OF_K = 0, 1, 2, 3
 
 
 def _layer(layer, mb):
@@ -56,6 +56,27 @@ def test_gives_up_and_the_resources_stay_usable(lost, sites, mb):
     conv.close()
 
 
+@pytest.mark.parametrize("mb", [1, 19])
+def test_calculate_k_gives_up_and_the_resources_stay_usable(mb):
+    conv, src, dst = _layer("A", mb)
+    torch.cuda.synchronize()
+    before = xb.kernel_launches()
+    assert conv.execute("calculate_k", src=src) == xb.SUCCESS
+    assert xb.kernel_launches() - before == 1  # the kernel this is about
+    want = conv.read(xb.SLOT_A, np.float32), conv.read(xb.SLOT_K, np.float32)
+    conv._set(xb.SLOT_USER_SRC, src)
+    conv._set(xb.SLOT_USER_DST, dst)
+    st = xb.lib().xnor_nn_b200_selftest_small_layer(C.byref(conv.c), conv.res, 5, TURN_OF_K)
+    assert st == xb.UNIMPLEMENTED
+    assert "gave up waiting (site 21)" in xb.last_error()
+    conv.synchronize()
+    assert conv.execute("calculate_k", src=src) == xb.SUCCESS
+    conv.synchronize()
+    assert np.array_equal(conv.read(xb.SLOT_A, np.float32), want[0])
+    assert np.array_equal(conv.read(xb.SLOT_K, np.float32), want[1])
+    conv.close()
+
+
 def test_hook_refuses_what_it_cannot_run():
     hook = xb.lib().xnor_nn_b200_selftest_small_layer
     conv, src, dst = _layer("A", 256)  # more tiles than SMs
@@ -71,4 +92,9 @@ def test_hook_refuses_what_it_cannot_run():
     conv._set(xb.SLOT_USER_DST, dst)
     assert hook(C.byref(conv.c), conv.res, 0, COMMIT) == xb.ERROR_INVALID_INPUT
     assert hook(C.byref(conv.c), conv.res, 5, 7) == xb.ERROR_INVALID_INPUT
+    conv.close()
+    conv, src, dst = _layer("D", 64)  # over 16 MB
+    conv._set(xb.SLOT_USER_SRC, src)
+    conv._set(xb.SLOT_USER_DST, dst)
+    assert hook(C.byref(conv.c), conv.res, 5, TURN_OF_K) == xb.ERROR_INVALID_INPUT
     conv.close()

@@ -284,8 +284,7 @@ xnor_nn_status_t exec_calculate_k(const xnor_nn_convolution_t *c, xnor_nn_resour
         if (maps_ok(*p)) {
             CU(launch_maps(*p, (const float *)src, (float *)res[xnor_nn_resource_a],
                            (float *)res[xnor_nn_resource_k], x->error_word, x->stream));
-            if (staged) CU(cudaStreamSynchronize(x->stream));
-            return xnor_nn_success;
+            return staged ? sync_and_check(x) : xnor_nn_success;
         }
         CU(launch_mean_abs(*p, (const float *)src, (float *)res[xnor_nn_resource_a], x->stream));
     }
@@ -1088,6 +1087,15 @@ xnor_nn_status_t xnor_nn_b200_selftest_small_layer(const xnor_nn_convolution_t *
     t.drop_commit = lost == xnor_nn_b200_lost_commit;
     t.drop_operand = lost == xnor_nn_b200_lost_operand;
     t.drop_turn = lost == xnor_nn_b200_lost_turn;
+    if (lost == xnor_nn_b200_lost_turn_of_k) {
+        if (!p->formats_ok || !maps_ok(*p) || p->ic <= 32) return xnor_nn_error_invalid_input;
+        t.drop_turn = 1;
+        x->staged_a_valid = false;
+        CU(launch_maps(*p, (const float *)res[xnor_nn_resource_user_src],
+                       (float *)res[xnor_nn_resource_a], (float *)res[xnor_nn_resource_k],
+                       x->error_word, x->stream, &t));
+        return sync_and_check(x);
+    }
     if (!p->formats_ok || !whole_ok(*p) || !(t.drop_commit || t.drop_operand || t.drop_turn) ||
         (t.drop_turn && p->ic <= 32))  // the channels of one task: nothing is handed on
         return xnor_nn_error_invalid_input;

@@ -91,6 +91,18 @@ __device__ __forceinline__ void dependency_wait() {
 }
 #endif
 
+// ---- self-tests ------------------------------------------------------------------------------
+// `test` (normally null) shortens a kernel's wait limit and makes one CTA lose the commit that
+// publishes its first accumulator, so that a test can watch a bounded wait run out: the kernel returns
+// by itself with *error_word set and the results of the call invalid. The one-launch pass can lose an
+// arrival of its packed operand instead, or, like the one-launch maps, the turns at which running sums
+// are handed on.
+struct ConvSelfTest {
+    unsigned long long wait_ns;  // 0: the normal limit (2 s)
+    int drop_commit;
+    int drop_operand, drop_turn;
+};
+
 // ---- activations -----------------------------------------------------------------------------
 // One pass over the fp32 source: sign bits into the family's packed layout and, when `a` is not
 // null, the per-pixel mean |x| map. Replaces upstream src/bcast_binarize_data.cpp:43-73 and the
@@ -109,7 +121,7 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
 // convolutions below.
 bool maps_ok(const Plan &p);
 cudaError_t launch_maps(const Plan &p, const float *src, float *a, float *k, int *error_word,
-                        cudaStream_t s);
+                        cudaStream_t s, const ConvSelfTest *test = nullptr);
 
 // ---- weights ---------------------------------------------------------------------------------
 // Sign-pack into the family's layout, alpha[oc] = mean |w|, op_c[oh][ow] = IC * taps inside.
@@ -149,15 +161,6 @@ struct ChainTarget {
     float *a;             // the next layer's res[a]
     int wp, hp, lead, icp;  // its frame geometry (Plan)
     float inv_ic;         // its Plan::inv_ic
-};
-// `test` (normally null) shortens a kernel's wait limit and makes one CTA lose the commit that
-// publishes its first accumulator, so that a test can watch a bounded wait run out: the kernel returns
-// by itself with *error_word set and the results of the call invalid. The one-launch pass can lose an
-// arrival of its packed operand instead, or the turns at which running sums are handed on.
-struct ConvSelfTest {
-    unsigned long long wait_ns;  // 0: the normal limit (2 s)
-    int drop_commit;
-    int drop_operand, drop_turn;
 };
 cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *bin_w,
                                 const float *alpha, const float *k, const float *a, float *k_out,

@@ -28,6 +28,7 @@ struct MapArgs {
     float *a, *k;
     int *error;
     unsigned long long wait_ns;
+    int turn_step;             // 1, 0 in a self-test (ConvSelfTest)
     float inv_ic, inv_khw;
     int ic, hw, ih, iw, vec;
     int oh, ow, kh, kw, sh, sw, ph, pw;
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(kThreads) maps_kernel(const MapArgs g) {
         if (col + 1 < g.columns) {
             sum[gr][lane] = acc;
             __syncwarp();
-            if (lane == 0) turn_pass(&summed[gr], col + 1);
+            if (lane == 0) turn_pass(&summed[gr], col + g.turn_step);
         } else if (px < b.last) {
             const int r = px - n * g.hw, y = (int)g.by_iw((uint32_t)r), x = r - y * g.iw;
             if (y >= own0 && y < own1) g.a[px] = acc;
@@ -139,10 +140,12 @@ bool maps_ok(const Plan &p) {
 }
 
 cudaError_t launch_maps(const Plan &p, const float *src, float *a, float *k, int *error_word,
-                        cudaStream_t s) {
+                        cudaStream_t s, const ConvSelfTest *test) {
     MapArgs g;
     if (!maps_shape(p, &g)) return cudaErrorNotSupported;
-    g.src = src; g.a = a; g.k = k; g.error = error_word; g.wait_ns = 2000000000ull;
+    g.src = src; g.a = a; g.k = k; g.error = error_word;
+    g.wait_ns = test && test->wait_ns ? test->wait_ns : 2000000000ull;
+    g.turn_step = test && test->drop_turn ? 0 : 1;
     g.inv_ic = p.inv_ic; g.inv_khw = p.inv_khw;
     g.ic = p.ic; g.hw = p.ih * p.iw; g.ih = p.ih; g.iw = p.iw;
     g.vec = p.src_nhwc && p.ic % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
