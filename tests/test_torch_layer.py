@@ -84,6 +84,30 @@ def test_backward_is_the_float_convolution_upstream_describes():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["channels_last", "transposed", "expanded"])
+def test_input_gradient_is_contiguous_whatever_the_input(layout):
+    """The result of torch.nn.grad.conv2d_input, which does not see the input's strides."""
+    torch.manual_seed(6)
+    layer = XnorConv2d(12, 32, 3, padding=1).cuda()
+    x = torch.randn(4, 12, 9, 9, device="cuda")
+    if layout == "channels_last":
+        x = x.to(memory_format=torch.channels_last)
+    elif layout == "transposed":
+        x = x.transpose(2, 3)
+    else:
+        x = x[:1].expand(4, -1, -1, -1)
+    x.requires_grad_()
+    y = layer(x)
+    gy = torch.randn_like(y)
+    got, = torch.autograd.grad(y, x, gy)
+    w = layer.weight.detach()
+    bw = torch.where(w >= 0, 1.0, -1.0) * w.double().mean().float()
+    want = torch.nn.grad.conv2d_input(x.shape, bw, gy, padding=1)
+    assert got.stride() == want.stride()
+    assert torch.allclose(got, want, rtol=1e-3, atol=1e-6 * float(gy.abs().max()))
+
+
+@pytest.mark.gpu
 def test_binarize_weights_float_on_the_device_matches_the_host_helper():
     """Signs exact; the mean within rounding of the index-order sum (the tolerance is relative
     to mean|w|, because the signed mean itself is a cancelling sum), and reproducible."""

@@ -14,7 +14,7 @@ already live on the GPU.
   `binarize_weights_float(weight)` = sign(w) * mean(w) in place of the weights; afterwards the
   weights count as changed. The float gradients are library calls (the operator behind
   `torch.nn.grad.conv2d_weight` and `conv2d_input`, which would each make a tensor to stand for the one
-  that the gradient does not depend on), as they are GEMM calls upstream; the binary forward pass is
+  that the gradient does not depend on; the input gradient is contiguous, as theirs is), as they are GEMM calls upstream; the binary forward pass is
   the part this library accelerates.
 
 torch is imported here only; the rest of the package does not need it.
@@ -52,7 +52,9 @@ class _XnorConvFunction(torch.autograd.Function):
             bweight = torch.empty_like(weight)
             layer._conv_for(x).binarize_weights_float(
                 weight.detach(), bweight, stream=torch.cuda.current_stream().cuda_stream)
-            grad_x = layer._float_backward(grad_y, x, bweight, (True, False, False))[0]
+            # only x's shape counts, but its strides would set the gradient's
+            like_x = x if x.is_contiguous() else grad_y.new_empty(1).expand(x.shape)
+            grad_x = layer._float_backward(grad_y, like_x, bweight, (True, False, False))[0]
         return grad_x, grad_w, grad_b, None
 
 
