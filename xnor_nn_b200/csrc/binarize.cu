@@ -321,12 +321,7 @@ __global__ void __launch_bounds__(TWARPS * 32) binarize_nibbles_kernel(const Bin
 // multiplied by 1/(KH*KW) (each term of upstream's sum is that product) and with zeros where the
 // window leaves the image (adding +0 to a sum of non-negative terms changes nothing), and a thread
 // adds up an output's terms in upstream's order. A staged row has its columns sorted by their
-// remainder modulo the stride, so that neighbouring outputs read neighbouring words, and tap j is word
-// j / SW of remainder j % SW, both known to the compiler for the widths and strides in use. A thread
-// keeps its column while it stages, eight lines at a time, and all its loads go out before the first is
-// used. AlexNet conv1 on 64 images (121 taps), launched alone: 18.8 us with the terms read from global memory
-// one after the other, 16.4 with them staged one by one (8.8 M warp instructions), 13.8 now (5.5 M); the
-// pass on one stream, of which the packer's rewrite is 2 to 3 us, 59.9 -> 55.7.
+// remainder modulo the stride, so that neighbouring outputs read neighbouring words.
 struct BoxArgs {
     const float *a;
     float *k;
@@ -335,12 +330,62 @@ struct BoxArgs {
     int rows, row_blocks;  // output rows per block, blocks per image
     int span, phase;       // columns of A an output row reads; words per remainder
     int lines;             // rows of A staged
-    int cols, line_step;   // threads side by side on a staged row; rows staged at a time
+    int cols, line_step;   // box_filter_columns_kernel: threads on a staged row; rows staged at a time
     FastDiv by_cols, by_sw, by_ow;
+};
+// Apart from the others' arguments: with the table among them those kernels, which do not read it, took up
+// to 3 % longer.
+struct BoxTapArgs {
+    BoxArgs box;
+    FastDiv by_span;
+    int tap[11];  // word of tap j, from the output's first
 };
 
 constexpr int kBoxThreads = 256, kBoxAhead = 8;
 constexpr int kBoxSmem = 40 * 1024;
+
+// An output a thread. Tap j is a fixed distance from the output's first word: three instructions per term
+// for the filter widths that are compiled in (KW). AlexNet conv1 on 64 images, 121 taps: 18.8 us with the
+// terms read from global memory one after the other, 16.4 like this.
+template <int KW>
+__global__ void __launch_bounds__(kBoxThreads) box_filter_kernel(const BoxTapArgs t) {
+    const BoxArgs &g = t.box;
+    extern __shared__ __align__(16) float tile[];
+    dependency_release();
+    dependency_wait();
+    const int n = blockIdx.x / g.row_blocks;
+    const int oy0 = (blockIdx.x - n * g.row_blocks) * g.rows;
+    const int n_out = min(g.rows, g.oh - oy0) * g.ow;
+    const int y0 = oy0 * g.sh - g.ph, pitch = g.phase * g.sw;
+    const float *img = g.a + (long)n * g.ih * g.iw;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < g.lines * g.span; i += kBoxThreads) {
+        const int line = (int)t.by_span((uint32_t)i), xx = i - line * g.span;
+        const int y = y0 + line, x = xx - g.pw, xs = (int)g.by_sw((uint32_t)xx);
+        float v = 0.f;
+        if (y >= 0 && y < g.ih && x >= 0 && x < g.iw)
+            v = __fmul_rn(__ldg(img + y * g.iw + x), g.inv_khw);
+        tile[line * pitch + (xx - xs * g.sw) * g.phase + xs] = v;
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < n_out; o += kBoxThreads) {
+        const int r = (int)g.by_ow((uint32_t)o), x = o - r * g.ow;
+        const float *row = tile + r * g.sh * pitch + x;
+        float acc = 0.f;
+        for (int i = 0; i < g.kh; i++, row += pitch) {
+            if (KW > 0) {
+#pragma unroll
+                for (int j = 0; j < KW; j++) acc = __fadd_rn(acc, row[t.tap[j]]);
+            } else {
+                for (int j = 0, at = 0, rem = 0; j < g.kw; j++) {
+                    acc = __fadd_rn(acc, row[rem * g.phase + at]);
+                    if (++rem == g.sw) { rem = 0; at++; }
+                }
+            }
+        }
+        g.k[((long)n * g.oh + oy0 + r) * g.ow + x] = acc;
+    }
+}
 
 // A line of the window of the thread's upper output (FIRST), of its lower one (SECOND), or of both.
 template <int KW, int SW, bool FIRST, bool SECOND>
@@ -362,9 +407,12 @@ __device__ __forceinline__ void add_line(const BoxArgs &g, const float *row, flo
     }
 }
 
-// TWO: a thread adds up two outputs, one below the other, and reads what their windows share once.
+// A thread keeps its column while it stages, eight lines at a time, and all its loads go out before the
+// first is used; tap j is word j / SW of remainder j % SW, known to the compiler. TWO: it adds up two
+// outputs, one below the other, and reads what their windows share once. AlexNet conv1 on 64 images,
+// launched alone: 16.4 us with the kernel above (8.8 M warp instructions), 13.8 like this (5.5 M).
 template <int KW, int SW, bool TWO>
-__global__ void __launch_bounds__(kBoxThreads) box_filter_kernel(const BoxArgs g) {
+__global__ void __launch_bounds__(kBoxThreads) box_filter_columns_kernel(const BoxArgs g) {
     extern __shared__ __align__(16) float tile[];
     dependency_release();
     dependency_wait();
@@ -445,18 +493,27 @@ __global__ void __launch_bounds__(kBoxThreads) box_filter_wide_kernel(const BoxA
     g.k[o] = acc;
 }
 
+using BoxTapFn = void (*)(BoxTapArgs);
+BoxTapFn box_kernel(int kw) {
+    return kw == 1    ? box_filter_kernel<1>
+           : kw == 3  ? box_filter_kernel<3>
+           : kw == 5  ? box_filter_kernel<5>
+           : kw == 7  ? box_filter_kernel<7>
+           : kw == 11 ? box_filter_kernel<11>
+                      : box_filter_kernel<0>;
+}
+// The same by columns; null where the other kernel is the better one.
 using BoxFn = void (*)(BoxArgs);
-template <bool TWO>
-BoxFn box_kernel(int kw, int sw) {
-    if (sw == 1 && kw == 1) return box_filter_kernel<1, 1, TWO>;
-    if (sw == 1 && kw == 3) return box_filter_kernel<3, 1, TWO>;
-    if (sw == 1 && kw == 5) return box_filter_kernel<5, 1, TWO>;
-    if (sw == 1 && kw == 7) return box_filter_kernel<7, 1, TWO>;
-    if (sw == 2 && kw == 3) return box_filter_kernel<3, 2, TWO>;
-    if (sw == 2 && kw == 5) return box_filter_kernel<5, 2, TWO>;
-    if (sw == 2 && kw == 7) return box_filter_kernel<7, 2, TWO>;
-    if (sw == 4 && kw == 11) return box_filter_kernel<11, 4, TWO>;
-    return box_filter_kernel<0, 1, TWO>;
+BoxFn box_columns_kernel(int kw, int sw, bool two) {
+    if (!two)
+        return kw == 5 && sw == 1   ? box_filter_columns_kernel<5, 1, false>
+               : kw == 5 && sw == 2 ? box_filter_columns_kernel<5, 2, false>
+                                    : nullptr;
+    if (kw == 7 && sw == 1) return box_filter_columns_kernel<7, 1, true>;
+    if (kw == 7 && sw == 2) return box_filter_columns_kernel<7, 2, true>;
+    if (kw == 11 && sw == 4) return box_filter_columns_kernel<11, 4, true>;
+    return kw == 1 || kw == 3 || kw == 5 || kw == 7 || kw == 11 ? nullptr
+                                                                : box_filter_columns_kernel<0, 1, true>;
 }
 
 BinArgs bin_args(const Plan &p, const float *src, void *out, float *a) {
@@ -563,10 +620,18 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
     g.by_sw = FastDiv((uint32_t)p.sw); g.by_ow = FastDiv((uint32_t)p.ow);
     auto lines = [&](int rows) { return (long)(rows - 1) * p.sh + p.kh; };
     auto bytes = [&](int rows) { return 4L * lines(rows) * g.phase * p.sw; };
-    // Two outputs a thread where their windows are large and share half of their lines at least (measured
-    // at 11 x 11 with stride 4: conv1 on 64 images 56.5 -> 55.7 us on one stream), else one; about one
-    // thread for each, if the rows that takes fit shared memory.
-    const int up = p.kh >= 2 * p.sh && p.kh * p.kw >= 49 && p.oh > 1 && bytes(2) <= kBoxSmem ? 2 : 1;
+    // By columns where an image's outputs are enough for half a block's threads; two outputs a thread where
+    // their windows are large and share half of their lines at least. calculate_k on 18 MB of one channel
+    // (150 us of it the mean |x|), an output a thread -> this: 5 x 5 on 56 x 56 198.6 -> 190.3 us, 7 x 7
+    // 209 -> 186, 9 x 9 295 -> 240, 9 x 9 with stride 2 191.5 -> 179, 13 x 13 412 -> 306; on 256 x 256
+    // 7 x 7 247 -> 202, 11 x 11 with stride 4 168.3 -> 167.9. Images of 49 outputs (14 x 14, stride 2)
+    // 174.8 -> 184.8 with 5 x 5, 178.8 -> 191.6 with 7 x 7; 7 x 7 images 232 to 266 -> 288 to 374.
+    // Widths that only the other kernel has compiled in: 3 x 3 178 -> 187 on 28 x 28, 203 -> 215 on 256 x
+    // 256, 11 x 11 246 -> 273 on 56 x 56, with stride 2 181 -> 191.
+    const bool two = p.kh >= 2 * p.sh && p.kh * p.kw >= 49 && p.oh > 1 && bytes(2) <= kBoxSmem;
+    const BoxFn by_columns = (long)p.oh * p.ow >= kBoxThreads / 2 ? box_columns_kernel(p.kw, p.sw, two) : nullptr;
+    const int up = by_columns && two ? 2 : 1;
+    // about one thread for each, if the rows that takes fit shared memory
     g.rows = up * (kBoxThreads / p.ow);
     if (g.rows > div_up_i(p.oh, up) * up) g.rows = div_up_i(p.oh, up) * up;
     if (g.rows < up) g.rows = up;
@@ -582,14 +647,20 @@ cudaError_t launch_box_filter(const Plan &p, const float *a, float *k, cudaStrea
     g.row_blocks = div_up_i(p.oh, g.rows);
     g.lines = (int)lines(g.rows);
     const unsigned blocks = (unsigned)(p.mb * g.row_blocks);
-    const int cols = div_up_i(g.span, 32) * 32;
-    g.cols = cols < kBoxThreads ? cols : kBoxThreads;
-    g.line_step = kBoxThreads / g.cols;
-    g.by_cols = FastDiv((uint32_t)g.cols);
-    auto kernel = up > 1 ? box_kernel<true>(p.kw, p.sw) : box_kernel<false>(p.kw, p.sw);
     // Launched under the tail of the packer, as the convolution is under its own: conv1 mb64 63.7 ->
     // 60.7 us a pass, the three upstream calls of an odd layer 20.6 -> 19.4.
-    return launch_overlapped(kernel, dim3(blocks), dim3(kBoxThreads), (size_t)bytes(g.rows), s, 1, g);
+    if (by_columns) {
+        const int cols = div_up_i(g.span, 32) * 32;
+        g.cols = cols < kBoxThreads ? cols : kBoxThreads;
+        g.line_step = kBoxThreads / g.cols;
+        g.by_cols = FastDiv((uint32_t)g.cols);
+        return launch_overlapped(by_columns, dim3(blocks), dim3(kBoxThreads), (size_t)bytes(g.rows), s, 1, g);
+    }
+    BoxTapArgs t;
+    t.box = g;
+    t.by_span = FastDiv((uint32_t)g.span);
+    for (int j = 0; j < 11; j++) t.tap[j] = j % p.sw * g.phase + j / p.sw;
+    return launch_overlapped(box_kernel(p.kw), dim3(blocks), dim3(kBoxThreads), (size_t)bytes(g.rows), s, 1, t);
 }
 
 }  // namespace xb200
