@@ -31,7 +31,7 @@ namespace xb200 {
 
 namespace {
 
-constexpr int kThreads = 256, kFewThreads = 128;
+constexpr int kThreads = 256;
 constexpr int kTasks = 8;   // few channels: warp loads per channel before the first is used
 
 struct FoldArgs {
@@ -70,11 +70,11 @@ struct NibbleTranspose {
 
 // IC channels (0: up to seven, four at a time); TWO: a row of a filter is two words of a column,
 // which are put together and stored as one.
-template <bool WITH_A, int IC, bool TWO>
-__global__ void __launch_bounds__(kFewThreads) fold_few_kernel(const FoldArgs g) {
+template <bool WITH_A, int IC, bool TWO, int THREADS>
+__global__ void __launch_bounds__(THREADS) fold_few_kernel(const FoldArgs g) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t *nibbles = reinterpret_cast<uint32_t *>(smem);  // [channel][row][pitch], eight columns a word
-    constexpr int kWarps = kFewThreads / 32;
+    constexpr int kWarps = THREADS / 32;
 
     const int n = blockIdx.x / g.row_blocks, hb = blockIdx.x - n * g.row_blocks;
     const int h0 = hb * g.sh - g.ph;  // input row of the block's first line
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kFewThreads) fold_few_kernel(const FoldArgs g)
     dependency_release();
     // rows outside the image and what a column reaches past it are zeros
     if (packs)
-        for (int i = threadIdx.x; i < g.ic * g.rows * g.pitch; i += kFewThreads) nibbles[i] = 0u;
+        for (int i = threadIdx.x; i < g.ic * g.rows * g.pitch; i += THREADS) nibbles[i] = 0u;
     __syncthreads();
     dependency_wait();
 
@@ -152,11 +152,11 @@ __global__ void __launch_bounds__(kFewThreads) fold_few_kernel(const FoldArgs g)
     // Item w of a column: a word, i.e. eight columns q of row i of channel c, or both of a row's two.
     // Threads are dealt whole columns' worth of items, so that a thread keeps its w.
     const int per = TWO ? 1 : (g.kw + 7) / 8;
-    const int groups = g.nw < kFewThreads ? (int)g.by_nw(kFewThreads) : 1;
-    const int group = g.nw < kFewThreads ? (int)g.by_nw(threadIdx.x) : 0;
+    const int groups = g.nw < THREADS ? (int)g.by_nw(THREADS) : 1;
+    const int group = g.nw < THREADS ? (int)g.by_nw(threadIdx.x) : 0;
     if (group >= groups) return;
     uint32_t *out = g.out + ((long)n * g.hb + hb) * g.ow * g.words;
-    for (int w = threadIdx.x - group * g.nw; w < g.nw; w += kFewThreads) {
+    for (int w = threadIdx.x - group * g.nw; w < g.nw; w += THREADS) {
         const int f = w / per, q = w - f * per;
         const uint32_t mask0 = first_nibbles(0xFFFFFFFFu, g.kw - 8 * q);
         const uint32_t mask1 = TWO ? first_nibbles(0xFFFFFFFFu, g.kw - 8) : 0u;
@@ -255,19 +255,20 @@ __global__ void __launch_bounds__(kThreads) fold_kernel(const FoldArgs g) {
 }
 
 using FoldFn = void (*)(FoldArgs);
-template <bool WITH_A, bool TWO>
+template <bool WITH_A, bool TWO, int THREADS>
 FoldFn few_kernel_of(int ic) {
     switch (ic) {
-        case 1: return fold_few_kernel<WITH_A, 1, TWO>;
-        case 2: return fold_few_kernel<WITH_A, 2, TWO>;
-        case 3: return fold_few_kernel<WITH_A, 3, TWO>;
-        case 4: return fold_few_kernel<WITH_A, 4, TWO>;
-        default: return fold_few_kernel<WITH_A, 0, TWO>;
+        case 1: return fold_few_kernel<WITH_A, 1, TWO, THREADS>;
+        case 2: return fold_few_kernel<WITH_A, 2, TWO, THREADS>;
+        case 3: return fold_few_kernel<WITH_A, 3, TWO, THREADS>;
+        case 4: return fold_few_kernel<WITH_A, 4, TWO, THREADS>;
+        default: return fold_few_kernel<WITH_A, 0, TWO, THREADS>;
     }
 }
+template <int THREADS>
 FoldFn few_kernel(bool with_a, bool two, int ic) {
-    return with_a ? (two ? few_kernel_of<true, true>(ic) : few_kernel_of<true, false>(ic))
-                  : (two ? few_kernel_of<false, true>(ic) : few_kernel_of<false, false>(ic));
+    return with_a ? (two ? few_kernel_of<true, true, THREADS>(ic) : few_kernel_of<true, false, THREADS>(ic))
+                  : (two ? few_kernel_of<false, true, THREADS>(ic) : few_kernel_of<false, false, THREADS>(ic));
 }
 
 }  // namespace
@@ -298,27 +299,31 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
     const int staged = 4 * (few ? p.ic : n8) * p.fold_rows * g.pitch;
     g.table_off = g.stage_off + div_up_i(staged, 16) * 16;
     const size_t smem = g.table_off + (few ? 0 : 8 * (size_t)g.nw);
-    void (*kernel)(FoldArgs) = few ? few_kernel(a != nullptr, two, p.ic)
-                               : a ? fold_kernel<true> : fold_kernel<false>;
-    static std::atomic<bool> opted_in[64][2];
+    const long blocks = (long)p.mb * g.row_blocks;
+    // Blocks of 256 threads where those of 128 would leave SMs with room for more of them (eight fit, four with
+    // five to seven channels) and each has more loads than a round or two. Packer alone, 128 -> 256 threads,
+    // us: 2048 columns of 3 channels, 406 blocks of 780 loads 27.6 -> 16.1, 805 of 390 18.4 -> 14.3; 1024
+    // columns, 812 blocks of 396 17.1 -> 13.1; 7 channels, 348 blocks of 924 28.2 -> 16.9. Slower: two images of
+    // 2048 columns, 116 blocks of 780, 9.4 -> 11.2 (one image 8.5 -> 6.3, four 18.3 -> 12.0).
+    const bool wide = few && blocks < (p.ic < 5 ? 148 * 8 : 148 * 4) && p.ic * p.sh * g.chunks > 320;
+    const FoldFn kernel = wide   ? few_kernel<256>(a != nullptr, two, p.ic)
+                          : few  ? few_kernel<128>(a != nullptr, two, p.ic)
+                          : a    ? fold_kernel<true>
+                                 : fold_kernel<false>;
+    // per device and kernel, once; few channels: fold_ok counts a bit a value, four of which take 192 KB at
+    // most
+    static std::atomic<bool> opted_in[64][2][2][2][6];
     int dev = 0;
     cudaGetDevice(&dev);
-    std::atomic<bool> &done = opted_in[dev & 63][a ? 1 : 0];
-    // Few channels: fold_ok counts a bit a value, four of which take 192 KB at most.
-    if (few && smem > 48 * 1024) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return e;
-    }
-    if (!few && !done.load(std::memory_order_acquire)) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    std::atomic<bool> &done = opted_in[dev & 63][wide ? 1 : 0][a ? 1 : 0][two ? 1 : 0][few ? (p.ic < 5 ? p.ic : 0) : 5];
+    if (smem > 48 * 1024 && !done.load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (few ? 200 : 160) * 1024);
         if (e != cudaSuccess) return e;
         done.store(true, std::memory_order_release);
     }
     note_launch();
-    return launch_overlapped(kernel, dim3((unsigned)(p.mb * g.row_blocks)),
-                             dim3(few ? kFewThreads : kThreads), smem, s, 1, g);
+    return launch_overlapped(kernel, dim3((unsigned)blocks), dim3(few && !wide ? 128 : kThreads), smem, s, 1, g);
 }
 
 }  // namespace xb200
