@@ -13,6 +13,7 @@ import pytest
 import cases
 import test_folded_gpu
 import test_long_filter_rows_gpu
+import test_long_tiles_gpu
 import test_position_columns_gpu
 import test_resident_filters_gpu
 import test_streamed_filters_gpu
@@ -38,10 +39,21 @@ FASTER_AS_ROWS = [
     cases._c("257_rows", 80, 256, 96, 3, 62, 3, 4, ph=1, pw=1),
 ]
 GPU_COLUMNS = test_position_columns_gpu.COLUMNS + test_resident_filters_gpu.COLUMNS
+# either side of the lines of the rule for eight epilogue warps
+EIGHT_WARPS = test_long_tiles_gpu.LONG_TILES + [
+    cases._c("conv2_eight_warps", 128, 256, 96, 27, 27, 5, 5, ph=2, pw=2),
+    cases._c("vgg_eight_warps", 64, 512, 512, 28, 28, 3, 3, ph=1, pw=1),
+]
+SIXTEEN_WARPS = [
+    cases._c("three_long_tiles_a_pair", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1),
+    cases._c("4608_cycles", 180, 256, 256, 28, 28, 3, 3, ph=1, pw=1),
+    cases._c("4224_cycles", 180, 256, 224, 28, 28, 3, 3, ph=1, pw=1),
+]
 LOST_COMMIT = cases._c("lost_commit", 64, 256, 96, 27, 27, 5, 5, ph=2, pw=2)
 LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + GPU_COLUMNS + test_position_columns_gpu.ROWS +
           test_resident_filters_gpu.ROWS + [LOST_COMMIT] + test_streamed_filters_gpu.STREAMED +
-          test_folded_gpu.FOLDED + test_long_filter_rows_gpu.LONG_ROWS + cases.SHAPE_CASES + [
+          test_folded_gpu.FOLDED + test_long_filter_rows_gpu.LONG_ROWS + EIGHT_WARPS + SIXTEEN_WARPS +
+          cases.SHAPE_CASES + [
               cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
               cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
 
@@ -104,6 +116,13 @@ def test_gpu_tests_of_position_columns_reach_them(launches):
     assert min(g["groups"] for g in got) < 8 < max(g["groups"] for g in got)
     assert 8 in {g["groups"] for g in got} and 1 in {g["shared_cols"] for g in got}
     assert not any(g["planes"] for g in _of(launches, test_position_columns_gpu.ROWS))
+
+
+def test_eight_epilogue_warps_on_long_tiles(launches):
+    assert [g["epilogue_warps"] for g in _of(launches, EIGHT_WARPS)] == [8] * len(EIGHT_WARPS)
+    assert [g["epilogue_warps"] for g in _of(launches, SIXTEEN_WARPS)] == [16] * len(SIXTEEN_WARPS)
+    got = _of(launches, test_long_tiles_gpu.LONG_TILES)
+    assert {g["shared_cols"] for g in got} == {0, 1} and {g["n_tiles"] for g in got} == {1, 2}
 
 
 def test_gpu_tests_of_long_filter_rows_reach_columns(launches):

@@ -1216,16 +1216,18 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     const int kk = p.kchunk / 32;
     // Eight epilogue warps instead of sixteen where a pair has four tiles or more and each keeps the tensor
-    // pipe busy for 4096 cycles or more: the stores have the next tile's MMAs to hide behind either way, all
-    // but the last tile's. A pass among others and on one stream, 16 and 8 warps, us: conv2 on 128 images (5120
-    // cycles, six tiles) 45.4 -> 44.2 and 47.9 -> 46.8, VGG (9216, six) 73.0 -> 72.2 and 75.4 -> 73.8. conv4 on
-    // 256 images (6912, three) 38.3 -> 38.8 in one set of runs, 37.6 -> 37.2 in another, chained layers that end
-    // in two such tiles 43.5 -> 43.8; conv3 (3456) 33.9 -> 34.0, 48 channels and 368 filters (864) on one stream
-    // 18.2 -> 19.1, one tap of 51 channels (16) 23.0 -> 24.2.
+    // pipe busy for 5000 cycles or more: the stores have the next tile's MMAs to hide behind either way, all
+    // but the last tile's. The time with sixteen over that with eight, layers of 28 x 28 with 128, 256 and 512
+    // filters and four to eight tiles a pair, a pass among others and on one stream (runs differ by 0.5 %):
+    //   5760 to 9216 cycles  0.98 to 1.02, mean 1.006   1.00 to 1.02, mean 1.012
+    //   4224 to 4608         0.94 to 1.01, mean 0.99    1.00 to 1.02, mean 1.004
+    //   fewer                0.98 to 1.03, mean 1.00    1.00 to 1.09, mean 1.013
+    // conv2 on 128 images (5120 cycles, six tiles) 43.3 -> 42.7 us among others, VGG (9216, six) 71.6 -> 71.2.
+    // With two or three tiles 0.90 to 1.07.
     const long tile_cycles =
         (long)g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last) * p.n_tile / 2;
     const int pair_tiles = div_up_i(((m_tiles + 1) / 2) * g.n_tiles, sms / 2);
-    const bool few = pair && kk == 4 && tile_cycles >= 4096 && pair_tiles >= 4;
+    const bool few = pair && kk == 4 && tile_cycles >= 5000 && pair_tiles >= 4;
     const int epi = few ? kFewEpiWarps : kEpiWarps;
     void (*kernel)(CUtensorMap, CUtensorMap, TcArgs) =
         few    ? conv_tcgen05_kernel<4, true, kFewEpiWarps>
