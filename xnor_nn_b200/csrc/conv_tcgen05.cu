@@ -938,7 +938,7 @@ __device__ __forceinline__ void producer_planes(const TcArgs &g, Control *ctl,
 // filters; the tensor pipe needs 128 an instruction on AlexNet conv2): working the starts out once instead of
 // dividing in every group took conv2 on 128 images from 42.9 to 42.0 us a pass among others, 96 channels on
 // 75 images from 27.7 to 27.1 and on one stream from 33.3 to 32.3. A table of 32 starts is one a lane.
-template <int KK>
+template <int KK, bool LONG>
 __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                                 uint32_t stage0, int who) {
     volatile int *abort_flag = &ctl->abort_flag;
@@ -955,13 +955,13 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
     const uint32_t afull0 = smem_u32(&ctl->a_full[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
     // Where the instructions of a filter row's chunks start, from its first position and column: a lane
     // works one out, so that no group has to divide. Rows of more than 32 instructions (over 1 KB) have
-    // the chunk's worked out by KK lanes in every group.
+    // the chunk's worked out by KK lanes in every group (LONG; with the question asked in the loop conv2
+    // took 43.6 us instead of 43.5).
     auto start_at = [&](int byte) {
         const int pos = byte / g.pos_bytes;
         return (uint32_t)((byte - pos * g.pos_bytes) >> 4) * lbo + (uint32_t)pos;
     };
     const int lane = threadIdx.x & 31;
-    const bool long_rows = g.chunks_per_tap * KK > 32;
     uint32_t start_of = start_at(lane / KK * g.kchunk + lane % KK * 32);
     int sa = 0, b = 0;
     uint32_t pa = 0, acc_phase = 0;
@@ -990,11 +990,11 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
                 fence_after();
             }
             const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
-            if (long_rows) start_of = start_at(chunk * g.kchunk + lane % KK * 32);
+            if (LONG) start_of = start_at(chunk * g.kchunk + lane % KK * 32);
             uint32_t start[KK];
 #pragma unroll
             for (int k = 0; k < KK; k++)
-                start[k] = __shfl_sync(0xffffffffu, start_of, (long_rows ? 0 : chunk * KK) + k);
+                start[k] = __shfl_sync(0xffffffffu, start_of, (LONG ? 0 : chunk * KK) + k);
             if (leader) {
                 const uint32_t at = tile + (uint32_t)(row * g.wp);
                 const uint64_t bdesc = b_hi | (uint64_t)(b_lo0 + (uint32_t)gr * b_units);
@@ -1111,7 +1111,10 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         const int who = warp == 1 ? 0 : 1;
         if (who < g.issuers && rank == 0) {
             if constexpr (PAIR) {
-                if (g.planes) mma_role_planes<KK>(g, ctl, tmem_base, stage0, who);
+                // filter rows of more than 32 instructions have chunks of 128 bytes
+                if (KK == 4 && g.planes && g.chunks_per_tap * KK > 32)
+                    mma_role_planes<KK, true>(g, ctl, tmem_base, stage0, who);
+                else if (g.planes) mma_role_planes<KK, false>(g, ctl, tmem_base, stage0, who);
                 else if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
                 else if (g.halo) mma_role_halo<KK>(g, ctl, tmem_base, stage0, who);
                 else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
@@ -1304,8 +1307,8 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         //   more, filters that would not be resident beside rows        0.94 to 1.10, median 1.00
         //   the others                                                  0.73 to 1.04, median 0.94
         // Only the last take columns; layers of the fourth kind stream their filters. Filters of ten and more
-        // columns, whose rows may be more than 1 KB, gain more, not less: 13 x 6 on 167 channels 241 us a
-        // pass, 315 as rows; 33 x 3 on 39 62 and 73; 25 x 3 on 214 142 and 174.
+        // columns, whose rows may be more than 1 KB, gain more, not less: 13 x 6 on 167 channels 218 us a
+        // pass, 315 as rows; 33 x 3 on 39 57 and 73; 25 x 3 on 214 129 and 174.
         const int columns = p.icp / 16, planes = columns + (columns & 1);
         const int rows = BM + (g.kh - 1) * p.wp + p.kw - 1;
         const int pitch = (rows + 7) & ~7;  // a load lands on a multiple of 128 bytes
