@@ -506,7 +506,9 @@ __device__ __forceinline__ void producer_ring(const TcArgs &g, Control *ctl,
 // i, i+2, ... of the running stage sequence, which continues across tiles), each commits its own
 // stages, and both commit to the accumulator's barrier (count 2) after their last stage of a
 // tile: a commit covers the MMAs of the committing thread only. The sum is over integers, so the
-// order in which the two threads' MMAs reach the pipe does not matter, except for the tile's
+// order in which the two threads' MMAs reach the pipe does not matter (that none of their sums is
+// lost is an assumption about the pipe, which executes them one after the other, and not documented
+// for several issuing threads; test_shared_accumulator_gpu.py watches it), except for the tile's
 // first instruction, which overwrites the accumulator: its issuer waits for the epilogue to have
 // drained the accumulator, and the other issuer waits until it has been executed (started[], a
 // commit: nothing orders the MMAs of two threads that have only been issued). The ring has an even
