@@ -10,13 +10,6 @@
 namespace xb200 {
 namespace tc {
 
-// (S * alpha) * K in upstream's order. The + 0 comes before the products: it makes a sum of zero +0
-// whatever sign the adder gave it, and leaves the -0 that a negative S times an alpha of zero is (a
-// filter of zeros; the next layer reads that sign).
-__device__ __forceinline__ float scaled(uint32_t s, float alpha, float k) {
-    return __fmul_rn(__fmul_rn(__fadd_rn(__uint_as_float(s), 0.f), alpha), k);
-}
-
 // The pixel and the filters that a lane stores.
 struct StoreAt {
     float *dst;
@@ -28,17 +21,11 @@ struct StoreAt {
 };
 
 // NCHW: for one filter the 32 lanes hold 32 neighbouring pixels, so a store instruction writes one
-// contiguous run. `al` = alpha from the tile's first filter on, in shared memory if `al_smem`;
-// columns_read(i) is called when the i-th load from tensor memory has completed, in reverse order of
-// the column groups if `reverse`.
-template <class F>
-__device__ __forceinline__ void store_nchw(const StoreAt &s, const float *al, bool al_smem, int n_tile,
-                                           uint32_t taddr, int cgroup, int cgroups, bool reverse,
-                                           F columns_read) {
+// contiguous run. `al` = alpha from the tile's first filter on, in shared memory.
+__device__ __forceinline__ void store_nchw(const StoreAt &s, const float *al, int n_tile, uint32_t taddr,
+                                           int cgroup, int cgroups) {
     float *out = s.dst + ((long)s.n * s.oc + s.oc0) * s.ohw + s.r;
-    const int steps = (n_tile - 32 * cgroup + 32 * cgroups - 1) / (32 * cgroups);
-    for (int i = 0; i < steps; i++) {
-        const int c0 = 32 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
+    for (int c0 = 32 * cgroup; c0 < n_tile; c0 += 32 * cgroups) {
         uint32_t v[32];
         if (c0 + 32 <= n_tile) {
             ld32(taddr + (uint32_t)c0, v);
@@ -46,11 +33,10 @@ __device__ __forceinline__ void store_nchw(const StoreAt &s, const float *al, bo
             ld16(taddr + (uint32_t)c0, v);
         }
         wait_ld();
-        columns_read(i);
         if (s.valid) {
             const int lim = s.n_valid - c0;
             float *o = out + (long)c0 * s.ohw;
-            if (al_smem && lim >= 32) {
+            if (lim >= 32) {
                 // full group: alpha by 16-byte shared loads, one running pointer
                 const float4 *a4 = reinterpret_cast<const float4 *>(al + c0);
 #pragma unroll
@@ -76,20 +62,16 @@ __device__ __forceinline__ void store_nchw(const StoreAt &s, const float *al, bo
 
 // NHWC, a number of filters that is a multiple of four and a result that starts on 16 bytes: a thread
 // owns one pixel and 16 neighbouring filters at a time, which are contiguous in the result.
-template <class F>
 __device__ __forceinline__ void store_nhwc(const StoreAt &s, const float *al, int n_tile, uint32_t taddr,
-                                           int cgroup, int cgroups, bool reverse, F columns_read) {
+                                           int cgroup, int cgroups) {
     float *out = s.dst + s.pix * s.oc + s.oc0;
     // 256-bit stores need 32-byte alignment: rows and tiles that are multiples of 8
     // floats on a result buffer aligned likewise
     const bool wide = (s.oc & 7) == 0 && (s.oc0 & 7) == 0 && ((uintptr_t)s.dst & 31) == 0;
-    const int steps = (n_tile - 16 * cgroup + 16 * cgroups - 1) / (16 * cgroups);
-    for (int i = 0; i < steps; i++) {
-        const int c0 = 16 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
+    for (int c0 = 16 * cgroup; c0 < n_tile; c0 += 16 * cgroups) {
         uint32_t v[16];
         ld16(taddr + (uint32_t)c0, v);
         wait_ld();
-        columns_read(i);
         if (s.valid && wide && c0 + 16 <= s.n_valid) {
             // 16 results = two whole 32-byte sectors, one 256-bit store each
             float x[16];
@@ -119,18 +101,13 @@ __device__ __forceinline__ void store_nhwc(const StoreAt &s, const float *al, in
 }
 
 // NHWC, any number of filters and any start of the result.
-template <class F>
 __device__ __forceinline__ void store_nhwc_odd(const StoreAt &s, const float *al, int n_tile,
-                                               uint32_t taddr, int cgroup, int cgroups, bool reverse,
-                                               F columns_read) {
+                                               uint32_t taddr, int cgroup, int cgroups) {
     float *out = s.dst + s.pix * s.oc + s.oc0;
-    const int steps = (n_tile - 16 * cgroup + 16 * cgroups - 1) / (16 * cgroups);
-    for (int i = 0; i < steps; i++) {
-        const int c0 = 16 * (cgroup + cgroups * (reverse ? steps - 1 - i : i));
+    for (int c0 = 16 * cgroup; c0 < n_tile; c0 += 16 * cgroups) {
         uint32_t v[16];
         ld16(taddr + (uint32_t)c0, v);
         wait_ld();
-        columns_read(i);
         if (s.valid) {
 #pragma unroll
             for (int j = 0; j < 16; j++)

@@ -135,13 +135,6 @@ struct Deal {
     }
 };
 
-// (S * alpha) * K in upstream's order. The + 0 comes before the products: it makes a sum of zero +0
-// whatever sign the adder gave it, and leaves the -0 that a negative S times an alpha of zero is (a
-// filter of zeros; the next layer reads that sign).
-__device__ __forceinline__ float scaled(uint32_t s, float alpha, float k) {
-    return __fmul_rn(__fmul_rn(__fadd_rn(__uint_as_float(s), 0.f), alpha), k);
-}
-
 // ---- epilogue role ---------------------------------------------------------------------------------
 // Warp w may touch TMEM lanes [32*(w%4), 32*(w%4)+32); several warps share a quadrant and split
 // its columns between them.

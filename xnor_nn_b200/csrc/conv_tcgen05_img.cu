@@ -422,12 +422,8 @@ conv_tcgen05_img_kernel(const __grid_constant__ CUtensorMap map_w,
                             const float4 k4 = *reinterpret_cast<const float4 *>(kk + c0 + j);
                             kv[j] = k4.x; kv[j + 1] = k4.y; kv[j + 2] = k4.z; kv[j + 3] = k4.w;
                         }
-                        // S + 0: a sum of zero is +0 whatever sign the adder gave it, and a
-                        // negative one times an alpha of zero stays -0
 #pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            v[j] = __float_as_uint(__fmul_rn(
-                                __fmul_rn(__fadd_rn(__uint_as_float(v[j]), 0.f), al), kv[j]));
+                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(scaled(v[j], al, kv[j]));
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; j++) v[j] = (uint32_t)(int)__uint_as_float(v[j]);

@@ -65,7 +65,6 @@ constexpr int kThreads = 32 * (1 + kWorkers + kIssuers);
 // Four tasks a worker. 7 x 402 channels of 29 x 29 (78 tasks): 7.1 -> 5.6 us among others, 16.3 -> 14.2 on
 // one stream, 27.0 -> 26.6 alone; 492 channels of 51 x 51 (128 tasks): 6.7 -> 7.1, 13.3 -> 20.2, 24.2 -> 32.
 constexpr int kMaxTasks = 4 * kWorkers;
-constexpr int kSms = 148;
 constexpr int kMaxStages = 36, kMaxParts = 8, kMaxGroups = 16, kMaxRows = 32 * kMaxGroups;
 
 struct WholeArgs {
@@ -360,13 +359,12 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
             fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
             const StoreAt to = {g.dst, g.oc, oc0, min(g.n_tile, g.oc - oc0), n, r, pix, ohw, kk, valid};
-            auto nothing = [](int) {};
             if (!g.dst_nhwc)
-                store_nchw(to, ctl->alpha, true, g.n_tile, taddr, cgroup, cgroups, false, nothing);
+                store_nchw(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups);
             else if ((g.oc & 3) == 0 && ((uintptr_t)g.dst & 15) == 0)
-                store_nhwc(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups, false, nothing);
+                store_nhwc(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups);
             else
-                store_nhwc_odd(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups, false, nothing);
+                store_nhwc_odd(to, ctl->alpha, g.n_tile, taddr, cgroup, cgroups);
         }
     }
     fence_before();
@@ -387,10 +385,10 @@ bool whole_shape(const Plan &p, WholeArgs *g, size_t *smem) {
     // take less time then and nothing else wants the SMs (one image, 2 tiles of 256 -> 16 of 32: 12.0 ->
     // 11.7 us on one stream).
     g->n_tile = div_up_i(div_up_i(p.oc, div_up_i(p.oc, 256)), 16) * 16;
-    while (g->n_tile / 2 >= 32 && m_tiles * div_up_i(p.oc, (g->n_tile / 2 + 15) / 16 * 16) <= kSms / 3)
+    while (g->n_tile / 2 >= 32 && m_tiles * div_up_i(p.oc, (g->n_tile / 2 + 15) / 16 * 16) <= sm_count() / 3)
         g->n_tile = (g->n_tile / 2 + 15) / 16 * 16;
     g->n_tiles = div_up_i(p.oc, g->n_tile);
-    if (m_tiles * g->n_tiles > kSms || 4L * p.mb * p.ic * p.ih * p.iw >= 1L << 32) return false;
+    if (m_tiles * g->n_tiles > sm_count() || 4L * p.mb * p.ic * p.ih * p.iw >= 1L << 32) return false;
     g->rows = BM + (p.kh - 1) * p.wp + p.kw - 1;
     g->columns = p.icp / 16;
     g->odd = p.cat && (g->columns & 1);

@@ -305,7 +305,7 @@ cudaError_t launch_fold(const Plan &p, const float *src, void *bin_src, float *a
     // us: 2048 columns of 3 channels, 406 blocks of 780 loads 27.6 -> 16.1, 805 of 390 18.4 -> 14.3; 1024
     // columns, 812 blocks of 396 17.1 -> 13.1; 7 channels, 348 blocks of 924 28.2 -> 16.9. Slower: two images of
     // 2048 columns, 116 blocks of 780, 9.4 -> 11.2 (one image 8.5 -> 6.3, four 18.3 -> 12.0).
-    const bool wide = few && blocks < (p.ic < 5 ? 148 * 8 : 148 * 4) && p.ic * p.sh * g.chunks > 320;
+    const bool wide = few && blocks < (p.ic < 5 ? 8 : 4) * sm_count() && p.ic * p.sh * g.chunks > 320;
     const FoldFn kernel = wide   ? few_kernel<256>(a != nullptr, two, p.ic)
                           : few  ? few_kernel<128>(a != nullptr, two, p.ic)
                           : a    ? fold_kernel<true>

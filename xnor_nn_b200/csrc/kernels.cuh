@@ -80,6 +80,13 @@ __device__ __forceinline__ uint32_t first_nibbles(uint32_t word, int n) {
     return n >= 8 ? word : n <= 0 ? 0u : word & (0xFFFFFFFFu >> (4 * (8 - n)));
 }
 
+// (S * alpha) * K in upstream's order, S as the bits of a float. The + 0 comes before the products: it
+// makes a sum of zero +0 whatever sign the adder gave it, and leaves the -0 that a negative S times an
+// alpha of zero is (a filter of zeros; the next layer reads that sign).
+__device__ __forceinline__ float scaled(uint32_t s, float alpha, float k) {
+    return __fmul_rn(__fmul_rn(__fadd_rn(__uint_as_float(s), 0.f), alpha), k);
+}
+
 // Lets the next kernel of the stream start its set-up now ...
 __device__ __forceinline__ void dependency_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

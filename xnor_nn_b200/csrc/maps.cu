@@ -107,7 +107,7 @@ bool maps_shape(const Plan &p, MapArgs *g) {
     if ((long)p.kh * p.kw > 64 || (long)p.oh * p.ow > 1 << 20) return false;
     g->columns = div_up_i(p.ic, 32);
     const long span = (long)(p.ow - 1) * p.sw + p.kw;
-    int rows = (int)((long)p.mb * p.oh / 148);
+    int rows = (int)((long)p.mb * p.oh / sm_count());
     if (rows < p.kh - 1) rows = p.kh - 1;
     if (rows < 1) rows = 1;
     if (rows > p.oh) rows = p.oh;

@@ -7,9 +7,7 @@
 
 namespace xb200 {
 
-// SMs of the current device (148 on B200); the same figure when no device can be asked, so that
-// plans made on a machine without a GPU come out as they would on the target.
-static int sm_count() {
+int sm_count() {
     static const int n = [] {
         int dev = 0, v = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||

@@ -122,6 +122,10 @@ long frame_slack(const Plan &p);
 
 int div_up_i(int a, int b);
 
+// SMs of the current device (148 on B200); the same figure when no device can be asked, so that
+// plans made on a machine without a GPU come out as they would on the target.
+int sm_count();
+
 // Fills a Plan from the descriptor fields and the requested family (kAuto: pick by shape).
 // Never fails: unknown formats are remembered and reported by the executors.
 void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested);
