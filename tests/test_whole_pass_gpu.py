@@ -33,12 +33,16 @@ ONE_LAUNCH = [
     cases._c("channels_last_odd", 3, 43, 91, 10, 11, 3, 3, ph=1, pw=1, fmt=CL),
     cases._c("channels_last_whole_sectors", 20, 256, 384, 13, 13, 3, 3, ph=1, pw=1, fmt=CL),
     cases._c("channels_last_source_only", 3, 44, 92, 10, 11, 3, 3, ph=1, pw=1, fmt=(1, 0, 0)),
+    cases._c("packed_twice_less_work", 10, 300, 256, 14, 14, 3, 3, ph=1, pw=1),
     cases._c("filter_of_zeros_and_ties", 2, 16, 6, 6, 7, 2, 2, ph=1, pw=1, fill="affine"),
 ]
 TWO_LAUNCHES = [
     cases._c("149_tiles", 149, 33, 40, 8, 16, 1, 1),
     cases._c("513_rows", 1, 20, 33, 5, 191, 3, 4, ph=1, pw=1),
     cases._c("81_tasks", 1, 20, 860, 9, 9, 1, 1),
+    # as long as the general path's work, half of it repeated; with a quarter of it one launch again
+    cases._c("packed_twice", 40, 300, 256, 14, 14, 3, 3, ph=1, pw=1),
+    cases._c("wide_halos", 16, 31, 229, 27, 27, 5, 5, ph=2, pw=2),
 ]
 
 

@@ -409,7 +409,20 @@ bool whole_shape(const Plan &p, WholeArgs *g, size_t *smem) {
     g->b_bytes = (uint32_t)(g->n_tile * p.kchunk);
     g->stage_bytes = (g->b_bytes + 1023u) & ~1023u;
     // a group of pixels is 32, or fewer if borders are in between
-    if (div_up_i(g->rows, 32) * g->columns > kMaxTasks) return false;
+    const int tasks = div_up_i(g->rows, 32) * g->columns;
+    if (tasks > kMaxTasks) return false;
+    // Not where pixels are packed more than 1.6 times (by neighbouring tiles, in halos, and by each filter tile)
+    // and the tiles, dealt to all SMs, come to more than 5.5 us in the cycles above: the general path does that
+    // work once, and with passes on several streams hides its second launch under it. The time of two launches
+    // over that of one, geometric means: of 275 layers that ran here before (drawn from 1 to 256 images, 16 to
+    // 512 channels and filters, 6 to 56 pixels) among others 1.33, on one stream 1.22, waited for 1.04; of the
+    // eleven that this rule takes out 0.90, 1.06 and 0.95; 384 filters on 256 channels of 13 x 13, 48 images,
+    // 0.75, 1.03 and 0.93. What stays slower alone is few tiles of many filters, which leave most SMs idle:
+    // conv4 on 16 to 48 images 1.2 to 1.4 among others, 0.82 to 0.99 on one stream, 0.87 to 0.95 waited for.
+    const long mma_cycles = (long)g->taps * ((g->chunks - 1) * (p.kchunk / 32) + g->kk_last) * g->n_tile / 2;
+    const long tile_cycles = 1200 + 4000 * div_up_i(tasks, kWorkers) + mma_cycles * 11 / 10 + 22 * g->n_tile;
+    const bool repeats = 10L * g->n_tiles * g->rows > 16L * BM;
+    if (repeats && m_tiles * g->n_tiles * tile_cycles > 10450L * sm_count()) return false;  // at 1.9 GHz
     const size_t operand = (size_t)g->planes * g->pitch * 16;
     g->b_off = (uint32_t)((kControlBytes + operand + 1023) & ~(size_t)1023);
     const size_t room = 227 * 1024 - 1024, want = 128 * 1024;
