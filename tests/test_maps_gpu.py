@@ -30,6 +30,9 @@ TWO_LAUNCHES = [
     cases._c("72_taps", 2, 16, 20, 14, 15, 9, 8, ph=4, pw=4),
     cases._c("over_16_megabytes", 65, 16, 64, 32, 32, 3, 3, ph=1, pw=1),
     cases._c("1025_channels_wide", 1, 16, 1025, 3, 64, 3, 3, ph=1, pw=1),
+    # longer than two launches take: bands of 60 tasks, many blocks of few
+    cases._c("long_bands", 19, 16, 464, 17, 17, 5, 5, ph=2, pw=2),
+    cases._c("many_bands", 5, 16, 3, 161, 161, 5, 5, ph=2, pw=2),
 ]
 
 

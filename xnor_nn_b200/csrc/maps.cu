@@ -99,6 +99,18 @@ __global__ void __launch_bounds__(kThreads) maps_kernel(const MapArgs g) {
     }
 }
 
+// What the launch takes, to a sixth (fitted to 78 layers of more than 5.9 us): a block's warps walk its tasks
+// one after the other, and all blocks share the SMs. Two launches take a host 5.7 us, most of which passes on
+// several streams hide. Over 285 layers (drawn from 1 to 256 images, 1 to 512 channels, 6 to 227 pixels, up to
+// 16 MB), the three upstream calls with two launches here over those with one: 1.02 on one stream and 1.14
+// among others if all take one, 1.035 and 1.14 with this rule; the 48 that it takes out 0.90 and 1.005 (19
+// images of 464 channels, 17 x 17, filters of 5 x 5: 44.6 and 60.6 us on one stream, calculate_k alone 7.0 and
+// 18.8).
+double launch_us(long blocks, long tasks, long outputs, int taps) {
+    return 3.6 + 0.58 * (double)(blocks * tasks) / (8.0 * sm_count()) + 0.74 * (double)((tasks + 7) / 8) +
+           0.58 * (double)((outputs + kThreads - 1) / kThreads) * taps / 25;
+}
+
 // Bands: as tall as leaves a block per SM, and at least so tall that most of what a band reads is its own.
 bool maps_shape(const Plan &p, MapArgs *g) {
     if (p.mb < 1 || p.oh < 1 || p.ow < 1 || p.ic < 1 || p.ih < 1 || p.iw < 1) return false;
@@ -126,7 +138,8 @@ bool maps_shape(const Plan &p, MapArgs *g) {
             g->bands = bands;
             g->lines = (int)lines;
             g->span = (int)span;
-            return (long)p.mb * bands < 1L << 30;
+            return (long)p.mb * bands < 1L << 30 &&
+                   launch_us((long)p.mb * bands, groups * g->columns, (long)rows * p.ow, p.kh * p.kw) <= 8.5;
         }
         if (rows == 1) return false;
     }
