@@ -16,8 +16,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("kernel", [xb.KERNEL_TCGEN05_I8, xb.KERNEL_TCGEN05_I8_ROWS],
                          ids=["tcgen05_i8", "tcgen05_i8_rows"])
-# one image; 40 images: one tile per thread block on many SMs; 256 images: several tiles per block,
-# the position-tile kernel on CTA pairs (the block that loses its commit is a pair's leader, so
+# The kernels behind the `forward` executor. (Passes of small layers in one call run on another one,
+# test_small_layer_waits_gpu.py.) One image; 40 images: one tile per thread block on many SMs; 256 images:
+# several tiles per block, the position-tile kernel on CTA pairs (the block that loses its commit is a pair's leader, so
 # both blocks of the pair give up, keep the epilogue's meetings and leave through the cluster
 # barrier). Layer D, 96 channels: the position-tile kernel with position tiles as columns beside
 # resident filters, two issuers on every tile of a pair

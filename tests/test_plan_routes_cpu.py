@@ -53,8 +53,8 @@ def test_rows_beyond_an_accumulator_run_on_popc():
 
 
 def test_strided_layers_of_few_channels_fold_while_their_bits_fit():
-    """The packer stages a bit per value, in 48 KB. Borders count in a row's pitch even where a wide
-    stride skips most of them."""
+    """The packer stages half a byte per value, in 192 KB (the rule counts a bit, in 48). Borders count in a
+    row's pitch even where a wide stride skips most of them."""
     assert _kernel(1, 8, 7, 16, 1000, 8, 8, sh=8, sw=8) == xb.KERNEL_TCGEN05_I8
     assert _kernel(1, 8, 7, 11, 1117, 11, 11, sh=11, sw=11, ph=1900, pw=1900) == xb.KERNEL_TCGEN05_I8
     assert _kernel(1, 8, 7, 11, 1117, 11, 11, sh=11, sw=11, ph=2000, pw=2000) == xb.KERNEL_POPC

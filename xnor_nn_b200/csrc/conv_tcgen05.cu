@@ -21,10 +21,10 @@
 //               N<=256, K=64 per instruction) into one of two to four accumulators in tensor
 //               memory, and tcgen05.commit hands buffers back / accumulators on
 //   warp 18     a second MMA issuer; the two take alternate ring buffers
-//   warps 2-17  (in pairs with long tiles 2-9, and the second issuer 10) epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions
-//               and a share of the columns), scale by alpha[filter] * K[position] in upstream's
-//               order and store; runs under the next tiles' MMAs thanks to the other
-//               accumulators
+//   warps 2-17  epilogue: tcgen05.ld the accumulator (a warp owns 32 TMEM lanes = 32 positions and a
+//               share of the columns), scale by alpha[filter] * K[position] in upstream's order
+//               and store; runs under the next tiles' MMAs thanks to the other accumulators.
+//               (In pairs with long tiles 2-9, and the second issuer 10.)
 //
 // Layers of more than one round of tiles run as clusters of two CTAs on tcgen05 cta_group::2:
 // the pair shares a tile of 256 positions x N filters, each CTA loads its own 128 positions and
@@ -1165,8 +1165,9 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // CTA pairs when the layer is more than one round of tiles (measured with 8-bit operands on
     // AlexNet conv4: 35.0 against 36.9 us at 256 images, 24.3 against 24.9 at 128). With a single
     // round the pair's longer hand-shakes cost more than its lighter loads save: a pass on one image
-    // 13.5 against 12.4 us with the present operands, on 32 images 17.5 against 16.6. Floats or sums out only (the chained epilogue carries per-pixel state across the
-    // filter tiles of one CTA), and a filter tile that splits into two UMMA-sized halves.
+    // 13.5 against 12.4 us with the present operands, on 32 images 17.5 against 16.6. Floats or sums out
+    // only (the chained epilogue carries per-pixel state across the filter tiles of one CTA), and a
+    // filter tile that splits into two UMMA-sized halves.
     const bool pair = !next && p.n_tile % 32 == 0 && m_tiles >= 2 &&
                       (long)m_tiles * (p.ocp16 / p.n_tile) > sms;
     const int b_rows = pair ? p.n_tile / 2 : p.n_tile;  // filter rows a CTA loads per stage

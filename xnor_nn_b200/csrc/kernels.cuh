@@ -137,8 +137,8 @@ cudaError_t launch_binarize_weights(const Plan &p, const float *w, void *bin_w, 
                                     int32_t *op_c, cudaStream_t s);
 
 // to = sign(from) * mean(from) over `elems` device floats (upstream
-// src/binarize_weights_float.cpp:3-25), with a fixed summation shape. Takes and returns a few
-// hundred bytes of stream-ordered scratch.
+// src/binarize_weights_float.cpp:3-25), with a fixed summation shape. Block sums pass through the
+// result, or, where it is small or also the source, through a kilobyte of stream-ordered scratch.
 cudaError_t launch_binarize_weights_float(long elems, const float *from, float *to,
                                           cudaStream_t s);
 

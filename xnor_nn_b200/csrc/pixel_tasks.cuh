@@ -10,8 +10,8 @@ namespace xb200 {
 namespace tasks {
 
 // 32 channels of 32 pixels, channels-last: eight lanes read a pixel's channels, four each (with 16-byte
-// loads where they are aligned) and four pixels at a time, and an 8 x 8 transposition of those quadruples leaves a lane with all channels of
-// pixel 4 (lane % 8) + lane / 8.
+// loads where they are aligned) and four pixels at a time, and an 8 x 8 transposition of those quadruples
+// leaves a lane with all channels of pixel 4 (lane % 8) + lane / 8.
 __device__ __forceinline__ void transpose8(float *v, int sub) {
 #pragma unroll
     for (int d = 4; d > 0; d >>= 1) {

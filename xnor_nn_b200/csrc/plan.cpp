@@ -57,9 +57,9 @@ int fold_bit_pitch(const Plan &p) {
     return pitch < (1L << 30) ? (int)pitch : 1 << 30;
 }
 
-// A strided layer is folded when its packer's working set (a row block of some channels, a bit per
-// value with fewer than eight of them, else half a byte, and the mean-|x| sums of the block's
-// pixels) fits shared memory. The popcount kernel it would otherwise run on needs 870 us for
+// A strided layer is folded when its packer's working set (a row block of some channels, half a byte a
+// value, and with eight channels or more the mean-|x| sums of the block's pixels) fits shared memory.
+// With fewer than eight channels the limit is a bit a value in 48 KB, which are 192 KB as staged. The popcount kernel it would otherwise run on needs 870 us for
 // AlexNet conv1 on 64 images.
 constexpr long kFoldStage = 48 * 1024, kFoldSums = 48 * 1024, kFoldWords = 4096;
 static bool fold_ok(const Plan &p) {
@@ -67,8 +67,8 @@ static bool fold_ok(const Plan &p) {
         return false;
     const int rows = p.kh < p.sh ? p.kh : p.sh, taps = div_up_i(p.kh, p.sh);
     const long span = (long)(p.ow - 1) * p.sw + p.kw;
-    // bytes staged at least, and words of a column they become: all of fewer than eight channels
-    // as bits, or eight channels as nibbles
+    // bytes staged at least, and words of a column they become: eight channels as nibbles, or all of
+    // fewer than eight, a quarter of whose nibbles' bytes count
     const long least = p.ic < 8 ? 4L * p.ic * rows * fold_bit_pitch(p) : 4 * rows * span;
     const long words = p.ic < 8 ? (long)p.ic * rows * div_up_i(p.kw, 8) : (long)rows * p.kw;
     return sums_exact(p) && least <= kFoldStage && 4L * p.sh * p.iw <= kFoldSums &&

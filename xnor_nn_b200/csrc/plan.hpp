@@ -114,8 +114,9 @@ struct Plan {
 // The layer the tensor-core kernel is launched on: the plan itself, or the unit-stride layer a
 // strided one was folded into. (The box filter K is the original layer's and computed apart.)
 Plan conv_view(const Plan &p);
-// 32-bit words between the rows of signs that the packer of a folded layer with fewer than eight
-// channels stages: all columns of the image with the border in front, and all that is read of them.
+// The row of signs that the packer of a folded layer with fewer than eight channels stages, in units of 32
+// columns (four words of nibbles): all columns of the image with the border in front, and all that is
+// read of them.
 int fold_bit_pitch(const Plan &p);
 // Rows behind the last position that tile loads may reach.
 long frame_slack(const Plan &p);
