@@ -1,5 +1,5 @@
-"""Bounded waits of the one-launch pass (conv_whole.cu) and of calculate_k in one launch (maps.cu) that run out, in the form that leaves the GPU
-healthy: the test hook shortens the limit and loses a commit, an arrival of the packed operand or the
+"""Bounded waits of the one-launch pass (conv_whole.cu) and of calculate_k in one launch (maps.cu) that run
+out, in the form that leaves the GPU healthy: the test hook shortens the limit and loses a commit, an arrival of the packed operand or the
 hand-over of running sums. Every role winds down, loads and MMAs in flight are waited for, the host turns
 the error word into a status, and the next pass on the same resources is right, bit for bit."""
 import ctypes as C

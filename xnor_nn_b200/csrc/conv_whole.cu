@@ -37,10 +37,10 @@
 // which come through the ring meanwhile), then 1000 to 5600 for the stores. One issuer needs about 500 cycles a
 // filter tile, mostly the chain of scalar instructions around its MMAs, hence four (MMAs of one image:
 // 6700 -> 5300). Times in us, two launches -> one: a pass among others on three streams, back to back on one
-// stream, alone: conv4 on one image 6.7 -> 4.7, 12.5 -> 10.9, 23.1 -> 22.9; on 32 images 8.2 -> 5.8,
-// 16.3 -> 16.0, 23.6 -> 28.1; on 64 images channels-last 12.2 -> 11.6, 21.0 -> 17.8, 29.4 -> 29.3; 16 channels
-// of 31 x 31, five images 6.7 -> 4.8, 8.0 -> 5.3, 19.4 -> 17.6. The first is bound by the host, for which a
-// launch is 2.0 us.
+// stream, waited for: conv4 on one image 7.2 -> 4.1, 12.8 -> 11.4, 23.6 -> 23.5; on 32 images 8.2 -> 5.9,
+// 16.4 -> 16.6, 25.0 -> 28.8; on 64 images channels-last 11.4 to 12.2 -> 11.9, 20.9 -> 18.0, 29.9 -> 29.9; 16
+// channels of 31 x 31, five images 8.7 -> 5.3, 7.5 -> 5.5, 20.0 -> 18.2. The first is bound by the host, for
+// which a launch is 2.0 us.
 #include <cuda.h>
 
 #include <atomic>

@@ -59,8 +59,8 @@ int fold_bit_pitch(const Plan &p) {
 
 // A strided layer is folded when its packer's working set (a row block of some channels, half a byte a
 // value, and with eight channels or more the mean-|x| sums of the block's pixels) fits shared memory.
-// With fewer than eight channels the limit is a bit a value in 48 KB, which are 192 KB as staged. The popcount kernel it would otherwise run on needs 870 us for
-// AlexNet conv1 on 64 images.
+// With fewer than eight channels the limit is a bit a value in 48 KB, which are 192 KB as staged. The
+// popcount kernel it would otherwise run on needs 870 us for AlexNet conv1 on 64 images.
 constexpr long kFoldStage = 48 * 1024, kFoldSums = 48 * 1024, kFoldWords = 4096;
 static bool fold_ok(const Plan &p) {
     if ((p.sh == 1 && p.sw == 1) || p.sh < 1 || p.sw < 1 || p.oh < 1 || p.ow < 1 || p.mb < 1)
