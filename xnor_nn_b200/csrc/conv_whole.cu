@@ -137,10 +137,13 @@ __device__ __forceinline__ bool finish_task(const WholeArgs &g, Control *ctl, ui
     const int q = (n * g.hp + h) * g.wp + w, row = q - tile.q0;
     const uint32_t *u = reinterpret_cast<const uint32_t *>(v);
     uint4 s;
-    s.x = first_nibbles(sign_nibbles(u), nc);
-    s.y = first_nibbles(sign_nibbles(u + 8), nc - 8);
-    s.z = first_nibbles(sign_nibbles(u + 16), nc - 16);
-    s.w = first_nibbles(sign_nibbles(u + 24), nc - 24);
+    s = make_uint4(sign_nibbles(u), sign_nibbles(u + 8), sign_nibbles(u + 16), sign_nibbles(u + 24));
+    if (nc < 32) {
+        s.x = first_nibbles(s.x, nc);
+        s.y = first_nibbles(s.y, nc - 8);
+        s.z = first_nibbles(s.z, nc - 16);
+        s.w = first_nibbles(s.w, nc - 24);
+    }
     if (live) {
         const int o = g.swizzled ? (((col >> 3) * g.pitch + row) << 7) + (((col ^ row) & 7) << 4)
                                  : (col * g.pitch + row) << 4;
@@ -286,9 +289,9 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
     const uint32_t b0 = smem_u32(base) + g.b_off;
     const int steps = g.taps * g.chunks;
     if (warp == 0) {
-        // ---- filter tiles ----
+        // ---- filter tiles ---- (not behind dependency_wait(): the kernels that write them let no dependent start
+        // early, so that whatever started before this grid came after them)
         const bool leader = elect_one();
-        dependency_wait();
         int stage = 0, sent = 0, tap = 0, chunk = 0;
         uint32_t phase = 0;
         bool ok = true;
