@@ -97,7 +97,10 @@ struct __align__(16) Control {
     uint32_t tmem_base;
     int abort_flag;
     alignas(16) float alpha[256];
-    int summed[kMaxGroups];                  // columns whose |x| have been added
+    // The channels before a task's have been added up. A barrier a task, used once: as counters in shared memory,
+    // polled with acquire loads and passed on with release stores, turns cost a pass of AlexNet conv4 on 32 images
+    // 15.6 us instead of 15.1 on one stream, one image 10.1 instead of 9.7.
+    unsigned long long turn[kMaxTasks];
     float sum[kMaxGroups][32];
     float a[kMaxRows];                       // mean |x| on the tile's rows of the frame
 };
@@ -156,14 +159,17 @@ __device__ __forceinline__ bool finish_task(const WholeArgs &g, Control *ctl, ui
     if (lane == 0) mbar_arrive(smem_u32(&ctl->packed[col / g.part_columns]));
     const bool mine = owner && live && q >> 7 == tile.mt;
     if (mine) *reinterpret_cast<uint4 *>(g.bin + (long)(g.lead + q) * g.icp + 16 * col) = s;
-    float acc;
-    if (!add_task(v, nc, col, g.inv_ic, &ctl->summed[gr], &ctl->sum[gr][lane], &ctl->abort_flag, g.error,
-                  g.wait_ns, &acc))
-        return false;
+    scale_task(v, g.inv_ic);
+    float acc = 0.f;
+    if (col > 0) {
+        if (!warp_wait(smem_u32(&ctl->turn[t]), 0, &ctl->abort_flag, g.error, 21, g.wait_ns)) return false;
+        acc = *(const volatile float *)&ctl->sum[gr][lane];
+    }
+    acc = sum_task(v, nc, acc);
     if (col + 1 < g.columns) {
         ctl->sum[gr][lane] = acc;
         __syncwarp();
-        if (lane == 0) turn_pass(&ctl->summed[gr], col + g.turn_step);
+        if (lane == 0 && g.turn_step) mbar_arrive(smem_u32(&ctl->turn[t + tile.groups]));
     } else if (live) {
         ctl->a[row] = acc;
         if (mine) g.a[px] = acc;
@@ -258,7 +264,6 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
             mbar_init(smem_u32(&ctl->packed[i]),
                       (uint32_t)(tile.groups * min(g.part_columns, g.columns - i * g.part_columns) +
                                  (blockIdx.x == 0 ? g.more_operand : 0)));
-        for (int i = 0; i < tile.groups; i++) ctl->summed[i] = 0;
         mbar_init(smem_u32(&ctl->acc_full), (uint32_t)(kIssuers + (blockIdx.x == 0 ? g.more_commits : 0)));
         mbar_init(smem_u32(&ctl->cleared), 4);
         for (int i = 0; i < kIssuers; i++) mbar_init(smem_u32(&ctl->drain[i]), 1);
@@ -266,6 +271,8 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     }
+    if (warp == kFirstIssuer)
+        for (int i = lane; i < kMaxTasks; i += 32) mbar_init(smem_u32(&ctl->turn[i]), 1);
     if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem_base), g.tmem_cols);
     const int worker = warp - 1;
     const bool works = worker >= 0 && worker < kWorkers;

@@ -1,6 +1,6 @@
 // Packing the source by tasks of 32 neighbouring pixels x 32 channels, a task a warp (conv_whole.cu,
 // maps.cu): loads, and the sum of |x| over the channels in upstream's order, which tasks of the same pixels
-// hand on from warp to warp.
+// hand on from warp to warp (the turns below are maps.cu's; conv_whole.cu has a barrier for each).
 #pragma once
 
 #include "kernels.cuh"
@@ -113,19 +113,12 @@ __device__ __forceinline__ void load_task(const Args &g, const Tile &tile, int t
     }
 }
 
-// Adds the task's |x| / IC to the sum of the channels before it, once those have been added; v is used
-// up. The caller passes the turn on (or has the mean, after the last channels).
-__device__ __forceinline__ bool add_task(float *v, int nc, int col, float inv_ic, const int *turn,
-                                         const float *sum, volatile int *abort_flag, int *error,
-                                         unsigned long long limit_ns, float *out) {
-    // |x| / IC = |x / IC|: two products an instruction, the sign goes with the addition
+// |x| / IC = |x / IC|: two products an instruction, the sign goes with the addition.
+__device__ __forceinline__ void scale_task(float *v, float inv_ic) {
 #pragma unroll
     for (int i = 0; i < 32; i += 2) mul2(v[i], v[i + 1], inv_ic);
-    float acc = 0.f;
-    if (col > 0) {
-        if (!turn_wait(turn, col, abort_flag, error, limit_ns)) return false;
-        acc = *(const volatile float *)sum;
-    }
+}
+__device__ __forceinline__ float sum_task(const float *v, int nc, float acc) {
     if (nc == 32) {
 #pragma unroll
         for (int i = 0; i < 32; i++) acc = __fadd_rn(acc, fabsf(v[i]));
@@ -134,7 +127,21 @@ __device__ __forceinline__ bool add_task(float *v, int nc, int col, float inv_ic
         for (int i = 0; i < 32; i++)
             if (i < nc) acc = __fadd_rn(acc, fabsf(v[i]));
     }
-    *out = acc;
+    return acc;
+}
+
+// Adds the task's |x| / IC to the sum of the channels before it, once those have been added; v is used
+// up. The caller passes the turn on (or has the mean, after the last channels).
+__device__ __forceinline__ bool add_task(float *v, int nc, int col, float inv_ic, const int *turn,
+                                         const float *sum, volatile int *abort_flag, int *error,
+                                         unsigned long long limit_ns, float *out) {
+    scale_task(v, inv_ic);
+    float acc = 0.f;
+    if (col > 0) {
+        if (!turn_wait(turn, col, abort_flag, error, limit_ns)) return false;
+        acc = *(const volatile float *)sum;
+    }
+    *out = sum_task(v, nc, acc);
     return true;
 }
 
