@@ -33,7 +33,7 @@
 // channel chunk, with a halo of the positions that follow it, and the taps of the row read that
 // tile at row offsets (producer_halo / mma_role_halo); filters that fit are loaded once and stay
 // (mma_role_resident), in layers of few channels beside position tiles that serve all taps of the
-// filter (mma_role_planes). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters)
+// filter (mma_role_planes, mma_role_block). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters)
 // or, when its loads share the way to L2 with the stores of the tile before it, those: AlexNet conv4
 // on 256 images takes 8200 cycles a tile without the other's stores and 10500 with them (pipe: 6900).
 //
@@ -787,8 +787,8 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
 }
 
-// Resident filters beside position tiles of rows: layers of more than 224 channels, one tap a filter
-// row, folded layers, and those that columns are no gain for. The only thing that arrives is position
+// Resident filters beside position tiles of rows, a tile for each filter row: rows of fewer than 128 bytes, a single
+// filter row, and what mma_role_block has no room or barriers for. The only thing that arrives is position
 // tiles, so a group (the taps of a filter row on one channel chunk) is one wait, kw * KK MMAs and one
 // commit, from one issuer: about 500 cycles a group and 30 an instruction (layers of 64 filters that
 // differ in nothing else), where the tensor pipe needs N / 2 an instruction. Wide tiles with several
@@ -842,6 +842,134 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
             __syncwarp();
             if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
             if (++chunk == g.chunks_per_tap) chunk = 0;
+        }
+        if (!ok) break;
+        if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
+            commit_pair(smem_u32(&ctl->acc_full[b]));
+        }
+        __syncwarp();
+        if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
+    }
+    if (leader) commit_pair_here(smem_u32(&ctl->drain[0]));
+    mbar_wait_quiet(smem_u32(&ctl->drain[0]), 0, g.wait_ns);
+}
+
+// Resident filters beside position tiles that serve all filter rows: a tile is the 128-byte rows of one K chunk
+// for every position that any tap reads, 128 + (kh-1) wp + kw-1 of them, and a tap is a row offset. Loaded once per
+// K chunk it is 20 KB for AlexNet conv3, where tiles for each filter row are 51 KB, beside which the results leave
+// the SM; and an issuer waits and commits once per chunk. Kernel alone, tiles for each filter row -> these: conv3 on
+// 256 images 22.9 -> 22.4 us, conv1 on 64 23.8 -> 21.4, and 1.00 to 1.11 times as fast, median 1.034, over 30
+// layers drawn from 16 to 256 images, 3 to 512 channels and filters, 6 to 56 pixels (first layers 60 to 227).
+__device__ __forceinline__ void producer_block(const TcArgs &g, Control *ctl, const CUtensorMap *map_a,
+                                               const CUtensorMap *map_b, uint32_t stage0, uint32_t rank) {
+    volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
+    const Deal<true> deal(g);
+    const int rounds = deal.rounds(g);
+    const uint32_t full_l = smem_u32(&ctl->full[0]), afull_l = smem_u32(&ctl->a_full[0]);
+    // a pair counts both CTAs' bytes on the leader's barriers
+    const uint32_t full0 = rank != 0 ? mapa(full_l, 0) : full_l;
+    const uint32_t afull0 = rank != 0 ? mapa(afull_l, 0) : afull_l;
+    const uint32_t aempty0 = smem_u32(&ctl->a_empty[0]);
+    const uint32_t a_bytes = (uint32_t)g.halo * (uint32_t)g.kchunk;
+    int sa = 0;
+    uint32_t pa = 0, armed = 0, parity = 0, b_armed = 0;
+    bool ok = true;
+    for (int it = 0; ok && it < rounds; it++) {
+        int mt, nt;
+        deal.at(g, it, mt, nt);
+        const int row = g.lead + mt * BM - g.ph * g.wp - g.pw;  // tap (0,0)
+        for (int chunk = 0; chunk < g.chunks_per_tap; chunk++) {
+            ok = warp_wait(aempty0 + 8u * (uint32_t)sa, pa ^ 1, abort_flag, g.error, 8, g.wait_ns);
+            if (!ok) break;
+            const uint32_t abar = afull0 + 8u * (uint32_t)sa;
+            if (leader) {
+                if (rank == 0) mbar_expect_tx(abar, 2u * a_bytes);  // abar is local here
+                tma_load_2d_pair(stage0 + (uint32_t)sa * g.a_slot_bytes, map_a, chunk * g.kchunk, row, abar);
+            }
+            armed |= 1u << sa;
+            parity = (parity & ~(1u << sa)) | (pa << sa);
+            if (++sa == g.n_a_slots) { sa = 0; pa ^= 1; }
+            // the chunk's filters, a barrier for each filter row (n_stages: kh * chunks)
+            for (int kh = 0; it == 0 && kh < g.kh; kh++) {
+                const int gr = kh * g.chunks_per_tap + chunk;
+                const uint32_t bar = full0 + 8u * (uint32_t)gr;
+                int brow = nt * g.n_tile + (int)rank * (g.n_tile >> 1) + kh * g.tap_kw * g.ocp16;
+                uint32_t bdst = stage0 + g.b_ring_off + (uint32_t)(gr * g.tap_kw) * g.b_slot_bytes;
+                if (leader) {
+                    if (rank == 0) mbar_expect_tx(bar, 2u * (uint32_t)g.tap_kw * g.b_bytes);
+                    for (int kw = 0; kw < g.tap_kw; kw++, brow += g.ocp16, bdst += g.b_slot_bytes)
+                        tma_load_2d_pair(bdst, map_b, chunk * g.kchunk, brow, bar);
+                }
+                b_armed |= 1u << gr;
+            }
+            __syncwarp();
+        }
+    }
+    if (rank == 0) {
+        // as in producer_ring: loads already issued land before the CTA may exit
+        for (int i = 0; i < g.n_stages; i++)
+            if (b_armed & (1u << i)) mbar_wait_quiet(full_l + 8u * (uint32_t)i, 0, g.wait_ns);
+        for (int i = 0; i < g.n_a_slots; i++)
+            if (armed & (1u << i))
+                mbar_wait_quiet(afull_l + 8u * (uint32_t)i, (parity >> i) & 1u, g.wait_ns);
+    }
+}
+
+template <int KK>
+__device__ __forceinline__ void mma_role_block(const TcArgs &g, Control *ctl, uint32_t tmem_base,
+                                               uint32_t stage0) {
+    volatile int *abort_flag = &ctl->abort_flag;
+    const bool leader = elect_one();
+    const int rounds = Deal<true>(g).rounds(g);
+    if (rounds == 0) return;
+    const uint64_t hi = (uint64_t)g.desc_hi << 32;
+    const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (1u << 16);
+    const uint32_t b_lo0 = (((stage0 + g.b_ring_off) >> 4) & 0x3FFF) | (1u << 16);
+    const uint32_t a_units = g.a_slot_bytes >> 4, b_units = g.b_slot_bytes >> 4;
+    const uint32_t row_units = (uint32_t)g.kchunk >> 4;  // one position further
+    const uint32_t full0 = smem_u32(&ctl->full[0]);
+    const uint32_t afull0 = smem_u32(&ctl->a_full[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
+    int sa = 0, b = 0;
+    uint32_t pa = 0, acc_phase = 0;
+    bool ok = true;
+    for (int it = 0; it < rounds; it++) {
+        const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
+        ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2, g.wait_ns);
+        if (ok && g.shared_cols && it > 0)
+            ok = warp_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag, g.error,
+                           7, g.wait_ns);
+        if (!ok) break;
+        for (int chunk = 0; chunk < g.chunks_per_tap; chunk++) {
+            ok = warp_wait(afull0 + 8u * (uint32_t)sa, pa, abort_flag, g.error, 9, g.wait_ns);
+            if (!ok) break;
+            const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
+            for (int kh = 0; kh < g.kh; kh++) {
+                const int gr = kh * g.chunks_per_tap + chunk;
+                if (it == 0)
+                    ok = warp_wait(full0 + 8u * (uint32_t)gr, 0, abort_flag, g.error, 3, g.wait_ns);
+                if (!ok) break;
+                fence_after();
+                if (leader) {
+                    uint64_t adesc =
+                        hi | (uint64_t)(a_lo0 + (uint32_t)sa * a_units + (uint32_t)(kh * g.wp) * row_units);
+                    uint64_t bdesc = hi | (uint64_t)(b_lo0 + (uint32_t)(gr * g.tap_kw) * b_units);
+                    for (int kw = 0; kw < g.tap_kw; kw++, adesc += row_units, bdesc += b_units) {
+#pragma unroll
+                        for (int k = 0; k < KK; k++) {
+                            if (k < kk) {
+                                mma_mxf4<true>(d_tmem, adesc + (uint64_t)(2 * k),
+                                               bdesc + (uint64_t)(2 * k), g.idesc,
+                                               tmem_base + kScaleCol, (chunk | kh | kw | k) == 0 ? 0u : 1u);
+                            }
+                        }
+                    }
+                    if (kh == g.kh - 1) commit_pair(aempty0 + 8u * (uint32_t)sa);
+                }
+                __syncwarp();
+            }
+            if (!ok) break;
+            if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
         }
         if (!ok) break;
         if (leader && !(g.drop_commit && it == 0 && blockIdx.x == 0)) {
@@ -1097,6 +1225,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         dependency_wait();
         if constexpr (PAIR) {
             if (g.planes) producer_planes(g, ctl, &map_a, &map_b, stage0, rank);
+            else if (g.block) producer_block(g, ctl, &map_a, &map_b, stage0, rank);
             else if (g.halo) producer_halo(g, ctl, &map_a, &map_b, stage0, rank);
             else producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
         } else {
@@ -1110,6 +1239,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 if (KK == 4 && g.planes && g.chunks_per_tap * KK > 32)
                     mma_role_planes<KK, true>(g, ctl, tmem_base, stage0, who);
                 else if (g.planes) mma_role_planes<KK, false>(g, ctl, tmem_base, stage0, who);
+                else if (KK == 4 && g.block) mma_role_block<KK>(g, ctl, tmem_base, stage0);
                 else if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
                 else if (g.halo) mma_role_halo<KK>(g, ctl, tmem_base, stage0, who);
                 else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
@@ -1274,7 +1404,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
     g.planes = 0; g.plane_rows = 0; g.plane_pitch = 0; g.pos_bytes = p.icp; g.plane_desc_hi = 0;
-    g.halo = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
+    g.halo = 0; g.block = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
     // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
     // (issue_probe checks that one). Narrower rows come with several taps a filter row when a layer
@@ -1312,6 +1442,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         const bool as_columns = p.cat && g.kh >= 3 && (walk >= 3 || p.icp == 16) &&
                                 !(p.icp == 32 && groups == 3 && p.n_tile <= 64) && rows <= 256 &&
                                 all_b + 2 * (size_t)col_slot <= room;
+        uint32_t tile_slot = row_slot;
         g.resident = 1;
         if (as_columns) {
             g.issuers = 2;
@@ -1320,10 +1451,17 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
             g.n_stages = groups < kMaxStages ? groups : kMaxStages;  // barriers of the filters
         } else {
             g.issuers = 1;
-            g.halo = (int)halo_rows;
-            g.n_stages = 2;
+            // A tile for all filter rows where they are rows of 128 bytes, in one box, with a barrier for each
+            // filter row's and chunk's filters, and two tiles fit. (A single filter row is the other form.)
+            const int block_rows = BM + (g.kh - 1) * p.wp + g.tap_kw - 1;
+            const uint32_t block_slot = (uint32_t)(block_rows * p.kchunk + 1023) & ~1023u;
+            g.block = g.kh > 1 && p.kchunk == 128 && block_rows <= 256 && groups <= kMaxStages &&
+                      all_b + 2 * (size_t)block_slot <= room;
+            g.halo = g.block ? block_rows : (int)halo_rows;
+            g.n_stages = g.block ? groups : 2;
+            if (g.block) tile_slot = block_slot;
         }
-        g.a_slot_bytes = as_columns ? col_slot : row_slot; g.b_slot_bytes = b_slot;
+        g.a_slot_bytes = as_columns ? col_slot : tile_slot; g.b_slot_bytes = b_slot;
         g.n_a_slots = (int)((room - all_b) / g.a_slot_bytes);
         if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
         g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
