@@ -1300,21 +1300,65 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // filter tile that splits into two UMMA-sized halves.
     const bool pair = !next && p.n_tile % 32 == 0 && m_tiles >= 2 &&
                       (long)m_tiles * (p.ocp16 / p.n_tile) > sms;
-    const int b_rows = pair ? p.n_tile / 2 : p.n_tile;  // filter rows a CTA loads per stage
     TcArgs g;
     g.alpha = alpha; g.kmap = k; g.amap = a; g.kmap_out = k_out; g.dst = dst; g.sums = sums;
     g.error = error_word;
     g.inv_khw = p.inv_khw; g.ih = p.ih; g.iw = p.iw; g.kh = p.kh;
     g.q_total = p.q_total;
     g.m_tiles = m_tiles;
-    g.n_tiles = p.ocp16 / p.n_tile;
-    g.n_tile = p.n_tile;
     // channels-wise: a tap, or the kw taps of a filter row one after the other
     const int tap_bytes = p.cat ? p.kw * p.icp : p.icp;
     const int tap_values = p.cat ? 2 * (p.kw - 1) * p.icp + p.ic : p.ic;
     g.tap_kw = p.cat ? 1 : p.kw;
     g.taps = p.kh * g.tap_kw;
     g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(tap_bytes, p.kchunk);
+    const int groups = g.kh * g.chunks_per_tap;
+    // as many ring buffers as fit beside the control block
+    const size_t room = 227 * 1024 - 1024 - kControlBytes;
+    // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
+    // (issue_probe checks that one). Narrower rows come with several taps a filter row when a layer
+    // that was asked onto the image-row kernel ends a chain; it takes the plain ring.
+    const bool row_offsets_ok = g.tap_kw == 1 || (g.tap_kw <= 9 && p.kchunk == 128);
+    // Position tiles of a filter row, and of all filter rows (where those are rows of 128 bytes, in one box,
+    // with a barrier for each filter row's and chunk's filters; a single filter row is the other form).
+    const uint32_t halo_rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
+    const int block_rows = BM + (g.kh - 1) * p.wp + g.tap_kw - 1;
+    const uint32_t row_slot = (halo_rows * p.kchunk + 1023) & ~1023u;
+    const uint32_t block_slot = (uint32_t)(block_rows * p.kchunk + 1023) & ~1023u;
+    const auto filter_bytes = [&](int n) {  // a CTA's filters of a tile of n, all of their operands
+        return (size_t)groups * g.tap_kw * (((pair ? n / 2 : n) * p.kchunk + 1023) & ~1023);
+    };
+    const auto filters_fit = [&](int n) { return filter_bytes(n) + 3 * (size_t)row_slot <= room; };
+    const auto block_fits = [&](int n) {
+        return g.kh > 1 && p.kchunk == 128 && block_rows <= 256 && groups <= kMaxStages &&
+               filter_bytes(n) + 2 * (size_t)block_slot <= room;
+    };
+    // A tile of half the filters, if that half stays in shared memory beside such tiles (below) and the whole
+    // would not: its filters are loaded once instead of for each position tile, which pays for reading the
+    // positions twice where
+    // - operand rows are an odd number of 16 bytes, so that every filter row loaded straddles sectors, or
+    // - a pair has three tiles or fewer and the accumulators of the whole share columns.
+    // Kernel alone, whole over half, 256 layers on 6 to 30 pixels, 270 to 512 channels, 120 to 768 filters, 1
+    // to 7 tiles a pair of the whole:
+    //   odd rows, tiles of 192 and 256, 3 x 3          0.98 to 1.49, mean 1.23
+    //   odd rows, tiles of 128, 4 x 4                  0.95 to 1.19, mean 1.06
+    //   others, up to three tiles, 256 filters a tile  0.99 to 1.29, mean 1.11
+    //   others, up to three tiles, 192                 0.91 to 1.16, mean 1.03
+    //   others, more tiles                             0.86 to 1.20, mean 1.04
+    //   2 x 2 filters on 640 to 768 channels           0.92 to 1.12, mean 0.98
+    // conv4 on 256 images, a pass: 41.6 -> 40.3 us on one stream.
+    int n_tile = p.n_tile;
+    const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
+    const int half_grid = sms / 2 - sms / 2 % half_tiles;
+    if (pair && !p.cat && g.kh >= 3 && n_tile >= 128 && n_tile % 64 == 0 && row_offsets_ok &&
+        !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
+        div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, sms / 2) &&
+        (p.icp % 32 != 0 ||
+         (n_tile > kAccStep && div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3)))
+        n_tile /= 2;
+    const int b_rows = pair ? n_tile / 2 : n_tile;  // filter rows a CTA loads per stage
+    g.n_tiles = p.ocp16 / n_tile;
+    g.n_tile = n_tile;
     g.kw = p.kw; g.ph = p.ph; g.pw = p.pw; g.wp = p.wp; g.hp = p.hp; g.lead = p.lead;
     g.oh = p.oh; g.ow = p.ow; g.oc = p.oc; g.ocp16 = p.ocp16;
     g.by_frame = FastDiv((uint32_t)(p.hp * p.wp)); g.by_wp = FastDiv((uint32_t)p.wp);
@@ -1330,9 +1374,9 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         g.n_inner = 1;
     }
     // M = 256 for a pair: 128 rows in each CTA
-    g.idesc = mxf4_idesc(pair ? 2 * BM : BM, (uint32_t)p.n_tile);
-    g.shared_cols = p.n_tile > kAccStep;
-    g.acc_step = (uint32_t)(p.n_tile < kAccStep ? p.n_tile : kAccStep);
+    g.idesc = mxf4_idesc(pair ? 2 * BM : BM, (uint32_t)n_tile);
+    g.shared_cols = n_tile > kAccStep;
+    g.acc_step = (uint32_t)(n_tile < kAccStep ? n_tile : kAccStep);
     // matrix descriptor, upper half: stride between 8-row groups (8 * kchunk bytes, in 16-byte
     // units), descriptor version 1, swizzle mode
     const uint32_t sbo = (uint32_t)(8 * p.kchunk) >> 4;
@@ -1354,7 +1398,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // conv2 on 128 images (5120 cycles, six tiles) 43.3 -> 42.7 us among others, VGG (9216, six) 71.6 -> 71.2.
     // With two or three tiles 0.90 to 1.07.
     const long tile_cycles =
-        (long)g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last) * p.n_tile / 2;
+        (long)g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last) * n_tile / 2;
     const int pair_tiles = div_up_i(((m_tiles + 1) / 2) * g.n_tiles, sms / 2);
     const bool few = pair && kk == 4 && tile_cycles >= 5000 && pair_tiles >= 4;
     const int epi = few ? kFewEpiWarps : kEpiWarps;
@@ -1401,25 +1445,16 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // Fewer pairs, if that costs no further round, so that each keeps to one filter tile.
     const int one_nt = grid - grid % g.n_tiles;
     const bool same_nt = pair && one_nt > 0 && div_up_i(units, one_nt) == div_up_i(units, grid);
-    // as many ring buffers as fit beside the control block
-    const size_t room = 227 * 1024 - 1024 - kControlBytes;
     g.planes = 0; g.plane_rows = 0; g.plane_pitch = 0; g.pos_bytes = p.icp; g.plane_desc_hi = 0;
     g.halo = 0; g.block = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
-    // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
-    // (issue_probe checks that one). Narrower rows come with several taps a filter row when a layer
-    // that was asked onto the image-row kernel ends a chain; it takes the plain ring.
-    const bool row_offsets_ok = g.tap_kw == 1 || (g.tap_kw <= 9 && p.kchunk == 128);
     bool halo = pair && g.tap_kw >= 2 && row_offsets_ok && g.issuers <= g.tap_kw;
     // Filters stay in shared memory if a pair works on several tiles of the same ones and their
     // operands leave room for three position tiles of 128-byte rows. Kernel alone, conv3 on 256 images
     // 25.4 -> 23.0 us (six such tiles in flight), conv1 on 64 images 26.1 -> 25.5 (eight).
-    const int groups = g.kh * g.chunks_per_tap;
     const int walk = same_nt ? div_up_i(units, one_nt) : 1;  // tiles of a pair
-    const uint32_t halo_rows = (uint32_t)(g.tap_kw > 1 ? BM + 8 : BM);
-    const uint32_t row_slot = (halo_rows * p.kchunk + 1023) & ~1023u, b_slot = (g.b_bytes + 1023u) & ~1023u;
-    const size_t all_b = (size_t)groups * g.tap_kw * b_slot;
-    if (walk > 1 && row_offsets_ok && all_b + 3 * (size_t)row_slot <= room) {
+    const size_t all_b = filter_bytes(n_tile);
+    if (walk > 1 && row_offsets_ok && filters_fit(n_tile)) {
         // Position tiles as 16-byte columns: layers whose filter rows are one operand row (Plan::cat), if
         // the positions of all taps are one box (256 rows) and two tiles fit. AlexNet conv2 on 128
         // images, kernel alone: 42.6 -> 40.3 us from loading 16 KB a tile instead of 160, 33.8 with two
@@ -1440,7 +1475,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         const int pitch = (rows + 7) & ~7;  // a load lands on a multiple of 128 bytes
         const uint32_t col_slot = (uint32_t)(planes * pitch * 16 + 1023) & ~1023u;
         const bool as_columns = p.cat && g.kh >= 3 && (walk >= 3 || p.icp == 16) &&
-                                !(p.icp == 32 && groups == 3 && p.n_tile <= 64) && rows <= 256 &&
+                                !(p.icp == 32 && groups == 3 && n_tile <= 64) && rows <= 256 &&
                                 all_b + 2 * (size_t)col_slot <= room;
         uint32_t tile_slot = row_slot;
         g.resident = 1;
@@ -1451,17 +1486,12 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
             g.n_stages = groups < kMaxStages ? groups : kMaxStages;  // barriers of the filters
         } else {
             g.issuers = 1;
-            // A tile for all filter rows where they are rows of 128 bytes, in one box, with a barrier for each
-            // filter row's and chunk's filters, and two tiles fit. (A single filter row is the other form.)
-            const int block_rows = BM + (g.kh - 1) * p.wp + g.tap_kw - 1;
-            const uint32_t block_slot = (uint32_t)(block_rows * p.kchunk + 1023) & ~1023u;
-            g.block = g.kh > 1 && p.kchunk == 128 && block_rows <= 256 && groups <= kMaxStages &&
-                      all_b + 2 * (size_t)block_slot <= room;
+            g.block = block_fits(n_tile);
             g.halo = g.block ? block_rows : (int)halo_rows;
             g.n_stages = g.block ? groups : 2;
             if (g.block) tile_slot = block_slot;
         }
-        g.a_slot_bytes = as_columns ? col_slot : tile_slot; g.b_slot_bytes = b_slot;
+        g.a_slot_bytes = as_columns ? col_slot : tile_slot; g.b_slot_bytes = (g.b_bytes + 1023u) & ~1023u;
         g.n_a_slots = (int)((room - all_b) / g.a_slot_bytes);
         if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
         g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
@@ -1509,8 +1539,12 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // images) took 41.3 us per pass, conv1 (64 images) 86, with two teams 37.7 and 79. The chained
     // epilogue carries per-pixel state from one filter tile to the next: one team.
     const int rounds = g.n_inner ? 1 : div_up_i(units, grid);
-    g.n_acc = g.shared_cols || g.n_inner ? 2 : (int)kScaleCol / p.n_tile;
+    g.n_acc = g.shared_cols || g.n_inner ? 2 : (int)kScaleCol / n_tile;
     if (g.n_acc > kMaxAcc) g.n_acc = kMaxAcc;
+    // Two instead of three beside position tiles for all filter rows: each is then one team's, which a lost
+    // commit cannot pass over to another. Kernel alone, three over two, 24 such layers: 0.99 to 1.01. (Tiles of
+    // columns, shorter, lose up to a tenth and keep three.)
+    if (g.block && g.n_acc == 3) g.n_acc = 2;
     g.teams = g.n_acc == 4 && rounds >= 4 && !few ? 4 : rounds >= 2 ? 2 : 1;
     g.by_acc = FastDiv((uint32_t)g.n_acc);
     note_launch();
