@@ -1,0 +1,39 @@
+"""Which chained layers run on CTA pairs, and in which form of the kernel (cpp/chain_launch.cpp)."""
+import json
+import os
+import subprocess
+
+import test_chain_pairs_gpu as gpu
+from xnor_nn_b200 import build
+
+MORE = {"conv3": (128, 256, 384, 13, 13, 3, 3, 1, 1), "conv4": (128, 384, 256, 13, 13, 3, 3, 1, 1)}
+
+
+def test_which_chained_layers_run_on_pairs(tmp_path):
+    build.build()
+    exe = str(tmp_path / "chain_launch")
+    here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cpp")
+    objs = [os.path.join(build.OBJ, n + ".o") for n in ("conv_tcgen05.cu", "plan.cpp", "tensormap.cpp")]
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", os.path.join(build.ROOT, "include"), "-I",
+                           build.CSRC, "-I", "/usr/local/cuda/include", os.path.join(here, "chain_launch.cpp")] +
+                          objs + ["-o", exe])
+    layers = {**gpu.PAIRS, **gpu.SINGLE, **MORE}
+    order = (0, 2, 1, 3, 4, 5, 6, 7, 8)  # filters before channels
+    out = subprocess.check_output([exe] + [",".join(str(d[i]) for i in order) for d in layers.values()],
+                                  text=True).splitlines()
+    got = dict(zip(layers, [json.loads(line) for line in out]))
+    assert all(g["served"] and g["epilogue_warps"] == 16 for g in got.values())
+    pairs = {name: g for name, g in got.items() if g["pair"]}
+    assert set(pairs) == set(gpu.PAIRS) | {"conv4"}
+    form = {name: "columns" if g["planes"] else "resident" if g["resident"] else "halo" if g["halo"] else "ring"
+            for name, g in pairs.items()}
+    assert form == {"columns": "columns", "rows_of_all_filter_rows": "resident",
+                    "rows_of_a_filter_row": "resident", "streamed": "halo", "streamed_two_filter_tiles": "halo",
+                    "streamed_four_tiles_odd_filters": "halo", "streamed_192_filters": "halo",
+                    "ring": "ring", "fewer_tiles_than_sms": "halo", "conv4": "halo"}, form
+    assert pairs["rows_of_all_filter_rows"]["halo"] > 136 >= pairs["rows_of_a_filter_row"]["halo"]
+    assert {g["n_tiles"] for g in pairs.values()} == {1, 2, 4}
+    assert {g["shared_cols"] for g in pairs.values()} == {0, 1}
+    assert {g["m_tiles"] % 2 for g in pairs.values()} == {0, 1}
+    # one position tile a pair at a time, all of its filter tiles in a row
+    assert all(g["grid"] == 2 * min(74, (g["m_tiles"] + 1) // 2) for g in pairs.values())

@@ -138,7 +138,9 @@ struct Deal {
 // ---- epilogue role ---------------------------------------------------------------------------------
 // Warp w may touch TMEM lanes [32*(w%4), 32*(w%4)+32); several warps share a quadrant and split
 // its columns between them.
-template <bool PAIR, int EPI>
+// EMITS: chained layers' results, and no others, on pairs. (On single CTAs both kinds have one kernel: the layers
+// of a chain then find its instructions in the caches. Two kernels: three layers on 64 images 23.0 -> 24.0 us.)
+template <bool PAIR, int EPI, bool EMITS>
 __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uint32_t tmem_base,
                                               int warp, int lane, bool alpha_in_smem) {
     volatile int *abort_flag = &ctl->abort_flag;
@@ -158,7 +160,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
     const int cgroup = ((warp - 2) >> 2) - team * cgroups;
     const int frame = g.hp * g.wp;
     const long ohw = (long)g.oh * g.ow;
-    const bool emits = !PAIR && g.emit_bin;  // chained layers do not run on pairs
+    const bool emits = EMITS || (!PAIR && g.emit_bin);
     bool ok = true;   // false once a wait ran out somewhere in the CTA
     float run = 0.f;  // chained layers: running sum of |y| over the filter tiles of a pixel
     for (int it = team; it < rounds; it += g.teams) {
@@ -174,7 +176,8 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
         const int r = oh * g.ow + ow;
         const long pix = (long)n * ohw + r;
         float kk = 0.f;
-        if (valid && !g.sums) {
+        // chained layers: K scales a pixel's mean |x|, which one column group writes after the last filter tile
+        if (valid && !g.sums && (!emits || (cgroup == 0 && nt == g.n_tiles - 1))) {
             if (g.kmap) {
                 kk = __ldg(g.kmap + pix);
             } else {
@@ -190,7 +193,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs &g, Control *ctl, uin
                         kk = __fadd_rn(kk, __fmul_rn(__ldg(img + y * g.iw + x), g.inv_khw));
                     }
                 }
-                if (g.kmap_out && cgroup == 0 && nt == 0) g.kmap_out[pix] = kk;
+                if (g.kmap_out && cgroup == 0 && (emits || nt == 0)) g.kmap_out[pix] = kk;
             }
         }
         const int oc0 = nt * g.n_tile;
@@ -1153,7 +1156,7 @@ __device__ __forceinline__ void mma_role_planes(const TcArgs &g, Control *ctl, u
 // own tensor memory. A stage is a third smaller per CTA that way (32 KB instead of 48 KB at
 // N = 256), which is what the kernel is short of: at one stage per 512 cycles a single CTA pulls
 // 94 B/clk from L2, four fifths of what the SM's port delivers.
-template <int KK, bool PAIR, int EPI>
+template <int KK, bool PAIR, int EPI, bool EMITS>
 __global__ void __launch_bounds__(threads_of(EPI), 1)
 conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const TcArgs g) {
@@ -1256,7 +1259,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 ctl->alpha[i] = i < g.oc ? __ldg(g.alpha + i) : 0.f;
             bar_sync(5, 32 * EPI);
         }
-        epilogue_role<PAIR, EPI>(g, ctl, tmem_base, warp, lane, alpha_in_smem);
+        epilogue_role<PAIR, EPI, EMITS>(g, ctl, tmem_base, warp, lane, alpha_in_smem);
     }
 
     fence_before();
@@ -1292,14 +1295,6 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         sm_count[d].store(sms, std::memory_order_relaxed);
     }
-    // CTA pairs when the layer is more than one round of tiles (measured with 8-bit operands on
-    // AlexNet conv4: 35.0 against 36.9 us at 256 images, 24.3 against 24.9 at 128). With a single
-    // round the pair's longer hand-shakes cost more than its lighter loads save: a pass on one image
-    // 13.5 against 12.4 us with the present operands, on 32 images 17.5 against 16.6. Floats or sums out
-    // only (the chained epilogue carries per-pixel state across the filter tiles of one CTA), and a
-    // filter tile that splits into two UMMA-sized halves.
-    const bool pair = !next && p.n_tile % 32 == 0 && m_tiles >= 2 &&
-                      (long)m_tiles * (p.ocp16 / p.n_tile) > sms;
     TcArgs g;
     g.alpha = alpha; g.kmap = k; g.amap = a; g.kmap_out = k_out; g.dst = dst; g.sums = sums;
     g.error = error_word;
@@ -1312,6 +1307,34 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.tap_kw = p.cat ? 1 : p.kw;
     g.taps = p.kh * g.tap_kw;
     g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(tap_bytes, p.kchunk);
+    g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
+    const int kk = p.kchunk / 32;
+    const int steps = g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last);  // MMAs of a tile
+    // CTA pairs when the layer is more than one round of tiles (measured with 8-bit operands on
+    // AlexNet conv4: 35.0 against 36.9 us at 256 images, 24.3 against 24.9 at 128) and a filter tile splits
+    // into two UMMA-sized halves. With a single round the pair's longer hand-shakes cost more than its lighter
+    // loads save: a pass on one image 13.5 against 12.4 us with the present operands, on 32 images 17.5
+    // against 16.6.
+    // Chained layers, whose CTAs carry a pixel's state across all of its filter tiles, store next to nothing,
+    // and a CTA alone keeps up with the tensor pipe while its loads are whole: pairs where they are not, which
+    // is where operand rows are an odd number of 16 bytes (each straddles sectors) or the last of several
+    // chunks of a row is partly empty (a stage's hand-over for fewer MMAs), and a position tile is enough work.
+    // Two layers chained, the first one's CTAs alone over pairs, 225 chains of 6 to 30 pixels a side, 32 to 512
+    // channels and 64 to 512 filters, on one stream and among others:
+    //   odd rows, 4000 cycles a tile and more              0.96 to 1.91, mean 1.31   0.91 to 1.90, mean 1.25
+    //   a partial chunk, the same, more tiles than SMs     1.02 to 1.38, mean 1.14   0.97 to 1.37, mean 1.11
+    //   a partial chunk, the same, fewer tiles             0.96 to 1.27, mean 1.07   0.94 to 1.41, mean 1.07
+    //   odd rows, fewer cycles                             0.92 to 1.48, mean 1.08   0.83 to 1.29, mean 1.02
+    //   a partial chunk, fewer cycles                      0.91 to 1.07, mean 0.99   0.79 to 1.03, mean 0.95
+    //   whole chunks and even rows                         0.79 to 1.04, mean 0.94   0.76 to 1.03, mean 0.93
+    // (conv4 on 64 images, of the third kind: 0.97 among others.) conv3, conv4 and conv5 on 128 images, conv4
+    // on pairs: 56.6 -> 53.4 us on one stream, 43.4 -> 43.1 among others.
+    const bool odd_rows = p.icp % 32 != 0;
+    const bool part_chunk = p.n_tile >= 96 && g.chunks_per_tap > 1 && tap_bytes % p.kchunk != 0;
+    const bool pair =
+        p.n_tile % 32 == 0 && m_tiles >= 2 &&
+        (next ? p.kh > 1 && (odd_rows || (part_chunk && m_tiles > sms)) && (long)steps * p.ocp16 / 2 >= 4000
+              : (long)m_tiles * (p.ocp16 / p.n_tile) > sms);
     const int groups = g.kh * g.chunks_per_tap;
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
@@ -1350,10 +1373,10 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     int n_tile = p.n_tile;
     const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
     const int half_grid = sms / 2 - sms / 2 % half_tiles;
-    if (pair && !p.cat && g.kh >= 3 && n_tile >= 128 && n_tile % 64 == 0 && row_offsets_ok &&
+    if (pair && !next && !p.cat && g.kh >= 3 && n_tile >= 128 && n_tile % 64 == 0 && row_offsets_ok &&
         !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
         div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, sms / 2) &&
-        (p.icp % 32 != 0 ||
+        (odd_rows ||
          (n_tile > kAccStep && div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3)))
         n_tile /= 2;
     const int b_rows = pair ? n_tile / 2 : n_tile;  // filter rows a CTA loads per stage
@@ -1386,8 +1409,6 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.tx_bytes = g.a_bytes + (uint32_t)(b_rows * p.kchunk);  // per CTA
     g.stage_bytes = (g.tx_bytes + 1023u) & ~1023u;
     g.issuers = g.taps * g.chunks_per_tap < 2 ? 1 : 2;
-    g.kk_last = (tap_values - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
-    const int kk = p.kchunk / 32;
     // Eight epilogue warps instead of sixteen where a pair has four tiles or more and each keeps the tensor
     // pipe busy for 5000 cycles or more: the stores have the next tile's MMAs to hide behind either way, all
     // but the last tile's. The time with sixteen over that with eight, layers of 28 x 28 with 128, 256 and 512
@@ -1397,32 +1418,32 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     //   fewer                0.98 to 1.03, mean 1.00    1.00 to 1.09, mean 1.013
     // conv2 on 128 images (5120 cycles, six tiles) 43.3 -> 42.7 us among others, VGG (9216, six) 71.6 -> 71.2.
     // With two or three tiles 0.90 to 1.07.
-    const long tile_cycles =
-        (long)g.taps * ((g.chunks_per_tap - 1) * kk + g.kk_last) * n_tile / 2;
+    const long tile_cycles = (long)steps * n_tile / 2;
     const int pair_tiles = div_up_i(((m_tiles + 1) / 2) * g.n_tiles, sms / 2);
-    const bool few = pair && kk == 4 && tile_cycles >= 5000 && pair_tiles >= 4;
+    const bool few = pair && !next && kk == 4 && tile_cycles >= 5000 && pair_tiles >= 4;
     const int epi = few ? kFewEpiWarps : kEpiWarps;
-    void (*kernel)(CUtensorMap, CUtensorMap, TcArgs) =
-        few    ? conv_tcgen05_kernel<4, true, kFewEpiWarps>
-        : pair ? (kk == 4   ? conv_tcgen05_kernel<4, true, kEpiWarps>
-                  : kk == 2 ? conv_tcgen05_kernel<2, true, kEpiWarps>
-                            : conv_tcgen05_kernel<1, true, kEpiWarps>)
-               : (kk == 4   ? conv_tcgen05_kernel<4, false, kEpiWarps>
-                  : kk == 2 ? conv_tcgen05_kernel<2, false, kEpiWarps>
-                            : conv_tcgen05_kernel<1, false, kEpiWarps>);
+    const int per_stage = kk == 4 ? 0 : kk == 2 ? 1 : 2, form = few ? 3 : !pair ? 0 : next ? 2 : 1;
+    using Kernel = void (*)(CUtensorMap, CUtensorMap, TcArgs);
+    static const Kernel kernels[3][4] = {
+        {conv_tcgen05_kernel<4, false, kEpiWarps, false>, conv_tcgen05_kernel<4, true, kEpiWarps, false>,
+         conv_tcgen05_kernel<4, true, kEpiWarps, true>, conv_tcgen05_kernel<4, true, kFewEpiWarps, false>},
+        {conv_tcgen05_kernel<2, false, kEpiWarps, false>, conv_tcgen05_kernel<2, true, kEpiWarps, false>,
+         conv_tcgen05_kernel<2, true, kEpiWarps, true>, nullptr},
+        {conv_tcgen05_kernel<1, false, kEpiWarps, false>, conv_tcgen05_kernel<1, true, kEpiWarps, false>,
+         conv_tcgen05_kernel<1, true, kEpiWarps, true>, nullptr}};
+    const Kernel kernel = kernels[per_stage][form];
     // per device and kernel, once: the opt-in to large dynamic shared memory, the SM count and
     // the number of CTA pairs that can be resident together
-    static std::atomic<bool> opted_in[64][3][3];
-    std::atomic<bool> &done = opted_in[d][kk == 4 ? 0 : kk == 2 ? 1 : 2][few ? 2 : pair ? 1 : 0];
+    static std::atomic<bool> opted_in[64][3][4];
+    std::atomic<bool> &done = opted_in[d][per_stage][form];
     if (!done.load(std::memory_order_acquire)) {
         const cudaError_t e = cudaFuncSetAttribute(
             kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
         done.store(true, std::memory_order_release);
     }
-    int units = g.n_inner ? m_tiles : m_tiles * g.n_tiles, slots = sms;
+    int units = (pair ? (m_tiles + 1) / 2 : m_tiles) * (next ? 1 : g.n_tiles), slots = sms;
     if (pair) {
-        units = ((m_tiles + 1) / 2) * g.n_tiles;
         slots = pair_count[d].load(std::memory_order_relaxed);
         if (!slots) {
             cudaLaunchConfig_t cfg = {};
@@ -1444,7 +1465,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     int grid = units < slots ? units : slots;
     // Fewer pairs, if that costs no further round, so that each keeps to one filter tile.
     const int one_nt = grid - grid % g.n_tiles;
-    const bool same_nt = pair && one_nt > 0 && div_up_i(units, one_nt) == div_up_i(units, grid);
+    const bool same_nt = pair && (!next || g.n_tiles == 1) && one_nt > 0 && div_up_i(units, one_nt) == div_up_i(units, grid);
     g.planes = 0; g.plane_rows = 0; g.plane_pitch = 0; g.pos_bytes = p.icp; g.plane_desc_hi = 0;
     g.halo = 0; g.block = 0; g.resident = 0; g.n_a_slots = 0; g.a_slot_bytes = 0; g.b_ring_off = 0; g.b_slot_bytes = 0;
     g.b_bytes = (uint32_t)(b_rows * p.kchunk);
