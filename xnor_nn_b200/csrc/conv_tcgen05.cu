@@ -1361,19 +1361,21 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // positions twice where
     // - operand rows are an odd number of 16 bytes, so that every filter row loaded straddles sectors, or
     // - a pair has three tiles or fewer and the accumulators of the whole share columns.
-    // Kernel alone, whole over half, 256 layers on 6 to 30 pixels, 270 to 512 channels, 120 to 768 filters, 1
-    // to 7 tiles a pair of the whole:
-    //   odd rows, tiles of 192 and 256, 3 x 3          0.98 to 1.49, mean 1.23
-    //   odd rows, tiles of 128, 4 x 4                  0.95 to 1.19, mean 1.06
-    //   others, up to three tiles, 256 filters a tile  0.99 to 1.29, mean 1.11
+    // Whole over half, 256 layers on 6 to 30 pixels, 270 to 512 channels, 120 to 768 filters, 1 to 7 tiles a pair
+    // of the whole, kernel alone, and 144 of the first three kinds, a pass among others:
+    //   odd rows, tiles of 192 and 256, 3 x 3          0.98 to 1.49, mean 1.23   0.98 to 1.21, mean 1.08
+    //   odd rows, tiles of 128, 4 x 4                  0.95 to 1.19, mean 1.06   0.75 to 1.02, mean 0.92
+    //   others, up to three tiles, 256 filters a tile  0.99 to 1.29, mean 1.11   0.98 to 1.08, mean 1.02
     //   others, up to three tiles, 192                 0.91 to 1.16, mean 1.03
     //   others, more tiles                             0.86 to 1.20, mean 1.04
     //   2 x 2 filters on 640 to 768 channels           0.92 to 1.12, mean 0.98
-    // conv4 on 256 images, a pass: 41.6 -> 40.3 us on one stream.
+    // conv4 on 256 images, a pass: 41.6 -> 40.3 us on one stream, 39.0 -> 37.7 among others. (Layers whose whole
+    // stays resident: half of 256 filters 1.06 with up to 1.4 tiles a pair on one stream, 0.95 to 1.05 among
+    // others; of 192 and 128 0.87 to 1.06.)
     int n_tile = p.n_tile;
     const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
     const int half_grid = sms / 2 - sms / 2 % half_tiles;
-    if (pair && !next && !p.cat && g.kh >= 3 && n_tile >= 128 && n_tile % 64 == 0 && row_offsets_ok &&
+    if (pair && !next && !p.cat && g.kh >= 3 && n_tile >= 192 && n_tile % 64 == 0 && row_offsets_ok &&
         !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
         div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, sms / 2) &&
         (odd_rows ||
