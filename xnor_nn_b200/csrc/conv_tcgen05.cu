@@ -602,7 +602,10 @@ __device__ __forceinline__ void mma_role(const TcArgs &g, Control *ctl, uint32_t
 // Step order inside a tile: filter row kh, channel chunk, filter column kw (the sums are integers:
 // any order gives the same result). A group = the kw steps of one (kh, chunk): one halo tile of
 // g.halo positions in slot G % n_a_slots (G counts groups across tiles), kw filter tiles in
-// consecutive slots of the filter ring. A descriptor that starts r rows into a 128-byte-swizzled
+// consecutive slots of the filter ring. With g.block a group is all kh kw steps of one chunk, whose
+// halo tile holds the positions of all of them, so that the positions are loaded once a tile instead of
+// once a filter row: the loads of a tile of conv3-sized layers go from 3 x 17 KB and 9 x 12 to 20 KB and
+// 9 x 12 a chunk. A descriptor that starts r rows into a 128-byte-swizzled
 // tile reads rows r .. r + 127 of it (the swizzle is a function of the shared-memory address), so
 // tap kw of the group is the halo tile's descriptor advanced by kw rows.
 __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
@@ -618,6 +621,7 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
     const uint32_t afull0 = rank != 0 ? mapa(afull_l, 0) : afull_l;
     const uint32_t empty0 = smem_u32(&ctl->empty[0]), aempty0 = smem_u32(&ctl->a_empty[0]);
     const int b_rows = g.n_tile >> 1;
+    const int kh_groups = g.block ? 1 : g.kh, group_taps = g.block ? g.taps : g.tap_kw;
     const uint32_t a_bytes = (uint32_t)g.halo * (uint32_t)g.kchunk;
     int sb = 0, sa = 0;
     uint32_t pb = 0, pa = 0;
@@ -628,7 +632,7 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
         deal.at(g, it, mt, nt);
         const int row0 = g.lead + mt * BM - g.ph * g.wp - g.pw;  // tap (0,0)
         const int brow0 = nt * g.n_tile + (int)rank * b_rows;
-        for (int kh = 0; ok && kh < g.kh; kh++) {
+        for (int kh = 0; ok && kh < kh_groups; kh++) {
             for (int chunk = 0; ok && chunk < g.chunks_per_tap; chunk++) {
                 const uint32_t aebar = aempty0 + 8u * (uint32_t)sa;
                 ok = warp_wait(aebar, pa ^ 1, abort_flag, g.error, 8, g.wait_ns);
@@ -661,7 +665,7 @@ __device__ __forceinline__ void producer_halo(const TcArgs &g, Control *ctl,
                     __syncwarp();
                     continue;
                 }
-                for (int kw = 0; kw < g.tap_kw; kw++, brow += g.ocp16) {
+                for (int tap = 0; tap < group_taps; tap++, brow += g.ocp16) {
                     const uint32_t ebar = empty0 + 8u * (uint32_t)sb;
                     ok = warp_wait(ebar, pb ^ 1, abort_flag, g.error, 1, g.wait_ns);
                     if (!ok) break;
@@ -697,7 +701,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     const int rounds = Deal<true>(g).rounds(g);
     if (rounds == 0) return;
     const int ksteps = g.taps * g.chunks_per_tap;  // >= g.issuers; a multiple of g.tap_kw
-    const int n_iss = g.issuers, kwn = g.tap_kw;
+    const int n_iss = g.issuers, kwn = g.block ? g.taps : g.tap_kw;
     const uint64_t hi = (uint64_t)g.desc_hi << 32;
     const uint32_t a_lo0 = ((stage0 >> 4) & 0x3FFF) | (1u << 16);
     const uint32_t b_lo0 = (((stage0 + g.b_ring_off) >> 4) & 0x3FFF) | (1u << 16);
@@ -712,6 +716,9 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
     int kw = who % kwn, sa = (who / kwn) % g.n_a_slots;
     uint32_t pa = ((who / kwn) / g.n_a_slots) & 1u;
     int chunk = (who / kwn) % g.chunks_per_tap;  // groups walk the chunks, then the filter rows
+    // the step's tap as a row of its position tile, and the filter columns left in its filter row
+    const int skip = g.wp - g.tap_kw;
+    int row = kw + kw / g.tap_kw * skip, to_go = g.tap_kw - kw % g.tap_kw;
     bool ok = true, entered = false, a_seen = false;
     int b = 0;  // the tile's accumulator and how often it has come round
     uint32_t acc_phase = 0;
@@ -742,7 +749,7 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
         fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
         const uint64_t adesc =
-            hi | (uint64_t)(a_lo0 + (uint32_t)sa * a_units + (uint32_t)kw * row_units);
+            hi | (uint64_t)(a_lo0 + (uint32_t)sa * a_units + (uint32_t)row * row_units);
         const uint64_t bdesc = hi | (uint64_t)(b_lo0 + (uint32_t)sb * b_units);
         const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
         if (leader) {
@@ -762,6 +769,9 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
         sb += n_iss;
         if (sb >= g.n_stages) { sb -= g.n_stages; pb ^= 1u; }
         kw += n_iss;
+        row += n_iss;
+        to_go -= n_iss;
+        if (to_go <= 0) { to_go += g.tap_kw; row += skip; }
         if (kw >= kwn) {
             // this thread's last step of the group is issued: its reads of the halo tile are
             // covered by this commit (both issuers commit: the barrier counts them)
@@ -773,6 +783,8 @@ __device__ __forceinline__ void mma_role_halo(const TcArgs &g, Control *ctl, uin
                 if (++sa == g.n_a_slots) { sa = 0; pa ^= 1u; }
                 if (++chunk == g.chunks_per_tap) chunk = 0;
             } while (kw >= kwn);
+            row = kw;
+            to_go = g.tap_kw - kw;
             a_seen = false;
         }
         ks += n_iss;
@@ -1228,7 +1240,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         dependency_wait();
         if constexpr (PAIR) {
             if (g.planes) producer_planes(g, ctl, &map_a, &map_b, stage0, rank);
-            else if (g.block) producer_block(g, ctl, &map_a, &map_b, stage0, rank);
+            else if (g.block && g.resident) producer_block(g, ctl, &map_a, &map_b, stage0, rank);
             else if (g.halo) producer_halo(g, ctl, &map_a, &map_b, stage0, rank);
             else producer_ring<PAIR>(g, ctl, &map_a, &map_b, stage0, rank);
         } else {
@@ -1242,7 +1254,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 if (KK == 4 && g.planes && g.chunks_per_tap * KK > 32)
                     mma_role_planes<KK, true>(g, ctl, tmem_base, stage0, who);
                 else if (g.planes) mma_role_planes<KK, false>(g, ctl, tmem_base, stage0, who);
-                else if (KK == 4 && g.block) mma_role_block<KK>(g, ctl, tmem_base, stage0);
+                else if (KK == 4 && g.block && g.resident) mma_role_block<KK>(g, ctl, tmem_base, stage0);
                 else if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
                 else if (g.halo) mma_role_halo<KK>(g, ctl, tmem_base, stage0, who);
                 else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
@@ -1522,15 +1534,23 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         halo = true;
     }
     if (halo && !g.resident) {
-        // three halo tiles of 136 positions, the rest of the room for filter tiles
-        g.halo = BM + 8;
+        // Three position tiles, for all filter rows where they are one box, else for one (136 positions); the
+        // rest of the room for filter tiles. For one over for all, 58 layers of 6 to 32 pixels, 300 to 1024
+        // channels and 192 to 768 filters, on one stream and among others:
+        //   2 x 2 and 3 x 3, tiles of 192 filters  1.02 to 1.08, mean 1.05   1.02 to 1.09, mean 1.05
+        //   2 x 2 and 3 x 3, tiles of 256          0.99 to 1.06, mean 1.02   0.98 to 1.07, mean 1.02
+        //   5 x 5, tiles of 192                    0.99 to 1.06, mean 1.02   1.00 to 1.06, mean 1.02
+        //   5 x 5, tiles of 256                    0.94 to 1.03, mean 0.99   0.99 to 1.02, mean 1.00
+        // The last keep theirs.
+        g.block = g.kh > 1 && p.kchunk == 128 && block_rows <= 256 && (g.kh < 5 || !g.shared_cols);
+        g.halo = g.block ? block_rows : BM + 8;
         g.n_a_slots = 3;
         g.a_slot_bytes = (uint32_t)(g.halo * p.kchunk + 1023) & ~1023u;
         g.b_slot_bytes = (g.b_bytes + 1023u) & ~1023u;
         g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
         g.n_stages = (int)((room - g.b_ring_off) / g.b_slot_bytes);
         if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
-        if (g.n_stages < 4) { g.halo = 0; halo = false; }
+        if (g.n_stages < 4) { g.halo = 0; g.block = 0; halo = false; }
     }
     if (!halo) {
         g.n_stages = (int)(room / g.stage_bytes);
@@ -1567,7 +1587,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // Two instead of three beside position tiles for all filter rows: each is then one team's, which a lost
     // commit cannot pass over to another. Kernel alone, three over two, 24 such layers: 0.99 to 1.01. (Tiles of
     // columns, shorter, lose up to a tenth and keep three.)
-    if (g.block && g.n_acc == 3) g.n_acc = 2;
+    if (g.block && g.resident && g.n_acc == 3) g.n_acc = 2;
     g.teams = g.n_acc == 4 && rounds >= 4 && !few ? 4 : rounds >= 2 ? 2 : 1;
     g.by_acc = FastDiv((uint32_t)g.n_acc);
     note_launch();

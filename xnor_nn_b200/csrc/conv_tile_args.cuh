@@ -49,7 +49,7 @@ struct TcArgs {
     // once, together with the first round's position tiles, and stay. Position tiles as in halo mode
     // (halo is 128 if there is one tap per filter row), or as columns:
     int resident;
-    int block;            // resident filters, a position tile of `halo` rows serves all filter rows (producer_block)
+    int block;            // a position tile of `halo` rows serves all filter rows (producer_block, producer_halo)
     // Resident filters with position tiles of 16-byte channel columns (producer_planes): columns of a
     // tile, positions of it and positions from one column to the next (a multiple of 8), bytes per
     // position and the upper half of its matrix descriptors. 0: not so.
