@@ -30,7 +30,8 @@ def test_which_chained_layers_run_on_pairs(tmp_path):
     assert form == {"columns": "columns", "rows_of_all_filter_rows": "resident",
                     "rows_of_a_filter_row": "resident", "streamed": "halo", "streamed_two_filter_tiles": "halo",
                     "streamed_four_tiles_odd_filters": "halo", "streamed_192_filters": "halo",
-                    "ring": "ring", "fewer_tiles_than_sms": "halo", "conv4": "halo"}, form
+                    "ring": "ring", "fewer_tiles_than_sms": "halo",
+                    "part_chunk_fewer_tiles_than_sms": "halo", "conv4": "halo"}, form
     assert pairs["rows_of_all_filter_rows"]["halo"] > 136 >= pairs["rows_of_a_filter_row"]["halo"]
     assert {g["n_tiles"] for g in pairs.values()} == {1, 2, 4}
     assert {g["shared_cols"] for g in pairs.values()} == {0, 1}

@@ -23,12 +23,12 @@ PAIRS = {
     "streamed_four_tiles_odd_filters": (801, 288, 1023, 4, 4, 3, 3, 1, 1),
     "streamed_192_filters": (801, 480, 192, 4, 4, 3, 3, 1, 1),
     "ring": (1101, 350, 511, 5, 4, 3, 1, 0, 0),
+    "part_chunk_fewer_tiles_than_sms": (41, 384, 256, 4, 4, 3, 3, 1, 1),
     "fewer_tiles_than_sms": (41, 288, 256, 4, 4, 3, 3, 1, 1),
 }
 SINGLE = {
     "even_rows_whole_chunks": (801, 256, 256, 4, 4, 3, 3, 1, 1),
     "part_chunk_64_filters": (801, 384, 64, 4, 4, 3, 3, 1, 1),
-    "part_chunk_fewer_tiles_than_sms": (41, 384, 256, 4, 4, 3, 3, 1, 1),
     "short_tiles": (801, 288, 160, 4, 4, 3, 3, 1, 1),
     "one_filter_row": (1200, 480, 512, 4, 4, 1, 1, 0, 0),
 }

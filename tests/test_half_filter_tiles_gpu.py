@@ -1,5 +1,5 @@
 """Filter tiles of half a layer's width, whose filters stay in shared memory where the whole tile's would not
-(conv_tcgen05.cu): 96 and 128 filters a tile, a half that is part padding, operand rows that straddle
+(conv_tcgen05.cu): a half that is part padding, operand rows that straddle
 sectors and that do not, the last such number of tiles a pair, an odd number of position tiles, both orders of
 the result; and the first layers beyond, which keep the whole width. test_half_filter_tiles_cpu.py pins which
 layers take which. Sums and K bit for bit against the oracle, floats to the parity contract's 1e-4. A commit
@@ -19,8 +19,6 @@ NHWC = (0, 0, 1)
 HALVED = [
     cases._c("256_filters_odd_rows", 1700, 256, 288, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("part_padding", 1601, 250, 270, 4, 4, 3, 3, ph=1, pw=1, fmt=NHWC),
-    cases._c("96_filters_a_tile", 2400, 192, 350, 4, 3, 3, 3, ph=1, pw=1),
-    cases._c("four_tiles_of_96", 1200, 384, 416, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("six_tiles_of_128", 700, 768, 290, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("even_rows_three_tiles_a_pair", 2200, 256, 512, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("odd_rows_four_tiles_a_pair", 3000, 256, 288, 4, 4, 3, 3, ph=1, pw=1),
@@ -28,6 +26,7 @@ HALVED = [
 WHOLE = [
     cases._c("128_filters", 3100, 128, 480, 4, 4, 4, 3, ph=1, pw=1),
     cases._c("even_rows_four_tiles_a_pair", 2400, 256, 320, 4, 4, 3, 3, ph=1, pw=1),
+    cases._c("odd_rows_192_filters", 2400, 192, 350, 4, 3, 3, 3, ph=1, pw=1),
     cases._c("even_rows_192_filters", 1601, 192, 384, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("two_filter_rows", 1601, 256, 608, 4, 4, 2, 3, ph=1, pw=1),
     cases._c("half_does_not_fit", 1200, 256, 544, 4, 4, 3, 3, ph=1, pw=1),
@@ -56,7 +55,7 @@ def test_against_the_oracle(oracle, case):
     conv.close()
 
 
-@pytest.mark.parametrize("case", HALVED[:3], ids=[c[0] for c in HALVED[:3]])
+@pytest.mark.parametrize("case", HALVED[:2], ids=[c[0] for c in HALVED[:2]])
 def test_lost_commit_times_out_and_the_resources_stay_usable(case):
     _, d, _, _ = case
     src, w = cases.make_inputs(case)

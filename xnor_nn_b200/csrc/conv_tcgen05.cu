@@ -1314,7 +1314,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.q_total = p.q_total;
     g.m_tiles = m_tiles;
     // channels-wise: a tap, or the kw taps of a filter row one after the other
-    const int tap_bytes = p.cat ? p.kw * p.icp : p.icp;
+    const int tap_bytes = p.cat ? p.kw * p.icp : p.row_bytes, tap_pitch = p.cat ? tap_bytes : p.icp;
     const int tap_values = p.cat ? 2 * (p.kw - 1) * p.icp + p.ic : p.ic;
     g.tap_kw = p.cat ? 1 : p.kw;
     g.taps = p.kh * g.tap_kw;
@@ -1331,21 +1331,21 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // and a CTA alone keeps up with the tensor pipe while its loads are whole: pairs where they are not, which
     // is where operand rows are an odd number of 16 bytes (each straddles sectors) or the last of several
     // chunks of a row is partly empty (a stage's hand-over for fewer MMAs), and a position tile is enough work.
-    // Two layers chained, the first one's CTAs alone over pairs, 225 chains of 6 to 30 pixels a side, 32 to 512
+    // Two layers chained, the first one's CTAs alone over pairs, 135 chains of 6 to 30 pixels a side, 32 to 512
     // channels and 64 to 512 filters, on one stream and among others:
-    //   odd rows, 4000 cycles a tile and more              0.96 to 1.91, mean 1.31   0.91 to 1.90, mean 1.25
-    //   a partial chunk, the same, more tiles than SMs     1.02 to 1.38, mean 1.14   0.97 to 1.37, mean 1.11
-    //   a partial chunk, the same, fewer tiles             0.96 to 1.27, mean 1.07   0.94 to 1.41, mean 1.07
-    //   odd rows, fewer cycles                             0.92 to 1.48, mean 1.08   0.83 to 1.29, mean 1.02
-    //   a partial chunk, fewer cycles                      0.91 to 1.07, mean 0.99   0.79 to 1.03, mean 0.95
-    //   whole chunks and even rows                         0.79 to 1.04, mean 0.94   0.76 to 1.03, mean 0.93
-    // (conv4 on 64 images, of the third kind: 0.97 among others.) conv3, conv4 and conv5 on 128 images, conv4
-    // on pairs: 56.6 -> 53.4 us on one stream, 43.4 -> 43.1 among others.
+    //   odd rows, 4000 cycles a tile and more            1.00 to 1.28, mean 1.15   0.99 to 1.26, mean 1.11
+    //   a partial chunk, the same, more tiles than SMs   0.99 to 1.76, mean 1.23   0.91 to 1.73, mean 1.19
+    //   a partial chunk, the same, fewer tiles           0.91 to 1.56, mean 1.08   0.94 to 1.62, mean 1.09
+    //   odd rows, fewer cycles                           0.92 to 1.10, mean 1.00   0.83 to 1.04, mean 0.96
+    //   a partial chunk, fewer cycles                    0.91 to 1.27, mean 1.08   0.80 to 1.19, mean 1.02
+    //   whole chunks and even rows                       0.78 to 1.10, mean 0.95   0.76 to 1.07, mean 0.93
+    // conv3, conv4 and conv5 on 128 images, conv4 on pairs: 56.6 -> 53.4 us on one stream, 43.4 -> 43.1 among
+    // others (on 64 images, conv4 on pairs: 37.8 -> 37.1 and 22.7 -> 23.1).
     const bool odd_rows = p.icp % 32 != 0;
     const bool part_chunk = p.n_tile >= 96 && g.chunks_per_tap > 1 && tap_bytes % p.kchunk != 0;
     const bool pair =
         p.n_tile % 32 == 0 && m_tiles >= 2 &&
-        (next ? p.kh > 1 && (odd_rows || (part_chunk && m_tiles > sms)) && (long)steps * p.ocp16 / 2 >= 4000
+        (next ? p.kh > 1 && (odd_rows || part_chunk) && (long)steps * p.ocp16 / 2 >= 4000
               : (long)m_tiles * (p.ocp16 / p.n_tile) > sms);
     const int groups = g.kh * g.chunks_per_tap;
     // as many ring buffers as fit beside the control block
@@ -1370,28 +1370,26 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     };
     // A tile of half the filters, if that half stays in shared memory beside such tiles (below) and the whole
     // would not: its filters are loaded once instead of for each position tile, which pays for reading the
-    // positions twice where
-    // - operand rows are an odd number of 16 bytes, so that every filter row loaded straddles sectors, or
-    // - a pair has three tiles or fewer and the accumulators of the whole share columns.
-    // Whole over half, 256 layers on 6 to 30 pixels, 270 to 512 channels, 120 to 768 filters, 1 to 7 tiles a pair
-    // of the whole, kernel alone, and 144 of the first three kinds, a pass among others:
-    //   odd rows, tiles of 192 and 256, 3 x 3          0.98 to 1.49, mean 1.23   0.98 to 1.21, mean 1.08
-    //   odd rows, tiles of 128, 4 x 4                  0.95 to 1.19, mean 1.06   0.75 to 1.02, mean 0.92
-    //   others, up to three tiles, 256 filters a tile  0.99 to 1.29, mean 1.11   0.98 to 1.08, mean 1.02
-    //   others, up to three tiles, 192                 0.91 to 1.16, mean 1.03
-    //   others, more tiles                             0.86 to 1.20, mean 1.04
-    //   2 x 2 filters on 640 to 768 channels           0.92 to 1.12, mean 0.98
-    // conv4 on 256 images, a pass: 41.6 -> 40.3 us on one stream, 39.0 -> 37.7 among others. (Layers whose whole
-    // stays resident: half of 256 filters 1.06 with up to 1.4 tiles a pair on one stream, 0.95 to 1.05 among
-    // others; of 192 and 128 0.87 to 1.06.)
+    // positions twice where the accumulators of the whole share columns and
+    // - a position's row ends inside a 32-byte sector, or
+    // - a pair has three tiles or fewer.
+    // Whole over half, 300 layers of 3 x 3 filters on 6 to 32 pixels, 270 to 512 channels, up to 7 tiles a pair of
+    // the whole, a pass on one stream and among others:
+    //   256 filters, such rows, up to three tiles  1.02 to 1.24, mean 1.12   0.99 to 1.09, mean 1.03
+    //   256 filters, such rows, more tiles         1.02 to 1.18, mean 1.10   1.00 to 1.09, mean 1.04
+    //   256 filters, others, up to three tiles     0.99 to 1.15, mean 1.05   0.94 to 1.04, mean 0.99
+    //   256 filters, others, more tiles            0.96 to 1.06, mean 1.01   0.96 to 0.99, mean 0.97
+    //   192 filters                                0.90 to 1.12, mean 0.99   0.85 to 0.99, mean 0.94
+    // conv4 on 256 images, of the third kind: 41.6 -> 40.3 us on one stream, 39.0 -> 37.7 among others. (Layers
+    // whose whole stays resident: half of 256 filters 1.06 with up to 1.4 tiles a pair on one stream, 0.95 to
+    // 1.05 among others; of 192 and 128 0.87 to 1.06.)
     int n_tile = p.n_tile;
     const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
     const int half_grid = sms / 2 - sms / 2 % half_tiles;
-    if (pair && !next && !p.cat && g.kh >= 3 && n_tile >= 192 && n_tile % 64 == 0 && row_offsets_ok &&
+    if (pair && !next && !p.cat && g.kh >= 3 && n_tile > kAccStep && n_tile % 64 == 0 && row_offsets_ok &&
         !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
         div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, sms / 2) &&
-        (odd_rows ||
-         (n_tile > kAccStep && div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3)))
+        (p.row_bytes % 32 != 0 || div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3))
         n_tile /= 2;
     const int b_rows = pair ? n_tile / 2 : n_tile;  // filter rows a CTA loads per stage
     g.n_tiles = p.ocp16 / n_tile;
@@ -1568,7 +1566,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
                                    (uint32_t)(halo ? g.halo : BM));
     if (!a_ok ||
         !encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
-                         (uint64_t)tap_bytes, (uint32_t)p.kchunk, (uint32_t)b_rows))
+                         (uint64_t)tap_pitch, (uint32_t)p.kchunk, (uint32_t)b_rows))
         return cudaErrorNotSupported;
 
     size_t smem = 1024 + kControlBytes +

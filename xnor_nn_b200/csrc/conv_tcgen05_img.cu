@@ -505,14 +505,14 @@ cudaError_t launch_conv_tcgen05_img(const Plan &p, const void *bin_src, const vo
     if (p.mb < 1 || p.img_tiles < 1) return cudaSuccess;
     const uint8_t *x0 = (const uint8_t *)bin_src + (size_t)p.lead * p.icp;  // pixel (0,0) of image 0
     CUtensorMap map_w, map_x, map_xh;
-    const uint64_t row = (uint64_t)p.icp;
+    const uint64_t row = (uint64_t)p.icp, bytes = (uint64_t)p.row_bytes;
     const uint32_t half_rows = p.img_half_rows ? (uint32_t)p.img_half_rows : (uint32_t)p.img_rows;
-    if (!encode_bytes_2d(&map_w, bin_w, (uint64_t)p.kh * p.kw * p.ocp16, row, row, (uint32_t)p.kchunk,
+    if (!encode_bytes_2d(&map_w, bin_w, (uint64_t)p.kh * p.kw * p.ocp16, bytes, row, (uint32_t)p.kchunk,
                          kFilters) ||
-        !encode_bytes_4d(&map_x, x0, row, (uint64_t)p.wp, (uint64_t)p.hp, (uint64_t)p.mb, row,
+        !encode_bytes_4d(&map_x, x0, bytes, (uint64_t)p.wp, (uint64_t)p.hp, (uint64_t)p.mb, row,
                          row * p.wp, row * p.wp * p.hp, (uint32_t)p.kchunk, (uint32_t)p.ow,
                          (uint32_t)p.img_rows) ||
-        !encode_bytes_4d(&map_xh, x0, row, (uint64_t)p.wp, (uint64_t)p.hp, (uint64_t)p.mb, row,
+        !encode_bytes_4d(&map_xh, x0, bytes, (uint64_t)p.wp, (uint64_t)p.hp, (uint64_t)p.mb, row,
                          row * p.wp, row * p.wp * p.hp, (uint32_t)p.kchunk, (uint32_t)p.ow,
                          half_rows))
         return cudaErrorNotSupported;
@@ -528,7 +528,7 @@ cudaError_t launch_conv_tcgen05_img(const Plan &p, const void *bin_src, const vo
     g.whole = p.img_whole;
     g.units = p.img_whole + 2 * (p.img_tiles - p.img_whole);
     g.half_rows = p.img_half_rows;
-    g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(p.icp, p.kchunk); g.taps = p.kh * p.kw;
+    g.kchunk = p.kchunk; g.chunks_per_tap = div_up_i(p.row_bytes, p.kchunk); g.taps = p.kh * p.kw;
     g.ocp16 = p.ocp16;
     g.kk_last = (p.ic - (g.chunks_per_tap - 1) * 2 * p.kchunk + 63) / 64;
     g.n_full = p.img_n;

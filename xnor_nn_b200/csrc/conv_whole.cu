@@ -404,13 +404,13 @@ bool whole_shape(const Plan &p, WholeArgs *g, size_t *smem) {
     g->n_tiles = div_up_i(p.oc, g->n_tile);
     if (m_tiles * g->n_tiles > sm_count() || 4L * p.mb * p.ic * p.ih * p.iw >= 1L << 32) return false;
     g->rows = BM + (p.kh - 1) * p.wp + p.kw - 1;
-    g->columns = p.icp / 16;
+    g->columns = p.row_bytes / 16;
     g->odd = p.cat && (g->columns & 1);
     g->planes = g->columns + (g->columns & 1);
     if (!p.cat && p.kchunk == 128) g->planes = (g->columns + 7) & ~7;
     g->pitch = (g->rows + 7 + 8) & ~7;
     g->swizzled = !p.cat && p.kchunk == 128;
-    const int tap_bytes = p.cat ? p.kw * p.icp : p.icp;
+    const int tap_bytes = p.cat ? p.kw * p.icp : p.row_bytes;
     g->tap_kw = p.cat ? 1 : p.kw;
     g->taps = p.kh * g->tap_kw;
     g->kchunk = p.kchunk;
@@ -493,9 +493,9 @@ cudaError_t launch_conv_whole(const Plan &p, const float *src, void *bin_src, co
     g.by_frame = FastDiv((uint32_t)(p.hp * p.wp)); g.by_wp = FastDiv((uint32_t)p.wp);
     g.by_hw = FastDiv((uint32_t)g.hw); g.by_iw = FastDiv((uint32_t)p.iw);
     CUtensorMap map_b;
-    const int tap_bytes = p.cat ? p.kw * p.icp : p.icp;
+    const int tap_bytes = p.cat ? p.kw * p.icp : p.row_bytes;
     if (!encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
-                         (uint64_t)tap_bytes, (uint32_t)p.kchunk, (uint32_t)g.n_tile))
+                         (uint64_t)(p.cat ? tap_bytes : p.icp), (uint32_t)p.kchunk, (uint32_t)g.n_tile))
         return cudaErrorNotSupported;
     int dev = 0;
     cudaGetDevice(&dev);

@@ -265,7 +265,16 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
         p->hp = p->oh + taps - 1;
         p->q_total = (long)p->mb * p->hp * p->wp;
     }
-    p->icp = div_up_i(channels, 32) * 16;
+    // Rows of several chunks start on 64 bytes: from elsewhere every row of a chunk's box straddles sectors, which
+    // the copy engine moves at down to half the rate. (The boxes end where the channels do: what lies between
+    // rows is not read.) Starting on 16 over starting on 64, 109 layers of 257 to 768 channels, 2 x 2 to 5 x 5
+    // filters, 6 to 40 pixels and 0.05 to 6 rounds of tiles, a pass on one stream and among others:
+    //   rows of an odd number of 16 bytes  0.96 to 1.72, mean 1.12   0.98 to 1.97, mean 1.12
+    //   of 32                              0.99 to 1.32, mean 1.04   0.97 to 1.31, mean 1.04
+    // 1 x 1 filters, bound by the packer and the stores, 0.97 to 1.06, mean 1.01, and 1.00. Starting on 128
+    // bytes instead: another 1.02 in the mean, but conv4 (192 bytes) packs slower, 14.8 -> 15.3 us.
+    p->row_bytes = div_up_i(channels, 32) * 16;
+    p->icp = !fold && taps > 1 && p->row_bytes > 128 ? div_up_i(p->row_bytes, 64) * 64 : p->row_bytes;
     p->kchunk = p->icp > 64 ? 128 : p->icp > 32 ? 64 : 32;
     // Filter tile of the position-tile kernel = its UMMA N: a multiple of 16, at most 256. The
     // filters are split into the fewest equal tiles and padded (with zero filters) to fill them,

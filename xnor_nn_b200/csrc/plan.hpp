@@ -56,7 +56,8 @@ struct Plan {
     //   lead + (n*(ih+ph) + h)*(iw+pw) + w
     // of a [rows][icp] byte matrix, and tap (kh,kw) of the output at q reads row
     //   q + (kh-ph)*(iw+pw) + (kw-pw).
-    int icp;        // bytes per position: two channels each, rounded up to 16
+    int icp;        // bytes from a position to the next: row_bytes, rounded up to 64 where that pays
+    int row_bytes;  // bytes of a position: two channels each, rounded up to 16
     int kchunk;     // bytes of K per pipeline stage: 128, 64 or 32 (= the swizzle span)
     int wp, hp;     // iw + pw, ih + ph
     int lead;       // zero rows in front of the first image
