@@ -1,7 +1,8 @@
-"""Positions of more than 128 bytes start on 64-byte boundaries (Plan::icp): every kernel that writes or reads
-such rows, at the least and the most that lies between them: the one-launch pass, both convolutions, both
-orders of the source and the weights, the upstream calls one by one, a chain into such rows, and frames left
-over from other values. Against the oracle: sums, A and K bit for bit, floats to the parity contract's 1e-4."""
+"""Positions of more than 128 bytes start on 64-byte boundaries (Plan::icp), and filter rows that hold several
+columns (Plan::tap_pitch): every kernel that writes or reads such rows, at the least and the most that lies
+between them: the one-launch pass, both convolutions, both orders of the source and the weights, the upstream
+calls one by one, a chain into such rows, and frames left over from other values. Against the oracle: sums, A and
+K bit for bit, floats to the parity contract's 1e-4."""
 import numpy as np
 import pytest
 
@@ -17,6 +18,9 @@ LAYERS = [  # channels of 144, 160, 176 and 192 bytes, 208 and 256
     cases._c("one_launch_nhwc_hwio_320", 3, 33, 320, 5, 5, 3, 3, ph=1, pw=1, fmt=(1, 1, 1)),
     cases._c("two_launches_352", 180, 96, 352, 13, 12, 3, 3, ph=1, pw=1),
     cases._c("two_launches_nhwc_hwio_390", 150, 48, 390, 11, 13, 2, 3, fmt=(1, 1, 0)),
+    cases._c("filter_rows_of_240_bytes", 2, 33, 96, 7, 8, 5, 5, ph=2, pw=2),
+    cases._c("filter_rows_of_144_bytes_hwio", 300, 40, 90, 9, 8, 3, 3, ph=1, pw=1, fmt=(1, 1, 1)),
+    cases._c("filter_rows_of_560_bytes", 60, 24, 150, 12, 14, 7, 7, ph=3, pw=3),
     cases._c("two_launches_512", 60, 64, 512, 14, 13, 3, 3, ph=1, pw=1),
 ]
 

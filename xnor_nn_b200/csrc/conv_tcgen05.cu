@@ -1314,7 +1314,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     g.q_total = p.q_total;
     g.m_tiles = m_tiles;
     // channels-wise: a tap, or the kw taps of a filter row one after the other
-    const int tap_bytes = p.cat ? p.kw * p.icp : p.row_bytes, tap_pitch = p.cat ? tap_bytes : p.icp;
+    const int tap_bytes = p.cat ? p.kw * p.icp : p.row_bytes;
     const int tap_values = p.cat ? 2 * (p.kw - 1) * p.icp + p.ic : p.ic;
     g.tap_kw = p.cat ? 1 : p.kw;
     g.taps = p.kh * g.tap_kw;
@@ -1566,7 +1566,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
                                    (uint32_t)(halo ? g.halo : BM));
     if (!a_ok ||
         !encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
-                         (uint64_t)tap_pitch, (uint32_t)p.kchunk, (uint32_t)b_rows))
+                         (uint64_t)p.tap_pitch, (uint32_t)p.kchunk, (uint32_t)b_rows))
         return cudaErrorNotSupported;
 
     size_t smem = 1024 + kControlBytes +

@@ -495,7 +495,7 @@ cudaError_t launch_conv_whole(const Plan &p, const float *src, void *bin_src, co
     CUtensorMap map_b;
     const int tap_bytes = p.cat ? p.kw * p.icp : p.row_bytes;
     if (!encode_bytes_2d(&map_b, bin_w, (uint64_t)g.taps * p.ocp16, (uint64_t)tap_bytes,
-                         (uint64_t)(p.cat ? tap_bytes : p.icp), (uint32_t)p.kchunk, (uint32_t)g.n_tile))
+                         (uint64_t)p.tap_pitch, (uint32_t)p.kchunk, (uint32_t)g.n_tile))
         return cudaErrorNotSupported;
     int dev = 0;
     cudaGetDevice(&dev);

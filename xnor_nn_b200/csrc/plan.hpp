@@ -58,6 +58,7 @@ struct Plan {
     //   q + (kh-ph)*(iw+pw) + (kw-pw).
     int icp;        // bytes from a position to the next: row_bytes, rounded up to 64 where that pays
     int row_bytes;  // bytes of a position: two channels each, rounded up to 16
+    int tap_pitch;  // bytes from a packed filter's row to the next filter's
     int kchunk;     // bytes of K per pipeline stage: 128, 64 or 32 (= the swizzle span)
     int wp, hp;     // iw + pw, ih + ph
     int lead;       // zero rows in front of the first image

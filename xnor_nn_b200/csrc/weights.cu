@@ -147,7 +147,7 @@ __device__ __forceinline__ void pack(const WArgs &g) {
         int c0 = word * span, from = tap;
         if (g.cat_words) {
             const int j = word / g.cat_words;
-            c0 -= j * g.cat_words * span;
+            c0 = j < g.kw ? c0 - j * g.cat_words * span : g.ic;  // past the last column nothing
             from = tap * g.kw + j;
         }
         if (g.fold_rows) {
@@ -224,12 +224,8 @@ cudaError_t launch_binarize_weights(const Plan &p, const float *w, void *bin_w, 
     g.out = (uint32_t *)bin_w;
     g.nibbles = p.family == kTcgen05;
     g.rows = g.nibbles ? p.ocp16 : p.ocp;
-    g.words = g.nibbles ? p.icp / 4 : p.icw;
-    g.cat_words = 0;
-    if (p.cat) {
-        g.cat_words = g.words;
-        g.words *= p.kw;
-    }
+    g.words = g.nibbles ? p.tap_pitch / 4 : p.icw;
+    g.cat_words = p.cat ? p.icp / 4 : 0;
     g.fold_rows = p.fold ? p.fold_rows : 0;
     g.fold_field = p.fold_field;
     g.taps = p.fold ? p.fold_taps : p.cat ? p.kh : p.kh * p.kw;
