@@ -33,9 +33,12 @@
 // channel chunk, with a halo of the positions that follow it, and the taps of the row read that
 // tile at row offsets (producer_halo / mma_role_halo); filters that fit are loaded once and stay
 // (mma_role_resident), in layers of few channels beside position tiles that serve all taps of the
-// filter (mma_role_planes, mma_role_block). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters)
+// filter (mma_role_planes). Where the positions of all filter rows are one box, a position tile is
+// loaded once a chunk for all of them, beside resident filters (mma_role_block) and streamed ones (producer_halo
+// with g.block). What bounds a tile is the tensor pipe (128 cycles per MMA of 256 filters)
 // or, when its loads share the way to L2 with the stores of the tile before it, those: AlexNet conv4
-// on 256 images takes 8200 cycles a tile without the other's stores and 10500 with them (pipe: 6900).
+// on 256 images, with 256 streamed filters a tile, took 8200 cycles a tile without the other's stores and 10500
+// with them (pipe: 6900); it has 128 resident ones now.
 //
 // The epilogue has three forms: floats in NCHW (a warp store is one contiguous run of a filter
 // plane), floats in NHWC (a thread owns whole 32-byte sectors and writes them with 256-bit

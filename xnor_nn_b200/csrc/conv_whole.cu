@@ -37,10 +37,16 @@
 // which come through the ring meanwhile), then 1000 to 5600 for the stores. One issuer needs about 500 cycles a
 // filter tile, mostly the chain of scalar instructions around its MMAs, hence four (MMAs of one image:
 // 6700 -> 5300). Times in us, two launches -> one: a pass among others on three streams, back to back on one
-// stream, waited for: conv4 on one image 7.2 -> 4.1, 12.8 -> 11.4, 23.6 -> 23.5; on 32 images 8.2 -> 5.9,
-// 16.4 -> 16.6, 25.0 -> 28.8; on 64 images channels-last 11.4 to 12.2 -> 11.9, 20.9 -> 18.0, 29.9 -> 29.9; 16
-// channels of 31 x 31, five images 8.7 -> 5.3, 7.5 -> 5.5, 20.0 -> 18.2. The first is bound by the host, for
-// which a launch is 2.0 us.
+// stream, waited for: conv4 on one image 7.2 -> 3.9, 12.8 -> 9.6, 23.6 -> 21.0; on 32 images 8.2 -> 5.3,
+// 16.4 -> 14.8, 25.0 -> 26.2; on 64 images channels-last 11.4 to 12.2 -> 11.4, 20.9 -> 18.0, 29.9 -> 29.9 (the
+// last two as measured before the next paragraph's changes); 16 channels of 31 x 31, five images 8.7 -> 5.3,
+// 7.5 -> 5.5, 20.0 -> 18.2 (the same). The first is bound by the host, for which a launch is 2.0 us.
+//
+// The cycles above are from before three changes to the packing, on one stream in us, one image and 32: one path
+// through a task's loads, whichever lanes have a pixel, 11.1 -> 10.0 and 16.4 -> 15.6; a barrier for each
+// hand-over of a running sum instead of counters that are polled, 10.1 -> 9.7 and 15.6 -> 15.1; the accumulator
+// cleared by the issuers, which have nothing to issue yet, instead of by packing warps, 9.7 -> 9.5 and 15.1 ->
+// 14.8.
 #include <cuda.h>
 
 #include <atomic>

@@ -70,7 +70,7 @@ struct Plan {
     // Layers of few channels: the kw taps of a filter row read neighbouring positions, and
     // positions are contiguous, so the operand row of position q can simply run on into the next
     // kw - 1 positions: one tap per filter row, kw*icp bytes deep, from the same activations (a
-    // tensor map whose rows overlap). Weights are then [kh][ocp16][kw*icp]. The copy engine moves
+    // tensor map whose rows overlap). Weights are then [kh][ocp16][tap_pitch]. The copy engine moves
     // full 128-byte rows instead of kw short ones, and 64-channel slices are not cut off at every tap.
     bool cat;
 
