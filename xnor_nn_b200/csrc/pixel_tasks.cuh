@@ -1,10 +1,9 @@
 // Packing the source by tasks of 32 neighbouring pixels x 32 channels, a task a warp (conv_whole.cu,
 // maps.cu): loads, and the sum of |x| over the channels in upstream's order, which tasks of the same pixels
-// hand on from warp to warp (the turns below are maps.cu's; conv_whole.cu has a barrier for each).
+// hand on from warp to warp.
 #pragma once
 
 #include "kernels.cuh"
-#include "tc_ptx.cuh"
 
 namespace xb200 {
 namespace tasks {
@@ -39,34 +38,6 @@ __device__ __forceinline__ void mul2(float &a, float &b, float by) {
         "mov.b64 {%0, %1}, x;\n\t}"
         : "+f"(a), "+f"(b)
         : "f"(by));
-}
-
-// Whose turn it is to add: a counter, since a warp may wait for it from several columns ahead, where an
-// mbarrier's parity says nothing. Bounded like every wait.
-__device__ __forceinline__ int turn_of(const int *turn) {
-    int v;
-    asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(tc::smem_u32(turn)) : "memory");
-    return v;
-}
-__device__ __forceinline__ void turn_pass(int *turn, int next) {
-    asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(turn)), "r"(next) : "memory");
-}
-__device__ __forceinline__ bool turn_wait(const int *turn, int want, volatile int *abort_flag, int *error,
-                                          unsigned long long limit_ns) {
-    bool ok = turn_of(turn) == want;
-    if (!ok) {
-        const unsigned long long t0 = tc::global_ns();
-        for (;;) {
-            for (int i = 0; i < 64 && !ok; i++) ok = turn_of(turn) == want;
-            if (ok || *abort_flag) break;
-            if (tc::global_ns() - t0 > limit_ns) {
-                *abort_flag = 1;
-                atomicCAS(error, 0, 21);
-                break;
-            }
-        }
-    }
-    return __all_sync(0xffffffffu, ok);
 }
 
 // `tile`: its pixels first .. last, in groups of 32; `g`: the source. Lane l has pixel l of the group,
@@ -128,21 +99,6 @@ __device__ __forceinline__ float sum_task(const float *v, int nc, float acc) {
             if (i < nc) acc = __fadd_rn(acc, fabsf(v[i]));
     }
     return acc;
-}
-
-// Adds the task's |x| / IC to the sum of the channels before it, once those have been added; v is used
-// up. The caller passes the turn on (or has the mean, after the last channels).
-__device__ __forceinline__ bool add_task(float *v, int nc, int col, float inv_ic, const int *turn,
-                                         const float *sum, volatile int *abort_flag, int *error,
-                                         unsigned long long limit_ns, float *out) {
-    scale_task(v, inv_ic);
-    float acc = 0.f;
-    if (col > 0) {
-        if (!turn_wait(turn, col, abort_flag, error, limit_ns)) return false;
-        acc = *(const volatile float *)sum;
-    }
-    *out = sum_task(v, nc, acc);
-    return true;
 }
 
 }  // namespace tasks
