@@ -50,5 +50,10 @@ def test_which_layers_have_blocks(launches):
     assert {g["halo"] for g in blocks} >= {256} and {g["a_slots"] for g in blocks} >= {2, 8}
     assert {g["groups"] for g in blocks} >= {2, 8} and {g["shared_cols"] for g in blocks} == {0, 1}
     assert {g["n_tiles"] for g in blocks} == {1, 2, 3} and {g["m_tiles"] % 2 for g in blocks} == {0, 1}
+    # one issuer where the taps of a filter row keep the tensor pipe for more than 800 cycles, else two
+    assert {n: g["issuers"] for n, g in launches.items() if n in [c[0] for c in gpu.BLOCKS] + ["alexnet_conv3"]} == {
+        "256_rows": 2, "eight_groups": 2, "two_tiles_in_flight": 2, "channel_tail_of_the_second_chunk": 2,
+        "two_filter_tiles": 1, "three_filter_tiles": 1, "overlapping_accumulators": 2, "a_filter_row_as_one": 2,
+        "folded": 2, "alexnet_conv3": 1}
     rows = [launches[c[0]] for c in gpu.ROWS]
     assert {g["kchunk"] for g in rows} == {64, 128} and 9 in {g["groups"] for g in rows}

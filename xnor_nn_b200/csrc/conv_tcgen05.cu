@@ -875,7 +875,8 @@ __device__ __forceinline__ void mma_role_resident(const TcArgs &g, Control *ctl,
 // Resident filters beside position tiles that serve all filter rows: a tile is the 128-byte rows of one K chunk
 // for every position that any tap reads, 128 + (kh-1) wp + kw-1 of them, and a tap is a row offset. Loaded once per
 // K chunk it is 20 KB for AlexNet conv3, where tiles for each filter row are 51 KB, beside which the results leave
-// the SM; and an issuer waits and commits once per chunk. Kernel alone, tiles for each filter row -> these: conv3 on
+// the SM; and an issuer waits and commits once per chunk. (The launcher says where two issuers
+// share a tile's filter rows.) One issuer, kernel alone, tiles for each filter row -> these: conv3 on
 // 256 images 22.9 -> 22.4 us, conv1 on 64 23.8 -> 21.4, and 1.00 to 1.11 times as fast, median 1.034, over 30
 // layers drawn from 16 to 256 images, 3 to 512 channels and filters, 6 to 56 pixels (first layers 60 to 227).
 __device__ __forceinline__ void producer_block(const TcArgs &g, Control *ctl, const CUtensorMap *map_a,
@@ -936,7 +937,7 @@ __device__ __forceinline__ void producer_block(const TcArgs &g, Control *ctl, co
 
 template <int KK>
 __device__ __forceinline__ void mma_role_block(const TcArgs &g, Control *ctl, uint32_t tmem_base,
-                                               uint32_t stage0) {
+                                               uint32_t stage0, int who) {
     volatile int *abort_flag = &ctl->abort_flag;
     const bool leader = elect_one();
     const int rounds = Deal<true>(g).rounds(g);
@@ -953,8 +954,11 @@ __device__ __forceinline__ void mma_role_block(const TcArgs &g, Control *ctl, ui
     bool ok = true;
     for (int it = 0; it < rounds; it++) {
         const uint32_t d_tmem = tmem_base + (uint32_t)b * g.acc_step;
-        ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2, g.wait_ns);
-        if (ok && g.shared_cols && it > 0)
+        if (who == 0)
+            ok = warp_wait(smem_u32(&ctl->acc_empty[b]), acc_phase ^ 1, abort_flag, g.error, 2, g.wait_ns);
+        else
+            ok = warp_wait(smem_u32(&ctl->started[b]), acc_phase, abort_flag, g.error, 6, g.wait_ns);
+        if (ok && who == 0 && g.shared_cols && it > 0)
             ok = warp_wait(smem_u32(&ctl->shared_free), (uint32_t)(it - 1) & 1u, abort_flag, g.error,
                            7, g.wait_ns);
         if (!ok) break;
@@ -962,7 +966,8 @@ __device__ __forceinline__ void mma_role_block(const TcArgs &g, Control *ctl, ui
             ok = warp_wait(afull0 + 8u * (uint32_t)sa, pa, abort_flag, g.error, 9, g.wait_ns);
             if (!ok) break;
             const int kk = chunk == g.chunks_per_tap - 1 ? g.kk_last : KK;
-            for (int kh = 0; kh < g.kh; kh++) {
+            // with two issuers each takes every other filter row of the tile (and some of each chunk: kh > 1)
+            for (int kh = g.issuers > 1 ? (chunk * g.kh + who) & 1 : 0; kh < g.kh; kh += g.issuers) {
                 const int gr = kh * g.chunks_per_tap + chunk;
                 if (it == 0)
                     ok = warp_wait(full0 + 8u * (uint32_t)gr, 0, abort_flag, g.error, 3, g.wait_ns);
@@ -981,8 +986,9 @@ __device__ __forceinline__ void mma_role_block(const TcArgs &g, Control *ctl, ui
                                                tmem_base + kScaleCol, (chunk | kh | kw | k) == 0 ? 0u : 1u);
                             }
                         }
+                        if ((chunk | kh | kw) == 0 && g.issuers > 1) commit_pair(smem_u32(&ctl->started[b]));
                     }
-                    if (kh == g.kh - 1) commit_pair(aempty0 + 8u * (uint32_t)sa);
+                    if (kh + g.issuers >= g.kh) commit_pair(aempty0 + 8u * (uint32_t)sa);
                 }
                 __syncwarp();
             }
@@ -996,8 +1002,8 @@ __device__ __forceinline__ void mma_role_block(const TcArgs &g, Control *ctl, ui
         __syncwarp();
         if (++b == g.n_acc) { b = 0; acc_phase ^= 1u; }
     }
-    if (leader) commit_pair_here(smem_u32(&ctl->drain[0]));
-    mbar_wait_quiet(smem_u32(&ctl->drain[0]), 0, g.wait_ns);
+    if (leader) commit_pair_here(smem_u32(&ctl->drain[who]));
+    mbar_wait_quiet(smem_u32(&ctl->drain[who]), 0, g.wait_ns);
 }
 
 // Position tiles of 16-byte columns (resident filters): the packed bytes of all positions that any tap
@@ -1257,7 +1263,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 if (KK == 4 && g.planes && g.chunks_per_tap * KK > 32)
                     mma_role_planes<KK, true>(g, ctl, tmem_base, stage0, who);
                 else if (g.planes) mma_role_planes<KK, false>(g, ctl, tmem_base, stage0, who);
-                else if (KK == 4 && g.block && g.resident) mma_role_block<KK>(g, ctl, tmem_base, stage0);
+                else if (KK == 4 && g.block && g.resident) mma_role_block<KK>(g, ctl, tmem_base, stage0, who);
                 else if (g.resident) mma_role_resident<KK>(g, ctl, tmem_base, stage0);
                 else if (g.halo) mma_role_halo<KK>(g, ctl, tmem_base, stage0, who);
                 else mma_role<KK, PAIR>(g, ctl, tmem_base, stage0, who);
@@ -1523,6 +1529,15 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         } else {
             g.issuers = 1;
             g.block = block_fits(n_tile);
+            // Two issuers where the taps of a filter row keep the tensor pipe for less time than one needs for them,
+            // about 500 cycles and 30 an instruction. One over two, 57 layers of 2 x 2 to 4 x 4 filters on 64 to
+            // 512 channels, 1 to 6 tiles a pair, on one stream and among others:
+            //   up to 800 cycles, three rows and more, or 96 filters and fewer  1.00 to 1.15   0.99 to 1.15
+            //   up to 800 cycles, two rows, 128 and more                        0.95 to 1.03   0.96 to 1.03
+            //   more                                                            0.98 to 1.00   0.99 to 1.00
+            // conv4 on 256 images 40.1 -> 35.6 us on one stream, 37 -> 33 among others; conv1 has
+            // three rows of 144 cycles.
+            if (g.block && g.tap_kw * kk * n_tile / 2 <= 800 && (g.kh > 2 || n_tile <= 96)) g.issuers = 2;
             g.halo = g.block ? block_rows : (int)halo_rows;
             g.n_stages = g.block ? groups : 2;
             if (g.block) tile_slot = block_slot;
@@ -1557,7 +1572,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         g.n_stages = (int)(room / g.stage_bytes);
         if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
     }
-    if (g.issuers == 2 && g.n_stages > 2 && !g.planes) g.n_stages &= ~1;
+    if (g.issuers == 2 && g.n_stages > 2 && !g.resident) g.n_stages &= ~1;
     if (g.n_stages < 2) return cudaErrorNotSupported;
     CUtensorMap map_a, map_b;
     // a position's row is tap_bytes long but only icp further than the one before it
