@@ -34,8 +34,8 @@ def launches(tmp_path_factory):
 
 def test_which_layers_have_half_the_width(launches):
     tiles = {name: got["n_tiles"] for name, got in launches.items()}
-    assert [tiles[c[0]] for c in gpu.HALVED] == [2, 2, 6, 2, 2]
-    assert [tiles[c[0]] for c in gpu.WHOLE] == [1, 1, 1, 1, 1, 1, 3, 1, 1]
+    assert [tiles[c[0]] for c in gpu.HALVED] == [2, 2, 2, 2, 6, 2, 2]
+    assert [tiles[c[0]] for c in gpu.WHOLE] == [1, 1, 1, 1, 1, 3, 1, 1]
     assert (tiles["alexnet_conv4"], tiles["alexnet_conv3"], tiles["vgg"]) == (2, 2, 2)
     halved = [launches[c[0]] for c in gpu.HALVED] + [launches["alexnet_conv4"]]
     # resident, with a tile for all filter rows and a barrier for each filter row's and chunk's filters

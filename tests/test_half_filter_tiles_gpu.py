@@ -19,6 +19,8 @@ NHWC = (0, 0, 1)
 HALVED = [
     cases._c("256_filters_odd_rows", 1700, 256, 288, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("part_padding", 1601, 250, 270, 4, 4, 3, 3, ph=1, pw=1, fmt=NHWC),
+    cases._c("odd_rows_192_filters", 2400, 192, 350, 4, 3, 3, 3, ph=1, pw=1),
+    cases._c("even_rows_192_filters", 1601, 192, 384, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("six_tiles_of_128", 700, 768, 290, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("even_rows_three_tiles_a_pair", 2200, 256, 512, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("odd_rows_four_tiles_a_pair", 3000, 256, 288, 4, 4, 3, 3, ph=1, pw=1),
@@ -26,8 +28,7 @@ HALVED = [
 WHOLE = [
     cases._c("128_filters", 3100, 128, 480, 4, 4, 4, 3, ph=1, pw=1),
     cases._c("even_rows_four_tiles_a_pair", 2400, 256, 320, 4, 4, 3, 3, ph=1, pw=1),
-    cases._c("odd_rows_192_filters", 2400, 192, 350, 4, 3, 3, 3, ph=1, pw=1),
-    cases._c("even_rows_192_filters", 1601, 192, 384, 4, 4, 3, 3, ph=1, pw=1),
+    cases._c("even_rows_192_filters_four_tiles", 3200, 192, 384, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("two_filter_rows", 1601, 256, 608, 4, 4, 2, 3, ph=1, pw=1),
     cases._c("half_does_not_fit", 1200, 256, 544, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("a_round_more_for_one_tile_a_pair", 500, 768, 290, 4, 4, 3, 3, ph=1, pw=1),

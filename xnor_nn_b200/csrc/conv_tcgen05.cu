@@ -1379,26 +1379,25 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     };
     // A tile of half the filters, if that half stays in shared memory beside such tiles (below) and the whole
     // would not: its filters are loaded once instead of for each position tile, which pays for reading the
-    // positions twice where the accumulators of the whole share columns and
+    // positions twice where
     // - a position's row ends inside a 32-byte sector, or
-    // - a pair has three tiles or fewer.
-    // Whole over half, 300 layers of 3 x 3 filters on 6 to 32 pixels, 270 to 512 channels, up to 7 tiles a pair of
-    // the whole, a pass on one stream and among others:
-    //   256 filters, such rows, up to three tiles  1.02 to 1.24, mean 1.12   0.99 to 1.09, mean 1.03
-    //   256 filters, such rows, more tiles         1.02 to 1.18, mean 1.10   1.00 to 1.09, mean 1.04
-    //   256 filters, others, up to three tiles     0.99 to 1.15, mean 1.05   0.94 to 1.04, mean 0.99
-    //   256 filters, others, more tiles            0.96 to 1.06, mean 1.01   0.96 to 0.99, mean 0.97
-    //   192 filters                                0.90 to 1.12, mean 0.99   0.85 to 0.99, mean 0.94
-    // conv4 on 256 images, of the third kind: 41.6 -> 40.3 us on one stream, 39.0 -> 37.7 among others. (Layers
-    // whose whole stays resident: half of 256 filters 1.06 with up to 1.4 tiles a pair on one stream, 0.95 to
-    // 1.05 among others; of 192 and 128 0.87 to 1.06.)
+    // - a pair has three tiles or fewer, or a tile keeps the tensor pipe for less than 5000 cycles (the others
+    //   have eight epilogue warps).
+    // Whole over half, 3 x 3 filters on 6 to 40 pixels, 288 to 512 channels, the halves with two issuers, a pass on
+    // one stream and among others:
+    //   256 filters, 3 to 6 tiles a pair  15 layers  1.05 to 1.15, mean 1.09   1.02 to 1.12, mean 1.05
+    //   192 filters, 1 to 6 tiles a pair  42 layers  1.05 to 1.24, mean 1.13   1.01 to 1.17, mean 1.08
+    // conv4 on 256 images 41.6 -> 35.6 us on one stream, 39.0 -> 35.6 among others. (Half of a whole that stays
+    // resident: of 256 filters with up to 1.4 tiles a pair 1.08 and 1.02, with more 0.96 and 0.93; of 192 1.02
+    // and 0.95; of 128 0.92 and 0.90.)
     int n_tile = p.n_tile;
     const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
     const int half_grid = sms / 2 - sms / 2 % half_tiles;
-    if (pair && !next && !p.cat && g.kh >= 3 && n_tile > kAccStep && n_tile % 64 == 0 && row_offsets_ok &&
+    if (pair && !next && !p.cat && g.kh >= 3 && n_tile >= 192 && n_tile % 64 == 0 && row_offsets_ok &&
         !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
         div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, sms / 2) &&
-        (p.row_bytes % 32 != 0 || div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3))
+        (p.row_bytes % 32 != 0 || div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3 ||
+         (long)steps * n_tile / 2 < 5000))
         n_tile /= 2;
     const int b_rows = pair ? n_tile / 2 : n_tile;  // filter rows a CTA loads per stage
     g.n_tiles = p.ocp16 / n_tile;
