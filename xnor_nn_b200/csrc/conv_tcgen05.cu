@@ -1387,7 +1387,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // one stream and among others:
     //   256 filters, 3 to 6 tiles a pair  15 layers  1.05 to 1.15, mean 1.09   1.02 to 1.12, mean 1.05
     //   192 filters, 1 to 6 tiles a pair  42 layers  1.05 to 1.24, mean 1.13   1.01 to 1.17, mean 1.08
-    // conv4 on 256 images 41.6 -> 35.6 us on one stream, 39.0 -> 35.6 among others. (Half of a whole that stays
+    // conv4 on 256 images 41.6 -> 35.6 us on one stream, 39 -> 36 among others. (Half of a whole that stays
     // resident: of 256 filters with up to 1.4 tiles a pair 1.08 and 1.02, with more 0.96 and 0.93; of 192 1.02
     // and 0.95; of 128 0.92 and 0.90.)
     int n_tile = p.n_tile;
@@ -1534,7 +1534,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
             //   up to 800 cycles, three rows and more, or 96 filters and fewer  1.00 to 1.15   0.99 to 1.15
             //   up to 800 cycles, two rows, 128 and more                        0.95 to 1.03   0.96 to 1.03
             //   more                                                            0.98 to 1.00   0.99 to 1.00
-            // conv4 on 256 images 40.1 -> 35.6 us on one stream, 37 -> 33 among others; conv1 has
+            // conv4 on 256 images 40.1 -> 35.6 us on one stream, 37.5 -> 36 among others; conv1 has
             // three rows of 144 cycles.
             if (g.block && g.tap_kw * kk * n_tile / 2 <= 800 && (g.kh > 2 || n_tile <= 96)) g.issuers = 2;
             g.halo = g.block ? block_rows : (int)halo_rows;
