@@ -26,6 +26,18 @@ ONE_LAUNCH = [
     cases._c("channels_last", 3, 44, 92, 10, 11, 3, 3, ph=1, pw=1, fmt=CL),
     cases._c("channels_last_odd", 3, 43, 91, 10, 11, 3, 3, ph=1, pw=1, fmt=CL),
 ]
+# The height of the result follows from the padding of the width: blocks whose windows lie below the image
+# altogether, which read nothing (test_map_bands_cpu.py walks what every block reads).
+BELOW_THE_IMAGE = [
+    cases._c("1x3_same", 8, 24, 64, 14, 14, 1, 3, ph=0, pw=1),
+    cases._c("1x7_same", 8, 24, 64, 14, 14, 1, 7, ph=0, pw=3),
+    cases._c("1x5_same", 4, 24, 64, 14, 14, 1, 5, ph=0, pw=2),
+    cases._c("1x3_one_image_512_channels", 1, 24, 512, 56, 56, 1, 3, ph=0, pw=1),
+    cases._c("3x3_no_rows_of_padding", 4, 24, 64, 9, 9, 3, 3, ph=0, pw=2),
+    cases._c("1x1_padding_2", 2, 24, 64, 10, 10, 1, 1, ph=2, pw=2),
+    cases._c("1x5_100x100", 1, 24, 64, 100, 100, 1, 5, ph=0, pw=2),
+    cases._c("1x3_channels_last", 8, 24, 64, 14, 14, 1, 3, ph=0, pw=1, fmt=CL),
+]
 TWO_LAUNCHES = [
     cases._c("72_taps", 2, 16, 20, 14, 15, 9, 8, ph=4, pw=4),
     cases._c("over_16_megabytes", 65, 16, 64, 32, 32, 3, 3, ph=1, pw=1),
@@ -54,7 +66,7 @@ def _run(oracle, case, launches):
     conv.close()
 
 
-@pytest.mark.parametrize("case", ONE_LAUNCH, ids=[c[0] for c in ONE_LAUNCH])
+@pytest.mark.parametrize("case", ONE_LAUNCH + BELOW_THE_IMAGE, ids=[c[0] for c in ONE_LAUNCH + BELOW_THE_IMAGE])
 def test_one_launch(oracle, case):
     _run(oracle, case, 1)
 

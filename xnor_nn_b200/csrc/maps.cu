@@ -8,6 +8,7 @@
 // others, a microsecond of it less work in the caller, and 16.5 instead of 17.0 on one stream; 15 images of 304
 // channels, 9 x 9, filters of 5 x 5, 9.9 instead of 13.0 among others, 24.6 and 24.4 on one stream.
 #include "kernels.cuh"
+#include "map_bands.cuh"
 #include "pixel_tasks.cuh"
 #include "tc_ptx.cuh"
 
@@ -15,31 +16,8 @@ namespace xb200 {
 
 namespace {
 
+using namespace bands;
 using namespace tasks;
-
-constexpr int kWarps = 8, kThreads = 32 * kWarps;
-constexpr int kMaxGroups = 32, kMaxTasks = 8 * kWarps, kTileFloats = 8 * 1024;
-// More source than this keeps the GPU busy for longer than a launch takes the host, and bands read what
-// their windows share more than once.
-constexpr long kMaxBytes = 16L << 20;
-
-struct MapArgs {
-    const float *src;
-    float *a, *k;
-    int *error;
-    unsigned long long wait_ns;
-    int turn_step;             // 1, 0 in a self-test (ConvSelfTest)
-    float inv_ic, inv_khw;
-    int ic, hw, ih, iw, vec;
-    int oh, ow, kh, kw, sh, sw, ph, pw;
-    int rows, bands;           // output rows of a block, blocks of an image
-    int lines, span, columns;  // rows and columns of A that a block's windows see; tasks of a group
-    FastDiv by_hw, by_iw, by_ow;
-};
-
-struct Band {
-    int first, last, groups, tasks;
-};
 
 template <bool NHWC>
 __global__ void __launch_bounds__(kThreads) maps_kernel(const MapArgs g) {
@@ -51,21 +29,13 @@ __global__ void __launch_bounds__(kThreads) maps_kernel(const MapArgs g) {
     __shared__ unsigned long long turn[kMaxTasks];
     __shared__ int abort_flag;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    const int n = (int)blockIdx.x / g.bands, band = (int)blockIdx.x - n * g.bands;
-    const int oy0 = band * g.rows, y0 = oy0 * g.sh - g.ph;
-    const int own0 = oy0 * g.sh, own1 = band + 1 < g.bands ? own0 + g.rows * g.sh : g.ih;
-    const int lo = max(0, y0), hi = min(g.ih, max(y0 + g.lines, own1));
+    const Band b = band_of(g, (int)blockIdx.x);
     for (int i = threadIdx.x; i < g.lines * g.span; i += kThreads) tile[i] = 0.f;
     if (threadIdx.x < kMaxTasks) tc::mbar_init(tc::smem_u32(&turn[threadIdx.x]), 1);
     if (threadIdx.x == 0) abort_flag = 0;
     dependency_release();
     __syncthreads();
     dependency_wait();
-    Band b;
-    b.first = n * g.hw + lo * g.iw;
-    b.last = n * g.hw + max(hi, lo) * g.iw;
-    b.groups = max(1, (b.last - b.first + 31) >> 5);
-    b.tasks = b.groups * g.columns;
     for (int t = warp; t < b.tasks; t += kWarps) {
         const int col = t / b.groups, gr = t - col * b.groups;
         const int nc = min(32, g.ic - 32 * col);
@@ -85,68 +55,22 @@ __global__ void __launch_bounds__(kThreads) maps_kernel(const MapArgs g) {
             __syncwarp();
             if (lane == 0 && g.turn_step) tc::mbar_arrive(tc::smem_u32(&turn[t + b.groups]));
         } else if (px < b.last) {
-            const int r = px - n * g.hw, y = (int)g.by_iw((uint32_t)r), x = r - y * g.iw;
-            if (y >= own0 && y < own1) g.a[px] = acc;
-            if (y - y0 < g.lines && x + g.pw < g.span)
-                tile[(y - y0) * g.span + x + g.pw] = __fmul_rn(acc, g.inv_khw);
+            const int r = px - b.n * g.hw, y = (int)g.by_iw((uint32_t)r), x = r - y * g.iw;
+            if (y >= b.own0 && y < b.own1) g.a[px] = acc;
+            if (y - b.y0 < g.lines && x + g.pw < g.span)
+                tile[(y - b.y0) * g.span + x + g.pw] = __fmul_rn(acc, g.inv_khw);
         }
     }
     __syncthreads();
     if (abort_flag) return;
-    const int n_out = min(g.rows, g.oh - oy0) * g.ow;
+    const int n_out = min(g.rows, g.oh - b.oy0) * g.ow;
     for (int o = threadIdx.x; o < n_out; o += kThreads) {
         const int r = (int)g.by_ow((uint32_t)o), x = o - r * g.ow;
         const float *row = tile + r * g.sh * g.span + x * g.sw;
         float acc = 0.f;
         for (int i = 0; i < g.kh; i++, row += g.span)
             for (int j = 0; j < g.kw; j++) acc = __fadd_rn(acc, row[j]);
-        g.k[((long)n * g.oh + oy0 + r) * g.ow + x] = acc;
-    }
-}
-
-// What the launch takes, to a sixth (fitted to 78 layers of more than 5.9 us): a block's warps walk its tasks
-// one after the other, and all blocks share the SMs. Two launches take a host 5.7 us, most of which passes on
-// several streams hide. Over 285 layers (drawn from 1 to 256 images, 1 to 512 channels, 6 to 227 pixels, up to
-// 16 MB), the three upstream calls with two launches here over those with one: 1.02 on one stream and 1.14
-// among others if all take one, 1.035 and 1.14 with this rule; the 48 that it takes out 0.90 and 1.005 (19
-// images of 464 channels, 17 x 17, filters of 5 x 5: 44.6 and 60.6 us on one stream, calculate_k alone 7.0 and
-// 18.8).
-double launch_us(long blocks, long tasks, long outputs, int taps) {
-    return 3.6 + 0.58 * (double)(blocks * tasks) / (8.0 * sm_count()) + 0.74 * (double)((tasks + 7) / 8) +
-           0.58 * (double)((outputs + kThreads - 1) / kThreads) * taps / 25;
-}
-
-// Bands: as tall as leaves a block per SM, and at least so tall that most of what a band reads is its own.
-bool maps_shape(const Plan &p, MapArgs *g) {
-    if (p.mb < 1 || p.oh < 1 || p.ow < 1 || p.ic < 1 || p.ih < 1 || p.iw < 1) return false;
-    if (4L * p.mb * p.ic * p.ih * p.iw > kMaxBytes) return false;
-    if (p.sh < 1 || p.sw < 1 || p.ph < 0 || p.pw < 0 || p.kh < 1 || p.kw < 1) return false;
-    if ((long)p.kh * p.kw > 64 || (long)p.oh * p.ow > 1 << 20) return false;
-    g->columns = div_up_i(p.ic, 32);
-    const long span = (long)(p.ow - 1) * p.sw + p.kw;
-    int rows = (int)((long)p.mb * p.oh / sm_count());
-    if (rows < p.kh - 1) rows = p.kh - 1;
-    if (rows < 1) rows = 1;
-    if (rows > p.oh) rows = p.oh;
-    for (;; rows--) {
-        const long lines = (long)(rows - 1) * p.sh + p.kh;
-        // input rows of a band, the rows below the last window with the last band
-        const int bands = div_up_i(p.oh, rows);
-        const long tail = p.ih - (long)(bands - 1) * rows * p.sh + p.ph;
-        const long reach = (long)rows * p.sh + p.ph;
-        long most = lines > reach ? lines : reach;
-        if (tail > most) most = tail;
-        if (most > p.ih) most = p.ih;
-        const long groups = (most * p.iw + 31) / 32;
-        if (groups <= kMaxGroups && groups * g->columns <= kMaxTasks && lines * span <= kTileFloats) {
-            g->rows = rows;
-            g->bands = bands;
-            g->lines = (int)lines;
-            g->span = (int)span;
-            return (long)p.mb * bands < 1L << 30 &&
-                   launch_us((long)p.mb * bands, groups * g->columns, (long)rows * p.ow, p.kh * p.kw) <= 8.5;
-        }
-        if (rows == 1) return false;
+        g.k[((long)b.n * g.oh + b.oy0 + r) * g.ow + x] = acc;
     }
 }
 

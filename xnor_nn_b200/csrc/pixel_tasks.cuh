@@ -8,6 +8,15 @@
 namespace xb200 {
 namespace tasks {
 
+// The pixel that lane `lane` reads of group `group` of a tile's pixels first .. last, channels-first: a lane behind
+// the last pixel reads that one, which has to be a pixel of the source (the first one serves a tile of none
+// in front of all).
+__host__ __device__ inline int lane_pixel(int first, int last, int group, int lane) {
+    const int px = first + 32 * group + lane < last ? first + 32 * group + lane : last - 1;
+    return px < 0 ? 0 : px;
+}
+
+#ifdef __CUDACC__
 // 32 channels of 32 pixels, channels-last: eight lanes read a pixel's channels, four each (with 16-byte
 // loads where they are aligned) and four pixels at a time, and an 8 x 8 transposition of those quadruples
 // leaves a lane with all channels of pixel 4 (lane % 8) + lane / 8.
@@ -63,11 +72,11 @@ __device__ __forceinline__ void load_task(const Args &g, const Tile &tile, int t
         }
         return;
     }
-    // A lane behind the last pixel reads that one, and what becomes of it is not used. With a path of their own
-    // such lanes took their warp through the loads twice: with one path, and no masks on full columns, passes of
-    // AlexNet conv4 in one launch (conv_whole.cu) on one image 11.1 -> 10.0 us on one stream, on 32 images 16.4 ->
-    // 15.6 and among others 5.97 -> 5.62.
-    const unsigned px = (unsigned)max(min(tile.first + 32 * gr + lane, tile.last - 1), 0);
+    // What becomes of a lane without a pixel is not used. With a path of their own such lanes took their warp
+    // through the loads twice: with one path, and no masks on full columns, passes of AlexNet conv4 in one launch
+    // (conv_whole.cu) on one image 11.1 -> 10.0 us on one stream, on 32 images 16.4 -> 15.6 and among others
+    // 5.97 -> 5.62.
+    const unsigned px = (unsigned)lane_pixel(tile.first, tile.last, gr, lane);
     // an address is a warp-uniform channel plane and a lane's 32-bit offset into it (the host checks
     // the range)
     const unsigned n = g.by_hw(px), r = px - n * g.hw;
@@ -100,6 +109,7 @@ __device__ __forceinline__ float sum_task(const float *v, int nc, float acc) {
     }
     return acc;
 }
+#endif
 
 }  // namespace tasks
 }  // namespace xb200
