@@ -101,3 +101,32 @@ def test_result_over_the_source():
         assert torch.equal(dst, want)
     assert counts == [1, 2, 2]
     conv.close()
+
+
+@pytest.mark.parametrize("between", [False, True], ids=["pass", "calculate_k_and_pass"])
+def test_new_weights_before_every_pass(between):
+    """Filters packed anew and the pass that reads them follow each other on the stream with nothing waited for in
+    between, alone and with a kernel that lets its successor start early: every pass has its own filters."""
+    torch = pytest.importorskip("torch")
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    conv = xb.Convolution(xb.ALGORITHM_BCAST, xb.NCHW, xb.OIHW, xb.NCHW, 2, 64, 96, 9, 9, 3, 3, 1, 1, 1, 1)
+    x = torch.randn(2, 96, 9, 9, generator=gen, device="cuda")
+    weights = [torch.randn(64, 96, 3, 3, generator=gen, device="cuda") for _ in range(2)]
+    conv.set_stream(torch.cuda.current_stream().cuda_stream or 1)  # 1: the legacy default stream
+    want = [torch.empty(conv.out_shape, device="cuda") for _ in weights]
+    for w, y in zip(weights, want):
+        conv.change_weights(w)
+        torch.cuda.synchronize()
+        conv.forward(x, y)
+        torch.cuda.synchronize()
+    assert not torch.equal(*want)
+    got = torch.empty((200, *conv.out_shape), device="cuda")
+    before = xb.kernel_launches()
+    for i in range(200):
+        conv.change_weights(weights[i % 2])
+        if between:
+            assert conv.execute("calculate_k", src=x) == xb.SUCCESS
+        conv.forward(x, got[i])
+    assert xb.kernel_launches() - before == 200 * (3 if between else 2)
+    assert all(torch.equal(got[i], want[i % 2]) for i in range(200))
+    conv.close()

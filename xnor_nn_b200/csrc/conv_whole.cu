@@ -314,9 +314,10 @@ conv_whole_kernel(const __grid_constant__ CUtensorMap map_b, const WholeArgs g) 
     const uint32_t b0 = smem_u32(base) + g.b_off;
     const int steps = g.taps * g.chunks;
     if (warp == 0) {
-        // ---- filter tiles ---- (not behind dependency_wait(): the kernels that write them let no dependent start
-        // early, so that whatever started before this grid came after them)
+        // ---- filter tiles ---- (the kernel before may have written them; the workers waited for it before the
+        // barrier above, so this returns at once)
         const bool leader = elect_one();
+        dependency_wait();
         int stage = 0, sent = 0, tap = 0, chunk = 0;
         uint32_t phase = 0;
         bool ok = true;

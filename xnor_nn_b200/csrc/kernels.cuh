@@ -17,9 +17,10 @@ inline void note_launch(int n = 1) { g_kernel_launches.fetch_add(n, std::memory_
 // Launch with programmatic stream serialisation: the grid may be scheduled while the previous
 // kernel of the stream is still draining, so that its set-up (and the launch latency itself)
 // runs under the predecessor's tail. Kernels launched this way call dependency_wait() before
-// they touch anything an earlier kernel may have written or may still be reading. The
-// tensor-core convolution and the tiled binarizer are launched like this (measured: 2-3 us per
-// forward pass for the convolution, another 0.8 us for the binarizer in back-to-back passes).
+// they touch anything an earlier kernel may have written (packed filters among it: that the kernel which
+// writes them has ended does not make them visible, the wait does) or may still be reading. All kernels of a
+// pass are launched like this (measured: 2-3 us per forward pass for the convolution, another 0.8 us for the
+// tiled binarizer in back-to-back passes); those that pack weights are not.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                      cudaStream_t s, int cluster, Args... args) {
