@@ -1,5 +1,6 @@
 // What the position-tile launcher hands the driver, without a GPU: its object files are linked against
-// stand-ins for the few CUDA runtime calls it makes (a device of 148 SMs and 74 pairs of them). For
+// stand-ins for the few CUDA runtime calls it makes (a device of 148 SMs and 74 pairs of them, or
+// as many pairs as the variable PAIRS says). For
 // each layer on the command line (mb,oc,ic,ih,iw,kh,kw,sh,sw,ph,pw) one line of JSON: the tensor
 // maps it asked for, the launch, and the parameters that say which form of the kernel runs.
 #include <cuda.h>
@@ -55,7 +56,8 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *, const cudaLaunchConfig_t *) {
-    *n = 74;
+    const char *pairs = getenv("PAIRS");
+    *n = pairs ? atoi(pairs) : 74;
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **args) {

@@ -17,7 +17,7 @@ LAYERS = gpu.HALVED + gpu.WHOLE + [
 
 
 @pytest.fixture(scope="module")
-def launches(tmp_path_factory):
+def launch(tmp_path_factory):
     build.build()
     exe = str(tmp_path_factory.mktemp("tile_launch") / "tile_launch")
     objs = [os.path.join(build.OBJ, n + ".o") for n in ("conv_tcgen05.cu", "plan.cpp", "tensormap.cpp")]
@@ -27,9 +27,17 @@ def launches(tmp_path_factory):
         objs + ["-o", exe])
     keys = ("mb", "oc", "ic", "ih", "iw", "kh", "kw", "sh", "sw", "ph", "pw")
     env = {k: v for k, v in os.environ.items() if k != "XNOR_NN_B200_KERNEL"}
-    out = subprocess.check_output([exe] + [",".join(str(c[1][k]) for k in keys) for c in LAYERS], text=True,
-                                  env=env).splitlines()
-    return dict(zip([c[0] for c in LAYERS], [json.loads(line) for line in out]))
+
+    def run(**more):
+        out = subprocess.check_output([exe] + [",".join(str(c[1][k]) for k in keys) for c in LAYERS], text=True,
+                                      env={**env, **more}).splitlines()
+        return dict(zip([c[0] for c in LAYERS], [json.loads(line) for line in out]))
+    return run
+
+
+@pytest.fixture(scope="module")
+def launches(launch):
+    return launch()
 
 
 def test_which_layers_have_half_the_width(launches):
@@ -43,3 +51,22 @@ def test_which_layers_have_half_the_width(launches):
     assert {g["m_tiles"] % 2 for g in halved} == {0, 1} and not any(g["shared_cols"] for g in halved)
     whole = [launches[c[0]] for c in gpu.WHOLE if c[0] != "whole_fits"] + [launches["vgg"]]
     assert all(g["pair"] and not g["resident"] for g in whole) and launches["whole_fits"]["resident"]
+
+
+def test_halves_are_resident_on_fewer_pairs(launch):
+    """Where fewer pairs than half the SMs can be resident, a layer is halved only if each of those that run keeps to
+    one filter tile: a halved layer that streams its filters would read its positions twice for nothing."""
+    names = [c[0] for c in gpu.HALVED] + ["alexnet_conv4"]
+    halved = whole = 0
+    for pairs in range(1, 75):
+        got = launch(PAIRS=str(pairs))
+        for name in names:
+            g = got[name]
+            assert g["served"] and g["pair"] and g["grid"] <= 2 * pairs
+            # these have filter tiles of 192 or 256, halved 96 or 128, and 2, 2, 2, 2, 6, 2, 2 and 2 of the latter
+            if g["n_tiles"] == (6 if name == "six_tiles_of_128" else 2):
+                assert g["resident"], (pairs, name, g)
+                halved += 1
+            else:
+                whole += 1
+    assert halved > 200 and whole > 100, (halved, whole)  # the line of three tiles a pair moves too

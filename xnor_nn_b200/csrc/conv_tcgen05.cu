@@ -1299,6 +1299,50 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 
 // ---- host side ---------------------------------------------------------------------------------
 
+using Kernel = void (*)(CUtensorMap, CUtensorMap, TcArgs);
+constexpr int kSingle = 0, kPair = 1, kPairEmits = 2, kPairFew = 3;  // forms; by MMAs of a chunk 4, 2 and 1
+const Kernel kKernels[3][4] = {
+    {conv_tcgen05_kernel<4, false, kEpiWarps, false>, conv_tcgen05_kernel<4, true, kEpiWarps, false>,
+     conv_tcgen05_kernel<4, true, kEpiWarps, true>, conv_tcgen05_kernel<4, true, kFewEpiWarps, false>},
+    {conv_tcgen05_kernel<2, false, kEpiWarps, false>, conv_tcgen05_kernel<2, true, kEpiWarps, false>,
+     conv_tcgen05_kernel<2, true, kEpiWarps, true>, nullptr},
+    {conv_tcgen05_kernel<1, false, kEpiWarps, false>, conv_tcgen05_kernel<1, true, kEpiWarps, false>,
+     conv_tcgen05_kernel<1, true, kEpiWarps, true>, nullptr}};
+
+// The opt-in to large dynamic shared memory, once per device and kernel.
+cudaError_t opt_in(int d, int per_stage, int form) {
+    static std::atomic<bool> opted_in[64][3][4];
+    std::atomic<bool> &done = opted_in[d][per_stage][form];
+    if (done.load(std::memory_order_acquire)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kKernels[per_stage][form],
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess) done.store(true, std::memory_order_release);
+    return e;
+}
+
+// CTA pairs that can be resident together, asked once per device (a CTA has an SM to itself in every form).
+int resident_pairs(int d, int sms) {
+    static std::atomic<int> pair_count[64];
+    int slots = pair_count[d].load(std::memory_order_relaxed);
+    if (slots) return slots;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (sms / 2));
+    cfg.blockDim = dim3(threads_of(kEpiWarps));
+    cfg.dynamicSmemBytes = 227 * 1024 - 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (opt_in(d, 0, kPair) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&slots, kKernels[0][kPair], &cfg) != cudaSuccess || slots <= 0) {
+        (void)cudaGetLastError();
+        slots = sms / 2;
+    }
+    pair_count[d].store(slots, std::memory_order_relaxed);
+    return slots;
+}
+
 }  // namespace
 
 cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *bin_w,
@@ -1309,7 +1353,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const int m_tiles = (int)((p.q_total + BM - 1) / BM);
     int dev = 0;
     cudaGetDevice(&dev);
-    static std::atomic<int> sm_count[64], pair_count[64];
+    static std::atomic<int> sm_count[64];
     const int d = dev & 63;
     int sms = sm_count[d].load(std::memory_order_relaxed);
     if (!sms) {
@@ -1392,11 +1436,13 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // and 0.95; of 128 0.92 and 0.90.)
     int n_tile = p.n_tile;
     const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
-    const int half_grid = sms / 2 - sms / 2 % half_tiles;
+    const int slots = pair ? resident_pairs(d, sms) : sms;
+    const int half_grid = slots - slots % half_tiles;  // pairs that keep to one filter tile, as below
     if (pair && !next && !p.cat && g.kh >= 3 && n_tile >= 192 && n_tile % 64 == 0 && row_offsets_ok &&
         !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
-        div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, sms / 2) &&
-        (p.row_bytes % 32 != 0 || div_up_i(pair_units * half_tiles / 2, sms / 2) <= 3 ||
+        pair_units * half_tiles > slots &&
+        div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, slots) &&
+        (p.row_bytes % 32 != 0 || div_up_i(pair_units * half_tiles / 2, slots) <= 3 ||
          (long)steps * n_tile / 2 < 5000))
         n_tile /= 2;
     const int b_rows = pair ? n_tile / 2 : n_tile;  // filter rows a CTA loads per stage
@@ -1442,46 +1488,12 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const int pair_tiles = div_up_i(((m_tiles + 1) / 2) * g.n_tiles, sms / 2);
     const bool few = pair && !next && kk == 4 && tile_cycles >= 5000 && pair_tiles >= 4;
     const int epi = few ? kFewEpiWarps : kEpiWarps;
-    const int per_stage = kk == 4 ? 0 : kk == 2 ? 1 : 2, form = few ? 3 : !pair ? 0 : next ? 2 : 1;
-    using Kernel = void (*)(CUtensorMap, CUtensorMap, TcArgs);
-    static const Kernel kernels[3][4] = {
-        {conv_tcgen05_kernel<4, false, kEpiWarps, false>, conv_tcgen05_kernel<4, true, kEpiWarps, false>,
-         conv_tcgen05_kernel<4, true, kEpiWarps, true>, conv_tcgen05_kernel<4, true, kFewEpiWarps, false>},
-        {conv_tcgen05_kernel<2, false, kEpiWarps, false>, conv_tcgen05_kernel<2, true, kEpiWarps, false>,
-         conv_tcgen05_kernel<2, true, kEpiWarps, true>, nullptr},
-        {conv_tcgen05_kernel<1, false, kEpiWarps, false>, conv_tcgen05_kernel<1, true, kEpiWarps, false>,
-         conv_tcgen05_kernel<1, true, kEpiWarps, true>, nullptr}};
-    const Kernel kernel = kernels[per_stage][form];
-    // per device and kernel, once: the opt-in to large dynamic shared memory, the SM count and
-    // the number of CTA pairs that can be resident together
-    static std::atomic<bool> opted_in[64][3][4];
-    std::atomic<bool> &done = opted_in[d][per_stage][form];
-    if (!done.load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return e;
-        done.store(true, std::memory_order_release);
-    }
-    int units = (pair ? (m_tiles + 1) / 2 : m_tiles) * (next ? 1 : g.n_tiles), slots = sms;
-    if (pair) {
-        slots = pair_count[d].load(std::memory_order_relaxed);
-        if (!slots) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(2 * (sms / 2));
-            cfg.blockDim = dim3(threads_of(epi));
-            cfg.dynamicSmemBytes = 227 * 1024 - 1024;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&slots, kernel, &cfg) != cudaSuccess || slots <= 0) {
-                (void)cudaGetLastError();
-                slots = sms / 2;
-            }
-            pair_count[d].store(slots, std::memory_order_relaxed);
-        }
-    }
+    const int per_stage = kk == 4 ? 0 : kk == 2 ? 1 : 2;
+    const int form = few ? kPairFew : !pair ? kSingle : next ? kPairEmits : kPair;
+    const Kernel kernel = kKernels[per_stage][form];
+    const cudaError_t opted = opt_in(d, per_stage, form);
+    if (opted != cudaSuccess) return opted;
+    const int units = (pair ? (m_tiles + 1) / 2 : m_tiles) * (next ? 1 : g.n_tiles);
     int grid = units < slots ? units : slots;
     // Fewer pairs, if that costs no further round, so that each keeps to one filter tile.
     const int one_nt = grid - grid % g.n_tiles;
