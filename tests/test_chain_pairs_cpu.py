@@ -4,6 +4,7 @@ import os
 import subprocess
 
 import test_chain_pairs_gpu as gpu
+import test_shared_accumulator_gpu
 from xnor_nn_b200 import build
 
 MORE = {"conv3": (128, 256, 384, 13, 13, 3, 3, 1, 1), "conv4": (128, 384, 256, 13, 13, 3, 3, 1, 1)}
@@ -38,3 +39,6 @@ def test_which_chained_layers_run_on_pairs(tmp_path):
     assert {g["m_tiles"] % 2 for g in pairs.values()} == {0, 1}
     # one position tile a pair at a time, all of its filter tiles in a row
     assert all(g["grid"] == 2 * min(74, (g["m_tiles"] + 1) // 2) for g in pairs.values())
+    # the test of two issuers on one accumulator repeats each form
+    assert all(pairs[name]["issuers"] == 2 for name in test_shared_accumulator_gpu.CHAINS)
+    assert {form[name] for name in test_shared_accumulator_gpu.CHAINS} == set(form.values())

@@ -3,7 +3,10 @@ conv_tcgen05.cu), whose two issuers take the taps of all rows in turn: an even a
 rows of two taps and of nine, a box of 256 rows, five filter rows, one, three and four chunks, the last one full
 and not, two filter tiles, accumulators that overlap, an odd number of position tiles; and the first layers
 beyond, which have a tile for each filter row. test_streamed_blocks_cpu.py pins which layers take which. Sums and
-K bit for bit against the oracle, floats to the parity contract's 1e-4."""
+K bit for bit against the oracle, floats to the parity contract's 1e-4. A commit that is lost makes a wait run out,
+and the next pass is right."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -46,4 +49,29 @@ def test_against_the_oracle(oracle, case):
         assert np.all(np.abs(dst.cpu().numpy() - want["dst"]) <= 1e-4 * np.abs(want["dst"]))
         assert np.array_equal(conv.forward_sums(), want["sums"])
         assert np.array_equal(conv.read(xb.SLOT_K, np.float32), want["k"])
+    conv.close()
+
+
+@pytest.mark.parametrize("name", ["odd_taps", "five_rows_192_filters", "five_rows_256_filters"])
+def test_lost_commit_times_out_and_the_resources_stay_usable(name):
+    case = next(c for c in BLOCKS + ROWS if c[0] == name)
+    _, d, _, _ = case
+    src, w = cases.make_inputs(case)
+    conv = xb.Convolution(xb.ALGORITHM_BCAST, xb.NCHW, xb.OIHW, xb.NCHW, d["mb"], d["oc"], d["ic"], d["ih"],
+                          d["iw"], d["kh"], d["kw"], d["sh"], d["sw"], d["ph"], d["pw"], w)
+    src = torch.from_numpy(src).cuda()
+    good = torch.zeros(int(np.prod(conv.out_shape)), device="cuda")
+    torch.cuda.synchronize()
+    conv.forward(src, good)
+    conv.synchronize()
+    junk, again = torch.zeros_like(good), torch.zeros_like(good)
+    torch.cuda.synchronize()
+    conv._set(xb.SLOT_USER_DST, junk)
+    st = xb.lib().xnor_nn_b200_selftest_lost_commit(C.byref(conv.c), conv.res, 5)
+    assert st == xb.UNIMPLEMENTED
+    assert "gave up waiting (site " in xb.last_error()
+    conv.synchronize()  # the error word was consumed
+    conv.forward(src, again)
+    conv.synchronize()
+    assert torch.equal(again, good)
     conv.close()

@@ -16,6 +16,7 @@ import test_long_filter_rows_gpu
 import test_long_tiles_gpu
 import test_position_columns_gpu
 import test_resident_filters_gpu
+import test_shared_accumulator_gpu
 import test_streamed_filters_gpu
 from xnor_nn_b200 import build
 
@@ -50,10 +51,11 @@ SIXTEEN_WARPS = [
     cases._c("4224_cycles", 180, 256, 224, 28, 28, 3, 3, ph=1, pw=1),
 ]
 LOST_COMMIT = cases._c("lost_commit", 64, 256, 96, 27, 27, 5, 5, ph=2, pw=2)
+SHARED_ACCUMULATOR = [c for c in test_shared_accumulator_gpu.LAYERS if not c[0].startswith("whole")]
 LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + GPU_COLUMNS + test_position_columns_gpu.ROWS +
           test_resident_filters_gpu.ROWS + [LOST_COMMIT] + test_streamed_filters_gpu.STREAMED +
           test_folded_gpu.FOLDED + test_long_filter_rows_gpu.LONG_ROWS + EIGHT_WARPS + SIXTEEN_WARPS +
-          cases.SHAPE_CASES + [
+          SHARED_ACCUMULATOR + cases.SHAPE_CASES + [
               cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
               cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
 
@@ -144,3 +146,18 @@ def test_gpu_tests_of_resident_rows_reach_them(launches):
 def test_gpu_tests_of_streamed_filters_reach_them(launches):
     got = _of(launches, test_streamed_filters_gpu.STREAMED)
     assert all(g["halo"] and not g["resident"] and g["issuers"] == 2 for g in got)
+
+
+def test_gpu_tests_of_shared_accumulators_reach_each_form_with_two_issuers(launches):
+    got = dict(zip([c[0] for c in SHARED_ACCUMULATOR], _of(launches, SHARED_ACCUMULATOR)))
+    assert all(g["issuers"] == 2 for g in got.values())
+    form = {name: ("pair " if g["pair"] else "single ") +
+                  ("columns" if g["planes"] else "resident" if g["resident"] else "streamed" if g["halo"] else "ring")
+            for name, g in got.items()}
+    assert form == {"pairs_columns": "pair columns", "pairs_resident": "pair resident",
+                    "pairs_streamed": "pair streamed", "pairs_streamed_192_filters": "pair streamed",
+                    "pairs_streamed_a_filter_row_at_a_time": "pair streamed", "single_ctas": "single ring"}
+    # a position tile for all filter rows, but where the name says otherwise
+    assert {name for name, g in got.items() if g["halo"] > 136} == {
+        "pairs_resident", "pairs_streamed", "pairs_streamed_192_filters"}
+    assert (got["pairs_streamed"]["shared_cols"], got["pairs_streamed_192_filters"]["shared_cols"]) == (1, 0)
