@@ -7,6 +7,18 @@ import test_chain_pairs_gpu as gpu
 import test_shared_accumulator_gpu
 from xnor_nn_b200 import build
 
+# Where a pair's longer hand-shakes cost more than its lighter loads save, either side of each line of the rule:
+# the same layer on more images or with more filters
+LINES = {  # name: (layer alone, layer on pairs)
+    "narrow_odd_rows_more_tiles": ((400, 96, 192, 7, 7, 5, 5, 2, 2), (400, 96, 224, 7, 7, 5, 5, 2, 2)),
+    "narrow_odd_rows_fewer_tiles": ((22, 160, 224, 18, 18, 5, 5, 2, 2), (22, 160, 256, 18, 18, 5, 5, 2, 2)),
+    "narrow_odd_rows_tiles": ((28, 96, 384, 23, 23, 5, 5, 2, 2), (60, 96, 384, 23, 23, 5, 5, 2, 2)),
+    "narrow_part_chunk_tiles": ((50, 100, 512, 18, 18, 3, 3, 1, 1), (100, 100, 1024, 18, 18, 3, 3, 1, 1)),
+    "wide_odd_rows_fewer_tiles": ((21, 416, 160, 22, 22, 3, 3, 1, 1), (21, 416, 192, 22, 22, 3, 3, 1, 1)),
+    "wide_part_chunk_more_tiles": ((200, 320, 192, 13, 13, 3, 3, 1, 1), (200, 320, 256, 13, 13, 3, 3, 1, 1)),
+    "wide_part_chunk_fewer_tiles": ((64, 384, 256, 13, 13, 3, 3, 1, 1), (64, 384, 320, 13, 13, 3, 3, 1, 1)),
+    "wide_part_chunk_few_tiles": ((20, 384, 192, 13, 13, 3, 3, 1, 1), (20, 384, 256, 13, 13, 3, 3, 1, 1)),
+}
 MORE = {"conv3": (128, 256, 384, 13, 13, 3, 3, 1, 1), "conv4": (128, 384, 256, 13, 13, 3, 3, 1, 1)}
 
 
@@ -18,12 +30,14 @@ def test_which_chained_layers_run_on_pairs(tmp_path):
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", os.path.join(build.ROOT, "include"), "-I",
                            build.CSRC, "-I", "/usr/local/cuda/include", os.path.join(here, "chain_launch.cpp")] +
                           objs + ["-o", exe])
-    layers = {**gpu.PAIRS, **gpu.SINGLE, **MORE}
+    lines = {(name, on): d for name, both in LINES.items() for on, d in zip((False, True), both)}
+    layers = {**gpu.PAIRS, **gpu.SINGLE, **MORE, **lines}
     order = (0, 2, 1, 3, 4, 5, 6, 7, 8)  # filters before channels
     out = subprocess.check_output([exe] + [",".join(str(d[i]) for i in order) for d in layers.values()],
                                   text=True).splitlines()
     got = dict(zip(layers, [json.loads(line) for line in out]))
     assert all(g["served"] and g["epilogue_warps"] == 16 for g in got.values())
+    assert {key for key in lines if got.pop(key)["pair"] != key[1]} == set()
     pairs = {name: g for name, g in got.items() if g["pair"]}
     assert set(pairs) == set(gpu.PAIRS) | {"conv4"}
     form = {name: "columns" if g["planes"] else "resident" if g["resident"] else "halo" if g["halo"] else "ring"

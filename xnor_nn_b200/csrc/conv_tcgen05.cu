@@ -1382,24 +1382,33 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // against 16.6.
     // Chained layers, whose CTAs carry a pixel's state across all of its filter tiles, store next to nothing,
     // and a CTA alone keeps up with the tensor pipe while its loads are whole: pairs where they are not, which
-    // is where operand rows are an odd number of 16 bytes (each straddles sectors) or the last of several
-    // chunks of a row is partly empty (a stage's hand-over for fewer MMAs), and a position tile is enough work.
-    // Two layers chained, the first one's CTAs alone over pairs, 135 chains of 6 to 30 pixels a side, 32 to 512
-    // channels and 64 to 512 filters, on one stream and among others:
-    //   odd rows, 4000 cycles a tile and more            1.00 to 1.28, mean 1.15   0.99 to 1.26, mean 1.11
-    //   a partial chunk, the same, more tiles than SMs   0.99 to 1.76, mean 1.23   0.91 to 1.73, mean 1.19
-    //   a partial chunk, the same, fewer tiles           0.91 to 1.56, mean 1.08   0.94 to 1.62, mean 1.09
-    //   odd rows, fewer cycles                           0.92 to 1.10, mean 1.00   0.83 to 1.04, mean 0.96
-    //   a partial chunk, fewer cycles                    0.91 to 1.27, mean 1.08   0.80 to 1.19, mean 1.02
-    //   whole chunks and even rows                       0.78 to 1.10, mean 0.95   0.76 to 1.07, mean 0.93
-    // conv3, conv4 and conv5 on 128 images, conv4 on pairs: 56.6 -> 53.4 us on one stream, 43.4 -> 43.1 among
-    // others (on 64 images, conv4 on pairs: 37.8 -> 37.1 and 22.7 -> 23.1).
-    const bool odd_rows = p.icp % 32 != 0;
+    // is where operand rows end inside a 32-byte sector or the last of several chunks of a row is partly empty
+    // (a stage's hand-over for fewer MMAs), and where a position tile is enough work for the pair's longer
+    // hand-shakes: cycles of the tensor pipe for all of its filter tiles. More are asked for with no more position
+    // tiles than SMs, which singles share out at once and without a second round. Two layers chained, the first
+    // one's CTAs alone over pairs, 603 chains of 5 to 34 pixels a side, 16 to 640 channels, 2 x 2 to 7 x 7 filters, 64
+    // to 512 of them, a pass on one stream and among others (narrow: positions of up to 128 bytes):
+    //   on pairs: odd rows, more tiles, narrow, 4000 cycles    107  0.92 to 1.21, mean 1.06   0.91 to 1.20, mean 1.04
+    //     the same, wide                                        58  0.99 to 1.55, mean 1.20   0.97 to 1.56, mean 1.15
+    //     odd rows, fewer tiles, narrow, 8000                   31  0.96 to 1.15, mean 1.05   0.94 to 1.14, mean 1.02
+    //     the same, wide, 5500                                  43  0.98 to 1.46, mean 1.11   0.94 to 1.57, mean 1.09
+    //     part of a chunk, more tiles, 5500                     63  0.96 to 1.19, mean 1.06   0.94 to 1.16, mean 1.04
+    //     the same, fewer, wide, 8000, 6000 below half the SMs  29  0.95 to 1.11, mean 1.01   0.96 to 1.30, mean 1.00
+    //   alone: the same kinds with fewer cycles, 4000 and more 142  0.91 to 1.15, mean 0.98   0.88 to 1.07, mean 0.96
+    //     with fewer than 4000                                  84  0.90 to 1.19, mean 0.96   0.82 to 1.11, mean 0.94
+    //     whole chunks and even rows                            46  0.86 to 1.25, mean 0.96   0.79 to 1.12, mean 0.94
+    // conv3, conv4 and conv5 on 128 images, conv4 on pairs: 57.4 -> 54.4 us on one stream, 43.4 among others
+    // either way.
+    const bool odd_rows = p.row_bytes % 32 != 0, wide = p.row_bytes > 128, more = m_tiles > sms;
     const bool part_chunk = p.n_tile >= 96 && g.chunks_per_tap > 1 && tap_bytes % p.kchunk != 0;
-    const bool pair =
-        p.n_tile % 32 == 0 && m_tiles >= 2 &&
-        (next ? p.kh > 1 && (odd_rows || part_chunk) && (long)steps * p.ocp16 / 2 >= 4000
-              : (long)m_tiles * (p.ocp16 / p.n_tile) > sms);
+    const long chained_cycles = (long)steps * p.ocp16 / 2;
+    const bool chained_pair =
+        p.kh > 1 && (p.icp % 32 != 0 || part_chunk) &&
+        (more     ? chained_cycles >= (odd_rows ? 4000 : 5500)
+         : wide   ? chained_cycles >= (odd_rows ? 5500 : m_tiles > sms / 2 ? 8000 : 6000)
+                  : odd_rows && chained_cycles >= 8000);
+    const bool pair = p.n_tile % 32 == 0 && m_tiles >= 2 &&
+                      (next ? chained_pair : (long)m_tiles * (p.ocp16 / p.n_tile) > sms);
     const int groups = g.kh * g.chunks_per_tap;
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
