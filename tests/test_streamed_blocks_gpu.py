@@ -23,12 +23,14 @@ BLOCKS = [
     cases._c("three_rows_of_nine", 300, 256, 256, 9, 12, 3, 9),
     cases._c("256_rows", 40, 512, 544, 9, 62, 3, 3, ph=1, pw=1),
     cases._c("five_rows_192_filters", 1200, 192, 300, 5, 5, 5, 5, ph=2, pw=2),
+    cases._c("25_taps_odd_rows_160_filters", 1200, 160, 340, 5, 5, 5, 5, ph=2, pw=2),
     cases._c("two_filter_tiles", 1000, 384, 600, 4, 4, 3, 3, ph=1, pw=1),
     cases._c("odd_filters", 1601, 251, 577, 4, 4, 3, 3, ph=1, pw=1),
 ]
 ROWS = [
     cases._c("257_rows", 40, 512, 800, 9, 64, 3, 2),
     cases._c("five_rows_256_filters", 1200, 256, 300, 5, 5, 5, 5, ph=2, pw=2),
+    cases._c("25_taps_odd_rows_192_filters", 1200, 192, 340, 5, 5, 5, 5, ph=2, pw=2),
     cases._c("one_filter_row", 1601, 512, 900, 4, 6, 1, 3),
 ]
 

@@ -1571,14 +1571,21 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     }
     if (halo && !g.resident) {
         // Three position tiles, for all filter rows where they are one box, else for one (136 positions); the
-        // rest of the room for filter tiles. For one over for all, 58 layers of 6 to 32 pixels, 300 to 1024
-        // channels and 192 to 768 filters, on one stream and among others:
-        //   2 x 2 and 3 x 3, tiles of 192 filters  1.02 to 1.08, mean 1.05   1.02 to 1.09, mean 1.05
-        //   2 x 2 and 3 x 3, tiles of 256          0.99 to 1.06, mean 1.02   0.98 to 1.07, mean 1.02
-        //   5 x 5, tiles of 192                    0.99 to 1.06, mean 1.02   1.00 to 1.06, mean 1.02
-        //   5 x 5, tiles of 256                    0.94 to 1.03, mean 0.99   0.99 to 1.02, mean 1.00
-        // The last keep theirs.
-        g.block = g.kh > 1 && p.kchunk == 128 && block_rows <= 256 && (g.kh < 5 || !g.shared_cols);
+        // rest of the room for filter tiles. For one over for all, 160 layers of 6 to 32 pixels, 230 to 1024
+        // channels and 144 to 768 filters, on one stream and among others (odd rows: those that end inside a
+        // 32-byte sector):
+        //   fewer than 25 taps, tiles of up to 192 filters  55  0.98 to 1.16, mean 1.06  1.01 to 1.16, mean 1.06
+        //   the same, of more, up to four filter rows       50  0.94 to 1.08, mean 1.02  0.97 to 1.10, mean 1.02
+        //   the same, five and six filter rows of 256        3  1.00 to 1.05, mean 1.03  1.00 to 1.04, mean 1.02
+        //   25 and 49 taps, even rows, up to 224            19  0.96 to 1.08, mean 1.03  0.96 to 1.06, mean 1.02
+        //   the same, tiles of 256                           6  1.00 to 1.01, mean 1.01  0.99 to 1.02, mean 1.00
+        //   25 and 49 taps, odd rows, fewer than 192         4  1.00 to 1.06, mean 1.03  1.01 to 1.05, mean 1.04
+        //   the same, 192 and more                          23  0.86 to 1.07, mean 0.95  0.91 to 1.04, mean 0.96
+        // The last keep theirs (probably since loads of a chunk that ends inside a sector are slow, as chained layers
+        // show too, and all taps of such a chunk would follow one another). So do 256 filters with five filter rows
+        // and more, for which it is no gain.
+        const bool long_runs = g.taps >= 25 && p.row_bytes % 32 != 0 && n_tile >= 192;
+        g.block = g.kh > 1 && p.kchunk == 128 && block_rows <= 256 && (g.kh < 5 || !g.shared_cols) && !long_runs;
         g.halo = g.block ? block_rows : BM + 8;
         g.n_a_slots = 3;
         g.a_slot_bytes = (uint32_t)(g.halo * p.kchunk + 1023) & ~1023u;
