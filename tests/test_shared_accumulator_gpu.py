@@ -3,7 +3,7 @@ position-tile kernel, on single CTAs and on pairs, beside streamed filters (posi
 all of them), resident ones, columns, and in chained layers. Sums of integers do not depend on the order, but none
 may be lost. Many passes of layers with the fewest and many K chunks, narrow and 256-wide filter tiles, results
 bit for bit the same and the sums those of the oracle. test_tile_launch_cpu.py and test_chain_pairs_cpu.py pin
-that the layers take the forms that they are called after."""
+which form each layer takes: the one it is called after, but for pairs_streamed, whose filters are resident."""
 import numpy as np
 import pytest
 
@@ -23,8 +23,8 @@ LAYERS = [
     cases._c("whole_256_one_chunk", 40, 256, 60, 13, 13, 3, 3, ph=1, pw=1),
     cases._c("whole_256_two_chunks", 30, 256, 384, 13, 13, 3, 3, ph=1, pw=1),
     cases._c("pairs_columns", 75, 256, 96, 27, 27, 3, 3, ph=1, pw=1),
-    cases._c("pairs_resident", 120, 256, 384, 13, 13, 3, 3, ph=1, pw=1),
-    cases._c("pairs_streamed", 120, 256, 640, 13, 13, 3, 3, ph=1, pw=1),
+    cases._c("pairs_streamed", 120, 256, 384, 13, 13, 3, 3, ph=1, pw=1),  # resident: halves of its filter tiles fit
+    cases._c("pairs_streamed_256_filters", 120, 256, 640, 13, 13, 3, 3, ph=1, pw=1),
     cases._c("pairs_streamed_192_filters", 120, 192, 640, 13, 13, 3, 3, ph=1, pw=1),
     cases._c("pairs_streamed_a_filter_row_at_a_time", 1200, 256, 300, 5, 5, 5, 5, ph=2, pw=2),
     cases._c("single_ctas", 120, 144, 300, 13, 13, 3, 3, ph=1, pw=1),

@@ -154,10 +154,10 @@ def test_gpu_tests_of_shared_accumulators_reach_each_form_with_two_issuers(launc
     form = {name: ("pair " if g["pair"] else "single ") +
                   ("columns" if g["planes"] else "resident" if g["resident"] else "streamed" if g["halo"] else "ring")
             for name, g in got.items()}
-    assert form == {"pairs_columns": "pair columns", "pairs_resident": "pair resident",
-                    "pairs_streamed": "pair streamed", "pairs_streamed_192_filters": "pair streamed",
+    assert form == {"pairs_columns": "pair columns", "pairs_streamed": "pair resident",
+                    "pairs_streamed_256_filters": "pair streamed", "pairs_streamed_192_filters": "pair streamed",
                     "pairs_streamed_a_filter_row_at_a_time": "pair streamed", "single_ctas": "single ring"}
     # a position tile for all filter rows, but where the name says otherwise
     assert {name for name, g in got.items() if g["halo"] > 136} == {
-        "pairs_resident", "pairs_streamed", "pairs_streamed_192_filters"}
-    assert (got["pairs_streamed"]["shared_cols"], got["pairs_streamed_192_filters"]["shared_cols"]) == (1, 0)
+        "pairs_streamed", "pairs_streamed_256_filters", "pairs_streamed_192_filters"}
+    assert (got["pairs_streamed_256_filters"]["shared_cols"], got["pairs_streamed_192_filters"]["shared_cols"]) == (1, 0)
