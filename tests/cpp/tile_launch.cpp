@@ -68,10 +68,10 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void 
              "\"grid\": %u, \"smem\": %zu, \"pair\": %s, \"planes\": %d, \"plane_rows\": %d, "
              "\"resident\": %d, \"halo\": %d, \"a_slots\": %d, \"stages\": %d, \"issuers\": %d, "
              "\"groups\": %d, \"kchunk\": %d, \"tap_kw\": %d, \"m_tiles\": %d, \"n_tiles\": %d, "
-             "\"shared_cols\": %d, \"epilogue_warps\": %u",
+             "\"shared_cols\": %d, \"accumulators\": %d, \"epilogue_warps\": %u",
              c->gridDim.x, c->dynamicSmemBytes, pair ? "true" : "false", g.planes, g.plane_rows,
              g.resident, g.halo, g.n_a_slots, g.n_stages, g.issuers, g.kh * g.chunks_per_tap, g.kchunk,
-             g.tap_kw, g.m_tiles, g.n_tiles, g.shared_cols,
+             g.tap_kw, g.m_tiles, g.n_tiles, g.shared_cols, g.n_acc,
              c->blockDim.x / 32 - 3);
     g_launch = text;
     return cudaSuccess;

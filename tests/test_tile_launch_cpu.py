@@ -18,6 +18,7 @@ import test_position_columns_gpu
 import test_resident_filters_gpu
 import test_shared_accumulator_gpu
 import test_streamed_filters_gpu
+import test_three_accumulators_gpu
 from xnor_nn_b200 import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -55,7 +56,7 @@ SHARED_ACCUMULATOR = [c for c in test_shared_accumulator_gpu.LAYERS if not c[0].
 LAYERS = (FASTER_AS_COLUMNS + FASTER_AS_ROWS + GPU_COLUMNS + test_position_columns_gpu.ROWS +
           test_resident_filters_gpu.ROWS + [LOST_COMMIT] + test_streamed_filters_gpu.STREAMED +
           test_folded_gpu.FOLDED + test_long_filter_rows_gpu.LONG_ROWS + EIGHT_WARPS + SIXTEEN_WARPS +
-          SHARED_ACCUMULATOR + cases.SHAPE_CASES + [
+          SHARED_ACCUMULATOR + test_three_accumulators_gpu.LAYERS + cases.SHAPE_CASES + [
               cases._c("alexnet_conv3_mb256", 256, 384, 256, 13, 13, 3, 3, ph=1, pw=1),
               cases._c("alexnet_conv4_mb256", 256, 256, 384, 13, 13, 3, 3, ph=1, pw=1)])
 
@@ -161,3 +162,10 @@ def test_gpu_tests_of_shared_accumulators_reach_each_form_with_two_issuers(launc
     assert {name for name, g in got.items() if g["halo"] > 136} == {
         "pairs_streamed", "pairs_streamed_256_filters", "pairs_streamed_192_filters"}
     assert (got["pairs_streamed_256_filters"]["shared_cols"], got["pairs_streamed_192_filters"]["shared_cols"]) == (1, 0)
+
+
+def test_gpu_tests_of_three_accumulators_reach_them(launches):
+    got = _of(launches, test_three_accumulators_gpu.LAYERS)
+    assert all(g["pair"] and g["resident"] and g["halo"] > 136 and g["accumulators"] == 3 for g in got)
+    assert [(g["issuers"], g["n_tiles"]) for g in got] == [(1, 1), (2, 1), (1, 2)]
+    assert all(g["m_tiles"] * g["n_tiles"] > 3 * g["grid"] for g in got)  # a fourth tile has the first one's
