@@ -1,8 +1,8 @@
 // What the position-tile launcher hands the driver, without a GPU: its object files are linked against
 // stand-ins for the few CUDA runtime calls it makes (a device of 148 SMs and 74 pairs of them, or
 // as many pairs as the variable PAIRS says). For
-// each layer on the command line (mb,oc,ic,ih,iw,kh,kw,sh,sw,ph,pw) one line of JSON: the tensor
-// maps it asked for, the launch, and the parameters that say which form of the kernel runs.
+// each layer on the command line (mb,oc,ic,ih,iw,kh,kw,sh,sw,ph,pw, and 1 for channels-last results) one line of
+// JSON: the tensor maps it asked for, the launch, and the parameters that say which form of the kernel runs.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -90,12 +90,14 @@ int main(int argc, char **argv) {
     for (int i = 1; i < argc; i++) {
         xnor_nn_convolution_t c;
         memset(&c, 0, sizeof c);
-        if (sscanf(argv[i], "%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d", &c.mb, &c.oc, &c.ic, &c.ih, &c.iw, &c.kh,
-                   &c.kw, &c.sh, &c.sw, &c.ph, &c.pw) != 11)
+        int last = 0;
+        if (sscanf(argv[i], "%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d", &c.mb, &c.oc, &c.ic, &c.ih, &c.iw, &c.kh,
+                   &c.kw, &c.sh, &c.sw, &c.ph, &c.pw, &last) < 11)
             return 2;
         c.oh = (c.ih + 2 * c.pw - c.kh) / c.sh + 1;
         c.ow = (c.iw + 2 * c.pw - c.kw) / c.sw + 1;
-        c.src_format = c.dst_format = xnor_nn_data_format_nchw;
+        c.src_format = xnor_nn_data_format_nchw;
+        c.dst_format = last ? xnor_nn_data_format_nhwc : xnor_nn_data_format_nchw;
         c.weights_format = xnor_nn_weights_format_oihw;
         xb200::Plan plan;
         xb200::make_plan(&plan, &c, xb200::kAuto);

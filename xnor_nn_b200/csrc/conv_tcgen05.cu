@@ -1416,6 +1416,18 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     const int groups = g.kh * g.chunks_per_tap;
     // as many ring buffers as fit beside the control block
     const size_t room = 227 * 1024 - 1024 - kControlBytes;
+    // Results that the epilogue stores float by float (channels-last, filters no multiple of four or a result between
+    // two 16-byte boundaries): a warp store is 4 bytes in each of 32 rows, and eight of them in turn fill a sector,
+    // which takes the longer the less L1 there is. That is what shared memory leaves of 256 KB: 28 KB beside more than
+    // 196 KB (with the system's 1 KB a block), 60 KB beside up to that. Position tiles for all filter rows are the
+    // larger ones and give up tiles in flight or filter buffers for it, if two and four are left. More than 196 KB
+    // over up to it, on one stream and among others, layers of 224 to 768 channels, 10 to 512 filters, 9 to 40 pixels:
+    //   resident filters (and three accumulators)  79  0.98 to 1.29, mean 1.10  1.00 to 1.21, mean 1.08
+    //   streamed ones, 224 and 256 a tile          18  1.00 to 1.21, mean 1.06  1.00 to 1.18, mean 1.06
+    // 210 filters on 448 channels of 37 x 37, 76 images, 217 -> 179 us on one stream, with a tile for each filter row
+    // 181. (Results in whole sectors, 40 layers: 0.97 to 1.02.)
+    const bool scattered = p.dst_nhwc && !next && ((p.oc & 3) != 0 || ((uintptr_t)dst & 15) != 0);
+    const size_t near_room = scattered ? 195 * 1024 - 1024 - kControlBytes : room;
     // A tap as a row offset into a position tile is known to work for the 128-byte swizzle only
     // (issue_probe checks that one). Narrower rows come with several taps a filter row when a layer
     // that was asked onto the image-row kernel ends a chain; it takes the plain ring.
@@ -1440,13 +1452,16 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
     // - a position's row ends inside a 32-byte sector, or
     // - a pair has three tiles or fewer, or a tile keeps the tensor pipe for less than 5000 cycles (the others
     //   have eight epilogue warps).
-    // Whole over half, 3 x 3 filters on 6 to 40 pixels, 288 to 512 channels, the halves with two issuers, a pass on
-    // one stream and among others:
-    //   256 filters, 3 to 6 tiles a pair  15 layers  1.05 to 1.15, mean 1.09   1.02 to 1.12, mean 1.05
-    //   192 filters, 1 to 6 tiles a pair  42 layers  1.05 to 1.24, mean 1.13   1.01 to 1.17, mean 1.08
-    // conv4 on 256 images 41.6 -> 35.6 us on one stream, 39 -> 36 among others. (Half of a whole that stays
-    // resident: of 256 filters with up to 1.4 tiles a pair 1.08 and 1.02, with more 0.96 and 0.93; of 192 1.02
-    // and 0.95; of 128 0.92 and 0.90.)
+    // Whole over half, 3 x 3 and 3 x 2 filters on 5 to 40 pixels, 257 to 512 channels, on one stream and among others:
+    //   rows that end inside a sector, 4 tiles a pair and more, 5000 cycles
+    //                                    44 layers  1.06 to 1.31, mean 1.15   1.03 to 1.24, mean 1.10
+    //   the others                       70 layers  1.02 to 1.22, mean 1.10   0.98 to 1.12, mean 1.05
+    // conv4 on 256 images 41.6 -> 35.6 us on one stream, 39 -> 36 among others. Even rows with four long tiles a pair
+    // are left out because the tests hold them to eight epilogue warps, with which halves have not been measured (VGG,
+    // half the width and sixteen warps: 1.055 and 1.025). (Half of a whole that stays resident: of 256 filters with up
+    // to 1.4 tiles a pair 1.08 and 1.02, with more 0.96 and 0.93; of 192 1.02 and 0.95; of 128 0.92 and 0.90.)
+    // Results stored float by float, of which halves make two stretches of a row: of 192 filters (8 layers) 1.01 to
+    // 1.21, mean 1.13, and 1.01 to 1.19, mean 1.07, of 256 (10) 0.88 to 1.11, mean 1.00, and 0.86 to 1.09, mean 0.99.
     int n_tile = p.n_tile;
     const int pair_units = (m_tiles + 1) / 2, half_tiles = 2 * (p.ocp16 / p.n_tile);
     const int slots = pair ? resident_pairs(d, sms) : sms;
@@ -1455,6 +1470,7 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         !filters_fit(n_tile) && filters_fit(n_tile / 2) && block_fits(n_tile / 2) && half_grid > 0 &&
         pair_units * half_tiles > slots &&
         div_up_i(pair_units * half_tiles, half_grid) == div_up_i(pair_units * half_tiles, slots) &&
+        !(scattered && n_tile == 256) &&
         (p.row_bytes % 32 != 0 || div_up_i(pair_units * half_tiles / 2, slots) <= 3 ||
          (long)steps * n_tile / 2 < 5000))
         n_tile /= 2;
@@ -1568,6 +1584,8 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         }
         g.a_slot_bytes = as_columns ? col_slot : tile_slot; g.b_slot_bytes = (g.b_bytes + 1023u) & ~1023u;
         g.n_a_slots = (int)((room - all_b) / g.a_slot_bytes);
+        if (g.block && near_room >= all_b + 2 * (size_t)g.a_slot_bytes)
+            g.n_a_slots = (int)((near_room - all_b) / g.a_slot_bytes);
         if (g.n_a_slots > kMaxASlots) g.n_a_slots = kMaxASlots;
         g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
         grid = one_nt;
@@ -1596,6 +1614,8 @@ cudaError_t launch_conv_tcgen05(const Plan &p, const void *bin_src, const void *
         g.b_slot_bytes = (g.b_bytes + 1023u) & ~1023u;
         g.b_ring_off = (uint32_t)g.n_a_slots * g.a_slot_bytes;
         g.n_stages = (int)((room - g.b_ring_off) / g.b_slot_bytes);
+        if (g.block && near_room >= g.b_ring_off + 4 * (size_t)g.b_slot_bytes)
+            g.n_stages = (int)((near_room - g.b_ring_off) / g.b_slot_bytes);
         if (g.n_stages > kMaxStages) g.n_stages = kMaxStages;
         if (g.n_stages < 4) { g.halo = 0; g.block = 0; halo = false; }
     }
