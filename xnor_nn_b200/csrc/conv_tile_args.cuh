@@ -40,16 +40,18 @@ struct TcArgs {
     int n_stages;         // ring buffers in use
     // Halo mode (pairs, filters at least two taps wide): the position tile of a
     // filter row is loaded once, with the kw - 1 positions that follow it, and serves all kw taps
-    // of the row (a tap is a row offset into the tile); the ring then holds filter tiles only.
-    int halo;             // 0, or rows of a halo tile (128 + 8; 128 with a single tap per row)
+    // of the row (a tap is a row offset into the tile), or, with `block`, those of all filter rows; the ring
+    // then holds filter tiles only.
+    int halo;             // 0, or rows of a position tile: 128 + 8 (128 with a single tap per row), up to 256 with block
     int n_a_slots;        // halo tiles in flight
     uint32_t a_slot_bytes, b_ring_off, b_slot_bytes, b_bytes;
     // Resident filters (pairs whose tiles all have the same filter tile, if its operands of all
     // taps fit shared memory beside three position tiles of 128-byte rows): filter tiles are loaded
-    // once, together with the first round's position tiles, and stay. Position tiles as in halo mode
-    // (halo is 128 if there is one tap per filter row), or as columns:
+    // once and stay. Position tiles as in halo mode or as columns:
     int resident;
-    int block;            // a position tile of `halo` rows serves all filter rows (producer_block, producer_halo)
+    // A position tile of `halo` rows serves all filter rows: beside resident filters (producer_block, which loads a
+    // chunk's filters behind the first tile's positions of that chunk) and streamed ones (producer_halo).
+    int block;
     // Resident filters with position tiles of 16-byte channel columns (producer_planes): columns of a
     // tile, positions of it and positions from one column to the next (a multiple of 8), bytes per
     // position and the upper half of its matrix descriptors. 0: not so.

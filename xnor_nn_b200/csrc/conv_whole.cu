@@ -30,19 +30,19 @@
 // columns have there (producer_planes), in which a tap is a start address.
 //
 // What bounds it, in cycles of a tile of AlexNet conv4 (136 pixels of 384 channels, 384 KB of filters per
-// 256, 1.9 GHz): 1200 until the first loads go out, 12000 of packing (three tasks a worker: 1300 to 2500 for
-// a task's loads, 1300 to 1900 of instructions; an SM takes floats in at 20 to 25 bytes a cycle, and 12, 16 or
-// 24 workers, or loads a task ahead, do not change that), which the filter loads share the way with, then the
-// MMAs (5300 with narrow filter tiles, all of which are in shared memory by then; 9500 with 256 filters,
-// which come through the ring meanwhile), then 1000 to 5600 for the stores. One issuer needs about 500 cycles a
-// filter tile, mostly the chain of scalar instructions around its MMAs, hence four (MMAs of one image:
-// 6700 -> 5300). Times in us, two launches -> one: a pass among others on three streams, back to back on one
+// 256, 1.9 GHz) in a pass that is waited for, on one image, on 32, and on 64 channels-last: 1700 to 1900 until the
+// kernel before has been waited for; 8800, 10300 and 13300 of packing (three tasks a worker; an SM takes floats in at
+// 20 to 25 bytes a cycle, and 12, 16 or 24 workers, or loads a task ahead, do not change that), which the filter loads
+// share the way with; 3100, 9000 and 8000 until the last MMA is done (one image has narrow filter tiles, all of which
+// are in shared memory by then; 256 filters come through the ring meanwhile); 1000, 5200 and 6200 of stores. One
+// issuer needs about 500 cycles a filter tile, mostly the chain of scalar instructions around its MMAs, hence four
+// (MMAs of one image, with the packing of then: 6700 -> 5300). Times in us, two launches -> one: a pass among others on three streams, back to back on one
 // stream, waited for: conv4 on one image 7.2 -> 3.9, 12.8 -> 9.6, 23.6 -> 21.0; on 32 images 8.2 -> 5.3,
 // 16.4 -> 14.8, 25.0 -> 26.2; on 64 images channels-last 11.4 to 12.2 -> 11.4, 20.9 -> 18.0, 29.9 -> 29.9 (the
 // last two as measured before the next paragraph's changes); 16 channels of 31 x 31, five images 8.7 -> 5.3,
 // 7.5 -> 5.5, 20.0 -> 18.2 (the same). The first is bound by the host, for which a launch is 2.0 us.
 //
-// The cycles above are from before three changes to the packing, on one stream in us, one image and 32: one path
+// What made the packing shorter (12000 cycles before), on one stream in us, one image and 32: one path
 // through a task's loads, whichever lanes have a pixel, 11.1 -> 10.0 and 16.4 -> 15.6; a barrier for each
 // hand-over of a running sum instead of counters that are polled, 10.1 -> 9.7 and 15.6 -> 15.1; the accumulator
 // cleared by the issuers, which have nothing to issue yet, instead of by packing warps, 9.7 -> 9.5 and 15.1 ->
@@ -433,13 +433,17 @@ bool whole_shape(const Plan &p, WholeArgs *g, size_t *smem) {
     const int tasks = div_up_i(g->rows, 32) * g->columns;
     if (tasks > kMaxTasks) return false;
     // Not where pixels are packed more than 1.6 times (by neighbouring tiles, in halos, and by each filter tile)
-    // and the tiles, dealt to all SMs, come to more than 5.5 us in the cycles above: the general path does that
+    // and the tiles, dealt to all SMs, come to more than 5.5 us: the general path does that
     // work once, and with passes on several streams hides its second launch under it. The time of two launches
     // over that of one, geometric means: of 275 layers that ran here before (drawn from 1 to 256 images, 16 to
     // 512 channels and filters, 6 to 56 pixels) among others 1.33, on one stream 1.22, waited for 1.04; of the
     // eleven that this rule takes out 0.90, 1.06 and 0.95; 384 filters on 256 channels of 13 x 13, 48 images,
     // 0.75, 1.03 and 0.93. What stays slower alone is few tiles of many filters, which leave most SMs idle:
     // conv4 on 16 to 48 images 1.2 to 1.4 among others, 0.82 to 0.99 on one stream, 0.87 to 0.95 waited for.
+    // The formula still gives a tile of conv4 what it takes (14900 cycles on one image, 26400 on 32; measured 14600
+    // and 26200), but those means are from before the packing got shorter, and the line is behind that: of 60 layers
+    // just beyond it (up to 14000 instead of 10450) one launch would now be 1.17 times as fast as two on one stream
+    // (0.84 to 1.49), 1.05 among others (0.81 to 1.36).
     const long mma_cycles = (long)g->taps * ((g->chunks - 1) * (p.kchunk / 32) + g->kk_last) * g->n_tile / 2;
     const long tile_cycles = 1200 + 4000 * div_up_i(tasks, kWorkers) + mma_cycles * 11 / 10 + 22 * g->n_tile;
     const bool repeats = 10L * g->n_tiles * g->rows > 16L * BM;

@@ -58,7 +58,8 @@ __host__ __device__ inline Band band_of(const MapArgs &g, int block) {
 // 16 MB), the three upstream calls with two launches here over those with one: 1.02 on one stream and 1.14
 // among others if all take one, 1.035 and 1.14 with this rule; the 48 that it takes out 0.90 and 1.005 (19
 // images of 464 channels, 17 x 17, filters of 5 x 5: 44.6 and 60.6 us on one stream, calculate_k alone 7.0 and
-// 18.8).
+// 18.8). That was with counters for the hand-overs of running sums. With barriers 70 layers just beyond the line (8.5
+// to 12 us by this formula) would take one launch 0.93 and 1.14 times as fast as two, 0.72 to 1.13 and 0.93 to 1.69.
 inline double launch_us(long blocks, long tasks, long outputs, int taps) {
     return 3.6 + 0.58 * (double)(blocks * tasks) / (8.0 * sm_count()) + 0.74 * (double)((tasks + 7) / 8) +
            0.58 * (double)((outputs + kThreads - 1) / kThreads) * taps / 25;

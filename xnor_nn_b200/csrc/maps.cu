@@ -4,7 +4,7 @@
 // (pixel_tasks.cuh), into shared memory; rows that two bands see are added by both, in the same order, and
 // left in the map by the one that owns them. Then a thread adds up an output's terms in upstream's order.
 // Bound by the latency of its few rounds of loads; what it is for is the launch it saves, 2 us of the host's:
-// the three upstream calls on 19 images of 75 channels, 31 x 27, take 10.2 instead of 12.8 us a pass among
+// the three upstream calls on 19 images of 75 channels, 31 x 27, take 9.6 instead of 12.8 us a pass among
 // others, a microsecond of it less work in the caller, and 16.5 instead of 17.0 on one stream; 15 images of 304
 // channels, 9 x 9, filters of 5 x 5, 9.9 instead of 13.0 among others, 24.6 and 24.4 on one stream.
 #include "kernels.cuh"

@@ -271,8 +271,11 @@ void make_plan(Plan *p, const xnor_nn_convolution_t *c, Family requested) {
     // filters, 6 to 40 pixels and 0.05 to 6 rounds of tiles, a pass on one stream and among others:
     //   rows of an odd number of 16 bytes  0.96 to 1.72, mean 1.12   0.98 to 1.97, mean 1.12
     //   of 32                              0.99 to 1.32, mean 1.04   0.97 to 1.31, mean 1.04
-    // 1 x 1 filters, bound by the packer and the stores, 0.97 to 1.06, mean 1.01, and 1.00. Starting on 128
-    // bytes instead: another 1.02 in the mean, but conv4 (192 bytes) packs slower, 14.8 -> 15.3 us.
+    // Filters of two to four taps on pairs, whose packer is the longer part, 78 layers of 60 to 230 MB of source: 0.98
+    // to 1.08, mean 1.015, on one stream, and 0.90 to 1.08, mean 0.995, among others, where what the rows add to the
+    // packed bytes counts for more (0.87 with 113 filters of 1 x 2 on 408 channels of 25 x 25, 190 images). 1 x 1
+    // filters, bound by the packer and the stores, 0.97 to 1.06, mean 1.01, and 1.00. Starting on 128 bytes instead:
+    // another 1.02 in the mean, but conv4 (192 bytes) packs slower, 14.8 -> 15.3 us.
     p->row_bytes = div_up_i(channels, 32) * 16;
     p->icp = !fold && taps > 1 && p->row_bytes > 128 ? div_up_i(p->row_bytes, 64) * 64 : p->row_bytes;
     p->kchunk = p->icp > 64 ? 128 : p->icp > 32 ? 64 : 32;
